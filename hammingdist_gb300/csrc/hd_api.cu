@@ -1312,7 +1312,7 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
           HD_CUDA(cudaMemGetInfo(&free_b, &total_b));
           const double need = (double)(R_max < 2 ? 1 : tri(R_max)) * dtype_bytes +
                               2.0 * (double)R_max * (double)words * 16.0 +
-                              (double)R_max * (double)words * (double)hd::kMmaOperandBytesPerWord;
+                              (double)hd::mma_operand_bytes(4, L, R_max);
           if (need > 0.5 * (double)free_b) return fallback();
         }
         owner = std::make_unique<hd_alignment>();

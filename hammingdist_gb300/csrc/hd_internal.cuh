@@ -63,9 +63,14 @@ struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
   cudaStream_t s = nullptr;
+  bool big = false;  // recycled by the library
   DevBuf() = default;
-  DevBuf(size_t n, cudaStream_t stream) : bytes(n), s(stream) {
-    if (n >= kBigBlock) p = big_alloc(n, stream);
+  // pool_only: from the pool whatever the size (a workspace whose size differs
+  // from launch to launch: a request that no released block fits returns them
+  // all to the pool)
+  DevBuf(size_t n, cudaStream_t stream, bool pool_only = false)
+      : bytes(n), s(stream), big(n >= kBigBlock && !pool_only) {
+    if (big) p = big_alloc(n, stream);
     else if (n) HD_CUDA(cudaMallocAsync(&p, n, stream));
   }
   DevBuf(const DevBuf &) = delete;
@@ -77,6 +82,7 @@ struct DevBuf {
       p = o.p;
       bytes = o.bytes;
       s = o.s;
+      big = o.big;
       o.p = nullptr;
       o.bytes = 0;
     }
@@ -85,7 +91,7 @@ struct DevBuf {
   ~DevBuf() { release(); }
   void release() {
     if (p) {
-      if (bytes >= kBigBlock) big_release(p, s);
+      if (big) big_release(p, s);
       else cudaFreeAsync(p, s);
     }
     p = nullptr;
@@ -119,11 +125,11 @@ struct Trace {
 struct TileConfig {
   int tile = 128;    // bit-plane engine: tile edge (64 or 128 rows)
   int stages = 3;    // bit-plane engine: TMA staging depth
-  int mma_band = 0;  // tensor-core engine: tile rows per L2 band (0: built-in)
-  int mma_rows = 0;  // tensor-core engine: row tiles per item, 1 or 2 (0: built-in 2)
+  int mma_band = 0;  // tensor-core engine: item rows (256 rows) per L2 band (0: built-in)
+  int mma_rows = 0;  // tensor-core engine: column halves per item, 1 or 2 (0: built-in 2)
 };
 // The autotuner's table: a configuration per (n bucket, L bucket, dtype),
-// and per L bucket the fewest single-row-tile items for which a launch goes
+// and per L bucket the smallest size (tiles of 128 x 240 pairs) at which a launch goes
 // to the tensor-core engine rather than the bit-plane engine.
 struct TuneTable {
   std::vector<std::pair<uint32_t, TileConfig>> entries;
@@ -209,9 +215,12 @@ struct hd_alignment {
   // alignment
   mutable hd::DevBuf op;
   mutable uint64_t op_rows = 0, op_cap = 0;
-  // per 256-site chunk of the operand (uint32 each): nonzero once an
+  // per 288-site chunk of the operand (uint32 each): nonzero once an
   // expanded row has a '-' in it (the chunks whose dash products count)
   mutable hd::DevBuf op_dash;
+  // the marked chunks' list and ranks after each extension of the operand,
+  // the last one current
+  mutable std::vector<hd::DevBuf> op_lists;
   // Freed on the null stream: every API call has synchronised its own stream
   // before returning, so no queued work still reads these buffers, and the
   // creating context (and its streams) may already be gone.
@@ -225,6 +234,10 @@ struct hd_alignment {
     for (auto *b : {&plane_buf[0], &plane_buf[1], &d_seqidx, &op, &op_dash}) {
       b->s = nullptr;
       b->release();
+    }
+    for (auto &b : op_lists) {
+      b.s = nullptr;
+      b.release();
     }
   }
 };
@@ -367,13 +380,19 @@ __device__ inline uint64_t global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// Waits for the barrier phase with a wall-clock limit; false = gave up.
+// A wait limit in SM clock cycles, at 2.125 cycles per ns (the SM clock ends at
+// 2.07 GHz, so at least limit_ns pass). Reading the cycle counter costs a few
+// cycles; %globaltimer costs hundreds, which a wait that ends meanwhile pays.
+__device__ inline long long wait_cycles(uint64_t limit_ns) {
+  return (long long)(limit_ns * 17 / 8);
+}
+// Waits for the barrier phase with a time limit; false = gave up.
 __device__ inline bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, uint64_t limit_ns) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = global_ns();
+  const long long t0 = clock64(), limit = wait_cycles(limit_ns);
   for (;;) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (global_ns() - t0 > limit_ns) return false;
+    if (clock64() - t0 > limit) return false;
   }
 }
 // 2-D tiled TMA load (global -> shared), completion counted on `bar`.
@@ -472,11 +491,9 @@ void query_distances_async(hd_ctx *ctx, const hd_alignment *aln, const uint8_t *
 void pairwise_tiles(hd_ctx *ctx, const hd_alignment *aln, int dtype_bytes, uint32_t max_dist,
                     void *d_out, uint64_t out_base, uint32_t tile_lo, uint32_t tile_hi);
 constexpr uint32_t kTile = 128;
-// columns of a tensor-core work item (the N of its MMAs)
+// the tensor-core engine's launch sizes are counted in tiles of 128 rows x
+// this many columns (the autotuner's thresholds)
 constexpr uint32_t kMmaCols = 240;
-// bytes of the tensor-core engine's E2M1 operand per 32-site word of a row
-// of the dense AND rule (6 blocks of 16 bytes: 4 planes and 2 dash blocks)
-constexpr uint32_t kMmaOperandBytesPerWord = 96;
 
 // Kernel configuration of one job: tile edge (64 or 128 rows; 4 or 8 rows
 // per thread) and TMA staging depth.
@@ -499,8 +516,14 @@ struct PairLaunchPlan {
     const void *d_jobs = nullptr;
     unsigned long long *d_counter = nullptr;
     bool mma = false;              // the tensor-core engine (hd_mma.cu): d_items holds
-    const void *d_items = nullptr; // its work items, `tiles` of them
-    bool queue = false;            // its CTAs draw items from d_counter (else round-robin)
+    const void *d_items = nullptr; // its work items, `items` of them
+    uint64_t items = 0;
+    bool queue = false;            // its CTA pairs draw items from d_counter, else
+                                   // pair u runs items u, u + pairs, ...
+    const void *d_tms = nullptr;   // its tensor maps
+    const void *d_fix = nullptr;   // tiles split along K, `fixes` of them, and
+    uint64_t fixes = 0;            // their pieces' workspace
+    void *d_ws = nullptr;
   };
   std::vector<Launch> launches;
   std::vector<DevBuf> blocks;  // job tables + tensor maps + tile counters
@@ -522,11 +545,11 @@ TileConfig default_tile_config(uint64_t n_rows, uint64_t length, int dtype_bytes
 bool tile_config_valid(int tile, int stages);
 // tune.cu: the autotuned table (or the default) for (n, L, dtype)
 TileConfig tile_config_for(hd_ctx *ctx, uint64_t n_rows, uint64_t length, int dtype_bytes);
-// the tensor-core engine's minimum launch size (single-row-tile items) for
+// the tensor-core engine's minimum launch size (tiles of 128 x 240 pairs) for
 // rows of `length` sites: HAMMINGDIST_MMA_MIN_ITEMS, else the table, else
 // the built-in value
 uint64_t mma_min_items_for(hd_ctx *ctx, uint64_t length);
-// mma.cu: the tensor-core engine's L2 band (tile rows) and row tiles per item
+// mma.cu: the tensor-core engine's L2 band (item rows) and column halves per item
 // for a configuration: HAMMINGDIST_MMA_BAND / HAMMINGDIST_MMA_ROWS, else the
 // configuration's own, else the built-in 16 and 2
 int mma_band_of(const TileConfig &c);
@@ -540,6 +563,8 @@ bool mma_eligible(const hd_alignment *aln);
 // operand cannot be allocated
 bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStream_t stream,
                 uint64_t cap_hint = 0);
+// bytes of that operand for `rows` rows of `sites` sites
+uint64_t mma_operand_bytes(uint32_t planes, uint64_t sites, uint64_t rows);
 // tile rows [tile_lo, tile_hi) (128 rows each) x all earlier columns into
 // d_out (lt index out_base at d_out[0]) on `stream`; sm_limit > 0 caps the
 // persistent grid. False when the alignment is not eligible (the caller

@@ -22,49 +22,66 @@
 // are kind::mxf4 with every UE8M0 scale factor 1.0 and FP32 accumulation,
 // exact while P L < 2^24. mismatches = L - matches.
 //
-// K order: first the P plane blocks of every 256-site chunk (partial sums up
+// K order: first the P plane blocks of every 288-site chunk (partial sums up
 // to P L), then the dash products, only for the chunks where some row of the
 // operand has a '-' (the expansion marks them): elsewhere every dash product
 // is 0. On aligned genomes the '-' sit mostly in leading and trailing runs, so
 // a row's P + 1 blocks per chunk shrink to about P.
 //
 // Operand (one buffer serves rows and columns): each row's bit planes are
-// expanded to packed E2M1, two sites per byte, K-major: for every 256 sites,
-// the P planes (1.0), the dash as 1.0 (read for rows) and the dash as -(P - 1)
-// (read for columns; -4 and -1 for P = 6), 128 bytes each; sites past L are
-// 0. An alignment caches its operand; a view of a resident alignment (a
-// serving window) gets one of its own rows.
+// expanded to packed E2M1, two sites per byte, in the layout the tensor
+// cores read without a swizzle: for 8 rows (a row group) and 288 sites, the P
+// planes (1.0), the dash as 1.0 (read for rows) and the dash as -(P - 1)
+// (read for columns; -4 and -1 for P = 6) are blocks of 1,152 bytes, each nine
+// 128-byte core matrices (8 rows x 16 bytes = 32 sites). Sites past L are 0. A
+// row group's blocks follow one another, so a TMA box of 16 groups brings one
+// block of 128 rows. An alignment caches its operand; a view of a resident
+// alignment (a serving window) gets one of its own rows.
 //
-// One launch serves a job table of matrices. Persistent CTAs (320 threads,
-// one per SM) walk a list of items: 240 columns J x one or two 128-row tiles
-// I of one job, in bands of 16 tile rows, column-major within a band, so
-// resident CTAs share operands in L2; the list ends with single-row-tile items
-// so that every CTA gets the same work to within a row tile.
-//  * warp 0 (one thread) issues TMA loads (128-byte swizzle) per stage of
-//    one 128-byte K block (256 sites) of the item's 128 or 256 rows and 240
-//    columns, 3 stages of 62 KB with full/empty mbarriers; warp 0 also
-//    allocates and frees the TMEM;
-//  * warp 1 (one thread) issues tcgen05.mma.cta_group::1.kind::mxf4
-//    .block_scale (M=128, N=240, K=64), four per row tile per stage, into
-//    TMEM (row tile h of the item at columns 256 h); the unit scale factors
-//    sit in the columns the accumulators leave, 240-255 (rows) and 496-511
-//    (columns), written once per CTA. Each stage's MMAs are
-//    committed to its empty barrier, an item's last ones to `done`;
-//  * warps 2-9, two per TMEM lane quarter, each read 32 rows x 128 or 112
-//    columns of each accumulator (tcgen05.ld, 64, 32 or 16 columns at a time),
-//    form min(L - matches, max_dist) (safe_int_cast,
-//    include/hamming/hamming_impl.hh:37-45), turn each 32 x 32 chunk around
-//    in a padded shared buffer and store it row by row, 32 consecutive
-//    entries of the job's dtype per store; they then release the
-//    accumulators (`tmem_free`) for the MMAs of the next item, whose first
-//    stages the producer has already loaded. The MMAs wait for this, so the
-//    epilogue's length is paid once per item.
+// One launch serves a job table of matrices. Persistent pairs of CTAs (a
+// cluster of two SMs, 320 threads each) walk a list of items: 256 rows x up to
+// 496 columns of one job, in bands of tile rows, column-major within a band,
+// so that resident pairs share operands in L2.
+//  * warp 0 (one thread) issues TMA loads per stage of one 144-byte K block of
+//    the CTA's 128 rows and of its half of the columns (128 + 120), 4 stages
+//    of 54,144 B; both CTAs' loads count on the first CTA's full barriers.
+//    The first CTA's producer also draws the items and hands their indices
+//    around; warp 0 allocates and frees the TMEM;
+//  * warp 1 of the first CTA (one thread) issues tcgen05.mma.cta_group::2
+//    .kind::mxf4.block_scale with K = 96 (the shape only sm_103a has: 1.5
+//    times the rate of K = 64), M = 256 and N = 256 and 240, three K steps per
+//    block, into both CTAs' TMEM (columns 0-255 and 256-495); the unit scale
+//    factors sit in columns 496-511. Each stage's MMAs are committed to both
+//    CTAs' empty barriers, an item's last ones to `done`;
+//  * warps 2-9, two per TMEM lane quarter, each read 32 rows x 248 columns
+//    (tcgen05.ld), form min(L - matches, max_dist) (safe_int_cast,
+//    include/hamming/hamming_impl.hh:37-45) as packed 16-bit values in
+//    registers and release the accumulators (`tmem_free`) at once: the next
+//    item's MMAs run while the warp turns 32 x 28 pieces around in shared
+//    memory and stores them row by row. 32-bit outputs are stored piece by
+//    piece before the release.
+// Where items do not divide evenly among the pairs (few rows, or the last
+// round), the rest is split along K at chunk boundaries: a piece leaves its
+// partial distances in a workspace, and k_pair_fix adds a tile's pieces.
 // Every wait is bounded; on a timeout the CTA records it in the status word,
 // waits (bounded) for its own copies and MMAs, frees its TMEM and returns.
+//
+// What bounds it (n = 14,000, L = 29,903, 8.05 FLOP per pair-site): the L2
+// reads. A pair's stage takes 745 cycles of MMAs and brings 108 KB; measured
+// alone, the loads reach 77 B per cycle and SM, the MMAs 14.4 PFLOP/s.
+//   form (K block x stages)                  operand in L2 / over 100 MB
+//   single CTAs, K = 96, 96 B x 3              9.1 / 8.0 PFLOP/s
+//   CTA pairs, K = 96, 96 B x 6               13.4 / 12.9
+//   CTA pairs, K = 96, 144 B x 4              14.5 / 12.6
+//   CTA pairs, K = 96, 192 B x 3              14.5 / 12.2
+// A 96-byte block's barrier traffic costs more than its MMAs last (536 of
+// 497 cycles); three stages of 192 hide less of the L2 latency. Pairs halve
+// the column bytes an SM loads and its MMAs read.
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "hd_internal.cuh"
@@ -74,77 +91,104 @@ namespace {
 
 constexpr int kEpiWarps = 8;      // two per TMEM lane quarter
 constexpr int kMmaThreads = 64 + 32 * kEpiWarps;  // warp 0: TMA, warp 1: MMA, warps 2-9: epilogue
-constexpr int kEpiThreads = 32 * kEpiWarps;
-constexpr int kMmaStages = 3;
-constexpr int kTM = 128, kTN = (int)kMmaCols;          // MMA tile: rows x columns (240)
-constexpr uint32_t kEpiSplit = 128;                   // epilogue halves: [0, 128), [128, kTN)
-// unit scale factors in the TMEM columns the two accumulators (columns
-// [0, kTN) and [256, 256 + kTN)) leave: the rows' at kTN, the columns' at
-// 256 + kTN, 16 columns each
-constexpr uint32_t kSfColA = kTN, kSfColB = 256 + kTN;
+constexpr int kMmaStages = 4;
+constexpr uint32_t kTM = 128;                          // rows of a tile row, and of a CTA in a pair
+constexpr uint32_t kRowsPerItem = 2 * kTM;             // M of a CTA pair's MMA
+constexpr uint32_t kN0 = 256, kN1 = 240;               // an item's column halves (N of its MMAs)
+constexpr uint32_t kItemCols = kN0 + kN1;
+constexpr uint32_t kChunkWords = 9;                    // 32-site words per chunk (288 sites)
+constexpr uint32_t kChunkSites = 32 * kChunkWords;
+constexpr uint32_t kBlockK = 16 * kChunkWords;         // bytes of K per row and block (144)
+constexpr uint32_t kGroupBytes = 8 * kBlockK;          // one block of 8 rows (1,152)
+constexpr uint32_t kKStep = 48;                        // bytes of K per MMA (96 values)
+constexpr uint32_t kABytes = kTM / 8 * kGroupBytes;              // 128 rows
+constexpr uint32_t kB0Bytes = kN0 / 16 * kGroupBytes;            // half of 256 columns
+constexpr uint32_t kB1Bytes = kN1 / 16 * kGroupBytes;            // half of 240 columns
+constexpr uint32_t kStageBytes = kABytes + kB0Bytes + kB1Bytes;  // 54,144
+// the epilogue warps' pieces: 32 rows x 14 words (28 16-bit columns), row r
+// at words 15 r (conflict-free by row and by column)
+constexpr uint32_t kPieceWords = 14, kPiecePitch = 15;
+constexpr uint32_t kEpiBytes = kEpiWarps * 32 * kPiecePitch * 4;
+constexpr int kMmaSmem = kMmaStages * kStageBytes + kEpiBytes + 128;
+static_assert(kBlockK % kKStep == 0 && kStageBytes % 128 == 0, "K steps and TMA destinations");
+static_assert(kMmaSmem + 256 <= 232448, "shared memory above the per-block limit");
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kHalfCols = kItemCols / 2;         // columns per epilogue warp (248)
+constexpr uint32_t kHalfWords = kHalfCols / 2;        // packed 16-bit pairs (124)
+constexpr uint32_t kSfColA = kItemCols, kSfColB = kItemCols + 8;  // unit scale factors
 constexpr uint32_t kSfWord = 0x7F7F7F7Fu;             // four UE8M0 scale factors of 2^0
-constexpr uint32_t kHalfBytes = kTM * 128;            // one 128-byte K block of 128 rows
-constexpr uint32_t kABytes = 2 * kHalfBytes;          // up to two row tiles
-constexpr uint32_t kBBytes = kTN * 128;
-constexpr uint32_t kStageBytes = kABytes + kBBytes;   // 62 KB, a multiple of 1 KB
-constexpr uint32_t kEpiPitch = 33;                    // words per row of an epilogue chunk
-constexpr uint32_t kEpiBytes = kEpiWarps * 32 * kEpiPitch * 4;  // 32 x 32 words per epilogue warp
-constexpr int kMmaSmem = kMmaStages * kStageBytes + kEpiBytes + 1024;
-static_assert(kStageBytes % 1024 == 0, "stages must stay 1 KB aligned for the 128-byte swizzle");
-static_assert(kMmaSmem <= 232448, "dynamic shared memory above the per-block limit");
-static_assert(kTN % 16 == 0 && kTN <= 240, "N of an M=128 MMA; 16 TMEM columns left for scales");
-constexpr uint32_t kTmemCols = 512;                   // row tile h at columns 256 h
 constexpr uint64_t kMmaWaitNs = 1000000000ull;        // 1 s
-constexpr uint32_t kMmaBand = 16;  // tile rows per L2 band (HAMMINGDIST_MMA_BAND overrides)
-constexpr int kItemRing = 4;                          // item indices handed to the consumers
-constexpr uint32_t kNoItem = 0xFFFFFFFFu;             // end of this CTA's items
-// 128-byte blocks per 256 sites of the operand: the P planes, the row side's
-// dash and the column side's dash (two blocks for P = 6: -4 and -1)
+constexpr uint32_t kMmaBand = 16;  // item rows (256 rows) per L2 band (HAMMINGDIST_MMA_BAND overrides)
+constexpr int kItemRing = 4;                          // item indices handed to the other warps
+// arrivals that free a ring slot: the MMA thread, the second CTA's producer
+// and both CTAs' epilogue warps
+constexpr uint32_t kRingReaders = 2 + 2 * kEpiWarps;
+constexpr uint32_t kNoItem = 0xFFFFFFFFu;             // end of this pair's items
+constexpr uint32_t kNoSlot = 0xFFFFFFFFu;             // an item that covers all of K
+// A split tile's partial distances of one K piece: 16-bit pairs, per CTA,
+// column half, lane quarter and word the 32 lanes of a warp
+constexpr uint64_t kSlotBytes = 2ull * 2 * 4 * kHalfWords * 32 * 4;
+// K pieces of fewer chunks than this cost more in barriers and workspace
+// traffic than they spread (two chunks of four planes run 3 us)
+constexpr uint32_t kMinPart = 2;
+// blocks of 288 sites per row and chunk in the operand: the P planes, the row
+// side's dash and the column side's dash (two blocks for P = 6: -4 and -1)
 __host__ __device__ constexpr uint32_t op_blocks(uint32_t planes) {
   return planes + (planes == 6 ? 3u : 2u);
 }
-// operand bytes per 32-site word: 16 bytes (32 sites of E2M1) per block
-__host__ __device__ constexpr uint64_t row_bytes_per_word(uint32_t planes) {
-  return (uint64_t)op_blocks(planes) * 16;
+__host__ __device__ constexpr uint32_t op_chunks(uint64_t sites) {
+  return (uint32_t)((sites + kChunkSites - 1) / kChunkSites);
 }
-static_assert(row_bytes_per_word(4) == kMmaOperandBytesPerWord, "operand size of the AND rule");
+// operand bytes of 8 rows
+__host__ __device__ constexpr uint64_t op_group_bytes(uint32_t planes, uint64_t sites) {
+  return (uint64_t)op_chunks(sites) * op_blocks(planes) * kGroupBytes;
+}
+uint64_t op_bytes(uint32_t planes, uint64_t sites, uint64_t rows) {
+  return ceil_div(rows, (uint64_t)8) * op_group_bytes(planes, sites);
+}
 // E2M1 codes: 1.0, and the column side's -(P - 1): -3 for P = 4, -4 else
 // (then -1 for P = 6)
 constexpr uint32_t kE2M1One = 0x2u, kE2M1Neg1 = 0xAu;
 __device__ __forceinline__ uint32_t dash_neg(uint32_t planes) { return planes == 4 ? 0xDu : 0xEu; }
 // instruction descriptor (block-scaled kinds): A and B E2M1 (1 at bits 7-9
 // and 10-12), both K-major, N >> 3 at bits 17-22, scale factors UE8M0 (bit
-// 23), M >> 4 at bits 24-28, scale factor ids 0, K = 64; D is FP32
+// 23), M >> 4 at bits 24-28, scale factor ids 0, K = 96 (bit 31); D is FP32
 __host__ __device__ constexpr uint32_t idesc_mxf4(uint32_t n) {
-  return (1u << 7) | (1u << 10) | ((n >> 3) << 17) | (1u << 23) | ((uint32_t)(kTM >> 4) << 24);
+  return (1u << 7) | (1u << 10) | ((n >> 3) << 17) | (1u << 23) |
+         ((kRowsPerItem >> 4) << 24) | (1u << 31);
 }
-constexpr uint32_t kIdesc = idesc_mxf4(kTN);
 
 }  // namespace
 
-// One matrix of a launch (device copy): its operand's tensor maps (boxes of
-// 256 and 128 rows for the row side, kTN rows for the column side) and its
-// output.
+// One matrix of a launch (device copy): its output and the chunks whose dash
+// products count. Its operand's tensor maps are at 2 job of the launch's maps
+// (boxes of one block of 128 and of 120 rows).
 struct MmaJob {
-  const CUtensorMap *tm256;
-  const CUtensorMap *tm128;
-  const CUtensorMap *tmb;
   void *out;                     // lt index out_base at out[0]
   unsigned long long out_base;
-  uint32_t n, nkb, sites, max_dist, dtype;  // rows, K blocks per side, L, cap, 1/2/4 bytes
+  uint32_t row_hi, sites, max_dist, dtype;  // rows end, L, cap, 1/2/4 bytes
   uint32_t planes;                          // P
-  uint32_t chunks;                          // 256-site chunks per row
+  uint32_t chunks;                          // 288-site chunks per row
   const uint32_t *dash_list;                // the chunks whose dash products count
-  const uint32_t *dash_marks;               // per chunk: some row has a '-' in it
+  const uint32_t *dash_rank;                // per chunk: listed chunks before it (chunks + 1)
   unsigned long long pairs;                 // lower-triangle pairs of this launch
 };
 
-// One work item: kTN columns J x row tiles [I, I + halves) of job `job`.
+// One work item: rows [row0, row0 + 256) x columns [col0, col0 + n0 + n1) of
+// job `job` over the chunks [c_lo, c_hi); a piece of a split tile leaves its
+// partial distances in workspace slot `slot`. n0 and n1, the N of the item's
+// MMAs, in units of 16; n1 > 0 only after n0 = 256 / 16.
 struct MmaItem {
-  uint32_t job;
-  uint32_t I;       // first 128-row tile
-  uint32_t J;       // kTN-column tile
-  uint32_t halves;  // row tiles in the item: 1 or 2
+  uint32_t job, row0, col0;  // job kNoItem: none (padding of the static order)
+  uint8_t n0_16, n1_16, planes, pad;
+  uint32_t c_lo, c_hi, slot, pad2;
+  __host__ __device__ uint32_t n0() const { return 16u * n0_16; }
+  __host__ __device__ uint32_t n1() const { return 16u * n1_16; }
+};
+static_assert(sizeof(MmaItem) == 32, "items are read as two 16-byte vectors");
+// One split tile: the workspace slots [slot, slot + parts) of its pieces.
+struct MmaFix {
+  uint32_t job, row0, col0, cols, slot, parts;
 };
 
 namespace {
@@ -168,59 +212,68 @@ __device__ __forceinline__ void put16(uint8_t *dst, uint32_t w, uint32_t v) {
 // Rows [row_lo, row_hi) of a P-plane alignment (P = 4: the AND rule; 5, 6:
 // the sparse rules, planes 4-5 in the second group) -> E2M1 operand rows.
 // One thread per (row, 32-site word): 16 or 32 bytes read, 16 bytes written
-// per block; eight consecutive words fill each 128-byte block of their 256
-// sites. The dash is the AND of the P planes ('-' has every plane); a chunk
-// of 256 sites where some row has a '-' is marked in dash_chunk.
+// per block. A warp takes one row group x 4 words, lane l row l % 8, so that
+// each of its stores fills whole 128-byte core matrices; a block of 256
+// threads takes 32 words. The words past the alignment's, up to whole chunks,
+// are written as 0. The dash is the AND of the P planes ('-' has every plane);
+// a chunk where some row has a '-' is marked in dash_chunk.
 __global__ void k_expand_op(const uint4 *__restrict__ g0, const uint4 *__restrict__ g1,
-                            uint32_t planes, uint64_t words, uint64_t row_lo, uint64_t row_hi,
+                            uint32_t planes, uint32_t words, uint64_t row_lo, uint64_t row_hi,
                             uint64_t L, uint8_t *__restrict__ x, uint32_t *dash_chunk) {
-  const uint32_t nb = op_blocks(planes);  // 128-byte blocks per 256 sites
-  // thread (x, y): word x of rows row_lo + y, row_lo + y + gridDim.y, ...
-  const uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (w >= words) return;
-  for (uint64_t r = row_lo + blockIdx.y; r < row_hi; r += gridDim.y) {
-    const uint4 p = g0[r * words + w];
-    const uint4 p1 = planes > 4 ? g1[r * words + w] : make_uint4(0u, 0u, 0u, 0u);
-    const uint64_t s0 = w * 32;
-    const uint32_t valid = s0 >= L ? 0u : (L - s0 >= 32 ? 0xffffffffu : ((1u << (L - s0)) - 1u));
+  const uint32_t nb = op_blocks(planes), chunks = op_chunks(L);
+  const uint32_t w = blockIdx.x * 32 + threadIdx.x / 8;
+  if (w >= chunks * kChunkWords) return;
+  const uint32_t c = w / kChunkWords;
+  const uint64_t s0 = (uint64_t)w * 32;
+  const uint32_t valid = s0 >= L ? 0u : (L - s0 >= 32 ? 0xffffffffu : ((1u << (L - s0)) - 1u));
+  const uint64_t in_group = (uint64_t)c * nb * kGroupBytes + (w - c * kChunkWords) * 128u +
+                            (threadIdx.x & 7u) * 16u;
+  const uint64_t group_bytes = op_group_bytes(planes, L);
+  for (uint64_t g = row_lo / 8 + blockIdx.y; g * 8 < row_hi; g += gridDim.y) {
+    const uint64_t r = g * 8 + (threadIdx.x & 7u);
+    if (r < row_lo || r >= row_hi) continue;
+    uint4 p = make_uint4(0u, 0u, 0u, 0u), p1 = p;
+    if (w < words) {
+      p = g0[r * words + w];
+      if (planes > 4) p1 = g1[r * words + w];
+    }
     uint32_t dash = p.x & p.y & p.z & p.w & valid;
     if (planes > 4) dash &= p1.x;
     if (planes > 5) dash &= p1.y;
-    uint8_t *blk = x + r * (words * row_bytes_per_word(planes)) + (w / 8) * (nb * 128) + (w % 8) * 16;
+    uint8_t *blk = x + g * group_bytes + in_group;
     put16(blk, p.x & valid, kE2M1One);
-    put16(blk + 128, p.y & valid, kE2M1One);
-    put16(blk + 256, p.z & valid, kE2M1One);
-    put16(blk + 384, p.w & valid, kE2M1One);
-    if (planes > 4) put16(blk + 512, p1.x & valid, kE2M1One);
-    if (planes > 5) put16(blk + 640, p1.y & valid, kE2M1One);
-    put16(blk + planes * 128, dash, kE2M1One);                // 1.0: the row side
-    put16(blk + (planes + 1) * 128, dash, dash_neg(planes));  // the column side
-    if (planes == 6) put16(blk + (planes + 2) * 128, dash, kE2M1Neg1);
+    put16(blk + kGroupBytes, p.y & valid, kE2M1One);
+    put16(blk + 2 * kGroupBytes, p.z & valid, kE2M1One);
+    put16(blk + 3 * kGroupBytes, p.w & valid, kE2M1One);
+    if (planes > 4) put16(blk + 4 * kGroupBytes, p1.x & valid, kE2M1One);
+    if (planes > 5) put16(blk + 5 * kGroupBytes, p1.y & valid, kE2M1One);
+    put16(blk + planes * kGroupBytes, dash, kE2M1One);                // 1.0: the row side
+    put16(blk + (planes + 1) * kGroupBytes, dash, dash_neg(planes));  // the column side
+    if (planes == 6) put16(blk + (planes + 2) * kGroupBytes, dash, kE2M1Neg1);
     // the chunk holds a '-': its dash products count (every writer stores 1)
-    if (dash && !dash_chunk[w / 8]) dash_chunk[w / 8] = 1u;
+    if (dash && !dash_chunk[c]) dash_chunk[c] = 1u;
   }
 }
 
 // ------------------------------------------------------- tcgen05 helpers
-// Shared-memory matrix descriptor, K-major, 128-byte swizzle: start address
-// >> 4 (bits 0-13), leading byte offset 16 B (unused for this layout, bits
-// 16-29), stride byte offset 1024 B between 8-row groups (bits 32-45),
-// descriptor version 1 (bits 46-47), layout SWIZZLE_128B = 2 (bits 61-63).
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+// Shared-memory matrix descriptor, K-major, no swizzle: start address >> 4
+// (bits 0-13), 128 B between the core matrices along K (bits 16-29), one
+// block between 8-row groups (bits 32-45), descriptor version 1 (bits 46-47).
+__device__ __forceinline__ uint64_t core_desc(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128 >> 4) << 16) |
+         ((uint64_t)(kGroupBytes >> 4) << 32) | ((uint64_t)1 << 46);
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                    smem_u32(dst)),
                "r"(ncols)
                : "memory");
 }
 __device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                : "memory");
 }
 __device__ __forceinline__ void tc_before_sync() {
@@ -229,18 +282,59 @@ __device__ __forceinline__ void tc_before_sync() {
 __device__ __forceinline__ void tc_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// D (+)= A B^T over K = 64 E2M1 values, every block of 32 scaled by the UE8M0
-// factors at TMEM addresses sfa and sfb
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// address, in the cluster's shared memory, of CTA `rank`'s copy of a local one
+__device__ __forceinline__ uint32_t map_rank(uint32_t saddr, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// the same without ordering memory: it does not wait for the stores in flight
+__device__ __forceinline__ void cluster_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed;\n\tbarrier.cluster.wait;" ::: "memory");
+}
+// D (+)= A B^T over K = 96 E2M1 values on the pair's tensor cores, every block
+// of 32 scaled by the UE8M0 factors at TMEM addresses sfa and sfb
 __device__ __forceinline__ void mma_f4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                        uint32_t idesc, uint32_t accumulate, uint32_t sfa,
                                        uint32_t sfb) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], "
+      "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], "
       "[%6], p;\n\t}" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
       : "memory");
+}
+// One K block (144 bytes a row) of an item: its three K steps against both
+// column halves, or the first alone.
+template <bool kSecond>
+__device__ __forceinline__ void mma_block(uint32_t tmem, uint64_t a_desc, uint32_t id0, uint32_t id1,
+                                          bool accumulate) {
+  constexpr uint64_t kStep = 128 * (kKStep / 16) >> 4;  // three core matrices
+  const uint64_t b0 = a_desc + (kABytes >> 4), b1 = b0 + (kB0Bytes >> 4);
+#pragma unroll
+  for (uint32_t k = 0; k < kBlockK / kKStep; ++k) {
+    const uint32_t acc = (accumulate || k) ? 1u : 0u;
+    mma_f4(tmem, a_desc + k * kStep, b0 + k * kStep, id0, acc, tmem + kSfColA, tmem + kSfColB);
+    if (kSecond)
+      mma_f4(tmem + kN0, a_desc + k * kStep, b1 + k * kStep, id1, acc, tmem + kSfColA, tmem + kSfColB);
+  }
+}
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
 }
 // The unit scale factors: this warp writes kSfWord to the NC TMEM columns
 // from col0 in its lane quarter (lane base `t_lane`) and waits for the
@@ -254,51 +348,62 @@ __device__ __forceinline__ void write_unit_scales(uint32_t t_lane, uint32_t col0
                  : "memory");
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// arrives on `bar` once every earlier tcgen05.mma of this thread has completed
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// 32 lanes x 64 consecutive 32-bit columns: thread t gets row (lane base + t)
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&v)[64]) {
+// arrives on both CTAs' barrier at `bar` once every earlier tcgen05.mma of
+// this thread has completed
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x64.b32 {"
-      "%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, "
-      "%19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, "
-      "%36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, "
-      "%53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63 "
-      "}, [%64];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]),
-        "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]),
-        "=r"(v[38]), "=r"(v[39]), "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]),
-        "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47]), "=r"(v[48]), "=r"(v[49]),
-        "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]),
-        "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]),
-        "=r"(v[62]), "=r"(v[63])
-      : "r"(taddr)
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
+      "[%0], %1;" ::"r"(bar),
+      "h"((uint16_t)3)
       : "memory");
 }
-// 32 lanes x 32 consecutive 32-bit columns
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+// bounded wait for a phase that the copies or the tensor cores complete, or
+// (kCluster) that a thread of either CTA completes to hand over what it wrote
+template <bool kCluster>
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  if (kCluster)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  return ok != 0;
+}
+template <bool kCluster = false>
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns) {
+  if (mbar_try<kCluster>(bar, parity)) return true;
+  const long long t0 = clock64(), limit = wait_cycles(limit_ns);
+  for (;;) {
+    if (mbar_try<kCluster>(bar, parity)) return true;
+    if (clock64() - t0 > limit) return false;
+  }
+}
+// TMA box of a pair's CTA: into its own shared memory, completion counted on
+// the barrier `bar` of the first CTA
+__device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap *map, int32_t x,
+                                              int32_t y, uint32_t bar) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {"
-      "%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, "
-      "%19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31 "
-      "}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
 // 32 lanes x 16 consecutive 32-bit columns
@@ -313,109 +418,169 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr)
       : "memory");
 }
+// 32 lanes x 8 consecutive 32-bit columns
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
+                 "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// min(sites - matches, max_dist) of accumulator columns OFF .. OFF + W - 1
-// (FP32 integers) into the warp's buffer, row `lane` at words 33 lane
-template <int OFF, int N, int W = 32>
-__device__ __forceinline__ void turn_chunk(uint32_t *buf, const uint32_t (&d)[N], uint32_t sites,
-                                           uint32_t max_dist, uint32_t lane) {
-  static_assert(OFF + W <= N, "columns outside the loaded registers");
+// min(sites - matches, cap) of two accumulator columns as packed 16-bit
+// values (cap <= 65535). FP32 throughout: every operand is an integer below
+// 2^24, and adding 2^23 leaves the value in the low mantissa bits, which
+// avoids the quarter-rate float-to-integer conversion while the accumulators
+// are held.
+__device__ __forceinline__ uint32_t pack2(uint32_t d0, uint32_t d1, float sites, float cap) {
+  const float m0 = fminf(sites - __uint_as_float(d0), cap) + 8388608.0f;
+  const float m1 = fminf(sites - __uint_as_float(d1), cap) + 8388608.0f;
+  return __byte_perm(__float_as_uint(m0), __float_as_uint(m1), 0x5410u);
+}
+
+// This warp's 32 rows x 248 columns from taddr, packed: word w holds columns
+// 2 w and 2 w + 1 of row `lane`.
+__device__ __forceinline__ void load_packed(uint32_t taddr, float sites, float cap,
+                                            uint32_t (&v)[kHalfWords]) {
 #pragma unroll
-  for (uint32_t j = 0; j < W; ++j) {
-    const uint32_t mism = sites - (uint32_t)__uint_as_float(d[OFF + j]);
-    buf[lane * kEpiPitch + j] = mism < max_dist ? mism : max_dist;
+  for (uint32_t g = 0; g < 7; ++g) {
+    uint32_t d[16], e[16];
+    tmem_ld16(taddr + 32 * g, d);
+    tmem_ld16(taddr + 32 * g + 16, e);
+    tmem_ld_wait();
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+      v[16 * g + k] = pack2(d[2 * k], d[2 * k + 1], sites, cap);
+      v[16 * g + 8 + k] = pack2(e[2 * k], e[2 * k + 1], sites, cap);
+    }
   }
+  uint32_t d[16], e[8];
+  tmem_ld16(taddr + 224, d);
+  tmem_ld8(taddr + 240, e);
+  tmem_ld_wait();
+#pragma unroll
+  for (uint32_t k = 0; k < 8; ++k) v[112 + k] = pack2(d[2 * k], d[2 * k + 1], sites, cap);
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k) v[120 + k] = pack2(e[2 * k], e[2 * k + 1], sites, cap);
 }
 
-// The buffered chunk of rows i0 .. i0 + rows - 1, columns j0 .. j0 + W - 1,
-// row by row: lane l < W stores column j0 + l of row i0 + r, lower-triangle
-// entry tri(i0 + r) + j0 + l = e0 + r i0 + r (r - 1) / 2, where it is below
-// the diagonal (j0 + l < i0 + r). The row loop is unrolled so that several
-// rows' loads and stores are in flight.
-template <typename T, uint32_t W = 32>
-__device__ __forceinline__ void store_chunk(T *out, unsigned long long e0, uint32_t i0,
-                                            uint32_t rows, uint32_t j0, const uint32_t *buf,
-                                            uint32_t lane) {
-#pragma unroll 8
-  for (uint32_t r = 0; r < 32; ++r)
-    if (r < rows && lane < W && j0 + lane < i0 + r)
-      out[e0 + (unsigned long long)r * i0 + r * (r - 1) / 2] = (T)buf[r * kEpiPitch + lane];
-}
-
-// One epilogue warp's share of an item: TMEM lanes of its quarter (rows
-// 32 sub + lane of each row tile) x its columns [c_lo, c_hi), read 64
-// columns at a time, then a last piece of 32 and one of 16 where the share
-// leaves them (112 = 64 + 32 + 16).
+// Rows i0 .. i0 + rows - 1 x columns j0 .. j0 + cols - 1 (cols <= 28) from the
+// warp's piece (row r's 16-bit values from word 15 r), row by row: lane l
+// stores column j0 + l of row i0 + r, lower-triangle entry tri(i0 + r) + j0 +
+// l = e0 + r i0 + r (r - 1) / 2, where it is below the diagonal. Eight rows
+// are read before they are stored: the compiler cannot tell the output from
+// the piece, and one row at a time waits for shared memory 32 times over (27 k
+// cycles for an item's 248 columns).
 template <typename T>
-__device__ __forceinline__ void epilogue_share(const MmaItem &tl, const MmaJob &job,
-                                               uint32_t t_lane, uint32_t c_lo, uint32_t c_hi,
-                                               uint32_t sub, uint32_t lane, uint32_t *buf) {
-  const uint32_t n = job.n, sites = job.sites, max_dist = job.max_dist;
-  T *out = static_cast<T *>(job.out);
-  for (uint32_t h = 0; h < tl.halves; ++h) {
-    const uint32_t i0 = (tl.I + h) * kTM + sub * 32;  // output row of lane 0
-    if (i0 >= n) continue;                           // warp-uniform
-    const uint32_t rows = n - i0 < 32u ? n - i0 : 32u;
-    const unsigned long long t0 = (unsigned long long)i0 * (i0 - 1) / 2 - job.out_base + lane;
-#pragma unroll 1
-    for (uint32_t c = c_lo; c < c_hi;) {
-      const uint32_t j0 = tl.J * kTN + c;  // first column of this group
-      if (j0 + 1 >= i0 + rows) break;      // no row reaches column j0 (warp-uniform)
-      __syncwarp();
-      if (c + 32 > c_hi) {  // a last piece of 16 columns
-        uint32_t d[16];
-        tmem_ld16(t_lane + 256u * h + c, d);
-        tmem_ld_wait();
-        turn_chunk<0, 16, 16>(buf, d, sites, max_dist, lane);
-        __syncwarp();
-        store_chunk<T, 16>(out, t0 + j0, i0, rows, j0, buf, lane);
-        __syncwarp();
-        break;
-      }
-      if (c + 64 > c_hi) {  // a piece of 32 columns
-        uint32_t d[32];
-        tmem_ld32(t_lane + 256u * h + c, d);
-        tmem_ld_wait();
-        turn_chunk<0>(buf, d, sites, max_dist, lane);
-        __syncwarp();
-        store_chunk<T>(out, t0 + j0, i0, rows, j0, buf, lane);
-        __syncwarp();
-        c += 32;
-        continue;
-      }
-      uint32_t d[64];
-      tmem_ld64(t_lane + 256u * h + c, d);
-      tmem_ld_wait();
-      turn_chunk<0>(buf, d, sites, max_dist, lane);
-      __syncwarp();
-      store_chunk<T>(out, t0 + j0, i0, rows, j0, buf, lane);
-      __syncwarp();  // the buffer is rewritten next
-      if (j0 + 33 >= i0 + rows) break;  // no row reaches column j0 + 32
-      turn_chunk<32>(buf, d, sites, max_dist, lane);
-      __syncwarp();
-      store_chunk<T>(out, t0 + j0 + 32, i0, rows, j0 + 32, buf, lane);
-      __syncwarp();
-      c += 64;
+__device__ __forceinline__ void store_piece(T *out, unsigned long long e0, uint32_t i0,
+                                            uint32_t rows, uint32_t j0, uint32_t cols,
+                                            const uint32_t *buf, uint32_t lane) {
+  // lanes past the columns read a column that is there (the piece has 30)
+  const uint16_t *h = reinterpret_cast<const uint16_t *>(buf) + (lane < cols ? lane : 0u);
+  // bit r: row i0 + r has column j0 + lane (rows first .. rows - 1)
+  const uint32_t first = j0 + lane < i0 ? 0u : j0 + lane + 1 - i0;
+  uint32_t on = rows >= 32 ? 0xffffffffu : (1u << rows) - 1u;
+  on = first < 32 ? on & (0xffffffffu << first) : 0u;
+  if (lane >= cols) on = 0;
+  T *o = out + e0;
+#pragma unroll
+  for (uint32_t r0 = 0; r0 < 32; r0 += 8) {
+    T x[8];
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) x[k] = (T)h[2 * kPiecePitch * (r0 + k)];
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+      if (on & (1u << (r0 + k))) *o = x[k];
+      o += i0 + r0 + k;  // tri(i + 1) - tri(i) = i
     }
   }
 }
 
-__global__ void __launch_bounds__(kMmaThreads, 1)
-    k_pairwise_mma(const MmaJob *__restrict__ jobs, const MmaItem *__restrict__ items,
-                   uint32_t n_items, unsigned *__restrict__ counter, uint32_t queue,
-                   int *status) {
+// The packed columns of one epilogue warp (rows i0 .., columns j0 .. j0 + 247,
+// those below col_end) to the output.
+template <typename T>
+__device__ __forceinline__ void store_packed(const MmaJob &job, uint32_t i0, uint32_t j0,
+                                             uint32_t col_end, const uint32_t (&v)[kHalfWords],
+                                             uint32_t lane, uint32_t *buf) {
+  const uint32_t rows = job.row_hi - i0 < 32u ? job.row_hi - i0 : 32u;
+  T *out = static_cast<T *>(job.out);
+  const unsigned long long t0 = (unsigned long long)i0 * (i0 - 1) / 2 - job.out_base + lane;
+#pragma unroll
+  for (uint32_t q = 0; q * kPieceWords < kHalfWords; ++q) {
+    constexpr uint32_t kAll = kHalfWords;
+    const uint32_t j = j0 + 2 * kPieceWords * q;
+    // no row reaches column j, or the item ends before it (warp-uniform)
+    if (j >= col_end || j + 1 >= i0 + rows) break;
+    const uint32_t words = kAll - q * kPieceWords < kPieceWords ? kAll - q * kPieceWords : kPieceWords;
+    const uint32_t cols = col_end - j < 2 * words ? col_end - j : 2 * words;
+    __syncwarp();  // the previous piece has been read
+#pragma unroll
+    for (uint32_t w = 0; w < words; ++w) buf[lane * kPiecePitch + w] = v[q * kPieceWords + w];
+    __syncwarp();
+    store_piece<T>(out, t0 + j, i0, rows, j, cols, buf, lane);
+  }
+}
+
+// 32-bit outputs: 8 columns at a time straight from the accumulators, four
+// rows per store.
+__device__ __forceinline__ void store_wide(const MmaJob &job, uint32_t taddr, uint32_t i0,
+                                           uint32_t j0, uint32_t col_end, uint32_t lane,
+                                           uint32_t *buf) {
+  const uint32_t rows = job.row_hi - i0 < 32u ? job.row_hi - i0 : 32u;
+  uint32_t *out = static_cast<uint32_t *>(job.out);
+  const unsigned long long t0 = (unsigned long long)i0 * (i0 - 1) / 2 - job.out_base;
+#pragma unroll 1
+  for (uint32_t c = 0; c < kHalfCols; c += 8) {
+    const uint32_t j = j0 + c;
+    if (j >= col_end || j + 1 >= i0 + rows) break;  // warp-uniform
+    uint32_t d[8];
+    tmem_ld8(taddr + c, d);
+    tmem_ld_wait();
+    __syncwarp();
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+      const uint32_t mism = job.sites - (uint32_t)__uint_as_float(d[k]);
+      buf[lane * 9 + k] = mism < job.max_dist ? mism : job.max_dist;
+    }
+    __syncwarp();
+    const uint32_t k = lane & 7u;
+#pragma unroll
+    for (uint32_t r = lane >> 3; r < 32; r += 4)
+      if (r < rows && j + k < col_end && j + k < i0 + r)
+        out[t0 + j + k + (unsigned long long)r * i0 + r * (r - 1) / 2] = buf[r * 9 + k];
+  }
+}
+static_assert(32 * 9 <= 32 * kPiecePitch, "the wide piece fits the warp's buffer");
+
+// Sites of a job in the chunks [c_lo, c_hi).
+__device__ __forceinline__ uint32_t sites_in(const MmaJob &job, uint32_t c_lo, uint32_t c_hi) {
+  const uint32_t hi = c_hi * kChunkSites, lo = c_lo * kChunkSites;
+  return (hi < job.sites ? hi : job.sites) - (lo < job.sites ? lo : job.sites);
+}
+// K blocks of the chunks [c_lo, c_hi): P per chunk, then the dash products of
+// the listed ones.
+__device__ __forceinline__ uint32_t blocks_in(const MmaJob &job, uint32_t c_lo, uint32_t c_hi) {
+  const uint32_t d = job.dash_rank[c_hi] - job.dash_rank[c_lo];
+  return job.planes * (c_hi - c_lo) + (job.planes == 6 ? 2 * d : d);
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMmaThreads, 1)
+    k_pairwise_mma(const CUtensorMap *__restrict__ tms, const MmaJob *__restrict__ jobs,
+                   uint32_t n_jobs, const MmaItem *__restrict__ items, uint32_t n_items,
+                   unsigned *__restrict__ counter, uint32_t queue, uint32_t *__restrict__ ws,
+                   unsigned long long *macs, int *status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full[kMmaStages], empty[kMmaStages], done, tmem_free, fin;
   __shared__ __align__(8) uint64_t item_full[kItemRing], item_empty[kItemRing];
   __shared__ uint32_t s_item[kItemRing];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
-  uint8_t *smem =
-      reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t smem = (smem_u32(smem_raw) + 127u) & ~127u;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_rank(), unit = blockIdx.x >> 1, units = gridDim.x >> 1;
   if (tid == 0) {
     for (int s = 0; s < kMmaStages; ++s) {
       mbar_init(&full[s], 1);
@@ -423,10 +588,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     }
     for (int r = 0; r < kItemRing; ++r) {
       mbar_init(&item_full[r], 1);
-      mbar_init(&item_empty[r], 1 + kEpiWarps);  // the MMA thread and each epilogue warp
+      mbar_init(&item_empty[r], kRingReaders);
     }
     mbar_init(&done, 1);
-    mbar_init(&tmem_free, kEpiThreads);
+    mbar_init(&tmem_free, 2 * kEpiWarps);
     mbar_init(&fin, 1);
     fence_mbar_init();
     s_abort = 0;
@@ -440,166 +605,210 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
   tc_after_sync();
   const uint32_t tmem = s_tmem;
   // the unit scale factors, once per CTA: warps 2-5 cover the lane quarters
-  if (warp >= 2 && warp < 6) {
-    write_unit_scales<16>(tmem + (((warp & 3u) * 32) << 16), kSfColA);
-    write_unit_scales<16>(tmem + (((warp & 3u) * 32) << 16), kSfColB);
-  }
+  if (warp >= 2 && warp < 6) write_unit_scales<16>(tmem + (((warp & 3u) * 32) << 16), kSfColA);
   tc_before_sync();
   __syncthreads();
+  cluster_sync();  // both CTAs' barriers and scale factors are ready
   tc_after_sync();
 
+  const uint32_t full0 = smem_u32(&full[0]), empty0 = smem_u32(&empty[0]);
+  const uint32_t ring_full0 = smem_u32(&item_full[0]);
+  // barriers of the first CTA, where both CTAs' threads arrive
+  const uint32_t lead_full0 = map_rank(full0, 0);
+  const uint32_t lead_ring_empty0 = map_rank(smem_u32(&item_empty[0]), 0);
   if (warp == 0) {
     if (lane == 0) {
-      // producer: draws this CTA's items from the launch's queue (its first
-      // item is blockIdx.x, later ones gridDim.x + an atomic count) or, with
-      // `queue` 0, round-robin (blockIdx.x + k gridDim.x); hands each item's
-      // index to the MMA and epilogue warps through the ring, then loads
-      // every K block of the item
-      uint32_t g = 0;  // K blocks issued (stage g % S, phase g / S)
+      // producer: loads its CTA's share of every K block of this pair's items.
+      // Static order: items unit, unit + units, ...; every warp walks them by
+      // itself. With `queue`, item `unit` and then the launch's counter: the
+      // first CTA's producer hands each index to the MMA warp and, in both
+      // CTAs, the epilogue warps and the second producer.
+      const uint32_t peer_item0 = map_rank(smem_u32(&s_item[0]), 1);
+      const uint32_t peer_ring_full0 = map_rank(ring_full0, 1);
+      uint32_t s = 0, ph = 1;  // stage, and the parity its empty barrier is waited for
       bool ok = true;
       for (uint32_t k = 0; ok; ++k) {
         const uint32_t r = k % kItemRing;
-        if (k >= (uint32_t)kItemRing &&
-            !mbar_wait_bounded(&item_empty[r], ((k / kItemRing) - 1) & 1u, kMmaWaitNs)) {
-          ok = false;
-          break;
-        }
-        uint32_t t = k == 0 ? blockIdx.x
-                            : (queue ? gridDim.x + atomicAdd(counter, 1u) : blockIdx.x + k * gridDim.x);
-        if (t >= n_items || *(volatile int *)&s_abort) t = kNoItem;
-        *(volatile uint32_t *)&s_item[r] = t;
-        mbar_arrive(&item_full[r]);  // releases the index to the waiting warps
-        if (t == kNoItem) break;
-        const MmaItem tl = items[t];
-        const MmaJob &job = jobs[tl.job];
-        const CUtensorMap *ta = tl.halves == 2 ? job.tm256 : job.tm128;
-        prefetch_tmap(ta);
-        prefetch_tmap(job.tmb);
-        const int32_t ya = (int32_t)(tl.I * kTM), yb = (int32_t)(tl.J * kTN);
-        const uint32_t bytes = kBBytes + tl.halves * kHalfBytes, nkb = job.nkb, P = job.planes;
-        const uint32_t NB = op_blocks(P), plane_kb = P * job.chunks;
-        for (uint32_t kb = 0; kb < nkb; ++kb) {
-          const uint32_t s = g % kMmaStages;
-          if ((g >= (uint32_t)kMmaStages &&
-               !mbar_wait_bounded(&empty[s], ((g / kMmaStages) - 1) & 1u, kMmaWaitNs)) ||
-              *(volatile int *)&s_abort) {
+        uint32_t t = unit + k * units;
+        if (queue && rank == 0) {
+          if (k >= (uint32_t)kItemRing &&
+              !mbar_wait<true>(smem_u32(&item_empty[r]), ((k / kItemRing) - 1) & 1u, 4 * kMmaWaitNs)) {
             ok = false;
             break;
           }
-          // K block kb: first the P plane blocks of every 256-site chunk,
-          // then the dash products of the chunks that hold a '-' (the rows'
-          // +1 block against the columns' -(P - 1) block; for P = 6 the +1
-          // block twice, against -4 and -1). Elsewhere the dash products are
-          // all 0, so those blocks are left out.
-          uint32_t blk_a, blk_b;
-          if (kb < plane_kb) {
-            blk_a = blk_b = NB * (kb / P) + kb % P;
-          } else {
-            const uint32_t j = kb - plane_kb, two = P == 6 ? 1u : 0u;
-            const uint32_t c = job.dash_list[j >> two];
-            blk_a = NB * c + P;
-            blk_b = NB * c + P + 1 + (j & two);
+          if (k) t = units + atomicAdd(counter, 1u);
+          if (t >= n_items || *(volatile int *)&s_abort) t = kNoItem;
+          *(volatile uint32_t *)&s_item[r] = t;
+          asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer_item0 + 4 * r), "r"(t) : "memory");
+          mbar_arrive_cluster(peer_ring_full0 + 8 * r);  // releases the index
+          mbar_arrive_cluster(map_rank(ring_full0 + 8 * r, 0));
+        } else if (queue) {
+          if (!mbar_wait<true>(ring_full0 + 8 * r, (k / kItemRing) & 1u, 4 * kMmaWaitNs)) {
+            ok = false;
+            break;
           }
-          const int32_t xa = (int32_t)(blk_a * 128), xb = (int32_t)(blk_b * 128);
-          uint8_t *st = smem + s * kStageBytes;
-          mbar_expect_tx(&full[s], bytes);
-          tma_load_2d(st, ta, xa, ya, &full[s]);
-          tma_load_2d(st + kABytes, job.tmb, xb, yb, &full[s]);
-          ++g;
+          t = *(volatile uint32_t *)&s_item[r];
+          mbar_arrive_cluster(lead_ring_empty0 + 8 * r);
+        }
+        if (t >= n_items) break;
+        const MmaItem it = items[t];
+        if (it.job == kNoItem) break;
+        const CUtensorMap *t128 = tms + 2 * it.job, *t120 = t128 + 1;
+        // row groups of this CTA's 128 rows, and of its half of each column half
+        const int32_t ya = (int32_t)(it.row0 / 8 + rank * (kTM / 8));
+        const int32_t yb0 = (int32_t)(it.col0 / 8 + rank * it.n0_16);
+        const int32_t yb1 = (int32_t)((it.col0 + it.n0()) / 8 + rank * it.n1_16);
+        const bool second = it.n1_16 != 0;
+        const uint32_t bytes = 2 * (kABytes + kB0Bytes + (second ? kB1Bytes : 0u));
+        auto issue = [&](int32_t xa, int32_t xb) {
+          if (!mbar_wait(empty0 + 8 * s, ph, kMmaWaitNs)) return false;
+          if (rank == 0) mbar_expect(full0 + 8 * s, bytes);
+          const uint32_t st = smem + s * kStageBytes, bar = lead_full0 + 8 * s;
+          tma_load_pair(st, t128, xa, ya, bar);
+          tma_load_pair(st + kABytes, t128, xb, yb0, bar);
+          if (second) tma_load_pair(st + kABytes + kB0Bytes, t120, xb, yb1, bar);
+          if (++s == (uint32_t)kMmaStages) {
+            s = 0;
+            ph ^= 1u;
+          }
+          return true;
+        };
+        // K order: the P plane blocks of every chunk, then the dash products
+        // of the listed chunks (the rows' +1 block against the columns'
+        // -(P - 1) block; for P = 6 the +1 block twice, against -4 and -1).
+        // Coordinates count 8-byte elements: a block is 144 of them.
+        const uint32_t P = it.planes, NB = op_blocks(P);
+        int32_t x = (int32_t)(it.c_lo * NB * kBlockK);
+        for (uint32_t c = it.c_lo; ok && c < it.c_hi; ++c, x += (int32_t)((NB - P) * kBlockK))
+          for (uint32_t p = 0; p < P; ++p, x += (int32_t)kBlockK)
+            if (!issue(x, x)) {
+              ok = false;
+              break;
+            }
+        const MmaJob &job = jobs[it.job];
+        const uint32_t d_hi = job.dash_rank[it.c_hi];
+        for (uint32_t d = job.dash_rank[it.c_lo]; ok && d < d_hi; ++d) {
+          const int32_t xd = (int32_t)((job.dash_list[d] * NB + P) * kBlockK);
+          ok = issue(xd, xd + (int32_t)kBlockK);
+          if (ok && P == 6) ok = issue(xd, xd + 2 * (int32_t)kBlockK);
         }
       }
       if (!ok) {
         atomicExch(&s_abort, 1);
         atomicExch(status, kStatusTmaTimeout);
+        // the copies in flight land (microseconds) before the CTA may leave
+        const uint64_t t0 = global_ns();
+        while (global_ns() - t0 < 10000000ull) {
+        }
       }
-      // the copies still in flight land before the CTA may leave
-      for (uint32_t q = g > (uint32_t)kMmaStages ? g - kMmaStages : 0; q < g; ++q)
-        mbar_wait_bounded(&full[q % kMmaStages], (q / kMmaStages) & 1u, kMmaWaitNs);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // MMA issuer
-      uint32_t g = 0;
+    if (rank == 0) {
+      // MMA issuer of the pair: the whole warp walks the loop, so that the
+      // descriptors stay in uniform registers, and one elected lane issues
+      const bool lead = elect_one();
+      uint32_t s = 0, ph = 0;
+      const uint64_t desc0 = core_desc(smem);
+      uint64_t desc = desc0;
       bool ok = true;
-      for (uint32_t it = 0; ok; ++it) {
-        const uint32_t r = it % kItemRing;
-        if (!mbar_wait_bounded(&item_full[r], (it / kItemRing) & 1u, 4 * kMmaWaitNs)) {
-          ok = false;
-          break;
+      for (uint32_t k = 0; ok; ++k) {
+        uint32_t t = unit + k * units;
+        if (queue) {
+          const uint32_t r = k % kItemRing;
+          if (!mbar_wait<true>(ring_full0 + 8 * r, (k / kItemRing) & 1u, 4 * kMmaWaitNs)) {
+            ok = false;
+            break;
+          }
+          t = __shfl_sync(0xffffffffu, *(volatile uint32_t *)&s_item[r], 0);
+          if (lead) mbar_arrive_cluster(lead_ring_empty0 + 8 * r);
         }
-        const uint32_t t = *(volatile uint32_t *)&s_item[r];
-        mbar_arrive(&item_empty[r]);
-        if (t == kNoItem) break;
-        const uint32_t halves = items[t].halves, nkb = jobs[items[t].job].nkb;
-        // the epilogue has read the previous item's accumulators
-        if (it > 0 && !mbar_wait_bounded(&tmem_free, (it - 1) & 1u, kMmaWaitNs)) {
+        if (t >= n_items) break;
+        const MmaItem it = items[t];
+        if (it.job == kNoItem) break;
+        const uint32_t nkb = __shfl_sync(0xffffffffu, blocks_in(jobs[it.job], it.c_lo, it.c_hi), 0);
+        const uint32_t n0 = __shfl_sync(0xffffffffu, it.n0(), 0);
+        const uint32_t n1 = __shfl_sync(0xffffffffu, it.n1(), 0);
+        const uint32_t id0 = idesc_mxf4(n0), id1 = idesc_mxf4(n1);
+        // both CTAs' epilogues have read the previous item's accumulators
+        if (k > 0 && !mbar_wait(smem_u32(&tmem_free), (k - 1) & 1u, kMmaWaitNs)) {
           ok = false;
           break;
         }
         tc_after_sync();
         for (uint32_t kb = 0; kb < nkb; ++kb) {
-          const uint32_t s = g % kMmaStages;
-          if (!mbar_wait_bounded(&full[s], (g / kMmaStages) & 1u, kMmaWaitNs) ||
-              *(volatile int *)&s_abort) {
+          if (!mbar_wait(full0 + 8 * s, ph, kMmaWaitNs)) {
             ok = false;
             break;
           }
           tc_after_sync();
-          const uint32_t a0 = smem_u32(smem + s * kStageBytes);
-          const uint64_t bd = sw128_desc(a0 + kABytes);
-          for (uint32_t h = 0; h < halves; ++h) {
-            const uint64_t ad = sw128_desc(a0 + h * kHalfBytes);
-#pragma unroll
-            for (uint32_t k = 0; k < 4; ++k)  // 32 bytes of K per MMA: +2 in 16-byte units
-              mma_f4(tmem + 256u * h, ad + 2 * k, bd + 2 * k, kIdesc, (kb | k) ? 1u : 0u,
-                     tmem + kSfColA, tmem + kSfColB);
+          if (lead) {
+            if (n1) mma_block<true>(tmem, desc, id0, id1, kb != 0);
+            else mma_block<false>(tmem, desc, id0, id1, kb != 0);
+            mma_commit(empty0 + 8 * s);
           }
-          mma_commit(&empty[s]);
-          ++g;
+          __syncwarp();
+          desc += kStageBytes >> 4;
+          if (++s == (uint32_t)kMmaStages) {
+            s = 0;
+            ph ^= 1u;
+            desc = desc0;
+          }
         }
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        mma_commit(&done);
+        if (lead) mma_commit(smem_u32(&done));
       }
-      if (!ok) {
-        atomicExch(&s_abort, 1);
-        atomicExch(status, kStatusTmaTimeout);
-        mma_commit(&done);  // releases an epilogue waiting for this item
+      if (lead) {
+        if (!ok) {
+          atomicExch(&s_abort, 1);
+          atomicExch(status, kStatusTmaTimeout);
+          mma_commit(smem_u32(&done));  // releases the epilogues waiting for this item
+        }
+        // every MMA of this thread has completed before TMEM is freed
+        mma_commit(smem_u32(&fin));
+        mbar_wait(smem_u32(&fin), 0, 4 * kMmaWaitNs);
       }
-      // every MMA of this thread has completed before TMEM is freed
-      mma_commit(&fin);
-      mbar_wait_bounded(&fin, 0, 4 * kMmaWaitNs);
+    } else if (unit == 0) {
+      // the launch's multiply-adds (pairs x 288 values per K block)
+      for (uint32_t q = lane; q < n_jobs; q += 32)
+        atomicAdd(macs, jobs[q].pairs * (unsigned long long)kChunkSites *
+                            blocks_in(jobs[q], 0, jobs[q].chunks));
     }
   } else {
-    // epilogue warps 2 .. 2 + kEpiWarps - 1: warp w reads TMEM lanes
-    // 32 (w % 4) .. + 31, which are rows 32 (w % 4) + lane of each row tile
-    // of the item, in columns [0, 128) (w < 6) or [128, kTN) (w >= 6). Each
-    // 32 x 32 chunk goes through the warp's padded shared buffer (row r at
-    // words 33 r: conflict-free both ways), so that one store instruction
-    // writes 32 consecutive entries of one row rather than one entry of 32
-    // rows.
-    const uint32_t sub = warp & 3u, c_lo = warp < 6 ? 0u : kEpiSplit, c_hi = warp < 6 ? kEpiSplit : (uint32_t)kTN;
-    const uint32_t t_lane = tmem + ((sub * 32) << 16);
-    uint32_t *buf = reinterpret_cast<uint32_t *>(smem + kMmaStages * kStageBytes) +
-                    (warp - 2) * 32 * kEpiPitch;
-    for (uint32_t it = 0;; ++it) {
-      const uint32_t r = it % kItemRing;
-      // lane 0 waits and reads the index; the warp takes its answer
-      uint32_t t = kNoItem;
+    // epilogue warps 2 .. 9: warp w reads TMEM lanes 32 (w % 4) .. + 31, which
+    // are rows 32 (w % 4) + lane of the CTA's 128, in columns [0, 248) (w < 6)
+    // or [248, 496) (w >= 6) of the item
+    const uint32_t sub = warp & 3u, half = warp < 6 ? 0u : 1u;
+    const uint32_t taddr = tmem + ((sub * 32) << 16) + half * kHalfCols;
+    const uint32_t lead_free = map_rank(smem_u32(&tmem_free), 0);
+    uint32_t *buf = reinterpret_cast<uint32_t *>(smem_raw + (smem - smem_u32(smem_raw)) +
+                                                 kMmaStages * kStageBytes) +
+                    (warp - 2) * 32 * kPiecePitch;
+    for (uint32_t k = 0;; ++k) {
+      uint32_t t = unit + k * units;
       bool got = true;
-      if (lane == 0) {
-        got = mbar_wait_bounded(&item_full[r], (it / kItemRing) & 1u, 4 * kMmaWaitNs);
-        if (got) t = *(volatile uint32_t *)&s_item[r];
+      if (queue) {
+        // lane 0 waits and reads the index; the warp takes its answer
+        const uint32_t r = k % kItemRing;
+        if (lane == 0) {
+          got = mbar_wait<true>(ring_full0 + 8 * r, (k / kItemRing) & 1u, 4 * kMmaWaitNs);
+          if (got) {
+            t = *(volatile uint32_t *)&s_item[r];
+            mbar_arrive_cluster(lead_ring_empty0 + 8 * r);
+          }
+        }
+        got = __shfl_sync(0xffffffffu, got ? 1u : 0u, 0) != 0;
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (!got) {
+          atomicExch(&s_abort, 1);
+          atomicExch(status, kStatusTmaTimeout);
+        }
       }
-      got = __shfl_sync(0xffffffffu, got ? 1u : 0u, 0) != 0;
-      t = __shfl_sync(0xffffffffu, t, 0);
-      if (got && lane == 0) mbar_arrive(&item_empty[r]);
-      if (!got) {
-        atomicExch(&s_abort, 1);
-        atomicExch(status, kStatusTmaTimeout);
-      }
-      // one decision per warp: tcgen05.ld needs the whole warp
-      if (__any_sync(0xffffffffu, t == kNoItem)) break;
-      got = mbar_wait_bounded(&done, it & 1u, 4 * kMmaWaitNs);
+      if (t >= n_items) break;
+      const MmaItem it = items[t];
+      if (it.job == kNoItem) break;
+      const MmaJob &job = jobs[it.job];
+      got = mbar_wait(smem_u32(&done), k & 1u, 4 * kMmaWaitNs);
       if (!got) {
         atomicExch(&s_abort, 1);
         atomicExch(status, kStatusTmaTimeout);
@@ -607,21 +816,42 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
       // one decision per warp: tcgen05.ld needs the whole warp
       if (__any_sync(0xffffffffu, !got || *(volatile int *)&s_abort)) break;
       tc_after_sync();
-      const MmaItem tl = items[t];
-      const MmaJob &job = jobs[tl.job];
-      if (job.dtype == 1)
-        epilogue_share<uint8_t>(tl, job, t_lane, c_lo, c_hi, sub, lane, buf);
-      else if (job.dtype == 2)
-        epilogue_share<uint16_t>(tl, job, t_lane, c_lo, c_hi, sub, lane, buf);
-      else
-        epilogue_share<uint32_t>(tl, job, t_lane, c_lo, c_hi, sub, lane, buf);
+      const uint32_t i0 = it.row0 + rank * kTM + sub * 32, j0 = it.col0 + half * kHalfCols;
+      const uint32_t col_end = it.col0 + it.n0() + it.n1();
+      // nothing below the diagonal, or past the rows or columns (warp-uniform)
+      const bool any = i0 < job.row_hi && j0 < col_end && j0 + 1 < i0 + 32;
+      if (job.dtype == 4) {
+        if (any) store_wide(job, taddr, i0, j0, col_end, lane, buf);
+        tc_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(lead_free);
+        continue;
+      }
+      uint32_t v[kHalfWords];
+      if (any) {
+        const uint32_t top = it.slot != kNoSlot ? 65535u : job.max_dist;
+        load_packed(taddr, (float)sites_in(job, it.c_lo, it.c_hi), (float)top, v);
+      }
       // the accumulators may be overwritten
       tc_before_sync();
-      mbar_arrive(&tmem_free);
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(lead_free);
+      if (!any) continue;
+      if (it.slot != kNoSlot) {
+        uint32_t *w = ws + (((uint64_t)it.slot * 2 + rank) * 8 + half * 4 + sub) * kHalfWords * 32 + lane;
+#pragma unroll
+        for (uint32_t q = 0; q < kHalfWords; ++q) w[32 * q] = v[q];
+      } else if (job.dtype == 1) {
+        store_packed<uint8_t>(job, i0, j0, col_end, v, lane, buf);
+      } else {
+        store_packed<uint16_t>(job, i0, j0, col_end, v, lane, buf);
+      }
     }
   }
   tc_before_sync();
   __syncthreads();
+  // neither CTA leaves while the other may still signal it or read its operands
+  cluster_sync_relaxed();
   tc_after_sync();
   if (warp == 0) {
     __syncwarp();
@@ -629,19 +859,78 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
   }
 }
 
-// FP4 (kind::mxf4) MMA rate from shared memory alone (no loads): one CTA per
-// SM (the shared-memory request keeps it alone) issues `rounds` x 4 MMAs of
-// M=128, N=256, K=64 on a zeroed stage (the values do not change the rate),
-// with unit scale factors in TMEM columns 256-287.
-constexpr uint32_t kPeakN = 256, kPeakSf = 256;
-__global__ void __launch_bounds__(128, 1) k_peak_mma(uint32_t rounds, int *status) {
+// The split tiles: each warp adds one piece (32 rows x 28 columns) of a tile
+// over the tile's K pieces, saturating at 65,535 (the results saturate at
+// max_dist <= 65,535 anyway), and stores it as the epilogue does. The
+// workspace was written just before and is read from L2.
+constexpr uint32_t kFixPieces = (kHalfWords + kPieceWords - 1) / kPieceWords;  // per 248 columns
+constexpr uint32_t kFixWarps = 2 * 8 * kFixPieces;                             // per tile
+constexpr uint32_t kLastWords = kHalfWords - (kFixPieces - 1) * kPieceWords;     // the last piece's
+__global__ void __launch_bounds__(256)
+    k_pair_fix(const MmaJob *__restrict__ jobs, const MmaFix *__restrict__ fix, uint32_t n_fix,
+               const uint32_t *__restrict__ ws) {
+  __shared__ uint32_t s_buf[8][32 * kPiecePitch];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t id = blockIdx.x * 8 + warp;
+  if (id >= n_fix * kFixWarps) return;
+  const MmaFix f = fix[id / kFixWarps];
+  const MmaJob &job = jobs[f.job];
+  const uint32_t q = id % kFixPieces, part = id / kFixPieces % 16;  // (rank, half, quarter)
+  const uint32_t i0 = f.row0 + (part >> 3) * kTM + (part & 3u) * 32;
+  const uint32_t j = f.col0 + (part >> 2 & 1u) * kHalfCols + 2 * kPieceWords * q;
+  if (i0 >= job.row_hi) return;
+  const uint32_t rows = job.row_hi - i0 < 32u ? job.row_hi - i0 : 32u;
+  if (j >= f.col0 + f.cols || j + 1 >= i0 + rows) return;
+  const uint32_t words = kHalfWords - q * kPieceWords < kPieceWords ? kHalfWords - q * kPieceWords
+                                                                    : kPieceWords;
+  uint32_t v[kPieceWords];
+#pragma unroll
+  for (uint32_t w = 0; w < kPieceWords; ++w) v[w] = 0;
+  const uint32_t *src = ws + (((uint64_t)f.slot * 16 + part) * kHalfWords + q * kPieceWords) * 32 + lane;
+  // the last piece's missing words repeat its last one (they are not stored),
+  // so that the loads of four parts go out together
+  auto add = [&](auto parts) {
+    constexpr uint32_t U = decltype(parts)::value;
+    uint32_t x[U][kPieceWords];
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u)
+#pragma unroll
+      for (uint32_t w = 0; w < kPieceWords; ++w)
+        x[u][w] = __ldcg(src + u * (kSlotBytes / 4) + 32 * (w < kLastWords ? w : min(w, words - 1)));
+#pragma unroll
+    for (uint32_t u = 0; u < U; ++u)
+#pragma unroll
+      for (uint32_t w = 0; w < kPieceWords; ++w) v[w] = __vaddus2(v[w], x[u][w]);
+    src += U * (kSlotBytes / 4);
+  };
+  uint32_t p = 0;
+  for (; p + 4 <= f.parts; p += 4) add(std::integral_constant<uint32_t, 4>());
+  for (; p < f.parts; ++p) add(std::integral_constant<uint32_t, 1>());
+  const uint32_t cap = job.max_dist * 0x10001u;
+  uint32_t *buf = s_buf[warp];
+#pragma unroll
+  for (uint32_t w = 0; w < kPieceWords; ++w) buf[lane * kPiecePitch + w] = __vminu2(v[w], cap);
+  __syncwarp();
+  const uint32_t cols = f.col0 + f.cols - j < 2 * words ? f.col0 + f.cols - j : 2 * words;
+  const unsigned long long e0 = (unsigned long long)i0 * (i0 - 1) / 2 - job.out_base + lane + j;
+  if (job.dtype == 1)
+    store_piece<uint8_t>(static_cast<uint8_t *>(job.out), e0, i0, rows, j, cols, buf, lane);
+  else
+    store_piece<uint16_t>(static_cast<uint16_t *>(job.out), e0, i0, rows, j, cols, buf, lane);
+}
+
+// FP4 (kind::mxf4) MMA rate from shared memory alone (no loads): CTA pairs
+// issue `rounds` K blocks of the engine's own MMAs (M = 256, N = 256 and 240,
+// K = 96) on zeroed stages (the values do not change the rate).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1)
+    k_peak_mma(uint32_t rounds, int *status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_tmem;
-  uint8_t *smem =
-      reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  for (uint32_t k = threadIdx.x; k < (kABytes + kPeakN * 128) / 16; k += blockDim.x)
-    reinterpret_cast<uint4 *>(smem)[k] = make_uint4(0, 0, 0, 0);
+  const uint32_t smem = (smem_u32(smem_raw) + 127u) & ~127u;
+  uint8_t *stage = smem_raw + (smem - smem_u32(smem_raw));
+  for (uint32_t k = threadIdx.x; k < kStageBytes / 16; k += blockDim.x)
+    reinterpret_cast<uint4 *>(stage)[k] = make_uint4(0, 0, 0, 0);
   // the generic-proxy writes above, before the tensor cores read them
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (threadIdx.x == 0) {
@@ -656,23 +945,23 @@ __global__ void __launch_bounds__(128, 1) k_peak_mma(uint32_t rounds, int *statu
   __syncthreads();
   tc_after_sync();
   const uint32_t tmem = s_tmem;
-  write_unit_scales<32>(tmem + (((threadIdx.x >> 5) * 32) << 16), kPeakSf);
+  write_unit_scales<16>(tmem + (((threadIdx.x >> 5) * 32) << 16), kSfColA);
   tc_before_sync();
   __syncthreads();
+  cluster_sync();
   tc_after_sync();
   if (threadIdx.x == 0) {
-    const uint32_t a0 = smem_u32(smem);
-    const uint64_t ad = sw128_desc(a0), bd = sw128_desc(a0 + kABytes);
-    for (uint32_t r = 0; r < rounds; ++r)
-#pragma unroll
-      for (uint32_t k = 0; k < 4; ++k)
-        mma_f4(tmem, ad + 2 * k, bd + 2 * k, idesc_mxf4(kPeakN), (r | k) ? 1u : 0u,
-               tmem + kPeakSf, tmem + kPeakSf + 16);
-    mma_commit(&bar);
-    if (!mbar_wait_bounded(&bar, 0, 4 * kMmaWaitNs)) atomicExch(status, kStatusTmaTimeout);
+    if (cluster_rank() == 0) {
+      const uint64_t desc = core_desc(smem);
+      for (uint32_t r = 0; r < rounds; ++r)
+        mma_block<true>(tmem, desc, idesc_mxf4(kN0), idesc_mxf4(kN1), r != 0);
+      mma_commit(smem_u32(&bar));
+    }
+    if (!mbar_wait(smem_u32(&bar), 0, 4 * kMmaWaitNs)) atomicExch(status, kStatusTmaTimeout);
   }
   tc_before_sync();
   __syncthreads();
+  cluster_sync();
   tc_after_sync();
   if (threadIdx.x < 32) {
     __syncwarp();
@@ -680,27 +969,22 @@ __global__ void __launch_bounds__(128, 1) k_peak_mma(uint32_t rounds, int *statu
   }
 }
 
-// One warp per job: the ascending list of the chunks whose mark is set, and
-// the job's K blocks (P per chunk, then one per listed chunk, two for P = 6);
-// the job's multiply-adds (pairs x 256 values per K block) are added to
-// *macs. A mark set concurrently by a later expansion (rows this launch does
-// not read) only adds dash products of 0.
-__global__ void k_dash_list(MmaJob *jobs, unsigned long long *macs) {
-  MmaJob &job = jobs[blockIdx.x];
-  const uint32_t lane = threadIdx.x;
-  uint32_t *list = const_cast<uint32_t *>(job.dash_list);
+// The ascending list of the chunks whose mark is set, and for every chunk the
+// listed ones before it (one block).
+__global__ void __launch_bounds__(512)
+    k_dash_list(const uint32_t *marks, uint32_t chunks, uint32_t *list, uint32_t *before) {
+  __shared__ uint32_t tmp[33];
   uint32_t n = 0;
-  for (uint32_t c0 = 0; c0 < job.chunks; c0 += 32) {
-    const uint32_t c = c0 + lane;
-    const bool on = c < job.chunks && *(volatile const uint32_t *)&job.dash_marks[c] != 0u;
-    const uint32_t bits = __ballot_sync(0xffffffffu, on);
-    if (on) list[n + __popc(bits & ((1u << lane) - 1u))] = c;
-    n += __popc(bits);
+  for (uint32_t c0 = 0; c0 < chunks; c0 += blockDim.x) {
+    const uint32_t c = c0 + threadIdx.x;
+    const uint32_t on = c < chunks && marks[c] != 0u ? 1u : 0u;
+    uint32_t total;
+    const uint32_t at = n + block_excl_scan<uint32_t>(on, tmp, total);
+    if (on) list[at] = c;
+    if (c < chunks) before[c] = at;
+    n += total;
   }
-  if (lane == 0) {
-    job.nkb = job.planes * job.chunks + n * (job.planes == 6 ? 2u : 1u);
-    atomicAdd(macs, job.pairs * 256ull * job.nkb);
-  }
+  if (threadIdx.x == 0) before[chunks] = n;
 }
 
 void set_smem_once() {
@@ -713,18 +997,39 @@ void set_smem_once() {
   HD_CUDA(err);
 }
 
-void make_tmap_u8(hd_ctx *ctx, CUtensorMap *tm, const void *base, uint64_t row_bytes,
+// Map of an operand's row groups: boxes of one block of `box_rows` rows.
+void make_tmap_op(hd_ctx *ctx, CUtensorMap *tm, const void *base, uint32_t planes, uint64_t sites,
                   uint64_t rows, uint32_t box_rows) {
-  cuuint64_t dims[2] = {row_bytes, rows};
-  cuuint64_t strides[1] = {row_bytes};
-  cuuint32_t box[2] = {128, box_rows};
+  const uint64_t group = op_group_bytes(planes, sites);
+  cuuint64_t dims[2] = {group / 8, ceil_div(rows, (uint64_t)8)};
+  cuuint64_t strides[1] = {group};
+  cuuint32_t box[2] = {kGroupBytes / 8, box_rows / 8};
   cuuint32_t es[2] = {1, 1};
-  CUresult r = ctx->encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base),
+  CUresult r = ctx->encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void *>(base),
                                  dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     fail(HD_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
+}
+
+// uint32s of the marks, and of the list and ranks k_dash_list makes of them
+uint64_t mark_words(uint64_t sites) { return op_chunks(sites); }
+uint64_t list_words(uint64_t sites) { return 2 * (uint64_t)op_chunks(sites) + 1; }
+
+// Expands rows [lo, hi) of the planes into the operand x, marks the chunks
+// and lists the marked ones.
+void expand_rows(hd_ctx *ctx, const uint4 *g0, const uint4 *g1, uint32_t planes, uint64_t words,
+                 uint64_t lo, uint64_t hi, uint64_t sites, uint8_t *x, uint32_t *marks,
+                 uint32_t *list, cudaStream_t stream) {
+  const uint64_t groups = ceil_div(hi, (uint64_t)8) - lo / 8;
+  const dim3 grid((unsigned)ceil_div((uint64_t)op_chunks(sites) * kChunkWords, (uint64_t)32),
+                  (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(groups, 65535)));
+  k_expand_op<<<grid, 256, 0, stream>>>(g0, g1, planes, (uint32_t)words, lo, hi, sites, x, marks);
+  HD_LAUNCHED(ctx);
+  const uint32_t chunks = op_chunks(sites);
+  k_dash_list<<<1, 512, 0, stream>>>(marks, chunks, list, list + chunks);
+  HD_LAUNCHED(ctx);
 }
 
 }  // namespace
@@ -754,21 +1059,22 @@ bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStr
   const hd_alignment *o = aln->base ? aln->base : aln;
   if (o->op_rows >= rows) return true;
   const uint32_t P = (uint32_t)o->planes;
-  const uint64_t words = o->words, rb = words * row_bytes_per_word(P);
+  const uint64_t words = o->words;
   if (rows > o->op_cap) {
     // room for the rows asked for, or for what the caller says will come
     const uint64_t plane_rows = o->plane_buf[0].bytes / (words * 16);
     const uint64_t cap = std::max(rows, std::min(cap_hint, plane_rows));
     DevBuf grown;
     try {
-      grown = DevBuf(cap * rb, stream);
+      grown = DevBuf(op_bytes(P, o->length, cap), stream);
     } catch (const Error &e) {
       if (e.code != HD_ERR_OOM) throw;
       cudaGetLastError();
       return false;  // the bit-plane engine needs no extra memory
     }
     if (o->op_rows) {
-      HD_CUDA(cudaMemcpyAsync(grown.p, o->op.p, o->op_rows * rb, cudaMemcpyDeviceToDevice, stream));
+      HD_CUDA(cudaMemcpyAsync(grown.p, o->op.p, op_bytes(P, o->length, o->op_rows),
+                              cudaMemcpyDeviceToDevice, stream));
       // launches on the context's other streams may still read the old
       // operand: they finish before it is freed
       for (cudaStream_t st : {ctx->side, ctx->stream}) HD_CUDA(cudaStreamSynchronize(st));
@@ -777,17 +1083,21 @@ bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStr
     o->op_cap = cap;
   }
   if (!o->op_dash.p) {
-    o->op_dash = DevBuf(words / 8 * 4, stream);
-    HD_CUDA(cudaMemsetAsync(o->op_dash.p, 0, words / 8 * 4, stream));
+    o->op_dash = DevBuf(mark_words(o->length) * 4, stream);
+    HD_CUDA(cudaMemsetAsync(o->op_dash.p, 0, mark_words(o->length) * 4, stream));
   }
-  const dim3 grid((unsigned)ceil_div(words, (uint64_t)256),
-                  (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(rows - o->op_rows, 65535)));
-  k_expand_op<<<grid, 256, 0, stream>>>(
-      o->plane_buf[0].as<uint4>(), P > 4 ? o->plane_buf[1].as<uint4>() : nullptr, P, words,
-      o->op_rows, rows, o->length, o->op.as<uint8_t>(), o->op_dash.as<uint32_t>());
-  HD_LAUNCHED(ctx);
+  // a list of its own for every extension: launches on other streams may
+  // still read an earlier one
+  o->op_lists.emplace_back(list_words(o->length) * 4, stream);
+  expand_rows(ctx, o->plane_buf[0].as<uint4>(), P > 4 ? o->plane_buf[1].as<uint4>() : nullptr, P,
+              words, o->op_rows, rows, o->length, o->op.as<uint8_t>(), o->op_dash.as<uint32_t>(),
+              o->op_lists.back().as<uint32_t>(), stream);
   o->op_rows = rows;
   return true;
+}
+
+uint64_t mma_operand_bytes(uint32_t planes, uint64_t sites, uint64_t rows) {
+  return op_bytes(planes, sites, rows);
 }
 
 double measure_mma_peak(hd_ctx *ctx) {
@@ -797,17 +1107,17 @@ double measure_mma_peak(hd_ctx *ctx) {
     err = cudaFuncSetAttribute(k_peak_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
   });
   HD_CUDA(err);
-  const uint32_t rounds = 4096;
-  k_peak_mma<<<ctx->sm_count, 128, kMmaSmem, ctx->stream>>>(256, ctx->d_status);  // warm-up
+  const uint32_t rounds = 4096, pairs = std::max(1, ctx->sm_count / 2);
+  k_peak_mma<<<2 * pairs, 128, kMmaSmem, ctx->stream>>>(256, ctx->d_status);  // warm-up
   HD_LAUNCHED(ctx);
   HD_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
-  k_peak_mma<<<ctx->sm_count, 128, kMmaSmem, ctx->stream>>>(rounds, ctx->d_status);
+  k_peak_mma<<<2 * pairs, 128, kMmaSmem, ctx->stream>>>(rounds, ctx->d_status);
   HD_LAUNCHED(ctx);
   HD_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
   HD_CUDA(cudaStreamSynchronize(ctx->stream));
   float ms = 0;
   HD_CUDA(cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
-  const double flop = (double)ctx->sm_count * rounds * 4 * 2.0 * kTM * kPeakN * 64;
+  const double flop = (double)pairs * rounds * 2.0 * kRowsPerItem * kItemCols * kChunkSites;
   return flop / (ms / 1e3);
 }
 
@@ -822,19 +1132,19 @@ bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLa
   if (!a->base) {
     if (!ensure_operand(ctx, a, a->n_rows, stream)) return false;
     op = a->op.as<uint8_t>();
-    dash = a->op_dash.as<uint32_t>();
+    dash = a->op_lists.back().as<uint32_t>();
     return true;
   }
   if (a->row0 == 0 && o->op.p && o->op_rows >= a->n_rows) {
-    // the base's chunk marks cover its other rows too: a chunk marked for
+    // the base's listed chunks cover its other rows too: a chunk listed for
     // them only adds dash products of 0
     op = o->op.as<uint8_t>();
-    dash = o->op_dash.as<uint32_t>();
+    dash = o->op_lists.back().as<uint32_t>();
     return true;
   }
   const uint32_t P = (uint32_t)o->planes;
-  const uint64_t rb = o->words * row_bytes_per_word(P), bytes = a->n_rows * rb;
-  const uint64_t flag_bytes = o->words / 8 * 4;
+  const uint64_t bytes = op_bytes(P, o->length, a->n_rows);
+  const uint64_t marks = mark_words(o->length), flag_bytes = (marks + list_words(o->length)) * 4;
   if (bytes > (8ull << 30)) return false;  // the bit-plane engine needs no extra memory
   DevBuf tmp;
   try {
@@ -845,35 +1155,176 @@ bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLa
     return false;
   }
   uint32_t *flags = reinterpret_cast<uint32_t *>(tmp.as<uint8_t>() + bytes);
-  HD_CUDA(cudaMemsetAsync(flags, 0, flag_bytes, stream));
-  const dim3 grid((unsigned)ceil_div(o->words, (uint64_t)256),
-                  (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(a->n_rows, 65535)));
-  k_expand_op<<<grid, 256, 0, stream>>>(
-      static_cast<const uint4 *>(a->planes_ptr(0)),
-      P > 4 ? static_cast<const uint4 *>(a->planes_ptr(1)) : nullptr, P, o->words, 0, a->n_rows,
-      o->length, tmp.as<uint8_t>(), flags);
-  HD_LAUNCHED(ctx);
+  HD_CUDA(cudaMemsetAsync(flags, 0, marks * 4, stream));
+  expand_rows(ctx, static_cast<const uint4 *>(a->planes_ptr(0)),
+              P > 4 ? static_cast<const uint4 *>(a->planes_ptr(1)) : nullptr, P, o->words, 0,
+              a->n_rows, o->length, tmp.as<uint8_t>(), flags, flags + marks, stream);
   op = tmp.as<uint8_t>();
-  dash = flags;
+  dash = flags + marks;
   plan->blocks.push_back(std::move(tmp));
   return true;
+}
+
+namespace {
+
+// The items of a launch and how the CTA pairs share them.
+struct MmaPlan {
+  // static order: pair u of `pairs` runs items u, u + pairs, ... up to the
+  // padding (job kNoItem)
+  std::vector<MmaItem> items;
+  std::vector<MmaFix> fix;
+  uint32_t slots = 0;
+  uint32_t pairs = 0;  // CTA pairs with work
+  // a tile's item, cut along K at the chunks `cuts` (first and last included)
+  void add_pieces(const MmaItem &tile, const std::vector<uint32_t> &cuts, std::vector<MmaItem> &out) {
+    if (cuts.size() <= 2) {
+      out.push_back(tile);
+      return;
+    }
+    fix.push_back({tile.job, tile.row0, tile.col0, tile.n0() + tile.n1(), slots,
+                   (uint32_t)cuts.size() - 1});
+    for (size_t k = 0; k + 1 < cuts.size(); ++k) {
+      MmaItem it = tile;
+      it.c_lo = cuts[k];
+      it.c_hi = cuts[k + 1];
+      it.slot = slots++;
+      out.push_back(it);
+    }
+  }
+};
+
+// Cost of an item per K block, in units of 250 cycles: 745 cycles of MMAs for
+// both column halves; one half alone waits for its loads (36.9 KB at the 72 B
+// per cycle and SM that the L2 gives), about 510.
+uint64_t block_cost(const MmaItem &it) { return it.n1_16 ? 3 : 2; }
+
+// One matrix: every pair of CTAs gets the same share of the work to within a
+// chunk. Whole items go round in list order while every pair has one more;
+// the rest is dealt out in K pieces that fill each pair up to the average.
+// Splitting costs the pieces' workspace traffic and one more launch, about 8
+// us, so it is left out where it would gain less (then the rest goes to the
+// least loaded pairs). n=1,000 x 29,903, 10 items: 35 us split, 160 us whole.
+void plan_static(std::vector<MmaItem> &list, uint32_t units, uint32_t planes, bool may_split,
+                 MmaPlan &plan) {
+  // The items of both column halves first: they all take the same time, so
+  // that the pairs working on one band stay at the same K and read its rows
+  // while the L2 holds them.
+  std::stable_partition(list.begin(), list.end(), [](const MmaItem &it) { return it.n1_16 != 0; });
+  const size_t m = list.size();
+  auto cost_of = [&](const MmaItem &it) {
+    return block_cost(it) * planes * (it.c_hi - it.c_lo);
+  };
+  uint64_t total = 0, most = 1;
+  for (const MmaItem &it : list) {
+    total += cost_of(it);
+    most = std::max(most, cost_of(it));
+  }
+  // a pair's share: the average, at least the shortest piece of a full tile
+  const uint64_t share = std::max<uint64_t>(ceil_div(total, units), 3ull * planes * kMinPart);
+  const size_t whole = std::min<size_t>(m, (size_t)(total / units / most) * units);
+  std::vector<std::vector<MmaItem>> of(units);
+  std::vector<uint64_t> load(units, 0);
+  for (size_t k = 0; k < whole; ++k) {
+    of[k % units].push_back(list[k]);
+    load[k % units] += cost_of(list[k]);
+  }
+  // 250 cycles are 0.12 us
+  const uint64_t unsplit = (whole / units + ceil_div(m - whole, (size_t)units)) * most;
+  const bool split = may_split && (double)(unsplit - std::min(unsplit, share)) * 0.12 > 8.0;
+  if (!split) {
+    for (size_t k = whole; k < m; ++k) {
+      const size_t u = std::min_element(load.begin(), load.end()) - load.begin();
+      of[u].push_back(list[k]);
+      load[u] += cost_of(list[k]);
+    }
+  } else {
+    // the rest as one row of chunks; pair u's end on it is the sum of the room
+    // up to u, so that rounding to whole chunks does not add up
+    auto room = [&](uint32_t v) { return load[v] < share ? share - load[v] : 0; };
+    uint32_t u = 0;
+    uint64_t at = 0, end = room(0);
+    for (size_t k = whole; k < m; ++k) {
+      const MmaItem &it = list[k];
+      const uint64_t per = block_cost(it) * planes;  // cost of one chunk
+      std::vector<uint32_t> cuts{it.c_lo}, owner;
+      for (uint32_t c = it.c_lo; c < it.c_hi;) {
+        const uint32_t left = it.c_hi - c;
+        uint64_t take = end > at ? (end - at + per / 2) / per : 0;
+        if (u + 1 < units && take < kMinPart && left > take) {
+          end += room(++u);  // this pair is full
+          continue;
+        }
+        if (u + 1 == units || take > left || left - take < kMinPart) take = left;
+        c += (uint32_t)take;
+        at += take * per;
+        cuts.push_back(c);
+        owner.push_back(u);
+      }
+      std::vector<MmaItem> pieces;
+      plan.add_pieces(it, cuts, pieces);
+      for (size_t q = 0; q < pieces.size(); ++q) of[owner[q]].push_back(pieces[q]);
+    }
+  }
+  size_t depth = 0;
+  for (uint32_t v = 0; v < units; ++v) {
+    depth = std::max(depth, of[v].size());
+    if (!of[v].empty()) plan.pairs = v + 1;
+  }
+  MmaItem none{};
+  none.job = kNoItem;
+  plan.items.assign(depth * plan.pairs, none);
+  for (uint32_t v = 0; v < plan.pairs; ++v)
+    for (size_t k = 0; k < of[v].size(); ++k) plan.items[k * plan.pairs + v] = of[v][k];
+}
+
+// Several matrices: the pairs draw items from a queue, the costliest first
+// (list order). Items longer than half of a pair's average share (a small
+// batch) are cut along K to about that length.
+void plan_queue(std::vector<MmaItem> &list, uint32_t units, const std::vector<uint32_t> &planes,
+                const std::vector<char> &may_split, MmaPlan &plan) {
+  uint64_t total = 0;
+  for (const MmaItem &it : list)
+    total += block_cost(it) * planes[it.job] * (it.c_hi - it.c_lo);
+  const uint64_t half = std::max<uint64_t>(1, total / units / 2);
+  for (const MmaItem &it : list) {
+    const uint32_t n = it.c_hi - it.c_lo;
+    const uint64_t cost = block_cost(it) * planes[it.job] * n;
+    uint64_t parts = may_split[it.job] ? std::min<uint64_t>(cost / half, n / kMinPart) : 1;
+    // below 8 us a split gains less than it costs
+    if ((double)(cost - std::min(cost, half)) * 0.12 < 8.0) parts = 1;
+    std::vector<uint32_t> cuts{it.c_lo};
+    for (uint64_t k = 1; k <= std::max<uint64_t>(parts, 1); ++k)
+      cuts.push_back(it.c_lo + (uint32_t)(n * k / std::max<uint64_t>(parts, 1)));
+    plan.add_pieces(it, cuts, plan.items);
+  }
+  plan.pairs = (uint32_t)std::min<uint64_t>(units, plan.items.size());
+}
+
+}  // namespace
+
+// Size of the tile rows [lo, hi) in tiles of 128 x kMmaCols pairs: what the
+// launch thresholds and the reported tile counts are in.
+static uint64_t size_tiles(uint64_t lo, uint64_t hi) {
+  uint64_t n = 0;
+  for (uint64_t I = lo; I < hi; ++I) n += ((I + 1) * kTM - 2) / kMmaCols + 1;
+  return n;
 }
 
 void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaStream_t stream,
                       PairLaunchPlan *plan, int sm_limit, std::vector<char> &taken) {
   taken.assign(specs.size(), 0);
   std::vector<const uint8_t *> ops(specs.size(), nullptr);  // each job's operand rows
-  std::vector<const uint32_t *> dash_marks(specs.size(), nullptr);  // and its chunk marks
+  std::vector<const uint32_t *> dash_lists(specs.size(), nullptr);  // and its listed chunks
   struct Job {
     size_t k;
     uint32_t t_lo, t_hi;
     double cost;
   };
   std::vector<Job> js;
-  // A launch with few items leaves SMs idle: below a minimum of single row
-  // tiles (128 x kTN) in all (mma_min_items_for, autotuned per row length),
-  // the bit-plane engine's finer tiles finish first; a batch of small
-  // matrices still goes here when together they are enough.
+  // A small launch leaves SMs idle: below a minimum size, counted in tiles of
+  // 128 x kMmaCols pairs (mma_min_items_for, autotuned per row length), the
+  // bit-plane engine's finer tiles finish first; a batch of small matrices
+  // still goes here when together they are enough.
   if (ctx->engine_force == 0) return;
   uint64_t items_total = 0, max_len = 0;
   for (const PairJobSpec &sp : specs) {
@@ -882,7 +1333,7 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     const uint64_t edge = sp.cfg.tile > 0 ? (uint64_t)sp.cfg.tile : kTile;
     const uint64_t lo = sp.tile_lo * edge / kTM;
     const uint64_t hi = ceil_div(std::min<uint64_t>(sp.tile_hi * edge, sp.aln->n_rows), kTM);
-    for (uint64_t I = lo; I < hi; ++I) items_total += ((I + 1) * kTM - 2) / kTN + 1;
+    items_total += size_tiles(lo, hi);
   }
   const uint64_t min_items = ctx->engine_force == 1 ? 0 : mma_min_items_for(ctx, max_len);
   if (items_total < min_items) return;
@@ -894,154 +1345,162 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     const uint64_t edge = sp.cfg.tile > 0 ? (uint64_t)sp.cfg.tile : kTile;
     const uint64_t row_lo = sp.tile_lo * edge, row_hi = std::min<uint64_t>(sp.tile_hi * edge, a->n_rows);
     if (row_lo % kTM || row_hi <= row_lo) continue;
-    if (!operand_for(ctx, a, stream, plan, ops[k], dash_marks[k])) continue;
+    if (!operand_for(ctx, a, stream, plan, ops[k], dash_lists[k])) continue;
     const uint32_t lo = (uint32_t)(row_lo / kTM), hi = (uint32_t)ceil_div(row_hi, kTM);
     js.push_back({k, lo, hi, (double)a->words * ((double)hi * hi - (double)lo * lo)});
     taken[k] = 1;
   }
   if (js.empty()) return;
   // Each job's K blocks: the P plane blocks of every chunk, and the dash
-  // products of the chunks its rows have a '-' in. The chunk list is built on
-  // the device from the expansion's marks (k_dash_list, below), in stream
-  // order after the operands; the host orders the jobs by the plane blocks.
-  std::vector<uint32_t> kcost(specs.size(), 0);
-  for (const Job &j : js) {
-    const hd_alignment *o = specs[j.k].aln->base ? specs[j.k].aln->base : specs[j.k].aln;
-    kcost[j.k] = (uint32_t)(o->planes * (o->words / 8));
-  }
-  // CTAs draw items from a queue in list order: the costliest items first
-  // (an item's cost is its K length), biggest jobs first among equals, so
-  // that the cheap items fill the tail
+  // products of the chunks its rows have a '-' in, whose list stays on the
+  // device (k_dash_list); the host orders the jobs by the plane blocks.
+  auto owner_of = [&](const Job &j) {
+    const hd_alignment *a = specs[j.k].aln;
+    return a->base ? a->base : a;
+  };
+  auto kcost = [&](const Job &j) {
+    const hd_alignment *o = owner_of(j);
+    return (uint64_t)o->planes * op_chunks(o->length);
+  };
+  // the costliest items first (an item's cost is its K length), biggest jobs
+  // first among equals, so that the cheap items fill the tail
   std::stable_sort(js.begin(), js.end(), [&](const Job &a, const Job &b) {
-    return kcost[a.k] != kcost[b.k] ? kcost[a.k] > kcost[b.k] : a.cost > b.cost;
+    return kcost(a) != kcost(b) ? kcost(a) > kcost(b) : a.cost > b.cost;
   });
-  // Items of each job: pairs of 128-row tiles (a single one where a range is
-  // odd; single ones throughout with mma_rows 1) x kTN-column tiles up to the
-  // last column any of their rows needs, in bands of mma_band tile rows,
-  // column-major within a band.
+  // Items of each job: 256 rows x 496 columns (with mma_rows 1, each column
+  // half by itself) up to the last column any of their rows needs, in bands of
+  // mma_band tile rows, column-major within a band. Near the diagonal an item
+  // is as wide as its rows need, in the 16 columns an MMA's N counts in.
+  const size_t nj = js.size();
   std::vector<MmaItem> list;
-  for (uint32_t q = 0; q < (uint32_t)js.size(); ++q) {
-    const TileConfig &cfg = specs[js[q].k].cfg;
-    const uint32_t band = (uint32_t)mma_band_of(cfg), rows = (uint32_t)mma_rows_of(cfg);
-    for (uint32_t b = js[q].t_lo; b < js[q].t_hi; b += band) {
-      const uint32_t e = std::min(b + band, js[q].t_hi);
-      const uint32_t j_end = (uint32_t)ceil_div((uint64_t)e * kTM - 1, kTN);
-      for (uint32_t J = 0; J < j_end; ++J)
-        for (uint32_t I = b; I < e; I += rows) {
-          const uint32_t h = std::min(rows, e - I);
-          // rows [128 I, 128 (I + h)) need columns < 128 (I + h) - 1; where
-          // only the second row tile reaches column tile J, it goes alone
-          if ((uint64_t)J * kTN >= (uint64_t)(I + h) * kTM - 1) continue;
-          if (h == 2 && (uint64_t)J * kTN >= (uint64_t)(I + 1) * kTM - 1)
-            list.push_back({q, I + 1, J, 1});
-          else
-            list.push_back({q, I, J, h});
+  std::vector<uint32_t> planes(nj);
+  std::vector<char> may_split(nj);
+  for (uint32_t q = 0; q < (uint32_t)nj; ++q) {
+    const PairJobSpec &sp = specs[js[q].k];
+    const hd_alignment *o = owner_of(js[q]);
+    planes[q] = (uint32_t)o->planes;
+    const uint32_t chunks = op_chunks(o->length);
+    may_split[q] = sp.dtype <= 2 && chunks >= 2 * kMinPart;
+    const uint32_t band = (uint32_t)mma_band_of(sp.cfg) * kRowsPerItem;
+    const bool halves = mma_rows_of(sp.cfg) == 1;
+    const uint32_t lo = js[q].t_lo * kTM;
+    const uint32_t hi = (uint32_t)std::min<uint64_t>((uint64_t)js[q].t_hi * kTM, sp.aln->n_rows);
+    for (uint32_t b = lo; b < hi; b += band) {
+      const uint32_t e = std::min(b + band, hi);
+      for (uint32_t col = 0; col + 1 < e; col += kItemCols)
+        for (uint32_t r = b; r < e; r += kRowsPerItem) {
+          const uint32_t last = std::min(r + kRowsPerItem, e);  // rows [r, last) need columns < last - 1
+          if (col + 1 >= last) continue;
+          const uint32_t need = (uint32_t)round_up(std::min(last - 1 - col, kItemCols), 16);
+          const uint32_t n0 = std::min(need, kN0), n1 = need - n0;
+          MmaItem it{q, r, col, (uint8_t)(n0 / 16), (uint8_t)(n1 / 16), (uint8_t)planes[q], 0, 0,
+                     chunks, kNoSlot, 0};
+          if (halves && n1) {
+            it.n1_16 = 0;
+            list.push_back(it);
+            it.col0 = col + n0;
+            it.n0_16 = (uint8_t)(n1 / 16);
+          }
+          list.push_back(it);
         }
     }
   }
-  // Work distribution. One matrix: every item costs the same, and the CTAs
-  // take them round-robin, the last pairs split into single row tiles until
-  // the count is a multiple of the grid, so that every CTA ends within one
-  // row tile of the others. Several matrices (items of unequal length): the
-  // CTAs draw items from a queue, and its last `grid` pairs are split, so
-  // that the CTAs finish within about half an item of each other.
-  // HAMMINGDIST_MMA_SCHEDULE=static|queue picks one for every launch. A
-  // short list splits every pair to fill more SMs.
+  // HAMMINGDIST_MMA_SCHEDULE=static|queue picks one for every launch (several
+  // matrices always go through the queue)
   const int sms = sm_limit > 0 && sm_limit < ctx->sm_count ? sm_limit : ctx->sm_count;
-  bool queue = js.size() > 1;
-  if (const char *e = std::getenv("HAMMINGDIST_MMA_SCHEDULE")) queue = std::string(e) == "queue";
-  uint64_t pairs = 0;
-  for (const MmaItem &m : list) pairs += m.halves == 2;
-  const uint64_t grid_n = std::min<uint64_t>(list.size() + pairs, (uint64_t)sms);
-  uint64_t split = list.size() < grid_n ? pairs
-                   : queue ? std::min<uint64_t>(pairs, grid_n)
-                           : (grid_n - list.size() % grid_n) % grid_n;
-  std::vector<MmaItem> tail;
-  for (size_t k = list.size(); k-- > 0 && split > 0;) {
-    if (list[k].halves != 2) continue;
-    tail.push_back({list[k].job, list[k].I + 1, list[k].J, 1});
-    list[k].halves = 1;
-    --split;
+  const uint32_t units = (uint32_t)std::max(1, sms / 2);
+  bool queue = nj > 1;
+  if (const char *e = std::getenv("HAMMINGDIST_MMA_SCHEDULE"))
+    queue = queue || std::string(e) == "queue";
+  MmaPlan mp;
+  DevBuf ws;
+  for (;;) {
+    if (queue) plan_queue(list, units, planes, may_split, mp);
+    else plan_static(list, units, planes[0], may_split[0], mp);
+    if (!mp.slots) break;
+    try {
+      ws = DevBuf(mp.slots * kSlotBytes, stream, true);
+      break;
+    } catch (const Error &e) {
+      if (e.code != HD_ERR_OOM) throw;
+      cudaGetLastError();
+      mp = MmaPlan();  // no room for the pieces: whole items
+      may_split.assign(nj, 0);
+    }
   }
-  list.insert(list.end(), tail.rbegin(), tail.rend());
-  // one device block: [tensor maps (3 per job)][jobs][items][queue counter]
-  // [dash chunk lists]
-  const size_t nj = js.size();
-  const size_t tm_bytes = nj * 3 * sizeof(CUtensorMap);
-  const size_t job_bytes = round_up(nj * sizeof(MmaJob), 64);
-  const size_t item_bytes = round_up(list.size() * sizeof(MmaItem), 16);
-  size_t dash_words = 0;
-  for (const Job &j : js) {
-    const hd_alignment *o = specs[j.k].aln->base ? specs[j.k].aln->base : specs[j.k].aln;
-    dash_words += o->words / 8;
-  }
-  const size_t dash_at = tm_bytes + job_bytes + item_bytes + 16;
-  std::vector<uint8_t> host(dash_at + dash_words * 4 + 4, 0);
+  // one device block: [tensor maps (2 per job)][jobs][items][split tiles]
+  // [queue counter]
+  const size_t tm_bytes = nj * 2 * sizeof(CUtensorMap);
+  const size_t job_at = tm_bytes, item_at = job_at + round_up(nj * sizeof(MmaJob), 64);
+  const size_t fix_at = item_at + mp.items.size() * sizeof(MmaItem);
+  const size_t counter_at = fix_at + round_up(mp.fix.size() * sizeof(MmaFix), 16);
+  std::vector<uint8_t> host(counter_at + 16, 0);
   DevBuf dev(host.size(), stream);
   auto *tms = reinterpret_cast<CUtensorMap *>(host.data());
-  auto *jobs = reinterpret_cast<MmaJob *>(host.data() + tm_bytes);
-  const auto *d_tms = reinterpret_cast<const CUtensorMap *>(dev.p);
-  size_t dash_off = 0;
+  auto *jobs = reinterpret_cast<MmaJob *>(host.data() + job_at);
   for (size_t q = 0; q < nj; ++q) {
     const PairJobSpec &sp = specs[js[q].k];
-    const hd_alignment *a = sp.aln;
-    const hd_alignment *o = a->base ? a->base : a;
-    const uint64_t rb = o->words * row_bytes_per_word((uint32_t)o->planes);
-    make_tmap_u8(ctx, &tms[3 * q], ops[js[q].k], rb, a->n_rows, 2 * kTM);
-    make_tmap_u8(ctx, &tms[3 * q + 1], ops[js[q].k], rb, a->n_rows, kTM);
-    make_tmap_u8(ctx, &tms[3 * q + 2], ops[js[q].k], rb, a->n_rows, kTN);
+    const hd_alignment *a = sp.aln, *o = owner_of(js[q]);
+    make_tmap_op(ctx, &tms[2 * q], ops[js[q].k], planes[q], o->length, a->n_rows, kTM);
+    make_tmap_op(ctx, &tms[2 * q + 1], ops[js[q].k], planes[q], o->length, a->n_rows, kN1 / 2);
     MmaJob &m = jobs[q];
-    m.tm256 = d_tms + 3 * q;
-    m.tm128 = d_tms + 3 * q + 1;
-    m.tmb = d_tms + 3 * q + 2;
     m.out = sp.d_out;
     m.out_base = sp.out_base;
-    m.n = (uint32_t)a->n_rows;
-    m.nkb = 0;  // set by k_dash_list
-    m.chunks = (uint32_t)(o->words / 8);
-    m.dash_list = reinterpret_cast<const uint32_t *>(static_cast<uint8_t *>(dev.p) + dash_at) + dash_off;
-    m.dash_marks = dash_marks[js[q].k];
-    dash_off += m.chunks;
+    m.chunks = op_chunks(o->length);
+    m.dash_list = dash_lists[js[q].k];
+    m.dash_rank = m.dash_list + m.chunks;
     // the launch's lower-triangle pairs (for its multiply-add count)
     const uint64_t r_lo = (uint64_t)js[q].t_lo * kTM, r_hi = std::min<uint64_t>((uint64_t)js[q].t_hi * kTM, a->n_rows);
+    m.row_hi = (uint32_t)r_hi;
     m.pairs = r_hi * (r_hi - 1) / 2 - (r_lo ? r_lo * (r_lo - 1) / 2 : 0);
-    m.planes = (uint32_t)o->planes;
+    m.planes = planes[q];
     m.sites = (uint32_t)a->length;
     m.max_dist = sp.max_dist;
     m.dtype = (uint32_t)sp.dtype;
   }
-  std::memcpy(host.data() + tm_bytes + job_bytes, list.data(), list.size() * sizeof(MmaItem));
+  std::memcpy(host.data() + item_at, mp.items.data(), mp.items.size() * sizeof(MmaItem));
+  std::memcpy(host.data() + fix_at, mp.fix.data(), mp.fix.size() * sizeof(MmaFix));
   // staged in pinned memory (pageable for a large table): `host` may go when this returns
   upload_table(ctx, dev.p, host.data(), host.size(), stream);
-  k_dash_list<<<(unsigned)nj, 32, 0, stream>>>(reinterpret_cast<MmaJob *>(dev.as<uint8_t>() + tm_bytes),
-                                              mma_mac_counter(ctx));
-  HD_LAUNCHED(ctx);
+  uint8_t *d = dev.as<uint8_t>();
   PairLaunchPlan::Launch L;
   L.mma = true;
   L.fn = reinterpret_cast<const void *>(k_pairwise_mma);
   L.smem = kMmaSmem;
   L.tile = kTM;
   L.jobs = nj;
-  L.tiles = list.size();
-  L.grid = grid_n;
-  L.d_jobs = dev.as<uint8_t>() + tm_bytes;
-  L.d_items = dev.as<uint8_t>() + tm_bytes + job_bytes;
-  L.d_counter = reinterpret_cast<unsigned long long *>(dev.as<uint8_t>() + tm_bytes + job_bytes +
-                                                       item_bytes);
+  for (const Job &j : js) L.tiles += size_tiles(j.t_lo, j.t_hi);
+  L.items = mp.items.size();
+  L.grid = 2 * mp.pairs;
+  L.d_jobs = d + job_at;
+  L.d_items = d + item_at;
+  L.d_tms = d;
+  L.d_fix = d + fix_at;
+  L.fixes = mp.fix.size();
+  L.d_ws = ws.p;
+  L.d_counter = reinterpret_cast<unsigned long long *>(d + counter_at);
   L.queue = queue;
   plan->launches.push_back(L);
   plan->blocks.push_back(std::move(dev));
+  if (ws.p) plan->blocks.push_back(std::move(ws));
 }
 
 void launch_mma(hd_ctx *ctx, const PairLaunchPlan::Launch &L, cudaStream_t stream) {
   set_smem_once();
   // the item queue starts empty at every launch (also when a graph replays it)
-  HD_CUDA(cudaMemsetAsync(L.d_counter, 0, sizeof(unsigned), stream));
+  if (L.queue) HD_CUDA(cudaMemsetAsync(L.d_counter, 0, sizeof(unsigned), stream));
   k_pairwise_mma<<<(unsigned)L.grid, kMmaThreads, kMmaSmem, stream>>>(
-      static_cast<const MmaJob *>(L.d_jobs), static_cast<const MmaItem *>(L.d_items),
-      (uint32_t)L.tiles, reinterpret_cast<unsigned *>(L.d_counter), L.queue ? 1u : 0u,
-      ctx->d_status);
+      static_cast<const CUtensorMap *>(L.d_tms), static_cast<const MmaJob *>(L.d_jobs),
+      (uint32_t)L.jobs, static_cast<const MmaItem *>(L.d_items), (uint32_t)L.items,
+      reinterpret_cast<unsigned *>(L.d_counter), L.queue ? 1u : 0u,
+      static_cast<uint32_t *>(L.d_ws), mma_mac_counter(ctx), ctx->d_status);
   HD_LAUNCHED(ctx);
+  if (L.fixes) {
+    k_pair_fix<<<(unsigned)ceil_div(L.fixes * kFixWarps, (uint64_t)8), 256, 0, stream>>>(
+        static_cast<const MmaJob *>(L.d_jobs), static_cast<const MmaFix *>(L.d_fix),
+        (uint32_t)L.fixes, static_cast<const uint32_t *>(L.d_ws));
+    HD_LAUNCHED(ctx);
+  }
   ctx->last_pair_tiles += L.tiles;
 }
 

@@ -2,9 +2,9 @@
 // dtype):
 //  * the bit-plane engine's tile edge (64 or 128 rows, i.e. 4 or 8 rows per
 //    thread) and TMA staging depth;
-//  * the tensor-core engine's L2 band (tile rows per band) and item shape
-//    (one or two 128-row tiles per item);
-// and per L bucket the launch size (single-row-tile items) from which a
+//  * the tensor-core engine's L2 band (item rows of 256 rows per band) and
+//    item shape (one or both column halves per item);
+// and per L bucket the launch size (tiles of 128 x 240 pairs) from which a
 // matrix launched alone goes to the tensor-core engine rather than the
 // bit-plane engine. The configurations are timed with the GPU filled (a batch
 // of copies of a synthetic packed alignment of the bucket's representative
@@ -40,7 +40,7 @@ int l_bucket(uint64_t L) {
   while (b < 3 && L > kLEdges[b]) ++b;
   return b;
 }
-// single-row-tile items of the tensor-core engine for one matrix of n rows
+// launch size of one matrix of n rows, in tiles of 128 x kMmaCols pairs
 uint64_t mma_items_of(uint64_t n) {
   uint64_t items = 0;
   for (uint64_t I = 0; I < ceil_div(n, (uint64_t)kTile); ++I)
@@ -179,7 +179,7 @@ extern "C" int hd_autotune(hd_ctx *ctx, uint64_t max_n_bucket) {
   if (!ctx) return HD_ERR_ARG;
   return tune_guard(ctx, [&] {
     const hd::TileConfig cands[] = {{128, 3}, {128, 2}, {128, 4}, {64, 3}, {64, 4}};
-    // tensor-core engine: (band, row tiles per item)
+    // tensor-core engine: (band, column halves per item)
     const int mma_cands[][2] = {{16, 2}, {8, 2}, {32, 2}, {16, 1}};
     const int nbmax = (int)std::min<uint64_t>(max_n_bucket, 6);
     hd::TuneTable table;
