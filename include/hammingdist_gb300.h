@@ -234,7 +234,7 @@ int hd_write_sparse(hd_ctx *ctx, const void *lt, uint64_t nsamples,
  * cudaFree (cudaFree synchronises the device). Same bytes as
  * hd_write_lower_triangular writes to a file.
  *  - Limit: nsamples <= 262144; larger inputs fail with HD_ERR_ARG before
- *    any work. The scratch is a fixed ~4.2 MB device array in the library,
+ *    any work. The scratch is a fixed ~130 KB device array in the library,
  *    held on every GPU that loads it until the process exits.
  *  - The first call on a device looks up that array's device address (once
  *    per device).
