@@ -22,7 +22,7 @@
 // are kind::mxf4 with every UE8M0 scale factor 1.0 and FP32 accumulation,
 // exact while P L < 2^24. mismatches = L - matches.
 //
-// K order: first the P plane blocks of every 288-site chunk (partial sums up
+// K order: first the P plane blocks of every 192-site chunk (partial sums up
 // to P L), then the dash products, only for the chunks where some row of the
 // operand has a '-' (the expansion marks them): elsewhere every dash product
 // is 0. On aligned genomes the '-' sit mostly in leading and trailing runs, so
@@ -30,9 +30,9 @@
 //
 // Operand (one buffer serves rows and columns): each row's bit planes are
 // expanded to packed E2M1, two sites per byte, in the layout the tensor
-// cores read without a swizzle: for 8 rows (a row group) and 288 sites, the P
+// cores read without a swizzle: for 8 rows (a row group) and 192 sites, the P
 // planes (1.0), the dash as 1.0 (read for rows) and the dash as -(P - 1)
-// (read for columns; -4 and -1 for P = 6) are blocks of 1,152 bytes, each nine
+// (read for columns; -4 and -1 for P = 6) are blocks of 768 bytes, each six
 // 128-byte core matrices (8 rows x 16 bytes = 32 sites). Sites past L are 0. A
 // row group's blocks follow one another, so a TMA box of 16 groups brings one
 // block of 128 rows. An alignment caches its operand; a view of a resident
@@ -42,14 +42,14 @@
 // cluster of two SMs, 320 threads each) walk a list of items: 256 rows x up to
 // 496 columns of one job, in bands of tile rows, column-major within a band,
 // so that resident pairs share operands in L2.
-//  * warp 0 (one thread) issues TMA loads per stage of one 144-byte K block of
-//    the CTA's 128 rows and of its half of the columns (128 + 120), 4 stages
-//    of 54,144 B; both CTAs' loads count on the first CTA's full barriers.
-//    The first CTA's producer also draws the items and hands their indices
-//    around; warp 0 allocates and frees the TMEM;
+//  * warps 0 and 10 (one thread each) take turns to issue the TMA loads of one
+//    96-byte K block of the CTA's 128 rows and of its half of the columns, 6
+//    stages of 36,096 B; both CTAs' loads count on the first CTA's full barriers.
+//    The first CTA's first producer also draws the items of a queued launch;
+//    warp 0 allocates and frees the TMEM;
 //  * warp 1 of the first CTA (one thread) issues tcgen05.mma.cta_group::2
 //    .kind::mxf4.block_scale with K = 96 (the shape only sm_103a has: 1.5
-//    times the rate of K = 64), M = 256 and N = 256 and 240, three K steps per
+//    times the rate of K = 64), M = 256 and N = 256 and 240, two K steps per
 //    block, into both CTAs' TMEM (columns 0-255 and 256-495); the unit scale
 //    factors sit in columns 496-511. Each stage's MMAs are committed to both
 //    CTAs' empty barriers, an item's last ones to `done`;
@@ -66,17 +66,19 @@
 // Every wait is bounded; on a timeout the CTA records it in the status word,
 // waits (bounded) for its own copies and MMAs, frees its TMEM and returns.
 //
-// What bounds it (n = 14,000, L = 29,903, 8.05 FLOP per pair-site): the L2
-// reads. A pair's stage takes 745 cycles of MMAs and brings 108 KB; measured
-// alone, the loads reach 77 B per cycle and SM, the MMAs 14.4 PFLOP/s.
-//   form (K block x stages)                  operand in L2 / over 100 MB
+// What bounds it (n = 14,000, L = 29,903, 8.05 FLOP per pair-site): the loads.
+// A pair's K block takes 497 cycles of MMAs and brings 72 KB; measured alone,
+// the loads reach 77 B per cycle and SM, the MMAs 14.4 PFLOP/s.
+//   form (K block x stages), alone             operand in L2 / over 100 MB
 //   single CTAs, K = 96, 96 B x 3              9.1 / 8.0 PFLOP/s
 //   CTA pairs, K = 96, 96 B x 6               13.4 / 12.9
 //   CTA pairs, K = 96, 144 B x 4              14.5 / 12.6
 //   CTA pairs, K = 96, 192 B x 3              14.5 / 12.2
-// A 96-byte block's barrier traffic costs more than its MMAs last (536 of
-// 497 cycles); three stages of 192 hide less of the L2 latency. Pairs halve
-// the column bytes an SM loads and its MMAs read.
+// The smaller blocks let the loads run further ahead of the MMAs, and two TMA
+// threads keep up with them: 4 x 144 B with one 1,985 us, 6 x 96 B with one
+// 1,940, with two 1,925 (531 cycles a block; 500 with every load from the same
+// rows), 84% of the FP4 rate hd_measure_mma_peak reports.
+// Pairs halve the column bytes an SM loads and its MMAs read.
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
@@ -90,21 +92,24 @@ namespace hd {
 namespace {
 
 constexpr int kEpiWarps = 8;      // two per TMEM lane quarter
-constexpr int kMmaThreads = 64 + 32 * kEpiWarps;  // warp 0: TMA, warp 1: MMA, warps 2-9: epilogue
-constexpr int kMmaStages = 4;
+// warp 0: TMA, warp 1: MMA, warps 2-9: epilogue, warp 10: TMA
+constexpr int kMmaThreads = 96 + 32 * kEpiWarps;
+constexpr uint32_t kProducers = 2;  // the TMA warps take K blocks in turn
+constexpr int kMmaStages = 6;
+static_assert(kMmaStages % kProducers == 0, "a stage always has the same producer");
 constexpr uint32_t kTM = 128;                          // rows of a tile row, and of a CTA in a pair
 constexpr uint32_t kRowsPerItem = 2 * kTM;             // M of a CTA pair's MMA
-constexpr uint32_t kN0 = 256, kN1 = 240;               // an item's column halves (N of its MMAs)
+constexpr uint32_t kN0 = 256, kN1 = 240;               // N of an item's two MMAs
 constexpr uint32_t kItemCols = kN0 + kN1;
-constexpr uint32_t kChunkWords = 9;                    // 32-site words per chunk (288 sites)
+constexpr uint32_t kChunkWords = 6;                    // 32-site words per chunk (192 sites)
 constexpr uint32_t kChunkSites = 32 * kChunkWords;
-constexpr uint32_t kBlockK = 16 * kChunkWords;         // bytes of K per row and block (144)
-constexpr uint32_t kGroupBytes = 8 * kBlockK;          // one block of 8 rows (1,152)
+constexpr uint32_t kBlockK = 16 * kChunkWords;         // bytes of K per row and block (96)
+constexpr uint32_t kGroupBytes = 8 * kBlockK;          // one block of 8 rows (768)
 constexpr uint32_t kKStep = 48;                        // bytes of K per MMA (96 values)
 constexpr uint32_t kABytes = kTM / 8 * kGroupBytes;              // 128 rows
-constexpr uint32_t kB0Bytes = kN0 / 16 * kGroupBytes;            // half of 256 columns
-constexpr uint32_t kB1Bytes = kN1 / 16 * kGroupBytes;            // half of 240 columns
-constexpr uint32_t kStageBytes = kABytes + kB0Bytes + kB1Bytes;  // 54,144
+constexpr uint32_t kB0Bytes = kN0 / 16 * kGroupBytes;            // a CTA's half of 256 columns
+constexpr uint32_t kBBytes = kItemCols / 16 * kGroupBytes;       // and of all 496
+constexpr uint32_t kStageBytes = kABytes + kBBytes;              // 36,096
 // the epilogue warps' pieces: 32 rows x 14 words (28 16-bit columns), row r
 // at words 15 r (conflict-free by row and by column)
 constexpr uint32_t kPieceWords = 14, kPiecePitch = 15;
@@ -113,25 +118,25 @@ constexpr int kMmaSmem = kMmaStages * kStageBytes + kEpiBytes + 128;
 static_assert(kBlockK % kKStep == 0 && kStageBytes % 128 == 0, "K steps and TMA destinations");
 static_assert(kMmaSmem + 256 <= 232448, "shared memory above the per-block limit");
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kHalfCols = kItemCols / 2;         // columns per epilogue warp (248)
+constexpr uint32_t kHalfCols = kItemCols / 2;         // columns per epilogue warp (248 at most)
 constexpr uint32_t kHalfWords = kHalfCols / 2;        // packed 16-bit pairs (124)
 constexpr uint32_t kSfColA = kItemCols, kSfColB = kItemCols + 8;  // unit scale factors
 constexpr uint32_t kSfWord = 0x7F7F7F7Fu;             // four UE8M0 scale factors of 2^0
 constexpr uint64_t kMmaWaitNs = 1000000000ull;        // 1 s
 constexpr uint32_t kMmaBand = 16;  // item rows (256 rows) per L2 band (HAMMINGDIST_MMA_BAND overrides)
 constexpr int kItemRing = 4;                          // item indices handed to the other warps
-// arrivals that free a ring slot: the MMA thread, the second CTA's producer
-// and both CTAs' epilogue warps
-constexpr uint32_t kRingReaders = 2 + 2 * kEpiWarps;
+// arrivals that free a ring slot: the MMA warp, the producers but the one that
+// fills it, and both CTAs' epilogue warps
+constexpr uint32_t kRingReaders = 1 + (2 * kProducers - 1) + 2 * kEpiWarps;
 constexpr uint32_t kNoItem = 0xFFFFFFFFu;             // end of this pair's items
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;             // an item that covers all of K
 // A split tile's partial distances of one K piece: 16-bit pairs, per CTA,
 // column half, lane quarter and word the 32 lanes of a warp
 constexpr uint64_t kSlotBytes = 2ull * 2 * 4 * kHalfWords * 32 * 4;
 // K pieces of fewer chunks than this cost more in barriers and workspace
-// traffic than they spread (two chunks of four planes run 3 us)
-constexpr uint32_t kMinPart = 2;
-// blocks of 288 sites per row and chunk in the operand: the P planes, the row
+// traffic than they spread (three chunks of four planes run 3 us)
+constexpr uint32_t kMinPart = 3;
+// blocks of 192 sites per row and chunk in the operand: the P planes, the row
 // side's dash and the column side's dash (two blocks for P = 6: -4 and -1)
 __host__ __device__ constexpr uint32_t op_blocks(uint32_t planes) {
   return planes + (planes == 6 ? 3u : 2u);
@@ -162,13 +167,13 @@ __host__ __device__ constexpr uint32_t idesc_mxf4(uint32_t n) {
 
 // One matrix of a launch (device copy): its output and the chunks whose dash
 // products count. Its operand's tensor maps are at 2 job of the launch's maps
-// (boxes of one block of 128 and of 120 rows).
+// (boxes of one block of 128 and of 248 rows).
 struct MmaJob {
   void *out;                     // lt index out_base at out[0]
   unsigned long long out_base;
   uint32_t row_hi, sites, max_dist, dtype;  // rows end, L, cap, 1/2/4 bytes
   uint32_t planes;                          // P
-  uint32_t chunks;                          // 288-site chunks per row
+  uint32_t chunks;                          // 192-site chunks per row
   const uint32_t *dash_list;                // the chunks whose dash products count
   const uint32_t *dash_rank;                // per chunk: listed chunks before it (chunks + 1)
   unsigned long long pairs;                 // lower-triangle pairs of this launch
@@ -313,13 +318,13 @@ __device__ __forceinline__ void mma_f4(uint32_t d_tmem, uint64_t a_desc, uint64_
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
       : "memory");
 }
-// One K block (144 bytes a row) of an item: its three K steps against both
+// One K block (96 bytes a row) of an item: its two K steps against both
 // column halves, or the first alone.
 template <bool kSecond>
 __device__ __forceinline__ void mma_block(uint32_t tmem, uint64_t a_desc, uint32_t id0, uint32_t id1,
                                           bool accumulate) {
   constexpr uint64_t kStep = 128 * (kKStep / 16) >> 4;  // three core matrices
-  const uint64_t b0 = a_desc + (kABytes >> 4), b1 = b0 + (kB0Bytes >> 4);
+  const uint64_t b0 = a_desc + (kABytes >> 4), b1 = b0 + (kB0Bytes >> 4);  // after 128 columns
 #pragma unroll
   for (uint32_t k = 0; k < kBlockK / kKStep; ++k) {
     const uint32_t acc = (accumulate || k) ? 1u : 0u;
@@ -441,15 +446,16 @@ __device__ __forceinline__ uint32_t pack2(uint32_t d0, uint32_t d1, float sites,
   return __byte_perm(__float_as_uint(m0), __float_as_uint(m1), 0x5410u);
 }
 
-// This warp's 32 rows x 248 columns from taddr, packed: word w holds columns
-// 2 w and 2 w + 1 of row `lane`.
-__device__ __forceinline__ void load_packed(uint32_t taddr, float sites, float cap,
+// This warp's 32 rows x 128 columns from t0 and 120 from t1, packed: word w
+// holds columns 2 w and 2 w + 1 of row `lane`.
+__device__ __forceinline__ void load_packed(uint32_t t0, uint32_t t1, float sites, float cap,
                                             uint32_t (&v)[kHalfWords]) {
 #pragma unroll
   for (uint32_t g = 0; g < 7; ++g) {
+    const uint32_t t = g < 4 ? t0 + 32 * g : t1 + 32 * (g - 4);
     uint32_t d[16], e[16];
-    tmem_ld16(taddr + 32 * g, d);
-    tmem_ld16(taddr + 32 * g + 16, e);
+    tmem_ld16(t, d);
+    tmem_ld16(t + 16, e);
     tmem_ld_wait();
 #pragma unroll
     for (uint32_t k = 0; k < 8; ++k) {
@@ -458,8 +464,8 @@ __device__ __forceinline__ void load_packed(uint32_t taddr, float sites, float c
     }
   }
   uint32_t d[16], e[8];
-  tmem_ld16(taddr + 224, d);
-  tmem_ld8(taddr + 240, e);
+  tmem_ld16(t1 + 96, d);
+  tmem_ld8(t1 + 112, e);
   tmem_ld_wait();
 #pragma unroll
   for (uint32_t k = 0; k < 8; ++k) v[112 + k] = pack2(d[2 * k], d[2 * k + 1], sites, cap);
@@ -526,7 +532,7 @@ __device__ __forceinline__ void store_packed(const MmaJob &job, uint32_t i0, uin
 
 // 32-bit outputs: 8 columns at a time straight from the accumulators, four
 // rows per store.
-__device__ __forceinline__ void store_wide(const MmaJob &job, uint32_t taddr, uint32_t i0,
+__device__ __forceinline__ void store_wide(const MmaJob &job, uint32_t t_lo, uint32_t t_hi, uint32_t i0,
                                            uint32_t j0, uint32_t col_end, uint32_t lane,
                                            uint32_t *buf) {
   const uint32_t rows = job.row_hi - i0 < 32u ? job.row_hi - i0 : 32u;
@@ -537,7 +543,7 @@ __device__ __forceinline__ void store_wide(const MmaJob &job, uint32_t taddr, ui
     const uint32_t j = j0 + c;
     if (j >= col_end || j + 1 >= i0 + rows) break;  // warp-uniform
     uint32_t d[8];
-    tmem_ld8(taddr + c, d);
+    tmem_ld8(c < kN0 / 2 ? t_lo + c : t_hi + (c - kN0 / 2), d);
     tmem_ld_wait();
     __syncwarp();
 #pragma unroll
@@ -616,21 +622,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMmaThreads, 1)
   // barriers of the first CTA, where both CTAs' threads arrive
   const uint32_t lead_full0 = map_rank(full0, 0);
   const uint32_t lead_ring_empty0 = map_rank(smem_u32(&item_empty[0]), 0);
-  if (warp == 0) {
+  if (warp == 0 || warp == 2 + kEpiWarps) {
     if (lane == 0) {
-      // producer: loads its CTA's share of every K block of this pair's items.
+      // producers: load their CTA's share of every K block of this pair's
+      // items, taking the blocks in turn (a block costs one thread about 460
+      // cycles of waits and issues; its MMAs last 497).
       // Static order: items unit, unit + units, ...; every warp walks them by
       // itself. With `queue`, item `unit` and then the launch's counter: the
-      // first CTA's producer hands each index to the MMA warp and, in both
-      // CTAs, the epilogue warps and the second producer.
+      // first CTA's first producer hands each index to all other warps.
       const uint32_t peer_item0 = map_rank(smem_u32(&s_item[0]), 1);
       const uint32_t peer_ring_full0 = map_rank(ring_full0, 1);
+      const bool fills = rank == 0 && warp == 0;  // the ring
+      uint32_t turn = warp == 0 ? 0u : 1u;        // blocks until this thread's next one
       uint32_t s = 0, ph = 1;  // stage, and the parity its empty barrier is waited for
       bool ok = true;
       for (uint32_t k = 0; ok; ++k) {
         const uint32_t r = k % kItemRing;
         uint32_t t = unit + k * units;
-        if (queue && rank == 0) {
+        if (queue && fills) {
           if (k >= (uint32_t)kItemRing &&
               !mbar_wait<true>(smem_u32(&item_empty[r]), ((k / kItemRing) - 1) & 1u, 4 * kMmaWaitNs)) {
             ok = false;
@@ -653,20 +662,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMmaThreads, 1)
         if (t >= n_items) break;
         const MmaItem it = items[t];
         if (it.job == kNoItem) break;
-        const CUtensorMap *t128 = tms + 2 * it.job, *t120 = t128 + 1;
-        // row groups of this CTA's 128 rows, and of its half of each column half
-        const int32_t ya = (int32_t)(it.row0 / 8 + rank * (kTM / 8));
-        const int32_t yb0 = (int32_t)(it.col0 / 8 + rank * it.n0_16);
-        const int32_t yb1 = (int32_t)((it.col0 + it.n0()) / 8 + rank * it.n1_16);
+        // boxes of one block of 128 rows, and of 248 for both MMAs' columns
         const bool second = it.n1_16 != 0;
-        const uint32_t bytes = 2 * (kABytes + kB0Bytes + (second ? kB1Bytes : 0u));
+        const CUtensorMap *ta = tms + 2 * it.job, *tb = ta + (second ? 1 : 0);
+        prefetch_tmap(ta);
+        prefetch_tmap(tb);
+        // row groups of this CTA's 128 rows, and of its half of the columns
+        const int32_t ya = (int32_t)(it.row0 / 8 + rank * (kTM / 8));
+        const int32_t yb = (int32_t)(it.col0 / 8 + rank * (it.n0_16 + it.n1_16));
+        const uint32_t bytes = 2 * (kABytes + (second ? kBBytes : kB0Bytes));
         auto issue = [&](int32_t xa, int32_t xb) {
-          if (!mbar_wait(empty0 + 8 * s, ph, kMmaWaitNs)) return false;
-          if (rank == 0) mbar_expect(full0 + 8 * s, bytes);
-          const uint32_t st = smem + s * kStageBytes, bar = lead_full0 + 8 * s;
-          tma_load_pair(st, t128, xa, ya, bar);
-          tma_load_pair(st + kABytes, t128, xb, yb0, bar);
-          if (second) tma_load_pair(st + kABytes + kB0Bytes, t120, xb, yb1, bar);
+          if (turn == 0) {
+            if (!mbar_wait(empty0 + 8 * s, ph, kMmaWaitNs)) return false;
+            if (rank == 0) mbar_expect(full0 + 8 * s, bytes);
+            const uint32_t st = smem + s * kStageBytes, bar = lead_full0 + 8 * s;
+            tma_load_pair(st, ta, xa, ya, bar);
+            tma_load_pair(st + kABytes, tb, xb, yb, bar);
+            turn = kProducers;
+          }
+          --turn;
           if (++s == (uint32_t)kMmaStages) {
             s = 0;
             ph ^= 1u;
@@ -676,7 +690,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMmaThreads, 1)
         // K order: the P plane blocks of every chunk, then the dash products
         // of the listed chunks (the rows' +1 block against the columns'
         // -(P - 1) block; for P = 6 the +1 block twice, against -4 and -1).
-        // Coordinates count 8-byte elements: a block is 144 of them.
+        // Coordinates count 8-byte elements: a block is 96 of them.
         const uint32_t P = it.planes, NB = op_blocks(P);
         int32_t x = (int32_t)(it.c_lo * NB * kBlockK);
         for (uint32_t c = it.c_lo; ok && c < it.c_hi; ++c, x += (int32_t)((NB - P) * kBlockK))
@@ -769,17 +783,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMmaThreads, 1)
         mbar_wait(smem_u32(&fin), 0, 4 * kMmaWaitNs);
       }
     } else if (unit == 0) {
-      // the launch's multiply-adds (pairs x 288 values per K block)
+      // the launch's multiply-adds (pairs x 192 values per K block)
       for (uint32_t q = lane; q < n_jobs; q += 32)
         atomicAdd(macs, jobs[q].pairs * (unsigned long long)kChunkSites *
                             blocks_in(jobs[q], 0, jobs[q].chunks));
     }
   } else {
     // epilogue warps 2 .. 9: warp w reads TMEM lanes 32 (w % 4) .. + 31, which
-    // are rows 32 (w % 4) + lane of the CTA's 128, in columns [0, 248) (w < 6)
-    // or [248, 496) (w >= 6) of the item
+    // are rows 32 (w % 4) + lane of the CTA's 128, in the columns that the
+    // first (w < 6) or the second CTA brings: `cols` of them, up to 128 in the
+    // first MMA's accumulators and the rest in the second's
     const uint32_t sub = warp & 3u, half = warp < 6 ? 0u : 1u;
-    const uint32_t taddr = tmem + ((sub * 32) << 16) + half * kHalfCols;
+    const uint32_t t_lane = tmem + ((sub * 32) << 16);
     const uint32_t lead_free = map_rank(smem_u32(&tmem_free), 0);
     uint32_t *buf = reinterpret_cast<uint32_t *>(smem_raw + (smem - smem_u32(smem_raw)) +
                                                  kMmaStages * kStageBytes) +
@@ -816,12 +831,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMmaThreads, 1)
       // one decision per warp: tcgen05.ld needs the whole warp
       if (__any_sync(0xffffffffu, !got || *(volatile int *)&s_abort)) break;
       tc_after_sync();
-      const uint32_t i0 = it.row0 + rank * kTM + sub * 32, j0 = it.col0 + half * kHalfCols;
-      const uint32_t col_end = it.col0 + it.n0() + it.n1();
+      const uint32_t cols = (it.n0() + it.n1()) / 2;
+      const uint32_t i0 = it.row0 + rank * kTM + sub * 32, j0 = it.col0 + half * cols;
+      const uint32_t col_end = j0 + cols;
+      const uint32_t t0 = t_lane + half * (it.n0() / 2), t1 = t_lane + kN0 + half * (it.n1() / 2);
       // nothing below the diagonal, or past the rows or columns (warp-uniform)
       const bool any = i0 < job.row_hi && j0 < col_end && j0 + 1 < i0 + 32;
       if (job.dtype == 4) {
-        if (any) store_wide(job, taddr, i0, j0, col_end, lane, buf);
+        if (any) store_wide(job, t0, t1, i0, j0, col_end, lane, buf);
         tc_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(lead_free);
@@ -830,7 +847,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMmaThreads, 1)
       uint32_t v[kHalfWords];
       if (any) {
         const uint32_t top = it.slot != kNoSlot ? 65535u : job.max_dist;
-        load_packed(taddr, (float)sites_in(job, it.c_lo, it.c_hi), (float)top, v);
+        load_packed(t0, t1, (float)sites_in(job, it.c_lo, it.c_hi), (float)top, v);
       }
       // the accumulators may be overwritten
       tc_before_sync();
@@ -877,10 +894,11 @@ __global__ void __launch_bounds__(256)
   const MmaJob &job = jobs[f.job];
   const uint32_t q = id % kFixPieces, part = id / kFixPieces % 16;  // (rank, half, quarter)
   const uint32_t i0 = f.row0 + (part >> 3) * kTM + (part & 3u) * 32;
-  const uint32_t j = f.col0 + (part >> 2 & 1u) * kHalfCols + 2 * kPieceWords * q;
+  const uint32_t half = (part >> 2 & 1u) * (f.cols / 2), end = f.col0 + half + f.cols / 2;
+  const uint32_t j = f.col0 + half + 2 * kPieceWords * q;
   if (i0 >= job.row_hi) return;
   const uint32_t rows = job.row_hi - i0 < 32u ? job.row_hi - i0 : 32u;
-  if (j >= f.col0 + f.cols || j + 1 >= i0 + rows) return;
+  if (j >= end || j + 1 >= i0 + rows) return;
   const uint32_t words = kHalfWords - q * kPieceWords < kPieceWords ? kHalfWords - q * kPieceWords
                                                                     : kPieceWords;
   uint32_t v[kPieceWords];
@@ -911,7 +929,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (uint32_t w = 0; w < kPieceWords; ++w) buf[lane * kPiecePitch + w] = __vminu2(v[w], cap);
   __syncwarp();
-  const uint32_t cols = f.col0 + f.cols - j < 2 * words ? f.col0 + f.cols - j : 2 * words;
+  const uint32_t cols = end - j < 2 * words ? end - j : 2 * words;
   const unsigned long long e0 = (unsigned long long)i0 * (i0 - 1) / 2 - job.out_base + lane + j;
   if (job.dtype == 1)
     store_piece<uint8_t>(static_cast<uint8_t *>(job.out), e0, i0, rows, j, cols, buf, lane);
@@ -1442,7 +1460,7 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     const PairJobSpec &sp = specs[js[q].k];
     const hd_alignment *a = sp.aln, *o = owner_of(js[q]);
     make_tmap_op(ctx, &tms[2 * q], ops[js[q].k], planes[q], o->length, a->n_rows, kTM);
-    make_tmap_op(ctx, &tms[2 * q + 1], ops[js[q].k], planes[q], o->length, a->n_rows, kN1 / 2);
+    make_tmap_op(ctx, &tms[2 * q + 1], ops[js[q].k], planes[q], o->length, a->n_rows, kItemCols / 2);
     MmaJob &m = jobs[q];
     m.out = sp.d_out;
     m.out_base = sp.out_base;
