@@ -403,8 +403,11 @@ bool all_cached(void *map, size_t len) {
 //     is copied.
 // host() holds the file's bytes [0, prefix_bytes()); wait_bytes(x) waits
 // until it holds [0, x); stream_wait_bytes(s, x) makes stream s wait for the
-// copies of [0, x) only, not for the copies queued after them. The destructor
-// stops the threads, joins them, waits for the copies, unmaps and closes.
+// copies of [0, x) only, not for the copies queued after them. Once the last
+// copy is done and host_done() says that the caller reads no more of host(),
+// the uploader unmaps the file (0.15 ms for 30 MB, 0.8 for 598) while the
+// caller's kernels run. The destructor stops the threads, joins them, waits
+// for the copies, unmaps what is left and closes.
 struct PartReader {
   hd_ctx *ctx;
   const char *path;
@@ -424,6 +427,7 @@ struct PartReader {
   std::vector<char> done;
   uint64_t prefix = 0;  // parts [0, prefix) on the host
   uint64_t queued = 0;  // parts [0, queued) copies queued on ctx->up, events recorded
+  bool unneeded = false;  // the caller reads no more of host()
   std::vector<std::thread> th;
 
   PartReader(hd_ctx *c, const char *p, uint64_t bytes, uint8_t *d)
@@ -546,6 +550,19 @@ struct PartReader {
       queued = k = e;
       cv.notify_all();
     }
+    if (!map) return;
+    {
+      std::unique_lock<std::mutex> lk(mu);
+      cv.wait(lk, [&] { return bad.load() || unneeded; });
+    }
+    if (cudaEventSynchronize(ctx->part_ev[parts - 1]) != cudaSuccess) return;
+    ::munmap(map, map_len);
+    map = nullptr;  // read again by the destructor only, after the join
+  }
+  void host_done() {
+    std::lock_guard<std::mutex> lk(mu);
+    unneeded = true;
+    cv.notify_all();
   }
   void fault(int code) {
     std::lock_guard<std::mutex> lk(mu);
@@ -572,11 +589,10 @@ struct PartReader {
     }
     return cudaStreamWaitEvent(s, ctx->part_ev[k - 1], 0) == cudaSuccess;
   }
-  // waits for the whole file: ctx->stream then waits for every copy; throws
+  // waits until every copy is queued: ctx->stream then waits for them; throws
   // HD_ERR_IO after a read error, HD_ERR_CUDA after a copy error
   void finish() {
     const bool ok = stream_wait_bytes(ctx->stream, n);
-    join();
     if (!ok || bad.load()) {
       if (bad.load() == 1) fail(HD_ERR_IO, open_failed(path));
       fail(HD_ERR_CUDA, "cudaMemcpyAsync of the FASTA file failed");
@@ -587,8 +603,11 @@ struct PartReader {
 // Reads a FASTA file into the context's device input buffer with a
 // PartReader: 8 MB parts are copied as they become ready, so the upload runs
 // under the read. If the buffer already holds this file, unchanged, nothing
-// is read or copied. Returns the device bytes; *nbytes = the file size.
-const uint8_t *stage_file(hd_ctx *ctx, const char *path, uint64_t *nbytes) {
+// is read or copied. Returns the device bytes; *nbytes = the file size. `rd`
+// holds the reader, which the caller lets go at the end of its work: its
+// threads end and the file is unmapped meanwhile.
+const uint8_t *stage_file(hd_ctx *ctx, const char *path, uint64_t *nbytes,
+                          std::unique_ptr<PartReader> &rd) {
   struct stat sb;
   if (!path || ::stat(path, &sb) != 0 || !S_ISREG(sb.st_mode)) fail(HD_ERR_IO, open_failed(path));
   const uint64_t n = (uint64_t)sb.st_size;
@@ -604,11 +623,10 @@ const uint8_t *stage_file(hd_ctx *ctx, const char *path, uint64_t *nbytes) {
     ctx->file = DevBuf(hd::round_up(n + 16, 1 << 20), ctx->stream);
   }
   uint8_t *dev = ctx->file.as<uint8_t>();
-  {
-    PartReader rd(ctx, path, n, dev);
-    rd.start();
-    rd.finish();
-  }
+  rd = std::make_unique<PartReader>(ctx, path, n, dev);
+  rd->start();
+  rd->host_done();
+  rd->finish();
   ctx->file_tag = tag;
   return dev;
 }
@@ -984,6 +1002,7 @@ void hd_ctx_destroy(hd_ctx *ctx) {
   cudaSetDevice(ctx->device);
   ctx->parsed.reset();  // its buffers are freed on ctx->stream
   ctx->file.release();
+  for (DevBuf &b : ctx->mma_ws) b.release();
   if (ctx->pin) cudaFreeHost(ctx->pin);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->d_status) cudaFree(ctx->d_status);
@@ -992,6 +1011,7 @@ void hd_ctx_destroy(hd_ctx *ctx) {
   for (cudaEvent_t e : ctx->trace.pool) cudaEventDestroy(e);
   if (ctx->up) cudaStreamSynchronize(ctx->up);
   for (cudaEvent_t e : ctx->part_ev) cudaEventDestroy(e);
+  for (cudaEvent_t e : ctx->call_ev) cudaEventDestroy(e);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->up) cudaStreamDestroy(ctx->up);
@@ -1056,7 +1076,8 @@ int hd_alignment_from_fasta_file(hd_ctx *ctx, const char *path, int remove_dupli
   return guard(ctx, [&] {
     hd::trace_begin(ctx, "hd_alignment_from_fasta_file");
     uint64_t nbytes = 0;
-    const uint8_t *d = stage_file(ctx, path, &nbytes);
+    std::unique_ptr<PartReader> rd;
+    const uint8_t *d = stage_file(ctx, path, &nbytes, rd);
     hd::trace_mark(ctx, "read + upload");
     hd::Records &rec = file_records(ctx, d, nbytes, n_limit);
     hd::trace_mark(ctx, "parse");
@@ -1082,7 +1103,8 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
     auto whole = [&] {
       hd_alignment *a = nullptr;
       uint64_t nbytes = 0;
-      const uint8_t *d = stage_file(ctx, path, &nbytes);
+      std::unique_ptr<PartReader> rd;
+      const uint8_t *d = stage_file(ctx, path, &nbytes, rd);
       hd::trace_mark(ctx, "read + upload");
       hd::Records &rec = file_records(ctx, d, nbytes, 0);
       hd::trace_mark(ctx, "parse");
@@ -1129,11 +1151,24 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
     }
     uint8_t *dev = ctx->file.as<uint8_t>();
     auto reader = std::make_unique<PartReader>(ctx, path, n, dev);
+    // the call's events (at most 12) are kept in the context, and made before
+    // the uploader starts: an event made between its copies, which hold the
+    // driver's lock, waited 0.3 ms
+    auto event_of = [ctx](size_t k) {
+      while (ctx->call_ev.size() <= k) {
+        cudaEvent_t e;
+        HD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        ctx->call_ev.push_back(e);
+      }
+      return ctx->call_ev[k];
+    };
+    event_of(11);
     reader->start();
     hd::trace_host(ctx, "readers started");
     const char *text = reader->host();
     hd::trace_mark(ctx, "setup");
     auto read_all = [&] {
+      reader->host_done();
       reader->finish();
       ctx->file_tag = tag;
     };
@@ -1200,18 +1235,13 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
     // waits for every stream the call uses before any of the above is freed
     struct Sync {
       hd_ctx *c;
-      std::vector<cudaEvent_t> ev;
-      cudaEvent_t make() {
-        cudaEvent_t e;
-        HD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        ev.push_back(e);
-        return e;
-      }
+      decltype(event_of) &event;
+      size_t used;
+      cudaEvent_t make() { return event(used++); }
       ~Sync() {
         for (cudaStream_t s : {c->stream, c->side, c->up}) cudaStreamSynchronize(s);
-        for (cudaEvent_t e : ev) cudaEventDestroy(e);
       }
-    } sync{ctx, {}};
+    } sync{ctx, event_of, 0};
     auto fallback = [&] {  // the whole matrix after the whole file
       HD_CUDA(cudaStreamSynchronize(ctx->side));
       read_all();
@@ -1657,7 +1687,8 @@ int hd_read_lower_triangular(hd_ctx *ctx, const char *path, int dtype_bytes, hd_
   if (parse_error) *parse_error = 0;
   return guard(ctx, [&] {
     uint64_t nbytes = 0;
-    const uint8_t *d = stage_file(ctx, path, &nbytes);
+    std::unique_ptr<PartReader> rd;
+    const uint8_t *d = stage_file(ctx, path, &nbytes, rd);
     hd::ParsedValues pv = hd::read_lower_triangular_device(ctx, d, nbytes, dtype_bytes);
     if (entries) *entries = pv.entries;
     if (nsamples) *nsamples = pv.nsamples;
@@ -1673,7 +1704,8 @@ int hd_read_csv(hd_ctx *ctx, const char *path, hd_output_fn out_fn, void *user, 
   if (parse_error) *parse_error = 0;
   return guard(ctx, [&] {
     uint64_t nbytes = 0;
-    const uint8_t *d = stage_file(ctx, path, &nbytes);
+    std::unique_ptr<PartReader> rd;
+    const uint8_t *d = stage_file(ctx, path, &nbytes, rd);
     hd::ParsedValues pv = hd::read_csv_device(ctx, d, nbytes);
     if (entries) *entries = pv.entries;
     if (nsamples) *nsamples = pv.nsamples;
@@ -1779,7 +1811,8 @@ int hd_reference_distances_file(hd_ctx *ctx, const char *ref, uint64_t ref_len, 
   return guard(ctx, [&] {
     hd::trace_begin(ctx, "hd_reference_distances_file");
     uint64_t nbytes = 0;
-    const uint8_t *d = stage_file(ctx, path, &nbytes);
+    std::unique_ptr<PartReader> rd;
+    const uint8_t *d = stage_file(ctx, path, &nbytes, rd);
     hd::trace_mark(ctx, "read + upload");
     reference_distances_of(ctx, d, nbytes, ref, ref_len, include_x, out, n_out, true);
   });
@@ -1820,7 +1853,8 @@ int hd_fasta_sequence_indices_file(hd_ctx *ctx, const char *path, uint64_t n_lim
   *n_out = 0;
   return guard(ctx, [&] {
     uint64_t nbytes = 0;
-    const uint8_t *d = stage_file(ctx, path, &nbytes);
+    std::unique_ptr<PartReader> rd;
+    const uint8_t *d = stage_file(ctx, path, &nbytes, rd);
     sequence_indices_of(ctx, d, nbytes, n_limit, out, n_out, true);
   });
 }
@@ -1956,6 +1990,7 @@ int hd_batch_run(hd_batch *b) {
         specs.push_back(s);
       }
       b->plan = hd::PairLaunchPlan();
+      b->plan.replayed = true;
       hd::prepare_pairwise_jobs(ctx, specs, st, &b->plan);
       HD_CUDA(cudaStreamSynchronize(st));
       for (auto &L : b->plan.launches) b->tiles += L.tiles;

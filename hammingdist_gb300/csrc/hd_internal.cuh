@@ -173,7 +173,12 @@ struct hd_ctx {
   // the page cache is copied directly (no CPU copy into `pin`).
   cudaStream_t up = nullptr;
   std::vector<cudaEvent_t> part_ev;
+  std::vector<cudaEvent_t> call_ev;  // a streamed call's other events (grows)
   int map_files = 0;
+  // the tensor-core engine's workspaces for launches on `stream` and `side`
+  // (K pieces of split tiles; grow, at most about 45 MB each): launches on one
+  // stream follow one another. A plan that is replayed from a graph has its own.
+  hd::DevBuf mma_ws[2];
   hd::Trace trace;
 };
 
@@ -527,6 +532,7 @@ struct PairLaunchPlan {
   };
   std::vector<Launch> launches;
   std::vector<DevBuf> blocks;  // job tables + tensor maps + tile counters
+  bool replayed = false;       // launched again later: keeps workspaces of its own
 };
 void prepare_pairwise_jobs(hd_ctx *ctx, std::vector<PairJobSpec> &specs, cudaStream_t stream,
                            PairLaunchPlan *plan,

@@ -1430,14 +1430,21 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
   bool queue = nj > 1;
   if (const char *e = std::getenv("HAMMINGDIST_MMA_SCHEDULE"))
     queue = queue || std::string(e) == "queue";
+  // the pieces' workspace: the context's for this stream, else the plan's own.
+  // (Allocated for each launch on the side stream, it held a streamed call up
+  // for 0.7 ms.)
   MmaPlan mp;
-  DevBuf ws;
+  DevBuf own;
+  DevBuf *ws = plan->replayed ? &own : stream == ctx->stream ? &ctx->mma_ws[0]
+               : stream == ctx->side ? &ctx->mma_ws[1] : &own;
   for (;;) {
     if (queue) plan_queue(list, units, planes, may_split, mp);
     else plan_static(list, units, planes[0], may_split[0], mp);
-    if (!mp.slots) break;
+    const uint64_t need = mp.slots * kSlotBytes;
+    if (need <= ws->bytes) break;
     try {
-      ws = DevBuf(mp.slots * kSlotBytes, stream, true);
+      ws->release();  // in stream order, after the launches that use it
+      *ws = DevBuf(round_up(need, 4ull << 20), stream, true);
       break;
     } catch (const Error &e) {
       if (e.code != HD_ERR_OOM) throw;
@@ -1495,12 +1502,12 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
   L.d_tms = d;
   L.d_fix = d + fix_at;
   L.fixes = mp.fix.size();
-  L.d_ws = ws.p;
+  L.d_ws = ws->p;
   L.d_counter = reinterpret_cast<unsigned long long *>(d + counter_at);
   L.queue = queue;
   plan->launches.push_back(L);
   plan->blocks.push_back(std::move(dev));
-  if (ws.p) plan->blocks.push_back(std::move(ws));
+  if (own.p) plan->blocks.push_back(std::move(own));
 }
 
 void launch_mma(hd_ctx *ctx, const PairLaunchPlan::Launch &L, cudaStream_t stream) {
