@@ -162,6 +162,12 @@ cudaEvent_t trace_event(hd_ctx *ctx, size_t k) {
 }
 }  // namespace
 
+uint64_t *pinned_words(hd_ctx *ctx) {
+  if (!ctx->words)
+    HD_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&ctx->words), 256, cudaHostAllocDefault));
+  return ctx->words;
+}
+
 void upload_table(hd_ctx *ctx, void *d_dst, const void *host, size_t bytes, cudaStream_t s) {
   constexpr int kSlots = 8;
   constexpr size_t kSlotBytes = 1u << 20;
@@ -1005,6 +1011,7 @@ void hd_ctx_destroy(hd_ctx *ctx) {
   for (DevBuf &b : ctx->mma_ws) b.release();
   if (ctx->pin) cudaFreeHost(ctx->pin);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  if (ctx->words) cudaFreeHost(ctx->words);
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
   if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);

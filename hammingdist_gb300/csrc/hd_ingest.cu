@@ -45,225 +45,390 @@ struct Table256 {
 // ------------------------------------------------------------ newline index
 constexpr int kNlThreads = 256;
 constexpr int kNlIters = 16;
+constexpr int kNlBatch = 8;                                               // vectors loaded at once
+constexpr int kNlWarps = kNlThreads / 32;
 constexpr uint64_t kNlWarpBytes = 32ull * 16 * kNlIters;                  // 8 KB
-constexpr uint64_t kNlBlockBytes = kNlWarpBytes * (kNlThreads / 32);      // 64 KB
+constexpr uint64_t kNlBlockBytes = kNlWarpBytes * kNlWarps;               // 64 KB
 
 __device__ inline uint32_t nl_nibble(uint32_t w) {
   uint32_t e = __vcmpeq4(w, 0x0a0a0a0au) & 0x01010101u;
   return (e | (e >> 7) | (e >> 14) | (e >> 21)) & 0xfu;
 }
+// 0x80 bits, nonzero exactly where some byte of w is '\n' (the lowest such
+// byte is exact, bytes above it may be flagged too: only whether there is one)
+__device__ inline uint32_t nl_any(uint32_t w) {
+  const uint32_t x = w ^ 0x0a0a0a0au;
+  return (x - 0x01010101u) & ~x & 0x80808080u;
+}
+// 16-bit mask of the '\n' bytes of a vector
+__device__ inline uint32_t nl_mask(uint4 v) {
+  if (!(nl_any(v.x) | nl_any(v.y) | nl_any(v.z) | nl_any(v.w))) return 0;
+  return nl_nibble(v.x) | (nl_nibble(v.y) << 4) | (nl_nibble(v.z) << 8) | (nl_nibble(v.w) << 12);
+}
 
 // 16-bit mask of '\n' bytes in p[off, off+16).
 __device__ inline uint32_t nl_mask16(const uint8_t *p, uint64_t off, uint64_t n) {
-  if (off + 16 <= n) {
-    uint4 v = __ldg(reinterpret_cast<const uint4 *>(p + off));
-    return nl_nibble(v.x) | (nl_nibble(v.y) << 4) | (nl_nibble(v.z) << 8) | (nl_nibble(v.w) << 12);
-  }
+  if (off + 16 <= n) return nl_mask(__ldg(reinterpret_cast<const uint4 *>(p + off)));
   uint32_t m = 0;
   for (int k = 0; k < 16; ++k)
     if (off + k < n && p[off + k] == '\n') m |= 1u << k;
   return m;
 }
 
-// Newlines per 64 KB block (counts) and per 8 KB warp span (warp_counts[w]).
-// A span with one or two newlines also records their offsets in the span
-// (warp_counts[W + 2 w] and [W + 2 w + 1], W = the launch's warps), so that
-// the write pass need not read it again: a FASTA line is usually longer than
-// a span. Each lane keeps the first two newlines of its own 16-byte slices,
+// Whether the line after the newline at `pos` is a header: it starts with '>'.
+__device__ inline bool header_after(const uint8_t *p, uint64_t pos, uint64_t n) {
+  return pos + 1 < n && p[pos + 1] == '>';
+}
+
+// Newlines and (kHdr) newlines that a header line follows: per 64 KB block
+// (counts: newlines | headers << 32) and per 8 KB warp span (warp_counts[w]:
+// newlines | headers << 16). A span with one or two newlines also records
+// their offsets in the span with their header flag (warp_counts[W + 2 w] and
+// [W + 2 w + 1] = offset << 1 | flag, W = the launch's warps), so that the
+// write pass need not read it again: a FASTA line is usually longer than a
+// span. Each lane keeps the first two newlines of its own 16-byte slices,
 // which it visits in increasing order; the span's first newline is the least
 // of the lanes' first ones, and its second the least of the rest.
-__global__ void k_nl_count(const uint8_t *p, uint64_t n, uint64_t *counts, uint32_t *warp_counts) {
-  __shared__ uint64_t tmp[33];
+// DRAM-bound: a lane has 8 vectors in flight, and a vector without a newline
+// costs 4 short tests: 598 MB in 83 us, 7.2 TB/s (4 in flight, with a full
+// mask of each: 112 us).
+template <bool kHdr>
+__global__ void __launch_bounds__(kNlThreads)
+    k_nl_count(const uint8_t *p, uint64_t n, uint64_t *counts, uint32_t *warp_counts) {
+  __shared__ uint32_t sums[kNlWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint64_t base = blockIdx.x * kNlBlockBytes + warp * kNlWarpBytes + lane * 16;
+  const uint64_t wbase = blockIdx.x * kNlBlockBytes + warp * kNlWarpBytes;
   constexpr uint32_t kNone = 0xFFFFFFFFu;
-  uint32_t c = 0, o0 = kNone, o1 = kNone;
-#pragma unroll 4
-  for (int it = 0; it < kNlIters; ++it) {
-    const uint32_t m = nl_mask16(p, base + it * 512ull, n);
-    if (m && c < 2) {
-      const uint32_t rel = (uint32_t)it * 512u + (uint32_t)lane * 16u;
-      const uint32_t a = rel + (uint32_t)(__ffs(m) - 1), m2 = m & (m - 1);
-      if (c == 0) {
-        o0 = a;
-        if (m2) o1 = rel + (uint32_t)(__ffs(m2) - 1);
-      } else {
-        o1 = a;
-      }
+  uint32_t c = 0, h = 0, o0 = kNone, o1 = kNone;
+  auto take = [&](uint32_t m, int it) {  // the newlines of slice `it`
+    const uint32_t rel = (uint32_t)it * 512u + (uint32_t)lane * 16u;
+    while (m) {
+      const uint32_t at = rel + (uint32_t)(__ffs(m) - 1);
+      m &= m - 1;
+      const uint32_t f = kHdr && header_after(p, wbase + at, n) ? 1u : 0u;
+      if (c == 0) o0 = at << 1 | f;
+      else if (c == 1) o1 = at << 1 | f;
+      ++c;
+      h += f;
     }
-    c += __popc(m);
+  };
+  const uint64_t lbase = wbase + lane * 16;
+  for (int i0 = 0; i0 < kNlIters; i0 += kNlBatch) {
+    uint4 v[kNlBatch];
+#pragma unroll
+    for (int k = 0; k < kNlBatch; ++k) {
+      const uint64_t at = lbase + (i0 + k) * 512ull;
+      v[k] = at + 16 <= n ? __ldg(reinterpret_cast<const uint4 *>(p + at)) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int k = 0; k < kNlBatch; ++k) {
+      const uint32_t m = nl_mask(v[k]);
+      if (m) take(m, i0 + k);
+    }
   }
-  const uint32_t cw = warp_sum(c);
-  const uint32_t wid = blockIdx.x * (kNlThreads / 32) + warp;
-  if (lane == 0) warp_counts[wid] = cw;
-  if (cw >= 1 && cw <= 2) {  // warp-uniform
+  // the input's last bytes, less than a vector: the last slice of their lane
+  if (n % 16 && n - n % 16 >= lbase && n - n % 16 - lbase < kNlWarpBytes &&
+      (n - n % 16 - lbase) % 512 == 0)
+    take(nl_mask16(p, n - n % 16, n), (int)((n - n % 16 - lbase) / 512));
+  const uint32_t cw = __reduce_add_sync(0xffffffffu, c | h << 16);  // at most 8,192 each
+  const uint32_t wid = blockIdx.x * kNlWarps + warp;
+  if (lane == 0) {
+    warp_counts[wid] = cw;
+    sums[warp] = cw;
+  }
+  const uint32_t cn = cw & 0xFFFFu;
+  if (cn >= 1 && cn <= 2) {  // warp-uniform
     const uint32_t q1 = __reduce_min_sync(0xffffffffu, o0);
     const uint32_t q2 = __reduce_min_sync(0xffffffffu, o0 == q1 ? o1 : o0);
     if (lane == 0) {
-      uint32_t *pos = warp_counts + gridDim.x * (kNlThreads / 32) + 2ull * wid;
+      uint32_t *pos = warp_counts + gridDim.x * kNlWarps + 2ull * wid;
       pos[0] = q1;
       pos[1] = q2;
     }
   }
-  uint64_t tot;
-  block_excl_scan<uint64_t>((uint64_t)c, tmp, tot);
-  if (threadIdx.x == 0) counts[blockIdx.x] = tot;
-}
-
-// Writes the positions of every '\n' in increasing order: each warp starts at
-// its block's offset plus the counts of the block's earlier warps; a span
-// with one or two newlines takes their offsets from the count pass, a span
-// with more scans its lanes' counts where some lane holds a newline.
-__global__ void k_nl_write(const uint8_t *p, uint64_t n, const uint64_t *block_off,
-                           const uint32_t *warp_counts, uint64_t *nl) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t wbase = blockIdx.x * kNlBlockBytes + warp * kNlWarpBytes;
-  const uint32_t wid = blockIdx.x * (kNlThreads / 32) + warp;
-  uint64_t off = block_off[blockIdx.x];
-  for (int w = 0; w < warp; ++w) off += warp_counts[blockIdx.x * (kNlThreads / 32) + w];
-  const uint32_t cw = warp_counts[wid];
-  if (cw == 0) return;
-  if (cw <= 2) {
-    const uint32_t *pos = warp_counts + gridDim.x * (kNlThreads / 32) + 2ull * wid;
-    if (lane < (int)cw) nl[off + lane] = wbase + pos[lane];
-    return;
-  }
-  for (int it = 0; it < kNlIters; ++it) {
-    uint64_t at = wbase + it * 512ull + lane * 16;
-    uint32_t m = nl_mask16(p, at, n);
-    if (!__any_sync(0xffffffffu, m != 0)) continue;
-    uint32_t cnt = __popc(m);
-    uint32_t inc = warp_incl_scan(cnt);
-    uint64_t pos = off + inc - cnt;
-    while (m) {
-      int k = __ffs(m) - 1;
-      nl[pos++] = at + k;
-      m &= m - 1;
-    }
-    off += __shfl_sync(0xffffffffu, inc, 31);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint64_t t = 0;
+#pragma unroll
+    for (int w = 0; w < kNlWarps; ++w) t += (uint64_t)(sums[w] & 0xFFFFu) | (uint64_t)(sums[w] >> 16) << 32;
+    counts[blockIdx.x] = t;
   }
 }
 
 struct ParseSummary {
   unsigned long long m_nl;      // newlines
   unsigned long long lines;     // M
+  unsigned long long headers;   // header lines after the first line
   unsigned long long R;         // records before the n limit
   unsigned long long Rk;        // records kept
   unsigned long long max_len;
   unsigned long long len0;
   unsigned long long skip;      // records left out at the start
+  unsigned long long n_limit;
   unsigned int unterminated;    // the last line has no '\n'
   unsigned int unequal;
   unsigned int multi;           // some record spans several non-empty lines
   unsigned int pad;
 };
 
-__global__ void k_nl_summary(const uint8_t *p, uint64_t n, const uint64_t *m_nl, ParseSummary *s) {
-  s->m_nl = *m_nl;
-  s->unterminated = (n > 0 && p[n - 1] != '\n') ? 1u : 0u;
-  s->lines = *m_nl + s->unterminated;
-}
-
-__device__ inline void line_range(uint64_t k, const uint64_t *nl, uint64_t m_nl, uint64_t n,
-                                  uint64_t &start, uint64_t &end) {
-  start = k ? nl[k - 1] + 1 : 0;
-  end = k < m_nl ? nl[k] : n;
-}
-
-// hdr[k] = line k (k >= 1) is a header: non-empty and starting with '>'.
-__global__ void k_lines(const uint8_t *p, uint64_t n, const uint64_t *nl, uint64_t m_nl, uint64_t M,
-                        uint32_t *hdr) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (k >= M) return;
-  uint64_t s, e;
-  line_range(k, nl, m_nl, n, s, e);
-  hdr[k] = (k >= 1 && e > s && p[s] == '>') ? 1u : 0u;
-}
-
 // Number of records the getline loop of read_fasta produces
 // (src/hamming_impl.cc:216-233): the first line is skipped; every later
 // header closes a record; the loop ends when the stream reaches its end,
-// which happens on reading an unterminated last line. first > 0: the bytes
-// before `first` (which follows a '\n') belong to records parsed before,
-// so the records up to the header that starts there are left out (s->skip:
-// record 0 and those whose header line starts before `first`).
-__global__ void k_rec_count(const uint64_t *H_total, const uint32_t *hdr, const uint64_t *H,
-                            const uint64_t *nl, uint64_t first, uint64_t n_limit,
-                            ParseSummary *s) {
-  uint64_t M = s->lines, R;
-  if (M == 0) R = 0;
-  else if (M == 1) R = s->unterminated ? 0 : 1;
-  else R = *H_total + 1 - ((hdr[M - 1] && s->unterminated) ? 1 : 0);
+// which happens on reading an unterminated last line (last_hdr: that line is
+// a header).
+__device__ inline void count_records(ParseSummary *s, bool last_hdr) {
+  const uint64_t M = s->lines;
+  const uint64_t R = M == 0 || (M == 1 && s->unterminated)
+                         ? 0 : s->headers + 1 - (last_hdr && s->unterminated ? 1 : 0);
+  uint64_t skip = s->skip;
+  if (skip == ~0ull) skip = R;
   s->R = R;
-  uint64_t skip = 0;
-  if (first) {
-    // the line that starts at `first` follows the newline at first - 1
-    uint64_t lo = 0, hi = s->m_nl;
-    while (lo < hi) {
-      const uint64_t mid = (lo + hi) / 2;
-      if (nl[mid] < first - 1) lo = mid + 1;
-      else hi = mid;
-    }
-    const uint64_t k0 = lo + 1;  // that line
-    skip = k0 < M ? H[k0] + 1 : R;
-  }
   s->skip = skip;
   const uint64_t after = R > skip ? R - skip : 0;
-  s->Rk = (n_limit && n_limit < after) ? n_limit : after;
+  s->Rk = (s->n_limit && s->n_limit < after) ? s->n_limit : after;
 }
 
-__global__ void k_records(const uint8_t *p, uint64_t n, const uint64_t *nl, uint64_t m_nl,
-                          uint64_t M, const uint32_t *hdr, const uint64_t *H,
-                          const ParseSummary *s, unsigned long long *rec_len,
-                          unsigned int *rec_nseg, uint64_t *rec_start) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (k == 0 || k >= M || hdr[k]) return;
-  uint64_t r = H[k];
-  const uint64_t skip = s->skip;
-  if (r < skip || r - skip >= s->Rk) return;
-  r -= skip;
-  uint64_t st, e;
-  line_range(k, nl, m_nl, n, st, e);
-  if (e == st) return;
-  atomicAdd(&rec_len[r], (unsigned long long)(e - st));
-  atomicAdd(&rec_nseg[r], 1u);
-  rec_start[r] = st;
+// One block: the newlines and headers before each block of k_nl_count (off[2 b]
+// and off[2 b + 1]) and the summary. first > 0: the bytes before `first`
+// (which follows a '\n') belong to records parsed before, so the records up
+// to the header that starts there are left out (s->skip: record 0 and those
+// whose header line starts before `first`). Latency-bound: a warp scans 512
+// counts from coalesced loads, all queued before the first is used, so up to
+// 1 GB of input takes one round.
+constexpr int kTopPer = 16;
+__global__ void __launch_bounds__(1024)
+    k_nl_top(const uint8_t *p, uint64_t n, const uint64_t *counts, uint64_t nblk, uint64_t first,
+             uint64_t n_limit, uint64_t *off, ParseSummary *s) {
+  __shared__ uint64_t tmp[33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint8_t last = threadIdx.x == 0 && n ? p[n - 1] : (uint8_t)'\n';
+  uint64_t before = 0;  // headers before the one at `first`
+  for (uint64_t q = threadIdx.x; q + 1 < first; q += blockDim.x)
+    before += p[q] == '\n' && p[q + 1] == '>' ? 1 : 0;
+  uint64_t nl = 0, hd = 0;
+  for (uint64_t b0 = 0; b0 < nblk; b0 += 1024 * kTopPer) {
+    // 16,384 blocks of at most 2^16 newlines: both sums fit 32 bits. The
+    // round's counts are spread over all warps, `per` rows of 32 each.
+    const uint64_t rows = (nblk - b0 + 1023) / 1024;
+    const int per = rows < kTopPer ? (int)rows : kTopPer;
+    const uint64_t i0 = b0 + (uint64_t)warp * 32 * per + lane;
+    uint64_t v[kTopPer], run = 0, tot;
+#pragma unroll
+    for (int k = 0; k < kTopPer; ++k)
+      v[k] = k < per && i0 + 32 * k < nblk ? counts[i0 + 32 * k] : 0;
+#pragma unroll
+    for (int k = 0; k < kTopPer; ++k) {
+      if (k >= per) break;
+      const uint64_t inc = warp_incl_scan(v[k]);
+      v[k] = run + inc - v[k];
+      run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    // the warps' sums, from lane 0 of each
+    const uint64_t ex = __shfl_sync(0xffffffffu, block_excl_scan<uint64_t>(lane ? 0 : run, tmp, tot), 0);
+#pragma unroll
+    for (int k = 0; k < kTopPer; ++k) {
+      const uint64_t x = ex + v[k];
+      if (k < per && i0 + 32 * k < nblk)
+        *reinterpret_cast<ulonglong2 *>(off + 2 * (i0 + 32 * k)) =
+            make_ulonglong2(nl + (x & 0xFFFFFFFFull), hd + (x >> 32));
+    }
+    nl += tot & 0xFFFFFFFFull;
+    hd += tot >> 32;
+  }
+  uint64_t tot = 0;
+  if (first) block_excl_scan<uint64_t>(before, tmp, tot);
+  if (threadIdx.x == 0) {
+    ParseSummary t{};
+    t.m_nl = nl;
+    t.headers = hd;
+    t.unterminated = last != '\n' ? 1u : 0u;
+    t.lines = nl + t.unterminated;
+    t.skip = !first ? 0 : first < n ? tot + 1 : ~0ull;
+    t.n_limit = n_limit;
+    if (nl == 0) count_records(&t, false);
+    *s = t;
+  }
 }
 
-__global__ void k_validate(const unsigned long long *rec_len, const unsigned int *rec_nseg,
-                           ParseSummary *s) {
-  uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (r >= s->Rk) return;
-  unsigned long long l = rec_len[r];
-  if (r == 0) s->len0 = l;
-  if (l != rec_len[0]) atomicOr(&s->unequal, 1u);
-  if (rec_nseg[r] > 1) atomicOr(&s->multi, 1u);
-  atomicMax(&s->max_len, l);
+// Writes the positions of every '\n' in increasing order, and (kHdr) for each
+// line k >= 1, which follows newline k - 1, the header lines before it and
+// whether it is one (lrec[k] = headers << 1 | flag), and the lines of the
+// headers (hline[0] = 0 and hline[h], h = 1, 2, ...): each warp starts at its
+// block's offsets plus the counts of the block's earlier warps; a span with
+// one or two newlines takes their offsets from the count pass, a span with
+// more scans its lanes' counts where some lane holds a newline. (A thread per
+// span, with the warp going through the spans of more than two newlines,
+// took 5 us instead of 17 on 598 MB of genomes, but leaves too few warps for
+// files of short lines: 0.45 ms instead of 0.25 for a 6 MB ingest.) The warp
+// that writes the last newline counts the records. Nothing is written when
+// there are more than `cap` newlines.
+template <bool kHdr>
+__global__ void __launch_bounds__(kNlThreads)
+    k_nl_write(const uint8_t *p, uint64_t n, const uint64_t *block_off, const uint32_t *warp_counts,
+               uint64_t cap, uint64_t *nl, uint64_t *lrec, uint64_t *hline, ParseSummary *s) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t wid = blockIdx.x * kNlWarps + warp;
+  // the block's spans, one a lane
+  uint32_t c = lane < kNlWarps ? warp_counts[blockIdx.x * kNlWarps + lane] : 0;
+  const uint32_t cw = __shfl_sync(0xffffffffu, c, warp), cn = cw & 0xFFFFu;
+  if (cn == 0) return;
+  const uint64_t m_nl = s->m_nl;
+  if (m_nl > cap) return;
+  const uint64_t wbase = blockIdx.x * kNlBlockBytes + warp * kNlWarpBytes;
+  if (lane >= warp) c = 0;
+  c = __reduce_add_sync(0xffffffffu, c);  // at most 7 x 8,192 newlines
+  uint64_t off = block_off[2 * blockIdx.x] + (c & 0xFFFFu);
+  uint64_t hoff = block_off[2 * blockIdx.x + 1] + (c >> 16);
+  auto put = [&](uint64_t j, uint64_t pos, uint64_t h, bool hdr) {
+    nl[j] = pos;
+    if (!kHdr) return;
+    lrec[j + 1] = h << 1 | (hdr ? 1u : 0u);
+    if (hdr) hline[h + 1] = j + 1;
+    if (j == 0) hline[0] = 0;
+    if (j + 1 == m_nl) count_records(s, hdr);
+  };
+  if (cn <= 2) {
+    const uint32_t *pos = warp_counts + gridDim.x * kNlWarps + 2ull * wid;
+    if (lane < (int)cn) {
+      const uint32_t a = pos[lane];
+      put(off + lane, wbase + (a >> 1), hoff + (lane == 1 ? pos[0] & 1u : 0u), a & 1u);
+    }
+    return;
+  }
+  for (int i0 = 0; i0 < kNlIters; i0 += kNlBatch) {
+    uint32_t ms[kNlBatch];
+#pragma unroll
+    for (int k = 0; k < kNlBatch; ++k)
+      ms[k] = nl_mask16(p, wbase + (i0 + k) * 512ull + lane * 16, n);
+#pragma unroll
+    for (int k = 0; k < kNlBatch; ++k) {
+      const uint64_t at = wbase + (i0 + k) * 512ull + lane * 16;
+      uint32_t m = ms[k];
+      if (!__any_sync(0xffffffffu, m != 0)) continue;
+      uint32_t hm = 0;  // the newlines a header follows
+      if (kHdr)
+        for (uint32_t t = m; t; t &= t - 1)
+          if (header_after(p, at + __ffs(t) - 1, n)) hm |= t & (0u - t);
+      const uint32_t cnt = __popc(m) | __popc(hm) << 16;
+      const uint32_t inc = warp_incl_scan(cnt);  // at most 512 each
+      uint64_t pos = off + ((inc - cnt) & 0xFFFFu), h = hoff + ((inc - cnt) >> 16);
+      for (; m; m &= m - 1) {
+        const bool hdr = hm & m & (0u - m);
+        put(pos++, at + __ffs(m) - 1, h, hdr);
+        h += hdr;
+      }
+      const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
+      off += all & 0xFFFFu;
+      hoff += all >> 16;
+    }
+  }
 }
 
-// Gather of multi-line records: masked line lengths, then line copies.
-__global__ void k_seqline_len(const uint64_t *nl, uint64_t m_nl, uint64_t n, uint64_t M,
-                              const uint32_t *hdr, const uint64_t *H, const ParseSummary *s,
-                              uint64_t *len) {
-  uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (k >= M) return;
-  uint64_t st, e;
-  line_range(k, nl, m_nl, n, st, e);
-  const uint64_t skip = s->skip;
-  len[k] = (k >= 1 && !hdr[k] && H[k] >= skip && H[k] - skip < s->Rk) ? e - st : 0;
+// The first line of a parse's lines [a, b) that is not empty, and the bytes of
+// all of them. The bytes up to the end of line k, line ends left out, only
+// grow with k: the first line that is not empty is found by bisection.
+struct LineSpan {
+  uint64_t start, len;  // of the first non-empty line (0 if none); of all lines
+  bool multi;           // several non-empty lines
+};
+__device__ inline uint64_t line_end(uint64_t k, const uint64_t *nl, uint64_t m_nl, uint64_t n) {
+  return k < m_nl ? nl[k] : n;
+}
+__device__ inline LineSpan record_span(uint64_t r, const uint64_t *nl, const uint64_t *hline,
+                                       uint64_t n, const ParseSummary *s) {
+  const uint64_t m_nl = s->m_nl;
+  const uint64_t a = hline[r] + 1, b = r < s->headers ? hline[r + 1] : s->lines;
+  if (a >= b) return {0, 0, false};
+  const uint64_t st = nl[a - 1] + 1;  // a >= 1
+  auto upto = [&](uint64_t k) { return line_end(k, nl, m_nl, n) - st - (k - a); };
+  const uint64_t len = upto(b - 1);
+  if (b - a == 1) return {len ? st : 0, len, false};
+  if (!len) return {0, 0, false};
+  uint64_t lo = a, hi = b - 1;
+  if (upto(a)) hi = a;
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) / 2;
+    if (upto(mid)) hi = mid;
+    else lo = mid + 1;
+  }
+  return {lo == a ? st : nl[lo - 1] + 1, len, upto(lo) != len};
 }
 
-__global__ void k_gather_lines(const uint8_t *p, const uint64_t *nl, uint64_t m_nl, uint64_t n,
-                               uint64_t M, const uint64_t *len, const uint64_t *dst_off,
-                               uint8_t *dst) {
-  uint64_t wid = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+// One thread per record: where it starts and its length, and in the summary
+// whether all lengths are equal, the largest one, and whether some record
+// spans several non-empty lines. The grid covers `cap` newlines.
+__global__ void __launch_bounds__(256)
+    k_records(const uint64_t *nl, const uint64_t *hline, uint64_t n, uint64_t cap, ParseSummary *s,
+              uint64_t *rec_len, uint64_t *rec_start) {
+  __shared__ uint64_t len0;
+  if (s->m_nl > cap) return;
+  const uint64_t Rk = s->Rk, skip = s->skip;
+  if (blockIdx.x * (uint64_t)blockDim.x >= Rk) return;  // block-uniform
+  const uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  LineSpan v{0, 0, false};
+  if (r < Rk) {
+    v = record_span(skip + r, nl, hline, n, s);
+    rec_len[r] = v.len;
+    rec_start[r] = v.start;
+  }
+  if (threadIdx.x == 0) {
+    len0 = blockIdx.x ? record_span(skip, nl, hline, n, s).len : v.len;
+    if (blockIdx.x == 0) {
+      s->len0 = v.len;
+      atomicMax(&s->max_len, (unsigned long long)v.len);
+    }
+  }
+  __syncthreads();
+  const bool differ = r < Rk && v.len != len0;
+  if (differ) atomicMax(&s->max_len, (unsigned long long)v.len);
+  const int unequal = __syncthreads_or(differ), multi = __syncthreads_or(v.multi);
+  if (threadIdx.x == 0) {
+    if (unequal) atomicOr(&s->unequal, 1u);
+    if (multi) atomicOr(&s->multi, 1u);
+  }
+}
+
+// Gather of multi-line records: a sequence line of a kept record r goes to its
+// place after the record's earlier lines, which start at dst_off[r - skip]. A
+// warp takes G neighbouring lines: the lanes find one line's place each, then
+// the warp copies line after line. G is about 2 KB of lines: the look-ups
+// are chains of four loads, which short lines share.
+__global__ void __launch_bounds__(256)
+    k_gather_lines(const uint8_t *p, const uint64_t *nl, const uint64_t *lrec,
+                   const uint64_t *hline, uint64_t n, const ParseSummary *s,
+                   const uint64_t *dst_off, uint8_t *dst, int G) {
+  const uint64_t wid = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
-  for (uint64_t k = wid; k < M; k += nwarps) {
-    uint64_t l = len[k];
-    if (!l) continue;
-    uint64_t st = k ? nl[k - 1] + 1 : 0;
-    for (uint64_t i = lane; i < l; i += 32) dst[dst_off[k] + i] = p[st + i];
+  const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+  const uint64_t M = s->lines, m_nl = s->m_nl, skip = s->skip, Rk = s->Rk;
+  for (uint64_t k0 = 1 + wid * G; k0 < M; k0 += nwarps * G) {
+    uint64_t st = 0, to = 0, l = 0;
+    const uint64_t k = k0 + lane;
+    if (lane < G && k < M) {
+      const uint64_t v = lrec[k], r = v >> 1;
+      if (!(v & 1) && r >= skip && r - skip < Rk) {
+        st = nl[k - 1] + 1;
+        l = line_end(k, nl, m_nl, n) - st;
+        const uint64_t a = hline[r] + 1;
+        to = dst_off[r - skip] + (st - (nl[a - 1] + 1) - (k - a));
+      }
+    }
+    for (int j = 0; j < G; ++j) {
+      const uint64_t lj = __shfl_sync(0xffffffffu, l, j);
+      const uint8_t *src = p + __shfl_sync(0xffffffffu, st, j);
+      uint8_t *out = dst + __shfl_sync(0xffffffffu, to, j);
+      uint64_t i = lane;
+      if (lj > 128) {
+        for (; i + 96 < lj; i += 128) {
+          const uint8_t b0 = src[i], b1 = src[i + 32], b2 = src[i + 64], b3 = src[i + 96];
+          out[i] = b0;
+          out[i + 32] = b1;
+          out[i + 64] = b2;
+          out[i + 96] = b3;
+        }
+      }
+      for (; i < lj; i += 32) out[i] = src[i];
+    }
   }
 }
 
@@ -272,83 +437,90 @@ static unsigned grid_for(uint64_t n, int threads) {
   return (unsigned)(g > 0x7fffffffull ? 0x7fffffffull : g);
 }
 
+namespace {
+// The scratch of a newline pass: [summary][offsets][counts][warp counts]
+struct NlScratch {
+  uint64_t nblk;
+  DevBuf buf;
+  ParseSummary *sum;
+  uint64_t *counts, *offs;
+  uint32_t *wcounts;
+  NlScratch(uint64_t nbytes, cudaStream_t st)
+      : nblk(ceil_div(nbytes ? nbytes : 1, kNlBlockBytes)),
+        buf(128 + nblk * (16 + 8 + 12 * kNlWarps), st) {
+    static_assert(sizeof(ParseSummary) <= 128, "summary");
+    uint8_t *b = buf.as<uint8_t>();
+    sum = reinterpret_cast<ParseSummary *>(b);
+    offs = reinterpret_cast<uint64_t *>(b + 128);
+    counts = offs + 2 * nblk;
+    wcounts = reinterpret_cast<uint32_t *>(counts + nblk);
+  }
+};
+// the summary, once every launch queued before has run
+ParseSummary summary_of(hd_ctx *ctx, const ParseSummary *d) {
+  ParseSummary *h = reinterpret_cast<ParseSummary *>(pinned_words(ctx));
+  HD_CUDA(cudaMemcpyAsync(h, d, sizeof(*h), cudaMemcpyDeviceToHost, ctx->stream));
+  HD_CUDA(cudaStreamSynchronize(ctx->stream));
+  return *h;
+}
+}  // namespace
+
 DevBuf newline_positions(hd_ctx *ctx, const uint8_t *d, uint64_t nbytes, uint64_t *m_nl) {
   cudaStream_t st = ctx->stream;
-  const uint64_t nblk = ceil_div(nbytes ? nbytes : 1, kNlBlockBytes);
-  DevBuf counts(nblk * 8, st), offs(nblk * 8, st), total(8, st), wcounts(nblk * 12 * (kNlThreads / 32), st);
-  k_nl_count<<<(unsigned)nblk, kNlThreads, 0, st>>>(d, nbytes, counts.as<uint64_t>(),
-                                                     wcounts.as<uint32_t>());
+  NlScratch sc(nbytes, st);
+  k_nl_count<false><<<(unsigned)sc.nblk, kNlThreads, 0, st>>>(d, nbytes, sc.counts, sc.wcounts);
   HD_LAUNCHED(ctx);
-  scan_exclusive<uint64_t>(ctx, counts.as<uint64_t>(), offs.as<uint64_t>(), nblk,
-                           total.as<uint64_t>());
-  uint64_t h = 0;
-  HD_CUDA(cudaMemcpyAsync(&h, total.p, 8, cudaMemcpyDeviceToHost, st));
-  HD_CUDA(cudaStreamSynchronize(st));
+  k_nl_top<<<1, 1024, 0, st>>>(d, nbytes, sc.counts, sc.nblk, 0, 0, sc.offs, sc.sum);
+  HD_LAUNCHED(ctx);
+  const uint64_t h = summary_of(ctx, sc.sum).m_nl;
   *m_nl = h;
   DevBuf nl((h + 1) * 8, st);
   if (h) {
-    k_nl_write<<<(unsigned)nblk, kNlThreads, 0, st>>>(d, nbytes, offs.as<uint64_t>(),
-                                                       wcounts.as<uint32_t>(), nl.as<uint64_t>());
+    k_nl_write<false><<<(unsigned)sc.nblk, kNlThreads, 0, st>>>(
+        d, nbytes, sc.offs, sc.wcounts, h, nl.as<uint64_t>(), nullptr, nullptr, sc.sum);
     HD_LAUNCHED(ctx);
   }
   return nl;
 }
 
+// Four launches and one wait: the tables of the lines and records are laid
+// out for one newline per 2 KB of input and 8,192 more, which holds records
+// of 4 KB and longer and every small file; an input with more newlines
+// repeats the last two launches, which wrote nothing, with tables of its size.
 Records parse_fasta(hd_ctx *ctx, const uint8_t *d_file, uint64_t nbytes, uint64_t n_limit,
                     uint64_t first) {
   cudaStream_t st = ctx->stream;
   Records rec;
-  uint64_t nblk = ceil_div(nbytes ? nbytes : 1, kNlBlockBytes);
-  DevBuf counts(nblk * 8, st), offs(nblk * 8, st), total(8, st), sumbuf(sizeof(ParseSummary), st);
-  DevBuf wcounts(nblk * 12 * (kNlThreads / 32), st);
-  ParseSummary *d_sum = sumbuf.as<ParseSummary>();
-  HD_CUDA(cudaMemsetAsync(d_sum, 0, sizeof(ParseSummary), st));
-  k_nl_count<<<(unsigned)nblk, kNlThreads, 0, st>>>(d_file, nbytes, counts.as<uint64_t>(),
-                                                     wcounts.as<uint32_t>());
+  NlScratch sc(nbytes, st);
+  k_nl_count<true><<<(unsigned)sc.nblk, kNlThreads, 0, st>>>(d_file, nbytes, sc.counts, sc.wcounts);
   HD_LAUNCHED(ctx);
-  scan_exclusive<uint64_t>(ctx, counts.as<uint64_t>(), offs.as<uint64_t>(), nblk,
-                           total.as<uint64_t>());
-  k_nl_summary<<<1, 1, 0, st>>>(d_file, nbytes, total.as<uint64_t>(), d_sum);
+  k_nl_top<<<1, 1024, 0, st>>>(d_file, nbytes, sc.counts, sc.nblk, first, n_limit, sc.offs, sc.sum);
   HD_LAUNCHED(ctx);
+  DevBuf tab;
+  uint64_t *nl = nullptr, *lrec = nullptr, *hline = nullptr;
   ParseSummary hs;
-  HD_CUDA(cudaMemcpyAsync(&hs, d_sum, sizeof(hs), cudaMemcpyDeviceToHost, st));
-  HD_CUDA(cudaStreamSynchronize(st));
-  const uint64_t m_nl = hs.m_nl, M = hs.lines;
-  DevBuf nl((m_nl + 1) * 8, st);
-  if (m_nl) {
-    k_nl_write<<<(unsigned)nblk, kNlThreads, 0, st>>>(d_file, nbytes, offs.as<uint64_t>(),
-                                                       wcounts.as<uint32_t>(), nl.as<uint64_t>());
+  uint64_t cap = std::min(nbytes, nbytes / 2048 + 8192);
+  for (bool again = false;; again = true) {
+    // newlines [0, cap), lines [0, cap + 1), headers [0, cap]; the sizes vary
+    // with the input: none of the large blocks kept for rows and results
+    tab = DevBuf((3 * cap + 5) * 8, st, true);
+    nl = tab.as<uint64_t>();
+    lrec = nl + cap + 1;
+    hline = lrec + cap + 2;
+    rec.rec_len = DevBuf((cap + 1) * 8, st, true);  // records <= newlines + 1
+    rec.rec_start = DevBuf((cap + 1) * 8, st, true);
+    k_nl_write<true><<<(unsigned)sc.nblk, kNlThreads, 0, st>>>(d_file, nbytes, sc.offs, sc.wcounts,
+                                                               cap, nl, lrec, hline, sc.sum);
     HD_LAUNCHED(ctx);
+    k_records<<<grid_for(cap + 1, 256), 256, 0, st>>>(nl, hline, nbytes, cap, sc.sum,
+                                                      rec.rec_len.as<uint64_t>(),
+                                                      rec.rec_start.as<uint64_t>());
+    HD_LAUNCHED(ctx);
+    hs = summary_of(ctx, sc.sum);
+    if (hs.m_nl <= cap) break;
+    if (again) fail(HD_ERR_CUDA, "newline counts changed between two passes");
+    cap = hs.m_nl;
   }
-  DevBuf hdr((M + 1) * 4, st), H((M + 1) * 8, st), htot(8, st);
-  HD_CUDA(cudaMemsetAsync(htot.p, 0, 8, st));
-  if (M) {
-    k_lines<<<grid_for(M, 256), 256, 0, st>>>(d_file, nbytes, nl.as<uint64_t>(), m_nl, M,
-                                              hdr.as<uint32_t>());
-    HD_LAUNCHED(ctx);
-    scan_exclusive<uint32_t>(ctx, hdr.as<uint32_t>(), H.as<uint64_t>(), M, htot.as<uint64_t>());
-  }
-  k_rec_count<<<1, 1, 0, st>>>(htot.as<uint64_t>(), hdr.as<uint32_t>(), H.as<uint64_t>(),
-                               nl.as<uint64_t>(), first, n_limit, d_sum);
-  HD_LAUNCHED(ctx);
-  const uint64_t cap = M + 1;  // records <= lines
-  rec.rec_len = DevBuf(cap * 8, st);
-  rec.rec_start = DevBuf(cap * 8, st);
-  DevBuf nseg(cap * 4, st);
-  HD_CUDA(cudaMemsetAsync(rec.rec_len.p, 0, cap * 8, st));
-  HD_CUDA(cudaMemsetAsync(rec.rec_start.p, 0, cap * 8, st));
-  HD_CUDA(cudaMemsetAsync(nseg.p, 0, cap * 4, st));
-  if (M) {
-    k_records<<<grid_for(M, 256), 256, 0, st>>>(
-        d_file, nbytes, nl.as<uint64_t>(), m_nl, M, hdr.as<uint32_t>(), H.as<uint64_t>(), d_sum,
-        rec.rec_len.as<unsigned long long>(), nseg.as<unsigned int>(), rec.rec_start.as<uint64_t>());
-    HD_LAUNCHED(ctx);
-    k_validate<<<grid_for(cap, 256), 256, 0, st>>>(rec.rec_len.as<unsigned long long>(),
-                                                   nseg.as<unsigned int>(), d_sum);
-    HD_LAUNCHED(ctx);
-  }
-  HD_CUDA(cudaMemcpyAsync(&hs, d_sum, sizeof(hs), cudaMemcpyDeviceToHost, st));
-  HD_CUDA(cudaStreamSynchronize(st));
   rec.n = hs.Rk;
   rec.len0 = hs.len0;
   rec.max_len = hs.max_len;
@@ -357,24 +529,20 @@ Records parse_fasta(hd_ctx *ctx, const uint8_t *d_file, uint64_t nbytes, uint64_
   rec.bytes = nbytes;
   if (hs.multi) {
     // records spanning several lines: concatenate them into one buffer
-    DevBuf len(M * 8, st), dst(M * 8, st), gtot(8, st);
-    k_seqline_len<<<grid_for(M, 256), 256, 0, st>>>(nl.as<uint64_t>(), m_nl, nbytes, M,
-                                                    hdr.as<uint32_t>(), H.as<uint64_t>(), d_sum,
-                                                    len.as<uint64_t>());
-    HD_LAUNCHED(ctx);
-    scan_exclusive<uint64_t>(ctx, len.as<uint64_t>(), dst.as<uint64_t>(), M, gtot.as<uint64_t>());
-    uint64_t total_bytes = 0;
-    HD_CUDA(cudaMemcpyAsync(&total_bytes, gtot.p, 8, cudaMemcpyDeviceToHost, st));
+    DevBuf gtot(8, st);
+    scan_exclusive<uint64_t>(ctx, rec.rec_len.as<uint64_t>(), rec.rec_start.as<uint64_t>(), rec.n,
+                             gtot.as<uint64_t>());
+    uint64_t *total = pinned_words(ctx);
+    HD_CUDA(cudaMemcpyAsync(total, gtot.p, 8, cudaMemcpyDeviceToHost, st));
     HD_CUDA(cudaStreamSynchronize(st));
+    const uint64_t total_bytes = *total;
     rec.gathered = DevBuf(total_bytes + 16, st);
-    k_gather_lines<<<grid_for(M * 32, 256), 256, 0, st>>>(d_file, nl.as<uint64_t>(), m_nl, nbytes,
-                                                          M, len.as<uint64_t>(),
-                                                          dst.as<uint64_t>(),
-                                                          rec.gathered.as<uint8_t>());
+    const uint64_t avg = total_bytes / hs.lines + 1;
+    const int G = (int)std::min<uint64_t>(32, 2048 / avg + 1);
+    k_gather_lines<<<grid_for(ceil_div(hs.lines, (uint64_t)G) * 32, 256), 256, 0, st>>>(
+        d_file, nl, lrec, hline, nbytes, sc.sum, rec.rec_start.as<uint64_t>(),
+        rec.gathered.as<uint8_t>(), G);
     HD_LAUNCHED(ctx);
-    if (rec.n)
-      scan_exclusive<uint64_t>(ctx, rec.rec_len.as<uint64_t>(), rec.rec_start.as<uint64_t>(),
-                               rec.n, gtot.as<uint64_t>());
     rec.base = rec.gathered.as<uint8_t>();
     rec.bytes = total_bytes;
   }

@@ -179,6 +179,8 @@ struct hd_ctx {
   // (K pieces of split tiles; grow, at most about 45 MB each): launches on one
   // stream follow one another. A plan that is replayed from a graph has its own.
   hd::DevBuf mma_ws[2];
+  // pinned words that small results are copied to (pinned_words)
+  uint64_t *words = nullptr;
   hd::Trace trace;
 };
 
@@ -191,6 +193,10 @@ namespace hd {
 // copy it last staged has run), so the copy is queued like a launch. Larger
 // tables go from pageable memory.
 void upload_table(hd_ctx *ctx, void *d_dst, const void *host, size_t bytes, cudaStream_t s);
+
+// 32 pinned words of the context for the next small device-to-host copy on
+// ctx->stream, which the caller waits for before it queues another
+uint64_t *pinned_words(hd_ctx *ctx);
 
 // tensor-core multiply-adds counted by the planning kernels (a 64-bit counter
 // in the context's status block, after the status word)
