@@ -33,6 +33,7 @@ SIGNATURES = {
     "hd_alignment_from_fasta": (ci, [vp, vp, u64, ci, ci, u64, ci, ci, P(vp)]),
     "hd_alignment_from_fasta_file": (ci, [vp, cp, ci, u64, ci, ci, P(vp)]),
     "hd_pairwise_lt_fasta_file": (ci, [vp, cp, ci, ci, i64, vp, vp, P(vp)]),
+    "hd_expect_pairwise": (ci, [vp]),
     "hd_alignment_from_sequences": (ci, [vp, vp, vp, u64, ci, ci, P(vp)]),
     "hd_alignment_info": (ci, [vp, P(u64), P(u64), P(u64), P(ci)]),
     "hd_alignment_sequence_indices": (ci, [vp, vp]),
@@ -202,6 +203,10 @@ class Context:
 
     def synchronize(self):
         self._check(lib().hd_ctx_synchronize(self.h))
+
+    def expect_pairwise(self) -> None:
+        """The next alignment built is compared whole (hd_expect_pairwise)."""
+        self._check(lib().hd_expect_pairwise(self.h))
 
     def alignment_from_fasta(self, data, nbytes=None, on_device=False, remove_duplicates=False,
                              n=0, include_x=False, semantics=SEM_GPU) -> Alignment:

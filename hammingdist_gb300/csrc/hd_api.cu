@@ -691,8 +691,9 @@ uint64_t words_for(uint64_t L) { return hd::round_up(hd::ceil_div(L ? L : 1, 32)
 
 // validate_data (src/hamming_impl.cc:80-91) + the include_x/use_gpu check
 // (include/hamming/hamming_impl.hh:99-102) + dedupe + rule choice + pack.
+// compared: the alignment's distances are wanted next
 hd_alignment *build_alignment(hd_ctx *ctx, hd::Records &rec, int remove_duplicates, int include_x,
-                              int semantics) {
+                              int semantics, bool compared) {
   if (rec.n == 0 || rec.len0 == 0) fail(HD_ERR_EMPTY, kMsgEmpty);
   if (!rec.all_equal) fail(HD_ERR_LENGTH, kMsgLength);
   if (semantics == HD_SEM_GPU && include_x) fail(HD_ERR_INCLUDE_X_GPU, kMsgIncludeX);
@@ -732,7 +733,7 @@ hd_alignment *build_alignment(hd_ctx *ctx, hd::Records &rec, int remove_duplicat
     aln->rule = rule;
     aln->planes = hd::planes_of(rule);
     aln->groups = aln->planes > 4 ? 2 : 1;
-    hd::pack_rows(ctx, rec, d_rows, aln);
+    hd::pack_rows(ctx, rec, d_rows, aln, compared);
     if (!aln->seqidx.empty()) {
       aln->d_seqidx = DevBuf(aln->seqidx.size() * 8, ctx->stream);
       HD_CUDA(cudaMemcpyAsync(aln->d_seqidx.p, aln->seqidx.data(), aln->seqidx.size() * 8,
@@ -1059,18 +1060,25 @@ int hd_ctx_synchronize(hd_ctx *ctx) {
   return guard(ctx, [&] { HD_CUDA(cudaStreamSynchronize(ctx->stream)); });
 }
 
+int hd_expect_pairwise(hd_ctx *ctx) {
+  if (!ctx) return HD_ERR_ARG;
+  ctx->expect_pairwise = true;
+  return HD_OK;
+}
+
 int hd_alignment_from_fasta(hd_ctx *ctx, const char *fasta, uint64_t nbytes, int fasta_on_device,
                             int remove_duplicates, uint64_t n_limit, int include_x, int semantics,
                             hd_alignment **out) {
   if (!ctx || !out || (!fasta && nbytes)) return HD_ERR_ARG;
   *out = nullptr;
+  const bool compared = std::exchange(ctx->expect_pairwise, false);
   return guard(ctx, [&] {
     hd::trace_begin(ctx, "hd_alignment_from_fasta");
     const uint8_t *d = stage_input(ctx, fasta, nbytes, fasta_on_device);
     hd::trace_mark(ctx, "upload");
     hd::Records rec = hd::parse_fasta(ctx, d, nbytes, n_limit);
     hd::trace_mark(ctx, "parse");
-    *out = build_alignment(ctx, rec, remove_duplicates, include_x, semantics);
+    *out = build_alignment(ctx, rec, remove_duplicates, include_x, semantics, compared);
     hd::trace_end(ctx);
   });
 }
@@ -1080,6 +1088,7 @@ int hd_alignment_from_fasta_file(hd_ctx *ctx, const char *path, int remove_dupli
                                  hd_alignment **out) {
   if (!ctx || !out || !path) return HD_ERR_ARG;
   *out = nullptr;
+  const bool compared = std::exchange(ctx->expect_pairwise, false);
   return guard(ctx, [&] {
     hd::trace_begin(ctx, "hd_alignment_from_fasta_file");
     uint64_t nbytes = 0;
@@ -1088,7 +1097,7 @@ int hd_alignment_from_fasta_file(hd_ctx *ctx, const char *path, int remove_dupli
     hd::trace_mark(ctx, "read + upload");
     hd::Records &rec = file_records(ctx, d, nbytes, n_limit);
     hd::trace_mark(ctx, "parse");
-    *out = build_alignment(ctx, rec, remove_duplicates, include_x, semantics);
+    *out = build_alignment(ctx, rec, remove_duplicates, include_x, semantics, compared);
     hd::trace_end(ctx);
   });
 }
@@ -1115,7 +1124,7 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
       hd::trace_mark(ctx, "read + upload");
       hd::Records &rec = file_records(ctx, d, nbytes, 0);
       hd::trace_mark(ctx, "parse");
-      a = build_alignment(ctx, rec, remove_duplicates, 0, HD_SEM_GPU);
+      a = build_alignment(ctx, rec, remove_duplicates, 0, HD_SEM_GPU, true);
       std::unique_ptr<hd_alignment> own(a);
       const uint64_t entries = a->n_rows < 2 ? 0 : tri(a->n_rows);
       void *host = out_fn(user, 0, a->n_rows, entries);
@@ -1407,10 +1416,15 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
           if (!hd::tile_config_valid(cfg.tile, cfg.stages)) cfg.stages = 3;
         }
       }
-      hd::pack_rows_and(ctx, all, rows + K, Kc - K, L, words, g0 + K * words,
-                        keep_planes.as<uint4>() + K * words);
+      // the new rows' planes and their tensor-core operand, before the
+      // launches of any stream read them
+      const bool with_op = use_mma && Kc >= 2 &&
+                           hd::pack_operand(ctx, all, rows + K, owner.get(), K, Kc,
+                                            keep_planes.as<uint4>(), ctx->stream, R_max);
+      if (!with_op)
+        hd::pack_rows_and(ctx, all, rows + K, Kc - K, L, words, g0 + K * words,
+                          keep_planes.as<uint4>() + K * words);
       hd::trace_host(ctx, "part " + std::to_string(c + 1) + " packing queued");
-      // the new rows' tensor-core operand, before the launches of any stream read it
       if (use_mma && Kc >= 2 && !hd::ensure_operand(ctx, owner.get(), Kc, ctx->stream, R_max)) {
         use_mma = false;
         T = (uint32_t)cfg.tile;
@@ -1542,11 +1556,12 @@ int hd_alignment_from_sequences(hd_ctx *ctx, const char *bytes, const uint64_t *
                                 int include_x, int semantics, hd_alignment **out) {
   if (!ctx || !out || (n && !offsets)) return HD_ERR_ARG;
   *out = nullptr;
+  const bool compared = std::exchange(ctx->expect_pairwise, false);
   return guard(ctx, [&] {
     const uint64_t nbytes = n ? offsets[n] - offsets[0] : 0;
     const uint8_t *d = stage_input(ctx, bytes ? bytes + (n ? offsets[0] : 0) : bytes, nbytes, 0);
     hd::Records rec = hd::records_from_offsets(ctx, d, offsets, n);
-    *out = build_alignment(ctx, rec, 0, include_x, semantics);
+    *out = build_alignment(ctx, rec, 0, include_x, semantics, compared);
   });
 }
 
@@ -1594,7 +1609,7 @@ int hd_pairwise_lt(hd_ctx *ctx, const hd_alignment *aln, int dtype_bytes, int64_
     // the tensor-core engine's operand and the launch plan (item lists,
     // tensor maps, job tables) first, so that the timing below is the
     // distance kernel's alone
-    if (!aln->base && hd::mma_eligible(aln) && hd::ensure_operand(ctx, aln, n, ctx->stream))
+    if (!aln->base && hd::mma_wanted(ctx, aln) && hd::ensure_operand(ctx, aln, n, ctx->stream))
       hd::trace_mark(ctx, "FP4 operand");
     hd::PairLaunchPlan plan;
     hd::plan_pairwise_tiles(ctx, aln, dtype_bytes, md, d_out, 0, 0, nb, &plan);
@@ -2441,6 +2456,7 @@ int hd_pairwise_lt_files(hd_ctx *ctx, uint64_t count, const char *const *paths,
         }
         hd_alignment *a = nullptr;
         int r;
+        hd_expect_pairwise(w);
         if (mapped) {  // from the device arena, after the file's copy
           r = cudaStreamWaitEvent(w->stream, ctx->part_ev[i], 0) == cudaSuccess ? HD_OK : HD_ERR_CUDA;
           if (r == HD_OK)

@@ -586,16 +586,6 @@ __device__ inline uint64_t mix64(uint64_t x) {
 constexpr unsigned long long kEmpty = ~0ull;
 constexpr int kHashU = 2;     // 512-byte blocks per warp per step of k_hash and k_tab_cmp
 
-// 16 bytes at the 16-byte aligned address x, bytes outside the readable
-// range [lo, hi) read as 0 (byte loads only at the ends of the range).
-__device__ inline uint4 load16_in(uint64_t x, uint64_t lo, uint64_t hi) {
-  if (x >= lo && x + 16 <= hi) return *reinterpret_cast<const uint4 *>(x);
-  uint32_t w[4] = {0u, 0u, 0u, 0u};
-  for (int k = 0; k < 16; ++k)
-    if (x + k >= lo && x + k < hi)
-      w[k >> 2] |= (uint32_t)*reinterpret_cast<const uint8_t *>(x + k) << (8 * (k & 3));
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
 __device__ inline uint32_t load4_in(uint64_t x, uint64_t lo, uint64_t hi) {
   if (x >= lo && x + 4 <= hi) return *reinterpret_cast<const uint32_t *>(x);
   uint32_t w = 0;
@@ -1289,7 +1279,8 @@ Records concat_records(hd_ctx *ctx, const Records &a, const Records &b, uint64_t
   return r;
 }
 
-void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_alignment *aln) {
+void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_alignment *aln,
+               bool compared) {
   Table256 t;
   int table = aln->rule == HD_RULE_AND ? kCodesAnd
               : aln->rule == HD_RULE_SPARSE ? kCodesSparse : kCodesSparseX;
@@ -1298,6 +1289,9 @@ void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_align
   aln->plane_buf[0] = DevBuf(bytes ? bytes : 16, ctx->stream);
   if (aln->groups > 1) aln->plane_buf[1] = DevBuf(bytes ? bytes : 16, ctx->stream);
   if (!aln->n_rows) return;
+  if (compared && aln->planes == 4 && mma_wanted(ctx, aln) &&
+      pack_operand(ctx, rec, d_rows, aln, 0, aln->n_rows, nullptr, ctx->stream))
+    return;
   const uint64_t jobs = aln->n_rows * hd::ceil_div((aln->words + 31) / 32, (uint64_t)kPackCPG);
   unsigned grid = grid_for(jobs * 32, kPackThreads);
   uint4 *g0 = aln->plane_buf[0].as<uint4>(), *g1 = aln->plane_buf[1].as<uint4>();
@@ -1322,7 +1316,6 @@ void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_align
 // other byte 0. The six symbols differ in their low three bits (X 0, A 1,
 // C 3, T 4, '-' 5, G 7), which pick each byte's code from code_lo:code_hi
 // and the symbol it must equal from a second table (both with __byte_perm).
-constexpr uint32_t kSymLo = 0x43004158u, kSymHi = 0x47002D54u;  // X A . C / T - . G
 __device__ __forceinline__ uint32_t site_codes(uint32_t w, uint32_t code_lo, uint32_t code_hi) {
   const uint32_t sel =
       (w & 0x7u) | ((w >> 4) & 0x70u) | ((w >> 8) & 0x700u) | ((w >> 12) & 0x7000u);

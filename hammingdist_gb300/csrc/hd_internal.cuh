@@ -179,6 +179,8 @@ struct hd_ctx {
   // (K pieces of split tiles; grow, at most about 45 MB each): launches on one
   // stream follow one another. A plan that is replayed from a graph has its own.
   hd::DevBuf mma_ws[2];
+  // the next alignment built is compared whole (hd_expect_pairwise)
+  bool expect_pairwise = false;
   // pinned words that small results are copied to (pinned_words)
   uint64_t *words = nullptr;
   hd::Trace trace;
@@ -226,8 +228,9 @@ struct hd_alignment {
   // alignment
   mutable hd::DevBuf op;
   mutable uint64_t op_rows = 0, op_cap = 0;
-  // per 288-site chunk of the operand (uint32 each): nonzero once an
-  // expanded row has a '-' in it (the chunks whose dash products count)
+  // per 192-site chunk of the operand (uint32 each): 0, or the extension of
+  // the operand (1, 2, ...) whose rows had the chunk's first '-' (the chunks
+  // whose dash products count, and whose dash blocks are written)
   mutable hd::DevBuf op_dash;
   // the marked chunks' list and ranks after each extension of the operand,
   // the last one current
@@ -360,6 +363,17 @@ void scan_exclusive(hd_ctx *ctx, const In *in, uint64_t *out, uint64_t n, uint64
   HD_LAUNCHED(ctx);
 }
 
+// 16 bytes at the 16-byte aligned address x, bytes outside the readable
+// range [lo, hi) read as 0 (byte loads only at the ends of the range).
+__device__ inline uint4 load16_in(uint64_t x, uint64_t lo, uint64_t hi) {
+  if (x >= lo && x + 16 <= hi) return *reinterpret_cast<const uint4 *>(x);
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+  for (int k = 0; k < 16; ++k)
+    if (x + k >= lo && x + k < hi)
+      w[k >> 2] |= (uint32_t)*reinterpret_cast<const uint8_t *>(x + k) << (8 * (k & 3));
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // ------------------------------------------------------- PTX helpers
 __device__ inline uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -438,6 +452,9 @@ struct Records {
 };
 
 // Character codes of the rules (bit p = bit plane p); '-' is all ones.
+// The six symbols of the rules differ in their low three bits (X 0, A 1, C 3,
+// T 4, '-' 5, G 7): the symbol a byte must equal, by those bits.
+constexpr uint32_t kSymLo = 0x43004158u, kSymHi = 0x47002D54u;  // X A . C / T - . G
 enum CodeTable { kCodesAnd = 0, kCodesSparse = 1, kCodesSparseX = 2, kNumCodeTables = 3 };
 void code_table(int table, uint8_t out[256]);
 inline int planes_of(int rule) { return rule == HD_RULE_AND ? 4 : rule == HD_RULE_SPARSE ? 5 : 6; }
@@ -475,7 +492,10 @@ struct IncDedupe {
 uint64_t consensus_matches(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows,
                            uint64_t n_rows);
 // Packs rows (record ids d_rows, or identity if null) into bit planes.
-void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_alignment *aln);
+// `compared`: the alignment's distances are wanted next, so the rows'
+// tensor-core operand is written along with the planes if they will use it
+void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_alignment *aln,
+               bool compared);
 // AND-rule planes of n_rows records (d_rows: record indices) into g0, and
 // into g1 too unless it is null (n_rows x words uint4 each, already allocated)
 void pack_rows_and(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, uint64_t n_rows,
@@ -575,6 +595,15 @@ bool mma_eligible(const hd_alignment *aln);
 // operand cannot be allocated
 bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStream_t stream,
                 uint64_t cap_hint = 0);
+// whether the distances of the whole alignment run on the tensor-core engine
+bool mma_wanted(hd_ctx *ctx, const hd_alignment *aln);
+// packs records d_rows[0 ..] (none: 0 ..) of the AND rule into rows [lo, hi) of
+// the alignment's planes (and of `copy`, if given) and of its operand, whose
+// earlier rows are there (op_rows == lo), in one pass over their text. False
+// (nothing is packed) if the operand cannot be allocated.
+bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const hd_alignment *aln,
+                  uint64_t lo, uint64_t hi, uint4 *copy, cudaStream_t stream,
+                  uint64_t cap_hint = 0);
 // bytes of that operand for `rows` rows of `sites` sites
 uint64_t mma_operand_bytes(uint32_t planes, uint64_t sites, uint64_t rows);
 // tile rows [tile_lo, tile_hi) (128 rows each) x all earlier columns into

@@ -215,16 +215,17 @@ __device__ __forceinline__ void put16(uint8_t *dst, uint32_t w, uint32_t v) {
 }
 
 // Rows [row_lo, row_hi) of a P-plane alignment (P = 4: the AND rule; 5, 6:
-// the sparse rules, planes 4-5 in the second group) -> E2M1 operand rows.
-// One thread per (row, 32-site word): 16 or 32 bytes read, 16 bytes written
-// per block. A warp takes one row group x 4 words, lane l row l % 8, so that
-// each of its stores fills whole 128-byte core matrices; a block of 256
-// threads takes 32 words. The words past the alignment's, up to whole chunks,
-// are written as 0. The dash is the AND of the P planes ('-' has every plane);
-// a chunk where some row has a '-' is marked in dash_chunk.
+// the sparse rules, planes 4-5 in the second group) -> the plane blocks of
+// their E2M1 operand rows. One thread per (row, 32-site word): 16 or 32 bytes
+// read, 16 bytes written per block. A warp takes one row group x 4 words, lane
+// l row l % 8, so that each of its stores fills whole 128-byte core matrices;
+// a block of 256 threads takes 32 words. The words past the alignment's, up to
+// whole chunks, are written as 0. The dash is the AND of the P planes ('-' has
+// every plane); a chunk where some row has its first '-' is marked with `ext`.
 __global__ void k_expand_op(const uint4 *__restrict__ g0, const uint4 *__restrict__ g1,
                             uint32_t planes, uint32_t words, uint64_t row_lo, uint64_t row_hi,
-                            uint64_t L, uint8_t *__restrict__ x, uint32_t *dash_chunk) {
+                            uint64_t L, uint8_t *__restrict__ x, uint32_t *dash_chunk,
+                            uint32_t ext) {
   const uint32_t nb = op_blocks(planes), chunks = op_chunks(L);
   const uint32_t w = blockIdx.x * 32 + threadIdx.x / 8;
   if (w >= chunks * kChunkWords) return;
@@ -252,11 +253,197 @@ __global__ void k_expand_op(const uint4 *__restrict__ g0, const uint4 *__restric
     put16(blk + 3 * kGroupBytes, p.w & valid, kE2M1One);
     if (planes > 4) put16(blk + 4 * kGroupBytes, p1.x & valid, kE2M1One);
     if (planes > 5) put16(blk + 5 * kGroupBytes, p1.y & valid, kE2M1One);
-    put16(blk + planes * kGroupBytes, dash, kE2M1One);                // 1.0: the row side
-    put16(blk + (planes + 1) * kGroupBytes, dash, dash_neg(planes));  // the column side
-    if (planes == 6) put16(blk + (planes + 2) * kGroupBytes, dash, kE2M1Neg1);
-    // the chunk holds a '-': its dash products count (every writer stores 1)
-    if (dash && !dash_chunk[c]) dash_chunk[c] = 1u;
+    if (dash && !dash_chunk[c]) dash_chunk[c] = ext;  // every writer stores the same
+  }
+}
+
+// The dash blocks of the marked chunks (list[0 .. *n)): of rows [row_lo,
+// row_hi), and for a chunk that extension `ext` marked first of the rows
+// before them, which have no '-' there. The other chunks' blocks are never
+// read, and stay unwritten: two of an operand's six blocks (four planes),
+// 0.4 of 1.3 GB for 14,000 rows of 29,903 sites. A thread per (row, word):
+// 48 threads take one row group of a chunk.
+constexpr uint32_t kDashGroups = 4;  // row groups per block
+__global__ void __launch_bounds__(kDashGroups * 8 * kChunkWords)
+    k_dash_blocks(const uint4 *__restrict__ g0, const uint4 *__restrict__ g1, uint32_t planes,
+                  uint32_t words, uint64_t row_lo, uint64_t row_hi, uint64_t L,
+                  uint8_t *__restrict__ x, const uint32_t *__restrict__ marks, uint32_t ext,
+                  const uint32_t *__restrict__ list, const uint32_t *__restrict__ n) {
+  const uint32_t sub = threadIdx.x / (8 * kChunkWords), u = threadIdx.x % (8 * kChunkWords);
+  const uint32_t nb = op_blocks(planes);
+  const uint64_t group_bytes = op_group_bytes(planes, L);
+  const uint64_t batches = ((row_hi + 7) / 8 + kDashGroups - 1) / kDashGroups;
+  const uint64_t jobs = batches * *n;
+  for (uint64_t job = blockIdx.x; job < jobs; job += gridDim.x) {
+    const uint64_t i = job / batches, g = (job - i * batches) * kDashGroups + sub;
+    const uint32_t c = list[i], w = c * kChunkWords + u / 8;
+    const uint64_t r = g * 8 + (u & 7u), s0 = (uint64_t)w * 32;
+    if (r >= row_hi || (r < row_lo && marks[c] != ext)) continue;
+    uint32_t dash = s0 >= L ? 0u : (L - s0 >= 32 ? 0xffffffffu : ((1u << (L - s0)) - 1u));
+    if (w < words) {
+      const uint4 p = g0[r * words + w];
+      dash &= p.x & p.y & p.z & p.w;
+      if (planes > 4) {
+        const uint4 p1 = g1[r * words + w];
+        dash &= p1.x;
+        if (planes > 5) dash &= p1.y;
+      }
+    }
+    uint8_t *blk = x + g * group_bytes + ((uint64_t)c * nb + planes) * kGroupBytes + u * 16u;
+    put16(blk, dash, kE2M1One);                       // 1.0: the row side
+    put16(blk + kGroupBytes, dash, dash_neg(planes));  // the column side
+    if (planes == 6) put16(blk + 2 * kGroupBytes, dash, kE2M1Neg1);
+  }
+}
+
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+// The AND rule's codes of 8 sites (bytes of w0 and w1, in order: A 1, C 2, G 4,
+// T 8, '-' 15, any other byte 0), one a byte, to c0 and c1. The low three bits
+// of a byte pick its symbol and the symbol's code; a byte unlike its symbol
+// has code 0 (0x80 of `ne`, spread over the byte).
+__device__ __forceinline__ void and_codes(uint32_t w0, uint32_t w1, uint32_t &c0, uint32_t &c1) {
+  constexpr uint32_t kCodeLo = 0x02000100u, kCodeHi = 0x04000F08u;  // X A . C / T - . G
+  uint32_t a = w0 & 0x07070707u, b = w1 & 0x07070707u;
+  a |= a >> 4;
+  b |= b >> 4;
+  const uint32_t sel = prmt(a, b, 0x6420u), sel1 = sel >> 16;  // a nibble a site
+  const uint32_t x0 = w0 ^ prmt(kSymLo, kSymHi, sel), x1 = w1 ^ prmt(kSymLo, kSymHi, sel1);
+  const uint32_t ne0 = ((x0 & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x0;
+  const uint32_t ne1 = ((x1 & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x1;
+  c0 = prmt(kCodeLo, kCodeHi, sel) & ~prmt(ne0, 0u, 0xBA98u);
+  c1 = prmt(kCodeLo, kCodeHi, sel1) & ~prmt(ne1, 0u, 0xBA98u);
+}
+
+// 32 sites, the bytes of v[0 .. 8] from bit db on -> their codes as nibbles z in
+// site order, 8 sites a word, and the plane words pl. kTail: the sites from
+// `valid` on are past L, '-' in the planes and 0 in z.
+template <bool kTail>
+__device__ __forceinline__ void pack_sites(const uint32_t *v, uint32_t db, uint32_t valid,
+                                           uint32_t *z, uint32_t *pl) {
+  uint32_t t[4];  // byte p: plane p's bits of 8 sites
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    uint32_t c0, c1;
+    and_codes(__funnelshift_r(v[2 * m], v[2 * m + 1], db),
+              __funnelshift_r(v[2 * m + 1], v[2 * m + 2], db), c0, c1);
+    const uint32_t k = valid > 8u * m ? valid - 8u * m : 0u;  // sites of these 8 and after
+    if (kTail && k < 8u) {
+      const uint32_t m0 = k >= 4u ? 0xFFFFFFFFu : (1u << (8u * k)) - 1u;
+      const uint32_t m1 = k <= 4u ? 0u : (1u << (8u * (k - 4u))) - 1u;
+      c0 = (c0 & m0) | (0x0F0F0F0Fu & ~m0);
+      c1 = (c1 & m1) | (0x0F0F0F0Fu & ~m1);
+    }
+    uint32_t y = c0 + (c1 << 4);  // bit 8 (s mod 4) + 4 (s / 4) + p
+    uint32_t q = (y ^ (y >> 14)) & 0x0000CCCCu;  // bit 4 of the index with bit 1
+    y ^= q ^ (q << 14);
+    q = (y ^ (y >> 7)) & 0x00AA00AAu;  // bit 3 with bit 0
+    t[m] = y ^ q ^ (q << 7);
+    z[m] = prmt(c0 | (c0 >> 4), c1 | (c1 >> 4), 0x6420u);
+    if (kTail && k < 8u) z[m] &= (1u << (4u * k)) - 1u;
+  }
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const uint32_t sel = (uint32_t)p | ((uint32_t)(4 + p) << 4);
+    pl[p] = prmt(prmt(t[0], t[1], sel), prmt(t[2], t[3], sel), 0x5410u);
+  }
+}
+
+// The text of rows [row_lo, row_hi) of the AND rule -> their plane words and
+// the plane blocks of their E2M1 operand rows, in one pass: row row_lo + i is
+// record rows[i] (none: i). Thread and store layout as in k_expand_op; the
+// sites past L are '-' in the planes and 0 in the operand. A thread reads the
+// 32 bytes of its sites as aligned 16-byte vectors. Eight sites' codes are
+// one word of nibbles z, in site order, in which plane p's E2M1 ones are the
+// bits p moved to bit 1 of each nibble; with the codes of sites k and k + 4
+// in a byte instead, two exchanges of bits leave plane p's 8 bits in byte p.
+// 14,000 rows of 29,903 sites move 1.47 GB (6.2 TB/s) in 238 us. Packing
+// and then expanding, with the planes read back and dash blocks written for
+// every chunk, took 198 + 212 us (1.9 GB).
+__global__ void __launch_bounds__(256, 6)
+    k_pack_op(const uint8_t *base, uint64_t bytes, const uint64_t *__restrict__ rs,
+              const uint64_t *__restrict__ rows, uint64_t row_lo, uint64_t row_hi, uint64_t L,
+              uint32_t words, uint4 *__restrict__ g0, uint4 *__restrict__ g1,
+              uint8_t *__restrict__ x, uint32_t *dash_chunk, uint32_t ext) {
+  constexpr uint32_t kPlanes = 4, nb = op_blocks(kPlanes);
+  const uint32_t op_words = op_chunks(L) * kChunkWords;
+  const uint32_t w = blockIdx.x * 32 + threadIdx.x / 8;
+  if (w >= words && w >= op_words) return;
+  const uint32_t c = w / kChunkWords;
+  const uint64_t s0 = (uint64_t)w * 32;
+  const uint32_t valid = s0 >= L ? 0u : L - s0 >= 32 ? 32u : (uint32_t)(L - s0);  // sites
+  const uint64_t in_group = (uint64_t)c * nb * kGroupBytes + (w - c * kChunkWords) * 128u +
+                            (threadIdx.x & 7u) * 16u;
+  const uint64_t group_bytes = op_group_bytes(kPlanes, L);
+  const uint64_t lo = reinterpret_cast<uint64_t>(base), hi = lo + bytes;
+  // the record starts of a group's rows are fetched one group ahead
+  auto start_of = [&](uint64_t r) -> uint64_t {
+    if (!valid || r < row_lo || r >= row_hi) return 0;
+    return lo + s0 + rs[rows ? rows[r - row_lo] : r - row_lo];
+  };
+  uint64_t r = row_lo / 8 * 8 + blockIdx.y * 8 + (threadIdx.x & 7u);
+  uint64_t next = start_of(r);
+  uint8_t *blk = x + (r / 8) * group_bytes + in_group;
+  const uint64_t blk_step = gridDim.y * group_bytes;
+  for (; (r & ~7ull) < row_hi; r += gridDim.y * 8, blk += blk_step) {
+    const uint64_t P = next;
+    next = start_of(r + gridDim.y * 8);
+    if (r < row_lo || r >= row_hi) continue;
+    uint32_t v[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = 0u;
+    uint32_t dw = 0, db = 0;
+    if (valid) {
+      const uint64_t A = P & ~15ull;
+      const uint32_t d = (uint32_t)(P - A);
+      dw = d >> 2;
+      db = 8u * (d & 3u);
+      uint4 a, b, e = make_uint4(0u, 0u, 0u, 0u);
+      if (A >= lo && A + 48 <= hi) {
+        const uint4 *q = reinterpret_cast<const uint4 *>(A);
+        a = __ldg(q);
+        b = __ldg(q + 1);
+        if (d) e = __ldg(q + 2);
+      } else {
+        a = load16_in(A, lo, hi);
+        b = load16_in(A + 16, lo, hi);
+        if (d) e = load16_in(A + 32, lo, hi);
+      }
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+      v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+      v[8] = e.x; v[9] = e.y; v[10] = e.z; v[11] = e.w;
+    }
+    // the words from byte 4 dw on
+#pragma unroll
+    for (int k = 0; k < 11; ++k) v[k] = (dw & 1u) ? v[k + 1] : v[k];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] = (dw & 2u) ? v[k + 2] : v[k];
+    uint32_t z[4], pl[4];
+    if (valid == 32u) pack_sites<false>(v, db, valid, z, pl);
+    else pack_sites<true>(v, db, valid, z, pl);
+    if (w < words) {
+      const uint4 o = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+      g0[r * words + w] = o;
+      if (g1) g1[r * words + w] = o;
+    }
+    if (w < op_words) {
+      constexpr uint32_t kOne = 0x22222222u;  // E2M1 1.0 in every nibble
+      uint4 *out = reinterpret_cast<uint4 *>(blk);
+      constexpr uint32_t kNext = kGroupBytes / 16;
+      out[0] = make_uint4((z[0] << 1) & kOne, (z[1] << 1) & kOne, (z[2] << 1) & kOne,
+                          (z[3] << 1) & kOne);
+      out[kNext] = make_uint4(z[0] & kOne, z[1] & kOne, z[2] & kOne, z[3] & kOne);
+      out[2 * kNext] = make_uint4((z[0] >> 1) & kOne, (z[1] >> 1) & kOne, (z[2] >> 1) & kOne,
+                                  (z[3] >> 1) & kOne);
+      out[3 * kNext] = make_uint4((z[0] >> 2) & kOne, (z[1] >> 2) & kOne, (z[2] >> 2) & kOne,
+                                  (z[3] >> 2) & kOne);
+      uint32_t dash = pl[0] & pl[1] & pl[2] & pl[3];
+      if (valid < 32u) dash &= (1u << valid) - 1u;
+      if (dash && !dash_chunk[c]) dash_chunk[c] = ext;  // every writer stores the same
+    }
   }
 }
 
@@ -1035,19 +1222,34 @@ void make_tmap_op(hd_ctx *ctx, CUtensorMap *tm, const void *base, uint32_t plane
 uint64_t mark_words(uint64_t sites) { return op_chunks(sites); }
 uint64_t list_words(uint64_t sites) { return 2 * (uint64_t)op_chunks(sites) + 1; }
 
-// Expands rows [lo, hi) of the planes into the operand x, marks the chunks
-// and lists the marked ones.
-void expand_rows(hd_ctx *ctx, const uint4 *g0, const uint4 *g1, uint32_t planes, uint64_t words,
-                 uint64_t lo, uint64_t hi, uint64_t sites, uint8_t *x, uint32_t *marks,
-                 uint32_t *list, cudaStream_t stream) {
-  const uint64_t groups = ceil_div(hi, (uint64_t)8) - lo / 8;
-  const dim3 grid((unsigned)ceil_div((uint64_t)op_chunks(sites) * kChunkWords, (uint64_t)32),
-                  (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(groups, 65535)));
-  k_expand_op<<<grid, 256, 0, stream>>>(g0, g1, planes, (uint32_t)words, lo, hi, sites, x, marks);
-  HD_LAUNCHED(ctx);
+// The list of the marked chunks, and their dash blocks (k_dash_blocks).
+void dash_rows(hd_ctx *ctx, const uint4 *g0, const uint4 *g1, uint32_t planes, uint64_t words,
+               uint64_t lo, uint64_t hi, uint64_t sites, uint8_t *x, uint32_t *marks, uint32_t ext,
+               uint32_t *list, cudaStream_t stream) {
   const uint32_t chunks = op_chunks(sites);
   k_dash_list<<<1, 512, 0, stream>>>(marks, chunks, list, list + chunks);
   HD_LAUNCHED(ctx);
+  const uint64_t jobs = ceil_div(ceil_div(hi, (uint64_t)8), (uint64_t)kDashGroups) * chunks;
+  k_dash_blocks<<<(unsigned)std::min<uint64_t>(jobs, (uint64_t)ctx->sm_count * 8),
+                  kDashGroups * 8 * kChunkWords, 0, stream>>>(
+      g0, g1, planes, (uint32_t)words, lo, hi, sites, x, marks, ext, list, list + 2 * chunks);
+  HD_LAUNCHED(ctx);
+}
+dim3 op_grid(uint64_t words, uint64_t lo, uint64_t hi) {
+  const uint64_t groups = ceil_div(hi, (uint64_t)8) - lo / 8;
+  return dim3((unsigned)ceil_div(words, (uint64_t)32),
+              (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(groups, 65535)));
+}
+
+// Expands rows [lo, hi) of the planes into the operand x, as its extension
+// `ext`, marks the chunks with a '-' and lists the marked ones.
+void expand_rows(hd_ctx *ctx, const uint4 *g0, const uint4 *g1, uint32_t planes, uint64_t words,
+                 uint64_t lo, uint64_t hi, uint64_t sites, uint8_t *x, uint32_t *marks,
+                 uint32_t ext, uint32_t *list, cudaStream_t stream) {
+  k_expand_op<<<op_grid((uint64_t)op_chunks(sites) * kChunkWords, lo, hi), 256, 0, stream>>>(
+      g0, g1, planes, (uint32_t)words, lo, hi, sites, x, marks, ext);
+  HD_LAUNCHED(ctx);
+  dash_rows(ctx, g0, g1, planes, words, lo, hi, sites, x, marks, ext, list, stream);
 }
 
 }  // namespace
@@ -1072,10 +1274,11 @@ bool mma_eligible(const hd_alignment *aln) {
          aln->n_rows < (1ull << 31);
 }
 
-bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStream_t stream,
-                uint64_t cap_hint) {
-  const hd_alignment *o = aln->base ? aln->base : aln;
-  if (o->op_rows >= rows) return true;
+namespace {
+// Room for `rows` rows in the operand of the alignment o, and for the list of
+// its next extension; false if there is no memory for it.
+bool grow_operand(hd_ctx *ctx, const hd_alignment *o, uint64_t rows, cudaStream_t stream,
+                  uint64_t cap_hint) {
   const uint32_t P = (uint32_t)o->planes;
   const uint64_t words = o->words;
   if (rows > o->op_cap) {
@@ -1107,10 +1310,44 @@ bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStr
   // a list of its own for every extension: launches on other streams may
   // still read an earlier one
   o->op_lists.emplace_back(list_words(o->length) * 4, stream);
+  return true;
+}
+}  // namespace
+
+bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStream_t stream,
+                    uint64_t cap_hint) {
+  const hd_alignment *o = aln->base ? aln->base : aln;
+  if (o->op_rows >= rows) return true;
+  if (!grow_operand(ctx, o, rows, stream, cap_hint)) return false;
+  const uint32_t P = (uint32_t)o->planes;
   expand_rows(ctx, o->plane_buf[0].as<uint4>(), P > 4 ? o->plane_buf[1].as<uint4>() : nullptr, P,
-              words, o->op_rows, rows, o->length, o->op.as<uint8_t>(), o->op_dash.as<uint32_t>(),
+              o->words, o->op_rows, rows, o->length, o->op.as<uint8_t>(),
+              o->op_dash.as<uint32_t>(), (uint32_t)o->op_lists.size(),
               o->op_lists.back().as<uint32_t>(), stream);
   o->op_rows = rows;
+  return true;
+}
+
+bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const hd_alignment *aln,
+                  uint64_t lo, uint64_t hi, uint4 *copy, cudaStream_t stream, uint64_t cap_hint) {
+  if (aln->base || aln->planes != 4 || aln->op_rows != lo || hi <= lo) return false;
+  if (!grow_operand(ctx, aln, hi, stream, cap_hint)) return false;
+  const uint32_t ext = (uint32_t)aln->op_lists.size();
+  uint4 *g0 = aln->plane_buf[0].as<uint4>();
+  uint8_t *x = aln->op.as<uint8_t>();
+  uint32_t *marks = aln->op_dash.as<uint32_t>();
+  const uint64_t op_words = (uint64_t)op_chunks(aln->length) * kChunkWords;
+  // up to 8 row groups a block, while that leaves four rounds of blocks
+  dim3 grid = op_grid(std::max(aln->words, op_words), lo, hi);
+  const uint64_t rounds = (uint64_t)grid.x * grid.y / ((uint64_t)ctx->sm_count * 6 * 4);
+  grid.y = (unsigned)ceil_div(grid.y, std::min<uint64_t>(8, std::max<uint64_t>(1, rounds)));
+  k_pack_op<<<grid, 256, 0, stream>>>(
+      rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), d_rows, lo, hi, aln->length,
+      (uint32_t)aln->words, g0, copy, x, marks, ext);
+  HD_LAUNCHED(ctx);
+  dash_rows(ctx, g0, nullptr, 4, aln->words, lo, hi, aln->length, x, marks, ext,
+            aln->op_lists.back().as<uint32_t>(), stream);
+  aln->op_rows = hi;
   return true;
 }
 
@@ -1176,7 +1413,7 @@ bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLa
   HD_CUDA(cudaMemsetAsync(flags, 0, marks * 4, stream));
   expand_rows(ctx, static_cast<const uint4 *>(a->planes_ptr(0)),
               P > 4 ? static_cast<const uint4 *>(a->planes_ptr(1)) : nullptr, P, o->words, 0,
-              a->n_rows, o->length, tmp.as<uint8_t>(), flags, flags + marks, stream);
+              a->n_rows, o->length, tmp.as<uint8_t>(), flags, 1, flags + marks, stream);
   op = tmp.as<uint8_t>();
   dash = flags + marks;
   plan->blocks.push_back(std::move(tmp));
@@ -1326,6 +1563,12 @@ static uint64_t size_tiles(uint64_t lo, uint64_t hi) {
   uint64_t n = 0;
   for (uint64_t I = lo; I < hi; ++I) n += ((I + 1) * kTM - 2) / kMmaCols + 1;
   return n;
+}
+
+bool mma_wanted(hd_ctx *ctx, const hd_alignment *aln) {
+  if (ctx->engine_force == 0 || !mma_eligible(aln)) return false;
+  const uint64_t min_items = ctx->engine_force == 1 ? 0 : mma_min_items_for(ctx, aln->length);
+  return size_tiles(0, ceil_div(aln->n_rows, (uint64_t)kTM)) >= min_items;
 }
 
 void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaStream_t stream,

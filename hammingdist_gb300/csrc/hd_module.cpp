@@ -335,6 +335,7 @@ DataSet<T> from_fasta(const std::string &filename, bool include_x, bool remove_d
     }
     return ds;
   }
+  check(hd_expect_pairwise(c));
   check(hd_alignment_from_fasta_file(c, filename.c_str(), remove_duplicates, n, include_x,
                                      use_gpu ? HD_SEM_GPU : HD_SEM_CPU, &a.p));
   say_trace();
@@ -374,6 +375,7 @@ py::dict from_fasta_device(uintptr_t fasta, uint64_t nbytes, uintptr_t out, uint
   {
     py::gil_scoped_release nogil;
     Aln a;
+    check(hd_expect_pairwise(c));
     check(hd_alignment_from_fasta(c, reinterpret_cast<const char *>(fasta), nbytes, 1,
                                   remove_duplicates, 0, 0, HD_SEM_GPU, &a.p));
     check(hd_alignment_info(a.p, &n_rows, nullptr, &n_in, nullptr));
@@ -416,6 +418,7 @@ DataSet<uint8_t> from_stringlist(const std::vector<std::string> &data, bool incl
   }
   py::gil_scoped_release nogil;
   Aln a;
+  check(hd_expect_pairwise(c));
   check(hd_alignment_from_sequences(c, cat.data(), offsets.data(), data.size(), include_x,
                                     use_gpu ? HD_SEM_GPU : HD_SEM_CPU, &a.p));
   return compute<uint8_t>(a.p, max_distance, false, "", std::chrono::steady_clock::now());
@@ -430,6 +433,7 @@ void from_fasta_to_lower_triangular(const std::string &in, const std::string &ou
   if (use_gpu) say("Using GPU...");
   py::gil_scoped_release nogil;
   Aln a;
+  check(hd_expect_pairwise(c));
   check(hd_alignment_from_fasta_file(c, in.c_str(), remove_duplicates, n, 0, HD_SEM_GPU, &a.p));
   say_trace();
   say("...pre-processing completed in " + std::to_string((long long)ms_since(t0)) + " ms...");

@@ -142,6 +142,12 @@ int hd_alignment_from_fasta_file(hd_ctx *ctx, const char *path, int remove_dupli
 int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicates,
                               int dtype_bytes, int64_t max_distance, hd_output_fn out_fn,
                               void *user, hd_alignment **aln_out);
+/* Says that the next alignment this context builds (hd_alignment_from_fasta,
+ * _from_fasta_file, _from_sequences) is compared whole afterwards
+ * (hd_pairwise_lt, hd_pairwise_lt_to_file): its rows' tensor-core operand is
+ * then written along with the packed rows, in one pass over their text,
+ * instead of from them on the first distances. Results do not depend on it. */
+int hd_expect_pairwise(hd_ctx *ctx);
 /* Same from n sequences held back to back in `bytes` with offsets[0..n]
  * (host memory). Replaces the DataSet(std::vector<std::string>&) path of
  * from_stringlist (src/hamming.cc:16-21). */

@@ -1,5 +1,5 @@
 """The tensor-core engine's items (256 rows x 496 columns on a pair of SMs,
-288-site chunks) at their edges, and tiles split along K, against the
+192-site chunks) at their edges, and tiles split along K, against the
 bit-plane engine bit for bit (whole numbers: no tolerance)."""
 import os
 
