@@ -1468,7 +1468,7 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
     if (remove_duplicates) {
       owner->d_seqidx = DevBuf(all.n * 8, ctx->stream);
       if (inc_rows) {
-        HD_CUDA(cudaMemcpyAsync(owner->d_seqidx.p, inc.rowid.p, all.n * 8, cudaMemcpyDeviceToDevice,
+        HD_CUDA(cudaMemcpyAsync(owner->d_seqidx.p, inc.rowid(), all.n * 8, cudaMemcpyDeviceToDevice,
                                 ctx->stream));
       } else {
         owner->seqidx = std::move(seq);
@@ -1491,7 +1491,7 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
       if (remove_duplicates) {
         all.row_of = DevBuf(all.n * 8, ctx->stream);
         if (inc_rows)
-          HD_CUDA(cudaMemcpyAsync(all.row_of.p, inc.rowid.p, all.n * 8, cudaMemcpyDeviceToDevice,
+          HD_CUDA(cudaMemcpyAsync(all.row_of.p, inc.rowid(), all.n * 8, cudaMemcpyDeviceToDevice,
                                   ctx->stream));
         else
           hd::upload_table(ctx, all.row_of.p, owner->seqidx.data(), all.n * 8, ctx->stream);

@@ -584,7 +584,7 @@ __device__ inline uint64_t mix64(uint64_t x) {
 }
 
 constexpr unsigned long long kEmpty = ~0ull;
-constexpr int kHashU = 2;     // 512-byte blocks per warp per step of k_hash and k_tab_cmp
+constexpr int kCmpFast = 4;  // 512-byte blocks per step of warp_equal
 
 __device__ inline uint32_t load4_in(uint64_t x, uint64_t lo, uint64_t hi) {
   if (x >= lo && x + 4 <= hi) return *reinterpret_cast<const uint32_t *>(x);
@@ -597,117 +597,161 @@ __device__ inline uint32_t load4_in(uint64_t x, uint64_t lo, uint64_t hi) {
 // Hash of each record's bytes: a sum over its 8-byte groups (at record
 // positions 8q; a short last group is zero-filled) of the 64-bit product of
 // the group's two 4-byte halves, each XORed with a position-keyed 32-bit
-// constant, then one 64-bit mix of the sum and the length (k_hash_fin).
+// constant, then one 64-bit mix of the sum and the length (k_tab_insert).
 // Different records rarely share a hash, and equal hashes are verified byte
 // by byte, so a collision costs a verify round, never a wrong answer. The sum
 // does not depend on the order of its terms, so a record is hashed in
-// segments of kHashSeg bytes, one warp each, that add their partial sums to
-// acc[r] (zeroed first): many warps per record keep enough loads in flight
-// however few records there are. Block (x, y) takes records 8x .. 8x + 7
-// (one per warp) from byte y kHashSeg on. A lane reads 16 aligned bytes per
-// step (two 512-byte blocks per warp and step) and the next lane's first 8;
-// the two groups starting in its 16 bytes start at byte d0 mod 8 of them (d0
-// = the segment's start mod 16) and are realigned with funnel shifts. Index
-// arithmetic within a segment is 32-bit, so that a 16-byte step costs about
-// 40 instructions.
-constexpr uint64_t kHashSeg = 4096;
+// segments of 4 KB of aligned memory (from its first byte's 16-byte vector
+// on), one warp each, that add their partial sums to acc[r] (zeroed first):
+// many warps per record keep enough loads in flight however few records there
+// are. Block (x, y) takes records 8x .. 8x + 7 (one per warp), segment y. A
+// lane reads 16 aligned bytes per step, four 512-byte steps at a time; the two
+// groups that start in them start at byte d0 mod 8 (d0 = the record's start
+// mod 16) and are realigned with funnel shifts, their last bytes from the next
+// lane, or for lane 31 from lane 0 of the next step. Only the record's last
+// steps mask bytes. 20,000 records of 29,903 bytes: 106 us, 5.7 TB/s (two
+// steps at a time, with masks and look-aheads in every step: 158).
+constexpr uint32_t kHashSeg = 4096;
 constexpr int kHashWarps = 8;
-__global__ void __launch_bounds__(32 * kHashWarps)
+constexpr int kHashSteps = 4;
+constexpr uint32_t kHashKx = 0x9e3779b9u, kHashKy = 0x85ebca6bu;  // per group, odd
+// Four steps (2 KB) of a record from the 16-byte aligned address A. kHi: the
+// lanes' groups start in the second word of their 8 bytes (d0 mod 8 >= 4); h8:
+// at this byte of them; sh: the funnel shift; span: bytes from A to the
+// record's end; q: the number of lane 0's first group; before: groups that
+// start before this byte are not the record's. kFast: all of the steps' groups
+// are whole and readable with the 8 bytes after them.
+template <bool kHi, bool kFast>
+__device__ __forceinline__ uint64_t hash_steps(uint64_t A, int64_t span, uint32_t h8, uint32_t sh,
+                                               uint32_t q, uint32_t before, uint64_t lo,
+                                               uint64_t hi, int lane) {
+  uint4 v[kHashSteps];
+  uint2 nx = make_uint2(0u, 0u);  // lane 31: the 8 bytes after its last 16
+#pragma unroll
+  for (int k = 0; k < kHashSteps; ++k) {
+    const uint32_t off = 512 * k + 16 * lane;
+    if (kFast) v[k] = __ldg(reinterpret_cast<const uint4 *>(A + off));
+    else v[k] = (int64_t)off < span ? load16_in(A + off, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (lane == 31) {
+    constexpr uint32_t off = 512 * kHashSteps;
+    if (kFast) nx = __ldg(reinterpret_cast<const uint2 *>(A + off));
+    else if ((int64_t)off < span) nx = make_uint2(load4_in(A + off, lo, hi), load4_in(A + off + 4, lo, hi));
+  }
+  uint32_t kx = (q + 2 * lane) * kHashKx + 0x7f4a7c15u;
+  uint32_t ky = (q + 2 * lane) * kHashKy + 0x165667b1u;
+  uint64_t h = 0;
+#pragma unroll
+  for (int k = 0; k < kHashSteps; ++k) {
+    constexpr int last = kHashSteps - 1;
+    // the next lane's first words: for lane 31 those of the next step's lane 0
+    const uint4 &vn = v[k < last ? k + 1 : k];
+    uint32_t n0 = __shfl_sync(0xffffffffu, lane == 0 ? vn.x : v[k].x, (lane + 1) & 31), n1 = 0;
+    if (kHi) n1 = __shfl_sync(0xffffffffu, lane == 0 ? vn.y : v[k].y, (lane + 1) & 31);
+    if (k == last && lane == 31) {
+      n0 = nx.x;
+      n1 = nx.y;
+    }
+    const uint32_t wd[5] = {kHi ? v[k].y : v[k].x, kHi ? v[k].z : v[k].y, kHi ? v[k].w : v[k].z,
+                            kHi ? n0 : v[k].w, kHi ? n1 : n0};
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      uint32_t x = __funnelshift_r(wd[2 * g], wd[2 * g + 1], sh);
+      uint32_t y = __funnelshift_r(wd[2 * g + 1], wd[2 * g + 2], sh);
+      bool on = k > 0 || 16 * lane + 8 * g + h8 >= before;
+      if (!kFast) {
+        const int64_t rem = span - (int64_t)(512 * k + 16 * lane + 8 * g + h8);  // bytes left
+        on = on && rem > 0;
+        if (rem > 0 && rem < 8) {  // the record's last group: bytes from rem on are 0
+          const uint32_t m = (uint32_t)rem;
+          y = m > 4u ? y & ((1u << (8u * (m - 4u))) - 1u) : 0u;
+          if (m < 4u) x &= (1u << (8u * m)) - 1u;
+        }
+      }
+      x ^= kx + (uint32_t)(64 * k + g) * kHashKx;
+      y ^= ky + (uint32_t)(64 * k + g) * kHashKy;
+      if (on) h += (uint64_t)x * y;
+    }
+  }
+  return h;
+}
+// One segment of a record (see k_hash) from its aligned address A
+template <bool kHi>
+__device__ __forceinline__ uint64_t hash_segment(uint64_t A, int64_t span, uint32_t h8, uint32_t sh,
+                                                 uint32_t q, uint32_t before, uint64_t lo,
+                                                 uint64_t hi, int lane) {
+  constexpr uint32_t kStep = 512 * kHashSteps;
+  uint64_t h = 0;
+#pragma unroll 1
+  for (uint32_t b = 0; b < kHashSeg && (int64_t)b < span; b += kStep) {
+    const uint64_t at = A + b;
+    const int64_t left = span - b;
+    const uint32_t qb = q + (b >> 3), bf = b ? 0u : before;
+    if (left >= (int64_t)(kStep + 8) && at >= lo && at + kStep + 16 <= hi)
+      h += hash_steps<kHi, true>(at, left, h8, sh, qb, bf, lo, hi, lane);
+    else
+      h += hash_steps<kHi, false>(at, left, h8, sh, qb, bf, lo, hi, lane);
+  }
+  return h;
+}
+__global__ void __launch_bounds__(32 * kHashWarps, 5)
     k_hash(const uint8_t *base, uint64_t bytes, const uint64_t *rs, const uint64_t *rl, uint64_t R,
            unsigned long long *acc) {
   const int lane = threadIdx.x & 31;
   const uint64_t r = (uint64_t)blockIdx.x * kHashWarps + (threadIdx.x >> 5);
   if (r >= R) return;  // warp-uniform
   const uint64_t lo = reinterpret_cast<uint64_t>(base), hi = lo + bytes;
-  const uint64_t len = rl[r];
-  for (uint64_t s_lo = (uint64_t)blockIdx.y * kHashSeg; s_lo < len;
-       s_lo += (uint64_t)gridDim.y * kHashSeg) {
-    const uint32_t seg = (uint32_t)(len - s_lo < kHashSeg ? len - s_lo : kHashSeg);
-    const uint64_t P = lo + rs[r] + s_lo;  // the record's byte s_lo
-    const uint64_t A = P & ~15ull;
-    const uint32_t d0 = (uint32_t)(P - A), h8 = d0 & 7u, sh = 8u * (d0 & 3u);
-    const bool hi_word = h8 >= 4u;  // the groups start in the lane's second word
-    const uint32_t span = d0 + seg, q0 = (uint32_t)(s_lo >> 3);
-    uint64_t h = 0;
-    for (uint32_t b0 = 0; b0 < span; b0 += 512 * kHashU) {
-      uint4 v[kHashU];
-      uint2 nx[kHashU];
-#pragma unroll
-      for (int k = 0; k < kHashU; ++k) {
-        const uint32_t off = b0 + 512 * k + 16 * lane;
-        v[k] = off < span ? load16_in(A + off, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
-        const uint32_t noff = b0 + 512 * k + 512;  // lane 31: the 8 bytes after its 16
-        nx[k] = (lane == 31 && noff < span)
-                    ? make_uint2(load4_in(A + noff, lo, hi), load4_in(A + noff + 4, lo, hi))
-                    : make_uint2(0u, 0u);
-      }
-#pragma unroll
-      for (int k = 0; k < kHashU; ++k) {
-        uint32_t n0 = __shfl_down_sync(0xffffffffu, v[k].x, 1);
-        uint32_t n1 = __shfl_down_sync(0xffffffffu, v[k].y, 1);
-        if (lane == 31) {
-          n0 = nx[k].x;
-          n1 = nx[k].y;
-        }
-        // words from the one the first group starts in
-        const uint32_t wd[5] = {hi_word ? v[k].y : v[k].x, hi_word ? v[k].z : v[k].y,
-                                hi_word ? v[k].w : v[k].z, hi_word ? n0 : v[k].w,
-                                hi_word ? n1 : n0};
-        const int32_t t0 = (int32_t)(b0 + 512 * k + 16 * lane + h8) - (int32_t)d0;
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          const int32_t t = t0 + 8 * g;  // the group's position in the segment
-          uint32_t x = __funnelshift_r(wd[2 * g], wd[2 * g + 1], sh);
-          uint32_t y = __funnelshift_r(wd[2 * g + 1], wd[2 * g + 2], sh);
-          const uint32_t rem = (uint32_t)((int32_t)seg - t);  // > 0 where valid
-          if (rem < 8u) {  // the record's last group: bytes from rem on are 0
-            y = rem > 4u ? y & ((1u << (8u * (rem - 4u))) - 1u) : 0u;
-            if (rem < 4u) x &= (1u << (8u * rem)) - 1u;
-          }
-          const uint32_t q = q0 + ((uint32_t)t >> 3);
-          x ^= q * 0x9e3779b9u + 0x7f4a7c15u;
-          y ^= q * 0x85ebca6bu + 0x165667b1u;
-          if ((uint32_t)t < seg) h += (uint64_t)x * y;
-        }
-      }
-    }
+  const uint64_t len = rl[r], P = lo + rs[r];
+  if (!len) return;
+  const uint32_t d0 = (uint32_t)(P & 15u), h8 = d0 & 7u, sh = 8u * (d0 & 3u);
+  for (uint64_t j = blockIdx.y; j * kHashSeg < d0 + len; j += gridDim.y) {
+    const uint64_t A = P - d0 + j * kHashSeg;
+    const int64_t span = (int64_t)(d0 + len - j * kHashSeg);  // to the record's end
+    // group numbers count from the record's start, d0 - h8 bytes into it
+    const uint32_t q = (uint32_t)(j * (kHashSeg / 8)) - (d0 >> 3);
+    const uint32_t before = j ? 0u : d0;
+    uint64_t h = (h8 & 4u) ? hash_segment<true>(A, span, h8, sh, q, before, lo, hi, lane)
+                           : hash_segment<false>(A, span, h8, sh, q, before, lo, hi, lane);
     h = warp_sum(h);
     if (lane == 0 && h) atomicAdd(&acc[r], (unsigned long long)h);
   }
 }
-// The record hashes from the sums k_hash left in h[r], in place.
-__global__ void k_hash_fin(const uint64_t *rl, uint64_t R, unsigned long long *h) {
-  const uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  const uint64_t v = mix64(h[r] ^ (rl[r] * 0xd6e8feb86659fd93ull));
-  h[r] = v == kEmpty ? v - 1 : v;
-}
-// Hashes of records [0, R) of rs/rl into out (R > 0).
+// Hash sums of records [0, R) of rs/rl into out (R > 0), which is zeroed.
 void hash_records(hd_ctx *ctx, const Records &rec, const uint64_t *rs, const uint64_t *rl,
                   uint64_t R, uint64_t *out) {
-  cudaStream_t st = ctx->stream;
-  HD_CUDA(cudaMemsetAsync(out, 0, R * 8, st));
-  unsigned long long *h = reinterpret_cast<unsigned long long *>(out);
-  if (rec.max_len) {
-    const uint64_t X = ceil_div(R, (uint64_t)kHashWarps), S = ceil_div(rec.max_len, kHashSeg);
-    if (X > 0x7fffffffull) fail(HD_ERR_ARG, "too many records");
-    // segments past 65,535 are taken by the warps' loop
-    k_hash<<<dim3((unsigned)X, (unsigned)std::min<uint64_t>(S, 65535)), 32 * kHashWarps, 0, st>>>(
-        rec.base, rec.bytes, rs, rl, R, h);
-    HD_LAUNCHED(ctx);
-  }
-  k_hash_fin<<<grid_for(R, 256), 256, 0, st>>>(rl, R, h);
+  if (!rec.max_len) return;
+  const uint64_t X = ceil_div(R, (uint64_t)kHashWarps), S = ceil_div(rec.max_len + 15, (uint64_t)kHashSeg);
+  if (X > 0x7fffffffull) fail(HD_ERR_ARG, "too many records");
+  // segments past 65,535 are taken by the warps' loop
+  k_hash<<<dim3((unsigned)X, (unsigned)std::min<uint64_t>(S, 65535)), 32 * kHashWarps, 0, ctx->stream>>>(
+      rec.base, rec.bytes, rs, rl, R, reinterpret_cast<unsigned long long *>(out));
   HD_LAUNCHED(ctx);
 }
 
 __device__ inline uint64_t slot_of(uint64_t h, uint64_t mask) { return (h ^ (h >> 29)) & mask; }
 
-__global__ void k_tab_insert(const uint64_t *hash, const uint64_t *list, uint64_t cnt,
+// The records of one round of duplicate removal: record list[i], or r0 + i
+// without a list, i < cnt.
+struct RoundList {
+  const uint64_t *list;
+  uint64_t r0, cnt;
+  __device__ uint64_t at(uint64_t i) const { return list ? list[i] : r0 + i; }
+};
+
+// The records' hashes into the table: each hash's lowest record index. A round
+// without a list is the records' first, and makes their hashes of k_hash's
+// sums in place.
+__global__ void k_tab_insert(uint64_t *hash, const uint64_t *rl, RoundList L,
                              unsigned long long *keys, unsigned long long *mins, uint64_t mask) {
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= cnt) return;
-  uint64_t r = list ? list[i] : i;
+  if (i >= L.cnt) return;
+  const uint64_t r = L.at(i);
   unsigned long long h = hash[r];
+  if (!L.list) {
+    h = mix64(h ^ (rl[r] * 0xd6e8feb86659fd93ull));
+    h = h == kEmpty ? h - 1 : h;
+    hash[r] = h;
+  }
   uint64_t slot = slot_of(h, mask);
   for (;;) {
     unsigned long long prev = atomicCAS(&keys[slot], kEmpty, h);
@@ -719,8 +763,19 @@ __global__ void k_tab_insert(const uint64_t *hash, const uint64_t *list, uint64_
   }
 }
 
-// Each record against the lowest-index record of equal hash: equal bytes ->
-// duplicate; different bytes (a hash collision) -> next round.
+// 16 bytes from byte 4 dw + sh / 8 on of the 32 bytes v, n (dw is warp-uniform)
+__device__ __forceinline__ uint4 shifted16(uint4 v, uint4 n, uint32_t dw, uint32_t sh) {
+  uint32_t w0, w1, w2, w3, w4;
+  switch (dw) {
+    case 0: w0 = v.x; w1 = v.y; w2 = v.z; w3 = v.w; w4 = n.x; break;
+    case 1: w0 = v.y; w1 = v.z; w2 = v.w; w3 = n.x; w4 = n.y; break;
+    case 2: w0 = v.z; w1 = v.w; w2 = n.x; w3 = n.y; w4 = n.z; break;
+    default: w0 = v.w; w1 = n.x; w2 = n.y; w3 = n.z; w4 = n.w; break;
+  }
+  return make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh),
+                    __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
+}
+
 // Whether the len bytes (len < 2^31) at Pa and at Pb, both inside [lo, hi),
 // are equal; called by a whole warp, same result in every lane. a is read
 // with aligned 16-byte loads; b's bytes at the same relative positions come
@@ -737,143 +792,265 @@ __device__ inline bool warp_equal(uint64_t Pa, uint64_t Pb, uint32_t len, uint64
   const uint32_t d = (uint32_t)(Bs - Ab), dw = d >> 2, sh = 8u * (d & 3u);
   const uint32_t span = da + len;                    // a's windows cover [0, span) from Aa
   const uint32_t b_end = (uint32_t)(Pb + len - Ab);  // b's bytes end there, from Ab
-  for (uint32_t b0 = 0; b0 < span; b0 += 512 * kHashU) {
+  // steps that end inside the span: all loads before the first use, and only
+  // the first window has bytes before a's first
+  uint32_t b0 = 0;
+  for (; b0 + 512 * kCmpFast <= span && Aa >= lo && Ab + b0 >= lo &&
+         Ab + b0 + 512 * kCmpFast + 16 <= hi;
+       b0 += 512 * kCmpFast) {
+    uint4 va[kCmpFast], vb[kCmpFast + 1];
+#pragma unroll
+    for (int k = 0; k < kCmpFast; ++k) {
+      const uint32_t off = b0 + 512 * k + 16 * lane;
+      va[k] = __ldg(reinterpret_cast<const uint4 *>(Aa + off));
+      vb[k] = __ldg(reinterpret_cast<const uint4 *>(Ab + off));
+    }
+    vb[kCmpFast] = make_uint4(0u, 0u, 0u, 0u);
+    if (d && lane == 0)  // lane 31 takes its next words from lane 0's next step
+      vb[kCmpFast] = __ldg(reinterpret_cast<const uint4 *>(Ab + b0 + 512 * kCmpFast));
     uint32_t diff = 0;
 #pragma unroll
-    for (int k = 0; k < kHashU; ++k) {
-      const uint32_t off = b0 + 512 * k + 16 * lane;
-      const bool in = off < span;
-      const uint4 va = in ? load16_in(Aa + off, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
-      const uint4 vb = off < b_end ? load16_in(Ab + off, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
-      uint4 vn;
-      vn.x = __shfl_down_sync(0xffffffffu, vb.x, 1);
-      vn.y = __shfl_down_sync(0xffffffffu, vb.y, 1);
-      vn.z = __shfl_down_sync(0xffffffffu, vb.z, 1);
-      vn.w = __shfl_down_sync(0xffffffffu, vb.w, 1);
-      if (lane == 31)
-        vn = (d && off + 16 < b_end) ? load16_in(Ab + off + 16, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
-      // words dw .. dw + 4 of b's 32 bytes (vb, vn)
-      uint32_t w0, w1, w2, w3, w4;
-      switch (dw) {  // warp-uniform
-        case 0: w0 = vb.x; w1 = vb.y; w2 = vb.z; w3 = vb.w; w4 = vn.x; break;
-        case 1: w0 = vb.y; w1 = vb.z; w2 = vb.w; w3 = vn.x; w4 = vn.y; break;
-        case 2: w0 = vb.z; w1 = vb.w; w2 = vn.x; w3 = vn.y; w4 = vn.z; break;
-        default: w0 = vb.w; w1 = vn.x; w2 = vn.y; w3 = vn.z; w4 = vn.w; break;
+    for (int k = 0; k < kCmpFast; ++k) {
+      uint4 x = vb[k];
+      if (d) {  // warp-uniform
+        const int to = (lane + 1) & 31;
+        uint4 vn;
+        vn.x = __shfl_sync(0xffffffffu, lane ? vb[k].x : vb[k + 1].x, to);
+        vn.y = __shfl_sync(0xffffffffu, lane ? vb[k].y : vb[k + 1].y, to);
+        vn.z = __shfl_sync(0xffffffffu, lane ? vb[k].z : vb[k + 1].z, to);
+        vn.w = __shfl_sync(0xffffffffu, lane ? vb[k].w : vb[k + 1].w, to);
+        x = shifted16(vb[k], vn, dw, sh);
       }
-      uint32_t x[4] = {va.x ^ __funnelshift_r(w0, w1, sh), va.y ^ __funnelshift_r(w1, w2, sh),
-                       va.z ^ __funnelshift_r(w2, w3, sh), va.w ^ __funnelshift_r(w3, w4, sh)};
-      if (!(off >= da && off + 16 <= span)) {
-        // a window at an end of the span: only the bytes at positions
-        // [0, len) from a's first byte count
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int32_t p = (int32_t)(off + 4 * j) - (int32_t)da;  // the word's first byte
-          uint32_t m = in ? 0xffffffffu : 0u;
-          if (p < 0) m &= p <= -4 ? 0u : (0xffffffffu << (8 * (uint32_t)(-p)));
-          if (p + 4 > (int32_t)len)
-            m &= p >= (int32_t)len ? 0u : (0xffffffffu >> (8 * (uint32_t)(p + 4 - (int32_t)len)));
-          x[j] &= m;
-        }
+      x.x ^= va[k].x;
+      x.y ^= va[k].y;
+      x.z ^= va[k].z;
+      x.w ^= va[k].w;
+      if (k == 0 && b0 == 0 && lane == 0 && da) {
+        x.x &= da >= 4 ? 0u : 0xffffffffu << (8 * da);
+        x.y &= da >= 8 ? 0u : da <= 4 ? 0xffffffffu : 0xffffffffu << (8 * (da - 4));
+        x.z &= da >= 12 ? 0u : da <= 8 ? 0xffffffffu : 0xffffffffu << (8 * (da - 8));
+        x.w &= da <= 12 ? 0xffffffffu : 0xffffffffu << (8 * (da - 12));
       }
-      diff |= x[0] | x[1] | x[2] | x[3];
+      diff |= x.x | x.y | x.z | x.w;
     }
     if (__any_sync(0xffffffffu, diff != 0)) return false;
+  }
+  for (; b0 < span; b0 += 512) {
+    const uint32_t off = b0 + 16 * lane;
+    const bool in = off < span;
+    const uint4 va = in ? load16_in(Aa + off, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
+    const uint4 vb = off < b_end ? load16_in(Ab + off, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
+    uint4 vn;
+    vn.x = __shfl_down_sync(0xffffffffu, vb.x, 1);
+    vn.y = __shfl_down_sync(0xffffffffu, vb.y, 1);
+    vn.z = __shfl_down_sync(0xffffffffu, vb.z, 1);
+    vn.w = __shfl_down_sync(0xffffffffu, vb.w, 1);
+    if (lane == 31)
+      vn = (d && off + 16 < b_end) ? load16_in(Ab + off + 16, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
+    const uint4 y = shifted16(vb, vn, dw, sh);
+    uint32_t x[4] = {va.x ^ y.x, va.y ^ y.y, va.z ^ y.z, va.w ^ y.w};
+    if (!(off >= da && off + 16 <= span)) {
+      // a window at an end of the span: only the bytes at positions
+      // [0, len) from a's first byte count
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int32_t p = (int32_t)(off + 4 * j) - (int32_t)da;  // the word's first byte
+        uint32_t m = in ? 0xffffffffu : 0u;
+        if (p < 0) m &= p <= -4 ? 0u : (0xffffffffu << (8 * (uint32_t)(-p)));
+        if (p + 4 > (int32_t)len)
+          m &= p >= (int32_t)len ? 0u : (0xffffffffu >> (8 * (uint32_t)(p + 4 - (int32_t)len)));
+        x[j] &= m;
+      }
+    }
+    if (__any_sync(0xffffffffu, (x[0] | x[1] | x[2] | x[3]) != 0)) return false;
   }
   return true;
 }
 
-// The verify step spread over segments: warp (i, seg) compares bytes
-// [seg * seg_bytes, +seg_bytes) of list record i with the lowest-index record
-// of its hash (rep_out[i]) and marks differs[i] on a difference; k_tab_resolve
-// then files each record as unique, a duplicate of rep, or (a hash collision)
-// a record for the next round. Many warps per record keep the loads in
-// flight when there are few duplicates.
-__global__ void k_tab_cmp(const uint8_t *base, uint64_t bytes, const uint64_t *rs,
-                          const uint64_t *rl, const uint64_t *hash, const uint64_t *list,
-                          uint64_t cnt, const unsigned long long *keys,
-                          const unsigned long long *mins, uint64_t mask, uint64_t seg_bytes,
-                          uint64_t segs, uint64_t *rep_out, uint32_t *differs) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t wid = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  if (wid >= cnt * segs) return;
-  const uint64_t i = wid / segs, seg = wid % segs;
-  const uint64_t r = list ? list[i] : i;
-  uint64_t rep = 0;
-  if (lane == 0) {
+// Each record's first record of equal hash (dup[r]); the records that are not
+// their own are listed to be compared with it (pairs[0 .. *n_pairs), any
+// order), those of another length marked as unlike it (differs[i]).
+__global__ void k_tab_find(const uint64_t *hash, const uint64_t *rl, RoundList L,
+                           const unsigned long long *keys, const unsigned long long *mins,
+                           uint64_t mask, uint64_t *dup, uint64_t *pairs,
+                           unsigned long long *n_pairs, uint32_t *differs) {
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  bool pair = false;
+  if (i < L.cnt) {
+    const uint64_t r = L.at(i);
     const unsigned long long h = hash[r];
     uint64_t slot = slot_of(h, mask);
     while (keys[slot] != h) slot = (slot + 1) & mask;
-    rep = mins[slot];
-    if (seg == 0) rep_out[i] = rep;
+    const uint64_t rep = mins[slot];
+    dup[r] = rep;
+    if (rep != r) {
+      pair = rl[r] == rl[rep];
+      if (!pair) differs[i] = 1u;
+    }
   }
-  rep = __shfl_sync(0xffffffffu, rep, 0);
-  if (rep == r) return;
-  const uint64_t len = rl[r];
-  if (len != rl[rep]) {
-    if (seg == 0 && lane == 0) differs[i] = 1u;
+  const uint32_t on = __ballot_sync(0xffffffffu, pair);
+  if (!on) return;
+  unsigned long long at = 0;
+  const int lane = threadIdx.x & 31;
+  if (lane == __ffs(on) - 1) at = atomicAdd(n_pairs, (unsigned long long)__popc(on));
+  at = __shfl_sync(0xffffffffu, at, __ffs(on) - 1);
+  if (pair) pairs[at + __popc(on & ((1u << lane) - 1u))] = i;
+}
+
+// The verify step: the listed records against their first record of equal
+// hash, byte by byte; differs[i] marks a difference (a hash collision, a
+// record for the next round). A warp compares segments of 4 KB, one after
+// another: few duplicates are spread over all SMs. 6,000 duplicates of
+// 29,903 bytes among 20,000 records: 67 us, 5 TB/s (a warp for every segment
+// of every record, most of which only looked their record up: 113).
+constexpr uint64_t kCmpSeg = 4096;
+constexpr int kCmpWarps = 8;
+__global__ void __launch_bounds__(32 * kCmpWarps)
+    k_tab_cmp(const uint8_t *base, uint64_t bytes, const uint64_t *rs, const uint64_t *rl,
+              RoundList L, const uint64_t *dup, const uint64_t *pairs,
+              const unsigned long long *n_pairs, uint64_t segs, uint32_t *differs) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t nwarps = (uint64_t)gridDim.x * kCmpWarps, jobs = *n_pairs * segs;
+  const uint64_t lo = reinterpret_cast<uint64_t>(base);
+  for (uint64_t job = (uint64_t)blockIdx.x * kCmpWarps + (threadIdx.x >> 5); job < jobs; job += nwarps) {
+    const uint64_t k = job / segs, i = pairs[k], r = L.at(i), rep = dup[r];
+    // the record's bytes in 4 KB of aligned memory
+    const uint64_t len = rl[r], P = lo + rs[r], j = job - k * segs;
+    const uint64_t o = j ? j * kCmpSeg - (P & 15u) : 0, e = (j + 1) * kCmpSeg - (P & 15u);
+    if (o >= len) continue;
+    const uint32_t sl = (uint32_t)((len < e ? len : e) - o);
+    const bool eq = warp_equal(P + o, lo + rs[rep] + o, sl, lo, lo + bytes, lane);
+    if (!eq && lane == 0) differs[i] = 1u;
+  }
+}
+
+// Which records are the first of their kind: a bit each (bits, a word per 32
+// records), those before each word in its tile of 256 (pre), and the tiles'
+// sums. A record unlike the first of its hash (differs) goes to `next` and is
+// none for now.
+constexpr int kDupTile = 256;
+__global__ void __launch_bounds__(kDupTile)
+    k_dup_flags(uint64_t r0, uint64_t R, const uint32_t *differs, uint64_t *dup, uint64_t *next,
+                unsigned long long *next_cnt, uint32_t *bits, uint32_t *pre, uint64_t *sums) {
+  __shared__ uint32_t warp_n[kDupTile / 32];
+  const uint64_t i = (uint64_t)blockIdx.x * kDupTile + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  bool first = false;
+  if (i < R) {
+    first = dup[r0 + i] == r0 + i;
+    if (differs && differs[i]) {
+      next[atomicAdd(next_cnt, 1ull)] = r0 + i;
+      dup[r0 + i] = kEmpty;
+    }
+  }
+  const uint32_t word = __ballot_sync(0xffffffffu, first);
+  if (lane == 0) warp_n[warp] = __popc(word);
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kDupTile / 32; ++w) {
+    if (w < warp) before += warp_n[w];
+    all += warp_n[w];
+  }
+  if (lane == 0 && i < R) {
+    bits[i >> 5] = word;
+    pre[i >> 5] = before;
+  }
+  if (threadIdx.x == 0) sums[blockIdx.x] = all;
+}
+
+// The records' rows: the first records numbered in order from k0 (their list
+// unique_rec and their rows), the others the row of their first record, which
+// may be one of the records before r0 (rowid of those is there).
+__global__ void k_dup_number(uint64_t r0, uint64_t R, uint64_t k0, const uint64_t *dup,
+                             const uint32_t *bits, const uint32_t *pre, const uint64_t *sums,
+                             uint64_t *rowid, uint64_t *unique_rec) {
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (i >= R) return;
+  const uint64_t d = dup[r0 + i];
+  if (d == kEmpty) return;  // of the next round
+  if (d < r0) {
+    rowid[r0 + i] = rowid[d];
     return;
   }
-  const uint64_t o = seg * seg_bytes;
-  if (o >= len) return;
-  const uint64_t sl = len - o < seg_bytes ? len - o : seg_bytes;
-  const uint64_t lo = reinterpret_cast<uint64_t>(base);
-  const bool eq = warp_equal(lo + rs[r] + o, lo + rs[rep] + o, (uint32_t)sl, lo, lo + bytes, lane);
-  if (!eq && lane == 0) differs[i] = 1u;
+  const uint64_t x = d - r0;
+  const uint64_t row =
+      k0 + sums[x / kDupTile] + pre[x >> 5] + __popc(bits[x >> 5] & ((1u << (x & 31)) - 1u));
+  rowid[r0 + i] = row;
+  if (d == r0 + i) unique_rec[row] = d;
 }
 
-__global__ void k_tab_resolve(const uint64_t *list, uint64_t cnt, const uint64_t *rep_out,
-                              const uint32_t *differs, uint64_t *dup, uint64_t *next,
-                              unsigned long long *next_cnt) {
+// The records of a round of equal hash but other bytes, for the next round
+__global__ void k_dup_next(RoundList L, const uint32_t *differs, uint64_t *next,
+                           unsigned long long *next_cnt) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= cnt) return;
-  const uint64_t r = list ? list[i] : i, rep = rep_out[i];
-  if (rep == r) {
-    dup[r] = r;
-  } else if (!differs[i]) {
-    dup[r] = rep;
-  } else {
-    next[atomicAdd(next_cnt, 1ull)] = r;
-  }
-}
-
-__global__ void k_unique_flags(const uint64_t *dup, uint64_t R, uint32_t *flag) {
-  uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (r < R) flag[r] = dup[r] == r ? 1u : 0u;
-}
-
-__global__ void k_number(const uint64_t *dup, const uint64_t *uidx, uint64_t R, uint64_t *seqidx,
-                         uint64_t *unique_rec) {
-  uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  seqidx[r] = uidx[dup[r]];
-  if (dup[r] == r) unique_rec[uidx[r]] = r;
+  if (i < L.cnt && differs[i]) next[atomicAdd(next_cnt, 1ull)] = L.at(i);
 }
 
 namespace {
-// One verify round over `cnt` list records (k_tab_cmp + k_tab_resolve).
-void verify_round(hd_ctx *ctx, const Records &rec, const uint64_t *hash, const uint64_t *list,
-                  uint64_t cnt, const unsigned long long *keys, const unsigned long long *mins,
-                  uint64_t mask, uint64_t *dup, uint64_t *next, unsigned long long *next_cnt) {
-  if (!cnt) return;
+// Scratch of duplicate removal for records [0, R): the counts (pairs to
+// compare, records for the next round, first records) and per-record marks,
+// zeroed together, then the rest
+struct DupScratch {
+  DevBuf buf;
+  unsigned long long *counts;  // 3
+  uint32_t *differs, *bits, *pre;
+  uint64_t *pairs, *next, *sums;
+  uint64_t zeroed;  // bytes from counts on
+  DupScratch(uint64_t R, cudaStream_t st) {
+    const uint64_t words = ceil_div(R, (uint64_t)32), tiles = ceil_div(R, (uint64_t)kDupTile);
+    zeroed = round_up(32 + R * 4, 16);
+    buf = DevBuf(zeroed + 2 * R * 8 + tiles * 8 + words * 8, st, true);
+    uint8_t *b = buf.as<uint8_t>();
+    counts = reinterpret_cast<unsigned long long *>(b);
+    differs = reinterpret_cast<uint32_t *>(b + 32);
+    pairs = reinterpret_cast<uint64_t *>(b + zeroed);
+    next = pairs + R;
+    sums = next + R;
+    bits = reinterpret_cast<uint32_t *>(sums + tiles);
+    pre = bits + words;
+  }
+};
+// Inserts a round's records, finds their first records and compares.
+void compare_round(hd_ctx *ctx, const Records &rec, const RoundList &L, uint64_t *hash,
+                   unsigned long long *keys, unsigned long long *mins, uint64_t mask, uint64_t *dup,
+                   const DupScratch &sc) {
   cudaStream_t st = ctx->stream;
-  constexpr uint64_t kSeg = 4096;  // bytes compared per warp
-  const uint64_t segs = ceil_div(rec.max_len ? rec.max_len : 1, kSeg);
-  DevBuf rep(cnt * 8, st), differs(cnt * 4, st);
-  HD_CUDA(cudaMemsetAsync(differs.p, 0, cnt * 4, st));
-  k_tab_cmp<<<grid_for(cnt * segs * 32, 256), 256, 0, st>>>(
-      rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), rec.rec_len.as<uint64_t>(), hash, list, cnt,
-      keys, mins, mask, kSeg, segs, rep.as<uint64_t>(), differs.as<uint32_t>());
+  const uint64_t *rs = rec.rec_start.as<uint64_t>(), *rl = rec.rec_len.as<uint64_t>();
+  k_tab_insert<<<grid_for(L.cnt, 256), 256, 0, st>>>(hash, rl, L, keys, mins, mask);
   HD_LAUNCHED(ctx);
-  k_tab_resolve<<<grid_for(cnt, 256), 256, 0, st>>>(list, cnt, rep.as<uint64_t>(),
-                                                   differs.as<uint32_t>(), dup, next, next_cnt);
+  k_tab_find<<<grid_for(L.cnt, 256), 256, 0, st>>>(hash, rl, L, keys, mins, mask, dup, sc.pairs,
+                                                   sc.counts, sc.differs);
+  HD_LAUNCHED(ctx);
+  const uint64_t segs = ceil_div(rec.max_len + 15, kCmpSeg);
+  const uint64_t blocks = ceil_div(L.cnt * segs, (uint64_t)kCmpWarps);
+  k_tab_cmp<<<(unsigned)std::min<uint64_t>(blocks, (uint64_t)ctx->sm_count * 8), 32 * kCmpWarps, 0,
+              st>>>(rec.base, rec.bytes, rs, rl, L, dup, sc.pairs, sc.counts, segs, sc.differs);
+  HD_LAUNCHED(ctx);
+}
+// Numbers the first records among [r0, r0 + R) from k0 on, from dup; those
+// marked in sc.differs are left for another round if `check`
+void number_round(hd_ctx *ctx, uint64_t r0, uint64_t R, uint64_t k0, uint64_t *dup, bool check,
+                  const DupScratch &sc, uint64_t *rowid, uint64_t *unique_rec) {
+  cudaStream_t st = ctx->stream;
+  const uint64_t tiles = ceil_div(R, (uint64_t)kDupTile);
+  k_dup_flags<<<(unsigned)tiles, kDupTile, 0, st>>>(r0, R, check ? sc.differs : nullptr, dup, sc.next,
+                                                    sc.counts + 1, sc.bits, sc.pre, sc.sums);
+  HD_LAUNCHED(ctx);
+  k_scan_top<void><<<1, 1024, 0, st>>>(sc.sums, tiles, reinterpret_cast<uint64_t *>(sc.counts) + 2);
+  HD_LAUNCHED(ctx);
+  k_dup_number<<<grid_for(R, 256), 256, 0, st>>>(r0, R, k0, dup, sc.bits, sc.pre, sc.sums, rowid,
+                                                 unique_rec);
   HD_LAUNCHED(ctx);
 }
 }  // namespace
 
+// One round and its numbering are queued together, with one wait: a second
+// round is needed only where two records of one hash differ.
 DevBuf dedupe(hd_ctx *ctx, const Records &rec, uint64_t *n_unique, std::vector<uint64_t> &seqidx) {
   cudaStream_t st = ctx->stream;
   const uint64_t R = rec.n;
-  seqidx.assign(R, 0);
+  seqidx.resize(R);
   DevBuf unique_rec((R ? R : 1) * 8, st);
   if (R == 0) {
     *n_unique = 0;
@@ -881,87 +1058,58 @@ DevBuf dedupe(hd_ctx *ctx, const Records &rec, uint64_t *n_unique, std::vector<u
   }
   uint64_t T = 64;
   while (T < 2 * R) T <<= 1;
-  DevBuf hash(R * 8, st), dup(R * 8, st), keys(T * 8, st), mins(T * 8, st);
-  DevBuf lists[2] = {DevBuf(R * 8, st), DevBuf(R * 8, st)};
-  DevBuf cnt(8, st);
-  hash_records(ctx, rec, rec.rec_start.as<uint64_t>(), rec.rec_len.as<uint64_t>(), R,
-               hash.as<uint64_t>());
-  uint64_t todo = R;
-  const uint64_t *list = nullptr;
-  for (int round = 0; todo; ++round) {
-    uint64_t *next = lists[round & 1].as<uint64_t>();
-    HD_CUDA(cudaMemsetAsync(keys.p, 0xff, T * 8, st));
-    HD_CUDA(cudaMemsetAsync(mins.p, 0xff, T * 8, st));
-    HD_CUDA(cudaMemsetAsync(cnt.p, 0, 8, st));
-    k_tab_insert<<<grid_for(todo, 256), 256, 0, st>>>(hash.as<uint64_t>(), list, todo,
-                                                      keys.as<unsigned long long>(),
-                                                      mins.as<unsigned long long>(), T - 1);
-    HD_LAUNCHED(ctx);
-    verify_round(ctx, rec, hash.as<uint64_t>(), list, todo, keys.as<unsigned long long>(),
-                 mins.as<unsigned long long>(), T - 1, dup.as<uint64_t>(), next,
-                 cnt.as<unsigned long long>());
-    uint64_t left = 0;
-    HD_CUDA(cudaMemcpyAsync(&left, cnt.p, 8, cudaMemcpyDeviceToHost, st));
+  DevBuf recs(3 * R * 8, st, true), table(2 * T * 8, st, true);
+  uint64_t *hash = recs.as<uint64_t>(), *dup = hash + R, *rowid = dup + R;
+  unsigned long long *keys = table.as<unsigned long long>(), *mins = keys + T;
+  DupScratch sc(R, st);
+  HD_CUDA(cudaMemsetAsync(hash, 0, R * 8, st));
+  HD_CUDA(cudaMemsetAsync(sc.counts, 0, sc.zeroed, st));
+  HD_CUDA(cudaMemsetAsync(keys, 0xff, 2 * T * 8, st));
+  hash_records(ctx, rec, rec.rec_start.as<uint64_t>(), rec.rec_len.as<uint64_t>(), R, hash);
+  compare_round(ctx, rec, RoundList{nullptr, 0, R}, hash, keys, mins, T - 1, dup, sc);
+  number_round(ctx, 0, R, 0, dup, true, sc, rowid, unique_rec.as<uint64_t>());
+  uint64_t *h = pinned_words(ctx);
+  auto fetch = [&] {
+    HD_CUDA(cudaMemcpyAsync(h, sc.counts, 24, cudaMemcpyDeviceToHost, st));
+    HD_CUDA(cudaMemcpyAsync(seqidx.data(), rowid, R * 8, cudaMemcpyDeviceToHost, st));
     HD_CUDA(cudaStreamSynchronize(st));
-    if (left >= todo) fail(HD_ERR_CUDA, "duplicate removal made no progress");
-    todo = left;
-    list = next;
+  };
+  fetch();
+  if (h[1]) {
+    DevBuf lists[2] = {DevBuf(h[1] * 8, st), DevBuf(h[1] * 8, st)};
+    HD_CUDA(cudaMemcpyAsync(lists[0].p, sc.next, h[1] * 8, cudaMemcpyDeviceToDevice, st));
+    uint64_t todo = h[1];
+    for (int round = 0; todo; ++round) {
+      const RoundList L{lists[round & 1].as<uint64_t>(), 0, todo};
+      HD_CUDA(cudaMemsetAsync(sc.counts, 0, 32 + todo * 4, st));
+      HD_CUDA(cudaMemsetAsync(keys, 0xff, 2 * T * 8, st));
+      compare_round(ctx, rec, L, hash, keys, mins, T - 1, dup, sc);
+      k_dup_next<<<grid_for(todo, 256), 256, 0, st>>>(
+          L, sc.differs, lists[(round + 1) & 1].as<uint64_t>(), sc.counts + 1);
+      HD_LAUNCHED(ctx);
+      HD_CUDA(cudaMemcpyAsync(h, sc.counts, 16, cudaMemcpyDeviceToHost, st));
+      HD_CUDA(cudaStreamSynchronize(st));
+      if (h[1] >= todo) fail(HD_ERR_CUDA, "duplicate removal made no progress");
+      todo = h[1];
+    }
+    number_round(ctx, 0, R, 0, dup, false, sc, rowid, unique_rec.as<uint64_t>());
+    fetch();
   }
-  DevBuf flag(R * 4, st), uidx(R * 8, st), tot(8, st), d_seqidx(R * 8, st);
-  k_unique_flags<<<grid_for(R, 256), 256, 0, st>>>(dup.as<uint64_t>(), R, flag.as<uint32_t>());
-  HD_LAUNCHED(ctx);
-  scan_exclusive<uint32_t>(ctx, flag.as<uint32_t>(), uidx.as<uint64_t>(), R, tot.as<uint64_t>());
-  k_number<<<grid_for(R, 256), 256, 0, st>>>(dup.as<uint64_t>(), uidx.as<uint64_t>(), R,
-                                             d_seqidx.as<uint64_t>(), unique_rec.as<uint64_t>());
-  HD_LAUNCHED(ctx);
-  HD_CUDA(cudaMemcpyAsync(n_unique, tot.p, 8, cudaMemcpyDeviceToHost, st));
-  HD_CUDA(cudaMemcpyAsync(seqidx.data(), d_seqidx.p, R * 8, cudaMemcpyDeviceToHost, st));
-  HD_CUDA(cudaStreamSynchronize(st));
+  *n_unique = h[2];
   return unique_rec;
 }
 
 // ------------------------------------------- incremental duplicate removal
-__global__ void k_iota(uint64_t *out, uint64_t start, uint64_t n) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i < n) out[i] = start + i;
-}
-__global__ void k_inc_flags(const uint64_t *dup, uint64_t r0, uint64_t m, uint32_t *flag) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i < m) flag[i] = dup[r0 + i] == r0 + i ? 1u : 0u;
-}
-// new unique record r0 + i gets row k0 + uidx[i]
-__global__ void k_inc_number(const uint64_t *dup, const uint64_t *uidx, uint64_t r0, uint64_t m,
-                             uint64_t k0, uint64_t *rowid, uint64_t *unique_rec) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= m || dup[r0 + i] != r0 + i) return;
-  rowid[r0 + i] = k0 + uidx[i];
-  unique_rec[k0 + uidx[i]] = r0 + i;
-}
-// a new duplicate gets the row of its first occurrence (earlier, or new and
-// numbered by k_inc_number)
-__global__ void k_inc_link(const uint64_t *dup, uint64_t r0, uint64_t m, uint64_t *rowid) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i < m && dup[r0 + i] != r0 + i) rowid[r0 + i] = rowid[dup[r0 + i]];
-}
-
 void IncDedupe::init(hd_ctx *ctx, uint64_t capacity) {
   cudaStream_t st = ctx->stream;
   cap = capacity ? capacity : 1;
   T = 64;
   while (T < 2 * cap) T <<= 1;
-  hash = DevBuf(cap * 8, st);
-  dup = DevBuf(cap * 8, st);
-  rowid = DevBuf(cap * 8, st);
-  unique_rec = DevBuf(cap * 8, st);
-  list = DevBuf(cap * 8, st);
-  next = DevBuf(cap * 8, st);
-  flag = DevBuf(cap * 4, st);
-  uidx = DevBuf(cap * 8, st);
-  keys = DevBuf(T * 8, st);
-  mins = DevBuf(T * 8, st);
-  cnt = DevBuf(16, st);
-  HD_CUDA(cudaMemsetAsync(keys.p, 0xff, T * 8, st));
-  HD_CUDA(cudaMemsetAsync(mins.p, 0xff, T * 8, st));
+  recs = DevBuf(3 * cap * 8, st, true);
+  unique_rec = DevBuf(cap * 8, st, true);
+  table = DevBuf(2 * T * 8, st, true);
+  HD_CUDA(cudaMemsetAsync(recs.p, 0, cap * 8, st));  // the hashes
+  HD_CUDA(cudaMemsetAsync(table.p, 0xff, 2 * T * 8, st));
   seen = 0;
   n_unique = 0;
 }
@@ -971,34 +1119,21 @@ bool IncDedupe::add(hd_ctx *ctx, const Records &rec) {
   const uint64_t r0 = seen, m = rec.n - seen;
   if (rec.n < seen || rec.n > cap) return false;
   if (m == 0) return true;
-  uint64_t *hp = hash.as<uint64_t>(), *lp = list.as<uint64_t>();
+  uint64_t *hash = recs.as<uint64_t>(), *dup = hash + cap, *rowid = dup + cap;
+  unsigned long long *keys = table.as<unsigned long long>(), *mins = keys + T;
+  DupScratch sc(m, st);
+  HD_CUDA(cudaMemsetAsync(sc.counts, 0, sc.zeroed, st));
   hash_records(ctx, rec, rec.rec_start.as<uint64_t>() + r0, rec.rec_len.as<uint64_t>() + r0, m,
-               hp + r0);
-  k_iota<<<grid_for(m, 256), 256, 0, st>>>(lp, r0, m);
-  HD_LAUNCHED(ctx);
+               hash + r0);
   // earlier records hold the smaller indices: they stay each hash's minimum
-  k_tab_insert<<<grid_for(m, 256), 256, 0, st>>>(hp, lp, m, keys.as<unsigned long long>(),
-                                                 mins.as<unsigned long long>(), T - 1);
-  HD_LAUNCHED(ctx);
-  HD_CUDA(cudaMemsetAsync(cnt.p, 0, 16, st));
-  verify_round(ctx, rec, hp, lp, m, keys.as<unsigned long long>(), mins.as<unsigned long long>(),
-               T - 1, dup.as<uint64_t>(), next.as<uint64_t>(), cnt.as<unsigned long long>());
-  k_inc_flags<<<grid_for(m, 256), 256, 0, st>>>(dup.as<uint64_t>(), r0, m, flag.as<uint32_t>());
-  HD_LAUNCHED(ctx);
-  scan_exclusive<uint32_t>(ctx, flag.as<uint32_t>(), uidx.as<uint64_t>(), m,
-                           cnt.as<uint64_t>() + 1);
-  uint64_t h[2] = {0, 0};  // unresolved records, new unique rows
-  HD_CUDA(cudaMemcpyAsync(h, cnt.p, 16, cudaMemcpyDeviceToHost, st));
+  compare_round(ctx, rec, RoundList{nullptr, r0, m}, hash, keys, mins, T - 1, dup, sc);
+  number_round(ctx, r0, m, n_unique, dup, true, sc, rowid, unique_rec.as<uint64_t>());
+  uint64_t *h = pinned_words(ctx);
+  HD_CUDA(cudaMemcpyAsync(h, sc.counts, 24, cudaMemcpyDeviceToHost, st));
   HD_CUDA(cudaStreamSynchronize(st));
   // a new record unlike the first record of its hash: the full dedupe decides
-  if (h[0]) return false;
-  k_inc_number<<<grid_for(m, 256), 256, 0, st>>>(dup.as<uint64_t>(), uidx.as<uint64_t>(), r0, m,
-                                                 n_unique, rowid.as<uint64_t>(),
-                                                 unique_rec.as<uint64_t>());
-  HD_LAUNCHED(ctx);
-  k_inc_link<<<grid_for(m, 256), 256, 0, st>>>(dup.as<uint64_t>(), r0, m, rowid.as<uint64_t>());
-  HD_LAUNCHED(ctx);
-  n_unique += h[1];
+  if (h[1]) return false;
+  n_unique += h[2];
   seen = rec.n;
   return true;
 }
@@ -1006,7 +1141,7 @@ bool IncDedupe::add(hd_ctx *ctx, const Records &rec) {
 void IncDedupe::rows(hd_ctx *ctx, std::vector<uint64_t> &seqidx) {
   seqidx.resize(seen);
   if (!seen) return;
-  HD_CUDA(cudaMemcpyAsync(seqidx.data(), rowid.p, seen * 8, cudaMemcpyDeviceToHost, ctx->stream));
+  HD_CUDA(cudaMemcpyAsync(seqidx.data(), rowid(), seen * 8, cudaMemcpyDeviceToHost, ctx->stream));
   HD_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 

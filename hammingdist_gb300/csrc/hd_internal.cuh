@@ -477,12 +477,15 @@ DevBuf dedupe(hd_ctx *ctx, const Records &rec, uint64_t *n_unique, std::vector<u
 // verifies only the records after them. Earlier records hold the smaller
 // indices, so they stay the first occurrences and their rows keep their
 // numbers; unique_rec lists the unique rows' records (n_unique of them) and
-// rowid (device) each record's row, which rows() copies to the host. A new
+// recs holds (device) each record's row, which rows() copies to the host. A new
 // record unlike the first record of its hash (a 64-bit collision), or more
 // records than the capacity, makes add() return false: the caller runs the
 // full dedupe.
 struct IncDedupe {
-  DevBuf hash, dup, rowid, unique_rec, list, next, flag, uidx, keys, mins, cnt;
+  DevBuf recs;        // hash, first record and row of each record (cap each)
+  DevBuf unique_rec;  // the unique rows' records
+  DevBuf table;       // T hashes and their first records
+  const uint64_t *rowid() const { return recs.as<uint64_t>() + 2 * cap; }
   uint64_t cap = 0, T = 0, seen = 0, n_unique = 0;
   void init(hd_ctx *ctx, uint64_t capacity);
   bool add(hd_ctx *ctx, const Records &rec);
