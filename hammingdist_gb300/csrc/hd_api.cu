@@ -1422,8 +1422,8 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
                            hd::pack_operand(ctx, all, rows + K, owner.get(), K, Kc,
                                             keep_planes.as<uint4>(), ctx->stream, R_max);
       if (!with_op)
-        hd::pack_rows_and(ctx, all, rows + K, Kc - K, L, words, g0 + K * words,
-                          keep_planes.as<uint4>() + K * words);
+        hd::pack_planes(ctx, all, rows + K, Kc - K, L, words, g0 + K * words,
+                        keep_planes.as<uint4>() + K * words);
       hd::trace_host(ctx, "part " + std::to_string(c + 1) + " packing queued");
       if (use_mma && Kc >= 2 && !hd::ensure_operand(ctx, owner.get(), Kc, ctx->stream, R_max)) {
         use_mma = false;
@@ -1609,7 +1609,9 @@ int hd_pairwise_lt(hd_ctx *ctx, const hd_alignment *aln, int dtype_bytes, int64_
     // the tensor-core engine's operand and the launch plan (item lists,
     // tensor maps, job tables) first, so that the timing below is the
     // distance kernel's alone
-    if (!aln->base && hd::mma_wanted(ctx, aln) && hd::ensure_operand(ctx, aln, n, ctx->stream))
+    if (hd::ensure_sites(ctx, aln, ctx->stream))
+      hd::trace_mark(ctx, "site lists");
+    else if (!aln->base && hd::mma_wanted(ctx, aln) && hd::ensure_operand(ctx, aln, n, ctx->stream))
       hd::trace_mark(ctx, "FP4 operand");
     hd::PairLaunchPlan plan;
     hd::plan_pairwise_tiles(ctx, aln, dtype_bytes, md, d_out, 0, 0, nb, &plan);

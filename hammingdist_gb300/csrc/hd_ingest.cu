@@ -1275,112 +1275,6 @@ __global__ void __launch_bounds__(kPackThreads)
   }
 }
 
-// AND-rule packer: a warp job is one 1024-site chunk of one row, and lane l
-// builds its 32-site word l from the chunk's bytes [32 l, 32 l + 32), read as
-// aligned 16-byte vectors (two of its own and the next lane's first;
-// realigned by the row's offset mod 16 with funnel shifts). A 256-entry table
-// in shared memory gives each byte its code (A, C, G, T one-hot, '-' 1111,
-// every other byte 0, as in src/hamming_impl.cc:23-44) with plane p's bit at
-// bit 8 p. Summed with weights 1, 2, 4, 8 over 4 sites, and 16 for the next 4,
-// byte p of the sum holds plane p's bits of 8 sites; four such sums give each
-// plane word by byte permutes. Sites past L get the '-' code.
-__global__ void __launch_bounds__(256)
-    k_pack_and(const uint8_t *base, uint64_t bytes, const uint64_t *rs, const uint64_t *rows,
-               uint64_t n_rows, uint64_t L, uint64_t words, uint4 *g0, uint4 *g1) {
-  __shared__ uint32_t spread[256];
-  {
-    const uint32_t b = threadIdx.x;  // the block has 256 threads
-    const uint32_t c = b == 'A' ? 1u : b == 'C' ? 2u : b == 'G' ? 4u : b == 'T' ? 8u : b == '-' ? 15u : 0u;
-    spread[b] = (c & 1u) | ((c & 2u) << 7) | ((c & 4u) << 14) | ((c & 8u) << 21);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const uint64_t lo = reinterpret_cast<uint64_t>(base), hi = lo + bytes;
-  const uint64_t chunks = (words + 31) / 32;
-  const uint64_t wid = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
-  for (uint64_t job = wid; job < n_rows * chunks; job += nwarps) {
-    const uint64_t u = job / chunks, q = job - u * chunks;
-    const uint64_t r = rows ? rows[u] : u;
-    const uint64_t P0 = lo + rs[r] + q * 1024;  // the chunk's first byte
-    const uint64_t A = P0 & ~15ull;
-    const uint32_t d = (uint32_t)(P0 - A), dw = d >> 2, db = d & 3u;
-    const int64_t rem64 = (int64_t)L - (int64_t)(q * 1024);
-    const uint32_t rem = rem64 <= 0 ? 0u : (rem64 >= 1024 ? 1024u : (uint32_t)rem64);
-    const uint64_t la = A + 32ull * lane;
-    uint32_t w[12];
-    {
-      const uint4 v0 = rem ? load16_in(la, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
-      const uint4 v1 = rem ? load16_in(la + 16, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
-      uint4 v2;
-      v2.x = __shfl_down_sync(0xffffffffu, v0.x, 1);
-      v2.y = __shfl_down_sync(0xffffffffu, v0.y, 1);
-      v2.z = __shfl_down_sync(0xffffffffu, v0.z, 1);
-      v2.w = __shfl_down_sync(0xffffffffu, v0.w, 1);
-      if (lane == 31) v2 = (rem && d) ? load16_in(la + 32, lo, hi) : make_uint4(0u, 0u, 0u, 0u);
-      w[0] = v0.x; w[1] = v0.y; w[2] = v0.z; w[3] = v0.w;
-      w[4] = v1.x; w[5] = v1.y; w[6] = v1.z; w[7] = v1.w;
-      w[8] = v2.x; w[9] = v2.y; w[10] = v2.z; w[11] = v2.w;
-    }
-    // the 36 bytes from byte 4 dw (dw is the same in the whole warp)
-    uint32_t x[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) x[k] = w[k];
-    if (dw == 1) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) x[k] = w[k + 1];
-    } else if (dw == 2) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) x[k] = w[k + 2];
-    } else if (dw == 3) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) x[k] = w[k + 3];
-    }
-    const uint32_t s0 = 32u * lane;  // chunk-relative site of this lane's first byte
-    uint32_t pair[4];  // byte p: plane p's bits of sites 8 m .. 8 m + 7
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      uint32_t e2 = 0;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int k = 2 * m + h;
-        uint32_t y = __funnelshift_r(x[k], x[k + 1], 8 * db);
-        const uint32_t sk = s0 + 4 * k;
-        if (sk + 4 > rem) {  // past the row's end: '-'
-          const uint32_t keep = sk >= rem ? 0u : (0xFFFFFFFFu >> (8 * (sk + 4 - rem)));
-          y = (y & keep) | (0x2D2D2D2Du & ~keep);
-        }
-        const uint32_t e = spread[y & 0xFFu] + 2u * spread[(y >> 8) & 0xFFu] +
-                           4u * spread[(y >> 16) & 0xFFu] + 8u * spread[y >> 24];
-        e2 += e << (4 * h);
-      }
-      pair[m] = e2;
-    }
-    uint32_t pl[4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const uint32_t lo2 = __byte_perm(pair[0], pair[1], (uint32_t)p | ((uint32_t)(4 + p) << 4));
-      const uint32_t hi2 = __byte_perm(pair[2], pair[3], (uint32_t)p | ((uint32_t)(4 + p) << 4));
-      pl[p] = __byte_perm(lo2, hi2, 0x5410u);
-    }
-    const uint64_t wi = q * 32 + lane;
-    if (wi < words) {
-      const uint4 v = make_uint4(pl[0], pl[1], pl[2], pl[3]);
-      g0[u * words + wi] = v;
-      if (g1) g1[u * words + wi] = v;
-    }
-  }
-}
-
-void pack_rows_and(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, uint64_t n_rows,
-                   uint64_t length, uint64_t words, uint4 *g0, uint4 *g1) {
-  if (!n_rows) return;
-  const uint64_t jobs = n_rows * ((words + 31) / 32);
-  k_pack_and<<<grid_for(jobs * 32, 256), 256, 0, ctx->stream>>>(
-      rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), d_rows, n_rows, length, words, g0, g1);
-  HD_LAUNCHED(ctx);
-}
-
 __global__ void k_concat_starts(const uint64_t *a, uint64_t na, const uint64_t *b, uint64_t nb,
                                 uint64_t b_off, uint64_t *out) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -1424,17 +1318,25 @@ void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_align
   aln->plane_buf[0] = DevBuf(bytes ? bytes : 16, ctx->stream);
   if (aln->groups > 1) aln->plane_buf[1] = DevBuf(bytes ? bytes : 16, ctx->stream);
   if (!aln->n_rows) return;
-  if (compared && aln->planes == 4 && mma_wanted(ctx, aln) &&
-      pack_operand(ctx, rec, d_rows, aln, 0, aln->n_rows, nullptr, ctx->stream))
+  if (aln->planes == 4) {
+    // Compared rows come with their tensor-core operand, unless a look at some
+    // of their sites says that site lists will do
+    uint4 *g = aln->plane_buf[0].as<uint4>();
+    const uint32_t stride = compared ? sites_sample_stride(ctx, aln) : 0;
+    if (stride) pack_planes(ctx, rec, d_rows, aln->n_rows, aln->length, aln->words, g, nullptr, stride);
+    const bool lists = stride && sites_likely(ctx, aln, ctx->stream);
+    if (lists && stride == 1) return;
+    if (compared && !lists && mma_wanted(ctx, aln) &&
+        pack_operand(ctx, rec, d_rows, aln, 0, aln->n_rows, nullptr, ctx->stream))
+      return;
+    pack_planes(ctx, rec, d_rows, aln->n_rows, aln->length, aln->words, g, nullptr);
     return;
+  }
   const uint64_t jobs = aln->n_rows * hd::ceil_div((aln->words + 31) / 32, (uint64_t)kPackCPG);
   unsigned grid = grid_for(jobs * 32, kPackThreads);
   uint4 *g0 = aln->plane_buf[0].as<uint4>(), *g1 = aln->plane_buf[1].as<uint4>();
   const uint64_t *rs = rec.rec_start.as<uint64_t>();
-  if (aln->planes == 4)
-    k_pack_and<<<grid_for(aln->n_rows * ((aln->words + 31) / 32) * 32, 256), 256, 0, ctx->stream>>>(
-        rec.base, rec.bytes, rs, d_rows, aln->n_rows, aln->length, aln->words, g0, nullptr);
-  else if (aln->planes == 5)
+  if (aln->planes == 5)
     k_pack<5><<<grid, kPackThreads, 0, ctx->stream>>>(rec.base, rs, d_rows, aln->n_rows, aln->length,
                                              aln->words, t, g0, g1);
   else

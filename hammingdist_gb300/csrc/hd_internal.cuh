@@ -207,6 +207,33 @@ inline unsigned long long *mma_mac_counter(const hd_ctx *ctx) {
 }
 }  // namespace hd
 
+namespace hd {
+// The lists of an alignment's sites where a row differs from a reference, by
+// tiles of rows and ranges of sites (hd_sites.cu), and what a sample of the
+// sites said about them.
+struct SiteLists {
+  int verdict = 0;  // 0: not looked at, 1: the distances use them, -1: they do not
+  double est_s = 0, est_d = 0, est_xd = 0;  // entries, and meetings with '-', from the sample
+  uint32_t tiles = 0, ranges = 0;           // tiles > 0: built
+  uint32_t zero = 0;                        // sites that every pair mismatches in
+  DevBuf base, off, es, ed, weight;
+  void release() {
+    for (DevBuf *b : {&base, &off, &es, &ed, &weight}) b->release();
+  }
+};
+// A launch over them (by value to its kernel)
+struct SiteJob {
+  const uint4 *base;
+  const uint16_t *off;
+  const uint32_t *es;
+  const uint8_t *ed;
+  const uint32_t *weight;
+  void *out;  // lt index out_base at out[0]
+  unsigned long long out_base, row_lo, row_hi, first, n;
+  uint32_t ranges, zero, max_dist, dtype;
+};
+}  // namespace hd
+
 struct hd_alignment {
   hd_ctx *ctx = nullptr;  // creating context; may be destroyed before the alignment
   int device = 0;
@@ -235,6 +262,8 @@ struct hd_alignment {
   // the marked chunks' list and ranks after each extension of the operand,
   // the last one current
   mutable std::vector<hd::DevBuf> op_lists;
+  // built on first use, where the distances use them (hd_sites.cu)
+  mutable std::unique_ptr<hd::SiteLists> sites;
   // Freed on the null stream: every API call has synchronised its own stream
   // before returning, so no queued work still reads these buffers, and the
   // creating context (and its streams) may already be gone.
@@ -253,6 +282,11 @@ struct hd_alignment {
       b.s = nullptr;
       b.release();
     }
+    if (sites)
+      for (auto *b : {&sites->base, &sites->off, &sites->es, &sites->ed, &sites->weight}) {
+        b->s = nullptr;
+        b->release();
+      }
   }
 };
 
@@ -499,10 +533,6 @@ uint64_t consensus_matches(hd_ctx *ctx, const Records &rec, const uint64_t *d_ro
 // tensor-core operand is written along with the planes if they will use it
 void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_alignment *aln,
                bool compared);
-// AND-rule planes of n_rows records (d_rows: record indices) into g0, and
-// into g1 too unless it is null (n_rows x words uint4 each, already allocated)
-void pack_rows_and(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, uint64_t n_rows,
-                   uint64_t length, uint64_t words, uint4 *g0, uint4 *g1 = nullptr);
 // records of a then b (b's starts shifted by b_off), one base; b parsed from
 // bytes that follow a's in the same buffer
 Records concat_records(hd_ctx *ctx, const Records &a, const Records &b, uint64_t b_off,
@@ -558,6 +588,8 @@ struct PairLaunchPlan {
     const void *d_fix = nullptr;   // tiles split along K, `fixes` of them, and
     uint64_t fixes = 0;            // their pieces' workspace
     void *d_ws = nullptr;
+    bool sites = false;            // by site lists (hd_sites.cu): one job, `grid` tile pairs
+    SiteJob site{};
   };
   std::vector<Launch> launches;
   std::vector<DevBuf> blocks;  // job tables + tensor maps + tile counters
@@ -590,6 +622,21 @@ uint64_t mma_min_items_for(hd_ctx *ctx, uint64_t length);
 int mma_band_of(const TileConfig &c);
 int mma_rows_of(const TileConfig &c);
 
+// sites.cu: distances from lists of the sites where a row differs from a
+// reference, for whole alignments of similar rows.
+// Whether the lists come into question for the alignment: 0, or the stride
+// (in four words) of the sites to look at. sites_likely looks at those words
+// of the planes (a wait); ensure_sites also builds the lists (another).
+uint32_t sites_sample_stride(hd_ctx *ctx, const hd_alignment *aln);
+bool sites_likely(hd_ctx *ctx, const hd_alignment *aln, cudaStream_t stream);
+bool ensure_sites(hd_ctx *ctx, const hd_alignment *aln, cudaStream_t stream);
+// launches for the specs that use them; taken[k] marks those
+void prepare_site_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaStream_t stream,
+                       PairLaunchPlan *plan, std::vector<char> &taken);
+void launch_sites(hd_ctx *ctx, const PairLaunchPlan::Launch &L, cudaStream_t stream);
+// size of the tensor-core engine's tile rows of rows [lo, hi), in tiles of 128 x 240 pairs
+uint64_t mma_size_tiles(uint64_t lo, uint64_t hi);
+
 // mma.cu: the tensor-core engine for every rule (4, 5 or 6 planes, with
 // P L < 2^24; HAMMINGDIST_KERNEL=lop3 turns it off).
 bool mma_eligible(const hd_alignment *aln);
@@ -600,6 +647,10 @@ bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStr
                 uint64_t cap_hint = 0);
 // whether the distances of the whole alignment run on the tensor-core engine
 bool mma_wanted(hd_ctx *ctx, const hd_alignment *aln);
+// packs records d_rows[0 .. n_rows) (none: 0 ..) of the AND rule into rows of
+// planes g0 (and g1, if given); stride > 1: only four words of every 4 stride
+void pack_planes(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, uint64_t n_rows,
+                 uint64_t length, uint64_t words, uint4 *g0, uint4 *g1, uint32_t stride = 1);
 // packs records d_rows[0 ..] (none: 0 ..) of the AND rule into rows [lo, hi) of
 // the alignment's planes (and of `copy`, if given) and of its operand, whose
 // earlier rows are there (op_rows == lo), in one pass over their text. False
@@ -621,6 +672,7 @@ double measure_mma_peak(hd_ctx *ctx);
 // One tensor-core launch for the specs it can take (dense AND rule, row
 // range starting on a 128-row tile, operand memory available); taken[k] marks
 // them. The plan keeps the launch's device block.
+// (specs already marked are left out).
 void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaStream_t stream,
                       PairLaunchPlan *plan, int sm_limit, std::vector<char> &taken);
 void launch_mma(hd_ctx *ctx, const PairLaunchPlan::Launch &L, cudaStream_t stream);

@@ -363,14 +363,18 @@ __device__ __forceinline__ void pack_sites(const uint32_t *v, uint32_t db, uint3
 // 14,000 rows of 29,903 sites move 1.47 GB (6.2 TB/s) in 238 us. Packing
 // and then expanding, with the planes read back and dash blocks written for
 // every chunk, took 198 + 212 us (1.9 GB).
+template <bool kOp>
 __global__ void __launch_bounds__(256, 6)
     k_pack_op(const uint8_t *base, uint64_t bytes, const uint64_t *__restrict__ rs,
               const uint64_t *__restrict__ rows, uint64_t row_lo, uint64_t row_hi, uint64_t L,
               uint32_t words, uint4 *__restrict__ g0, uint4 *__restrict__ g1,
-              uint8_t *__restrict__ x, uint32_t *dash_chunk, uint32_t ext) {
+              uint8_t *__restrict__ x, uint32_t *dash_chunk, uint32_t ext, uint32_t stride) {
   constexpr uint32_t kPlanes = 4, nb = op_blocks(kPlanes);
-  const uint32_t op_words = op_chunks(L) * kChunkWords;
-  const uint32_t w = blockIdx.x * 32 + threadIdx.x / 8;
+  const uint32_t op_words = kOp ? op_chunks(L) * kChunkWords : 0u;
+  // without the operand a warp takes 32 words of one row instead
+  const uint32_t k = blockIdx.x * 32 + (kOp ? threadIdx.x / 8 : threadIdx.x & 31u);
+  const uint32_t w = kOp ? k : (k >> 2) * 4 * stride + (k & 3u);
+  const uint32_t row = kOp ? threadIdx.x & 7u : threadIdx.x >> 5;
   if (w >= words && w >= op_words) return;
   const uint32_t c = w / kChunkWords;
   const uint64_t s0 = (uint64_t)w * 32;
@@ -384,7 +388,7 @@ __global__ void __launch_bounds__(256, 6)
     if (!valid || r < row_lo || r >= row_hi) return 0;
     return lo + s0 + rs[rows ? rows[r - row_lo] : r - row_lo];
   };
-  uint64_t r = row_lo / 8 * 8 + blockIdx.y * 8 + (threadIdx.x & 7u);
+  uint64_t r = row_lo / 8 * 8 + blockIdx.y * 8 + row;
   uint64_t next = start_of(r);
   uint8_t *blk = x + (r / 8) * group_bytes + in_group;
   const uint64_t blk_step = gridDim.y * group_bytes;
@@ -417,10 +421,21 @@ __global__ void __launch_bounds__(256, 6)
       v[8] = e.x; v[9] = e.y; v[10] = e.z; v[11] = e.w;
     }
     // the words from byte 4 dw on
+    if (kOp) {
 #pragma unroll
-    for (int k = 0; k < 11; ++k) v[k] = (dw & 1u) ? v[k + 1] : v[k];
+      for (int k = 0; k < 11; ++k) v[k] = (dw & 1u) ? v[k + 1] : v[k];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) v[k] = (dw & 2u) ? v[k + 2] : v[k];
+      for (int k = 0; k < 9; ++k) v[k] = (dw & 2u) ? v[k + 2] : v[k];
+    } else {  // the same for the whole warp but its words past the row's end, which read 0
+      if (__any_sync(__activemask(), dw & 1u)) {
+#pragma unroll
+        for (int k = 0; k < 11; ++k) v[k] = v[k + 1];
+      }
+      if (__any_sync(__activemask(), dw & 2u)) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v[k] = v[k + 2];
+      }
+    }
     uint32_t z[4], pl[4];
     if (valid == 32u) pack_sites<false>(v, db, valid, z, pl);
     else pack_sites<true>(v, db, valid, z, pl);
@@ -429,7 +444,7 @@ __global__ void __launch_bounds__(256, 6)
       g0[r * words + w] = o;
       if (g1) g1[r * words + w] = o;
     }
-    if (w < op_words) {
+    if (kOp && w < op_words) {
       constexpr uint32_t kOne = 0x22222222u;  // E2M1 1.0 in every nibble
       uint4 *out = reinterpret_cast<uint4 *>(blk);
       constexpr uint32_t kNext = kGroupBytes / 16;
@@ -1328,6 +1343,26 @@ bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStr
   return true;
 }
 
+namespace {
+// up to 8 row groups a block, while that leaves four rounds of blocks
+dim3 pack_grid(hd_ctx *ctx, uint64_t words, uint64_t lo, uint64_t hi) {
+  dim3 grid = op_grid(words, lo, hi);
+  const uint64_t rounds = (uint64_t)grid.x * grid.y / ((uint64_t)ctx->sm_count * 6 * 4);
+  grid.y = (unsigned)ceil_div(grid.y, std::min<uint64_t>(8, std::max<uint64_t>(1, rounds)));
+  return grid;
+}
+}  // namespace
+
+void pack_planes(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, uint64_t n_rows,
+                 uint64_t length, uint64_t words, uint4 *g0, uint4 *g1, uint32_t stride) {
+  if (!n_rows) return;
+  const uint64_t w = 4 * ceil_div(words, (uint64_t)4 * stride);
+  k_pack_op<false><<<pack_grid(ctx, w, 0, n_rows), 256, 0, ctx->stream>>>(
+      rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), d_rows, 0, n_rows, length,
+      (uint32_t)words, g0, g1, nullptr, nullptr, 0, stride);
+  HD_LAUNCHED(ctx);
+}
+
 bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const hd_alignment *aln,
                   uint64_t lo, uint64_t hi, uint4 *copy, cudaStream_t stream, uint64_t cap_hint) {
   if (aln->base || aln->planes != 4 || aln->op_rows != lo || hi <= lo) return false;
@@ -1337,13 +1372,9 @@ bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const
   uint8_t *x = aln->op.as<uint8_t>();
   uint32_t *marks = aln->op_dash.as<uint32_t>();
   const uint64_t op_words = (uint64_t)op_chunks(aln->length) * kChunkWords;
-  // up to 8 row groups a block, while that leaves four rounds of blocks
-  dim3 grid = op_grid(std::max(aln->words, op_words), lo, hi);
-  const uint64_t rounds = (uint64_t)grid.x * grid.y / ((uint64_t)ctx->sm_count * 6 * 4);
-  grid.y = (unsigned)ceil_div(grid.y, std::min<uint64_t>(8, std::max<uint64_t>(1, rounds)));
-  k_pack_op<<<grid, 256, 0, stream>>>(
+  k_pack_op<true><<<pack_grid(ctx, std::max(aln->words, op_words), lo, hi), 256, 0, stream>>>(
       rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), d_rows, lo, hi, aln->length,
-      (uint32_t)aln->words, g0, copy, x, marks, ext);
+      (uint32_t)aln->words, g0, copy, x, marks, ext, 1);
   HD_LAUNCHED(ctx);
   dash_rows(ctx, g0, nullptr, 4, aln->words, lo, hi, aln->length, x, marks, ext,
             aln->op_lists.back().as<uint32_t>(), stream);
@@ -1565,6 +1596,10 @@ static uint64_t size_tiles(uint64_t lo, uint64_t hi) {
   return n;
 }
 
+uint64_t mma_size_tiles(uint64_t lo, uint64_t hi) {
+  return size_tiles(lo / kTM, ceil_div(hi, (uint64_t)kTM));
+}
+
 bool mma_wanted(hd_ctx *ctx, const hd_alignment *aln) {
   if (ctx->engine_force == 0 || !mma_eligible(aln)) return false;
   const uint64_t min_items = ctx->engine_force == 1 ? 0 : mma_min_items_for(ctx, aln->length);
@@ -1573,7 +1608,7 @@ bool mma_wanted(hd_ctx *ctx, const hd_alignment *aln) {
 
 void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaStream_t stream,
                       PairLaunchPlan *plan, int sm_limit, std::vector<char> &taken) {
-  taken.assign(specs.size(), 0);
+  taken.resize(specs.size(), 0);
   std::vector<const uint8_t *> ops(specs.size(), nullptr);  // each job's operand rows
   std::vector<const uint32_t *> dash_lists(specs.size(), nullptr);  // and its listed chunks
   struct Job {
@@ -1588,8 +1623,9 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
   // still goes here when together they are enough.
   if (ctx->engine_force == 0) return;
   uint64_t items_total = 0, max_len = 0;
-  for (const PairJobSpec &sp : specs) {
-    if (!mma_eligible(sp.aln) || sp.tile_hi <= sp.tile_lo) continue;
+  for (size_t k = 0; k < specs.size(); ++k) {
+    const PairJobSpec &sp = specs[k];
+    if (taken[k] || !mma_eligible(sp.aln) || sp.tile_hi <= sp.tile_lo) continue;
     max_len = std::max<uint64_t>(max_len, sp.aln->length);
     const uint64_t edge = sp.cfg.tile > 0 ? (uint64_t)sp.cfg.tile : kTile;
     const uint64_t lo = sp.tile_lo * edge / kTM;
@@ -1601,7 +1637,7 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
   for (size_t k = 0; k < specs.size(); ++k) {
     const PairJobSpec &sp = specs[k];
     const hd_alignment *a = sp.aln;
-    if (!mma_eligible(a) || sp.tile_hi <= sp.tile_lo) continue;
+    if (taken[k] || !mma_eligible(a) || sp.tile_hi <= sp.tile_lo) continue;
     // the caller's tile rows are in units of its configuration's tile edge
     const uint64_t edge = sp.cfg.tile > 0 ? (uint64_t)sp.cfg.tile : kTile;
     const uint64_t row_lo = sp.tile_lo * edge, row_hi = std::min<uint64_t>(sp.tile_hi * edge, a->n_rows);

@@ -362,8 +362,10 @@ bool tile_config_valid(int tile, int stages) {
 // a batch captures only the launch step and replays it.
 void prepare_pairwise_jobs(hd_ctx *ctx, std::vector<PairJobSpec> &specs, cudaStream_t stream,
                            PairLaunchPlan *plan, int sm_limit) {
-  // the dense AND rule goes to the tensor-core engine, one launch for all of it
-  std::vector<char> taken;
+  // large alignments of similar rows by their site lists, the rest to the
+  // tensor-core engine, one launch for all of it
+  std::vector<char> taken(specs.size(), 0);
+  prepare_site_jobs(ctx, specs, stream, plan, taken);
   prepare_mma_jobs(ctx, specs, stream, plan, sm_limit, taken);
   struct Group {
     const Variant *v;
@@ -444,6 +446,10 @@ void prepare_pairwise_jobs(hd_ctx *ctx, std::vector<PairJobSpec> &specs, cudaStr
 
 void launch_pairwise_plan(hd_ctx *ctx, PairLaunchPlan &plan, cudaStream_t stream) {
   for (auto &L : plan.launches) {
+    if (L.sites) {
+      launch_sites(ctx, L, stream);
+      continue;
+    }
     if (L.mma) {
       launch_mma(ctx, L, stream);
       continue;
