@@ -1267,6 +1267,7 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
     uint64_t L = 0, words = 0, R_max = 0, K = 0, B_prev = 0, tiles = 0;
     uint32_t T = 0, t_done = 0;
     bool use_mma = false;  // tensor-core engine: 128-row tiles
+    bool use_sites = false;  // site lists, for all rows once the last ones are here
     // SMs left to the next part's ingest while a band runs
     // (HAMMINGDIST_STREAM_FREE_SMS, default 16)
     int free_sms = 16;
@@ -1309,6 +1310,31 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
       hd::trace_at(ctx, rows_text + " done", s);
       b->done = sync.make();
       HD_CUDA(cudaEventRecord(b->done, s));
+      bands.push_back(std::move(b));
+    };
+    // rows [lo, hi) (lo a multiple of 128) by the owner's site lists
+    auto launch_rows = [&](uint64_t lo, uint64_t hi) {
+      auto b = std::make_unique<Band>();
+      b->row_lo = lo;
+      b->row_hi = hi;
+      const std::string rows_text = "rows " + std::to_string(lo) + "-" + std::to_string(hi);
+      hd::trace_at(ctx, rows_text + " start", ctx->stream);
+      std::vector<hd::PairJobSpec> specs(1);
+      specs[0].aln = owner.get();
+      specs[0].dtype = dtype_bytes;
+      specs[0].max_dist = md;
+      specs[0].d_out = d_lt.p;
+      specs[0].cfg = cfg;
+      specs[0].cfg.tile = (int)hd::kTile;
+      specs[0].tile_lo = (uint32_t)(lo / hd::kTile);
+      specs[0].tile_hi = (uint32_t)hd::ceil_div(hi, hd::kTile);
+      ctx->last_pair_tiles = 0;
+      hd::prepare_pairwise_jobs(ctx, specs, ctx->stream, &b->plan);
+      hd::launch_pairwise_plan(ctx, b->plan, ctx->stream);
+      tiles += ctx->last_pair_tiles;
+      hd::trace_at(ctx, rows_text + " done", ctx->stream);
+      b->done = sync.make();
+      HD_CUDA(cudaEventRecord(b->done, ctx->stream));
       bands.push_back(std::move(b));
     };
     for (int c = 0;; ++c) {
@@ -1416,16 +1442,32 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
           if (!hd::tile_config_valid(cfg.tile, cfg.stages)) cfg.stages = 3;
         }
       }
+      if (c == 0) {
+        // a look at some words of the first part's rows
+        const uint64_t total = std::min<uint64_t>(R_max, (uint64_t)((double)Kc * ((double)n / (double)B)));
+        const hd::Words sel = Kc >= 512 ? hd::sites_sample(ctx, owner.get(), total) : hd::Words{};
+        if (sel.stride > 1) {
+          hd::pack_planes(ctx, all, rows, Kc, L, words, g0, nullptr, &sel);
+          use_sites = hd::sites_likely(ctx, owner.get(), ctx->stream, Kc, total);
+          hd::trace_host(ctx, "sites looked at");
+        }
+      }
       // the new rows' planes and their tensor-core operand, before the
       // launches of any stream read them
-      const bool with_op = use_mma && Kc >= 2 &&
+      const bool with_op = use_mma && !use_sites && Kc >= 2 &&
                            hd::pack_operand(ctx, all, rows + K, owner.get(), K, Kc,
                                             keep_planes.as<uint4>(), ctx->stream, R_max);
       if (!with_op)
         hd::pack_planes(ctx, all, rows + K, Kc - K, L, words, g0 + K * words,
                         keep_planes.as<uint4>() + K * words);
       hd::trace_host(ctx, "part " + std::to_string(c + 1) + " packing queued");
-      if (use_mma && Kc >= 2 && !hd::ensure_operand(ctx, owner.get(), Kc, ctx->stream, R_max)) {
+      if (last && use_sites) {
+        owner->n_rows = Kc;
+        use_sites = hd::ensure_sites(ctx, owner.get(), ctx->stream);
+        hd::trace_host(ctx, "site lists built");
+      }
+      if (use_mma && !use_sites && Kc >= 2 &&
+          !hd::ensure_operand(ctx, owner.get(), Kc, ctx->stream, R_max)) {
         use_mma = false;
         T = (uint32_t)cfg.tile;
         if (t_done) fail(HD_ERR_OOM, "no memory for the tensor-core operand of a streamed call");
@@ -1435,7 +1477,7 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
       K = Kc;
       if (!last) {
         const uint32_t t_end = (uint32_t)(K / T);
-        if (t_end > t_done) {
+        if (t_end > t_done && !use_sites) {
           cudaEvent_t packed = sync.make();
           HD_CUDA(cudaEventRecord(packed, ctx->stream));
           launch(t_done, t_end, K, ctx->side, std::max(1, ctx->sm_count - free_sms), packed);
@@ -1446,7 +1488,18 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
         continue;
       }
       const uint32_t t_end = K >= 2 ? (uint32_t)hd::ceil_div(K, T) : t_done;
-      if (t_end > t_done) {
+      if (use_sites) {
+        // four ranges of rows with about as many entries each, so that their
+        // copies overlap the later ones, at multiples of the lists' tiles of
+        // 224 rows and the specs' of 128
+        uint64_t lo = 0;
+        for (int q = 1; q <= 4 && lo < K; ++q) {
+          const uint64_t hi =
+              q < 4 ? std::max<uint64_t>(lo, (uint64_t)((double)K * std::sqrt(0.25 * q)) / 896 * 896) : K;
+          if (hi > lo) launch_rows(lo, hi);
+          lo = hi;
+        }
+      } else if (t_end > t_done) {
         const uint32_t t_split =
             std::max(t_done + 1, (uint32_t)std::ceil(0.9 * (double)t_end));
         // one after the other on the context's stream: launched on two

@@ -1322,10 +1322,12 @@ void pack_rows(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, hd_align
     // Compared rows come with their tensor-core operand, unless a look at some
     // of their sites says that site lists will do
     uint4 *g = aln->plane_buf[0].as<uint4>();
-    const uint32_t stride = compared ? sites_sample_stride(ctx, aln) : 0;
-    if (stride) pack_planes(ctx, rec, d_rows, aln->n_rows, aln->length, aln->words, g, nullptr, stride);
-    const bool lists = stride && sites_likely(ctx, aln, ctx->stream);
-    if (lists && stride == 1) return;
+    const Words sel = compared ? sites_sample(ctx, aln) : Words{};
+    if (sel.stride)
+      pack_planes(ctx, rec, d_rows, aln->n_rows, aln->length, aln->words, g, nullptr,
+                  sel.stride > 1 ? &sel : nullptr);
+    const bool lists = sel.stride && sites_likely(ctx, aln, ctx->stream);
+    if (lists && sel.stride == 1) return;
     if (compared && !lists && mma_wanted(ctx, aln) &&
         pack_operand(ctx, rec, d_rows, aln, 0, aln->n_rows, nullptr, ctx->stream))
       return;

@@ -221,6 +221,28 @@ struct SiteLists {
     for (DevBuf *b : {&base, &off, &es, &ed, &weight}) b->release();
   }
 };
+// A selection of a row's 32-site words: with stride 1 all of them, else the
+// first and the last 32 (an alignment's ends have most of its '-') and four
+// neighbouring ones of every 4 stride between them.
+struct Words {
+  uint32_t words, stride, count;  // of a row; selected (some may be past the last: at >= words)
+  static constexpr uint32_t kEdge = 32;
+  __host__ __device__ uint32_t edges() const { return stride == 1 ? 0u : 2 * kEdge; }
+  __host__ __device__ uint32_t at(uint32_t k) const {
+    if (stride == 1) return k;
+    if (k < kEdge) return k;
+    if (k < 2 * kEdge) return words - 2 * kEdge + k;
+    k -= 2 * kEdge;
+    const uint32_t w = kEdge + (k >> 2) * 4 * stride + (k & 3u);
+    return w < words - kEdge ? w : words;
+  }
+  // stride > 1 needs more than 64 words
+  static Words of(uint32_t words, uint32_t stride) {
+    Words s{words, stride, words};
+    if (stride > 1) s.count = 2 * kEdge + 4 * ((words - 2 * kEdge + 4 * stride - 1) / (4 * stride));
+    return s;
+  }
+};
 // A launch over them (by value to its kernel)
 struct SiteJob {
   const uint4 *base;
@@ -624,11 +646,13 @@ int mma_rows_of(const TileConfig &c);
 
 // sites.cu: distances from lists of the sites where a row differs from a
 // reference, for whole alignments of similar rows.
-// Whether the lists come into question for the alignment: 0, or the stride
-// (in four words) of the sites to look at. sites_likely looks at those words
-// of the planes (a wait); ensure_sites also builds the lists (another).
-uint32_t sites_sample_stride(hd_ctx *ctx, const hd_alignment *aln);
-bool sites_likely(hd_ctx *ctx, const hd_alignment *aln, cudaStream_t stream);
+// Whether the lists come into question for the alignment (with `rows` rows, 0:
+// its own): stride 0, or the words of a row to look at. sites_likely looks at
+// those words of the planes' first `have` rows (0: all; a wait) for an
+// alignment that will have `rows`; ensure_sites also builds the lists (another).
+Words sites_sample(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows = 0);
+bool sites_likely(hd_ctx *ctx, const hd_alignment *aln, cudaStream_t stream, uint64_t have = 0,
+                  uint64_t rows = 0);
 bool ensure_sites(hd_ctx *ctx, const hd_alignment *aln, cudaStream_t stream);
 // launches for the specs that use them; taken[k] marks those
 void prepare_site_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaStream_t stream,
@@ -648,9 +672,10 @@ bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStr
 // whether the distances of the whole alignment run on the tensor-core engine
 bool mma_wanted(hd_ctx *ctx, const hd_alignment *aln);
 // packs records d_rows[0 .. n_rows) (none: 0 ..) of the AND rule into rows of
-// planes g0 (and g1, if given); stride > 1: only four words of every 4 stride
+// planes g0 (and g1, if given); sel: only those words
 void pack_planes(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, uint64_t n_rows,
-                 uint64_t length, uint64_t words, uint4 *g0, uint4 *g1, uint32_t stride = 1);
+                 uint64_t length, uint64_t words, uint4 *g0, uint4 *g1,
+                 const Words *sel = nullptr);
 // packs records d_rows[0 ..] (none: 0 ..) of the AND rule into rows [lo, hi) of
 // the alignment's planes (and of `copy`, if given) and of its operand, whose
 // earlier rows are there (op_rows == lo), in one pass over their text. False

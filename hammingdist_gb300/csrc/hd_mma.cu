@@ -368,12 +368,12 @@ __global__ void __launch_bounds__(256, 6)
     k_pack_op(const uint8_t *base, uint64_t bytes, const uint64_t *__restrict__ rs,
               const uint64_t *__restrict__ rows, uint64_t row_lo, uint64_t row_hi, uint64_t L,
               uint32_t words, uint4 *__restrict__ g0, uint4 *__restrict__ g1,
-              uint8_t *__restrict__ x, uint32_t *dash_chunk, uint32_t ext, uint32_t stride) {
+              uint8_t *__restrict__ x, uint32_t *dash_chunk, uint32_t ext, Words sel) {
   constexpr uint32_t kPlanes = 4, nb = op_blocks(kPlanes);
   const uint32_t op_words = kOp ? op_chunks(L) * kChunkWords : 0u;
   // without the operand a warp takes 32 words of one row instead
   const uint32_t k = blockIdx.x * 32 + (kOp ? threadIdx.x / 8 : threadIdx.x & 31u);
-  const uint32_t w = kOp ? k : (k >> 2) * 4 * stride + (k & 3u);
+  const uint32_t w = kOp ? k : sel.at(k);
   const uint32_t row = kOp ? threadIdx.x & 7u : threadIdx.x >> 5;
   if (w >= words && w >= op_words) return;
   const uint32_t c = w / kChunkWords;
@@ -1354,12 +1354,13 @@ dim3 pack_grid(hd_ctx *ctx, uint64_t words, uint64_t lo, uint64_t hi) {
 }  // namespace
 
 void pack_planes(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, uint64_t n_rows,
-                 uint64_t length, uint64_t words, uint4 *g0, uint4 *g1, uint32_t stride) {
+                 uint64_t length, uint64_t words, uint4 *g0, uint4 *g1, const Words *sel) {
   if (!n_rows) return;
-  const uint64_t w = 4 * ceil_div(words, (uint64_t)4 * stride);
-  k_pack_op<false><<<pack_grid(ctx, w, 0, n_rows), 256, 0, ctx->stream>>>(
+  const Words all = Words::of((uint32_t)words, 1);
+  if (!sel) sel = &all;
+  k_pack_op<false><<<pack_grid(ctx, sel->count, 0, n_rows), 256, 0, ctx->stream>>>(
       rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), d_rows, 0, n_rows, length,
-      (uint32_t)words, g0, g1, nullptr, nullptr, 0, stride);
+      (uint32_t)words, g0, g1, nullptr, nullptr, 0, *sel);
   HD_LAUNCHED(ctx);
 }
 
@@ -1374,7 +1375,7 @@ bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const
   const uint64_t op_words = (uint64_t)op_chunks(aln->length) * kChunkWords;
   k_pack_op<true><<<pack_grid(ctx, std::max(aln->words, op_words), lo, hi), 256, 0, stream>>>(
       rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), d_rows, lo, hi, aln->length,
-      (uint32_t)aln->words, g0, copy, x, marks, ext, 1);
+      (uint32_t)aln->words, g0, copy, x, marks, ext, Words::of(0, 1));
   HD_LAUNCHED(ctx);
   dash_rows(ctx, g0, nullptr, 4, aln->words, lo, hi, aln->length, x, marks, ext,
             aln->op_lists.back().as<uint32_t>(), stream);

@@ -59,12 +59,6 @@ __device__ __forceinline__ uint32_t e_code(uint32_t e) { return (e >> 18) & 63u;
 __device__ __forceinline__ uint32_t e_run(uint32_t e) { return e >> 26; }
 constexpr uint32_t kMeetsDash = 1u << 24, kRefZero = 1u << 25;
 
-// A selection of the 32-site words: four neighbouring ones of every 4 stride
-struct Words {
-  uint32_t words, stride, count;  // of the rows; 1: all; selected (the last may be past words)
-  __host__ __device__ uint32_t at(uint32_t k) const { return (k >> 2) * 4 * stride + (k & 3u); }
-};
-
 struct Planes {
   const uint4 *g0, *g1;
   uint32_t planes;
@@ -190,29 +184,33 @@ __global__ void __launch_bounds__(256)
   }
 }
 // One block: the entries (s, x, d), the pairs of s entries of one site that
-// meet, and the pairs of an x and a d entry
+// meet, and the pairs of an x and a d entry: of the sites before `edge` in
+// out[0 .. 5), of the others in out[5 .. 10)
 __global__ void __launch_bounds__(1024)
-    k_site_cost(const uint32_t *counts, uint32_t sites, unsigned long long *out) {
-  __shared__ unsigned long long sum[5];
-  if (threadIdx.x < 5) sum[threadIdx.x] = 0;
+    k_site_cost(const uint32_t *counts, uint32_t edge, uint32_t sites, unsigned long long *out) {
+  __shared__ unsigned long long sum[10];
+  if (threadIdx.x < 10) sum[threadIdx.x] = 0;
   __syncthreads();
-  unsigned long long v[5] = {0, 0, 0, 0, 0};
-  for (uint32_t i = threadIdx.x; i < sites; i += blockDim.x) {
-    const unsigned long long s = counts[4 * i], x = counts[4 * i + 1], d = counts[4 * i + 2];
-    const unsigned long long l = counts[4 * i + 3];
-    v[0] += s;
-    v[1] += x;
-    v[2] += d;
-    v[3] += (s * s - l * l) / 2;
-    v[4] += x * d;
-  }
+  for (int part = 0; part < 2; ++part) {
+    unsigned long long v[5] = {0, 0, 0, 0, 0};
+    const uint32_t end = part ? sites : edge;
+    for (uint32_t i = (part ? edge : 0u) + threadIdx.x; i < end; i += blockDim.x) {
+      const unsigned long long s = counts[4 * i], x = counts[4 * i + 1], d = counts[4 * i + 2];
+      const unsigned long long l = counts[4 * i + 3];
+      v[0] += s;
+      v[1] += x;
+      v[2] += d;
+      v[3] += (s * s - l * l) / 2;
+      v[4] += x * d;
+    }
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    v[k] = warp_sum(v[k]);
-    if ((threadIdx.x & 31) == 0 && v[k]) atomicAdd(&sum[k], v[k]);
+    for (int k = 0; k < 5; ++k) {
+      v[k] = warp_sum(v[k]);
+      if ((threadIdx.x & 31) == 0 && v[k]) atomicAdd(&sum[5 * part + k], v[k]);
+    }
   }
   __syncthreads();
-  if (threadIdx.x < 5) out[threadIdx.x] = sum[threadIdx.x];
+  if (threadIdx.x < 10) out[threadIdx.x] = sum[threadIdx.x];
 }
 
 // What building the lists leaves (device)
@@ -611,65 +609,68 @@ int forced() {
   if (const char *e = std::getenv("HAMMINGDIST_SITE_LISTS")) return std::atoi(e) ? 1 : -1;
   return 0;
 }
-bool usable(hd_ctx *ctx, const hd_alignment *a) {
-  return !a->base && ctx->engine_force < 0 && a->n_rows >= 2 && a->n_rows < (1ull << 31) &&
+bool usable(hd_ctx *ctx, const hd_alignment *a, uint64_t rows) {
+  return !a->base && ctx->engine_force < 0 && rows >= 2 && rows < (1ull << 31) &&
          a->length >= 1 && a->length <= (uint64_t)kMaxRanges * kRange &&
          (a->planes == 4 || a->groups == 2);
 }
 
 }  // namespace
 
-uint32_t sites_sample_stride(hd_ctx *ctx, const hd_alignment *a) {
+Words sites_sample(hd_ctx *ctx, const hd_alignment *a, uint64_t rows) {
+  if (!rows) rows = a->n_rows;
   const int f = forced();
-  if (f < 0 || !usable(ctx, a)) return 0;
+  if (f < 0 || !usable(ctx, a, rows)) return Words{};
   // below this the launches and waits that build lists for one call cost what
   // they save (about 100 us)
-  if (f == 0 && dense_us(a->n_rows, a->length, (uint32_t)a->planes) < 200.0) return 0;
-  const uint64_t w = ceil_div(a->length, (uint64_t)32);
-  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(8, w / 64));
+  if (f == 0 && dense_us(rows, a->length, (uint32_t)a->planes) < 200.0) return Words{};
+  const uint32_t w = (uint32_t)ceil_div(a->length, (uint64_t)32);
+  return Words::of(w, w < 256 ? 1 : 8);
 }
 
-bool sites_likely(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
-  const uint32_t stride = sites_sample_stride(ctx, a);
-  if (!stride) return false;
+bool sites_likely(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st, uint64_t have, uint64_t rows) {
+  if (!rows) rows = a->n_rows;
+  if (!have) have = rows;
+  const Words sel = sites_sample(ctx, a, rows);
+  if (!sel.stride) return false;
   if (a->sites && a->sites->verdict) return a->sites->verdict > 0;
   if (!a->sites) a->sites = std::make_unique<SiteLists>();
   SiteLists &S = *a->sites;
   if (forced() > 0) {
     S.verdict = 1;
-    S.est_s = (double)a->n_rows * (double)a->length;  // room for anything (tests)
+    S.est_s = (double)rows * (double)a->length;  // room for anything (tests)
     S.est_d = S.est_s;
     return true;
   }
-  const uint32_t words = (uint32_t)ceil_div(a->length, (uint64_t)32);
-  const uint32_t quads = (uint32_t)ceil_div((uint64_t)words, (uint64_t)4 * stride);
-  const Words sel{words, stride, quads * 4};
+  const uint32_t quads = (uint32_t)ceil_div((uint64_t)sel.count, (uint64_t)4);
   const uint64_t count_bytes = (uint64_t)quads * 128 * 4 * 4;
-  DevBuf buf(ref_bytes(a) + 64 + count_bytes, st);
+  DevBuf buf(ref_bytes(a) + 80 + count_bytes, st);
   uint4 *r0 = buf.as<uint4>();
   uint2 *r1 = reinterpret_cast<uint2 *>(r0 + a->words);
   auto *sums = reinterpret_cast<unsigned long long *>(r1 + a->words);
-  uint32_t *counts = reinterpret_cast<uint32_t *>(sums + 8);
+  uint32_t *counts = reinterpret_cast<uint32_t *>(sums + 10);
   HD_CUDA(cudaMemsetAsync(counts, 0, count_bytes, st));
   const Planes p = planes_of(a);
-  k_site_ref<<<(unsigned)ceil_div((uint64_t)sel.count, (uint64_t)2), 256, 0, st>>>(
-      p, a->n_rows, sel, r0, r1);
+  k_site_ref<<<(unsigned)ceil_div((uint64_t)sel.count, (uint64_t)2), 256, 0, st>>>(p, have, sel, r0,
+                                                                                   r1);
   HD_LAUNCHED(ctx);
-  const uint64_t shares = std::min<uint64_t>(ceil_div(a->n_rows, (uint64_t)512), 64);
-  k_site_count<<<dim3(quads, (unsigned)shares), 256, 0, st>>>(p, a->n_rows, a->length, sel, r0, r1,
-                                                              counts);
+  const uint64_t shares = std::min<uint64_t>(ceil_div(have, (uint64_t)512), 64);
+  k_site_count<<<dim3(quads, (unsigned)shares), 256, 0, st>>>(p, have, a->length, sel, r0, r1, counts);
   HD_LAUNCHED(ctx);
-  k_site_cost<<<1, 1024, 0, st>>>(counts, quads * 128, sums);
+  k_site_cost<<<1, 1024, 0, st>>>(counts, 32 * sel.edges(), quads * 128, sums);
   HD_LAUNCHED(ctx);
   uint64_t *h = pinned_words(ctx);
-  HD_CUDA(cudaMemcpyAsync(h, sums, 40, cudaMemcpyDeviceToHost, st));
+  HD_CUDA(cudaMemcpyAsync(h, sums, 80, cudaMemcpyDeviceToHost, st));
   HD_CUDA(cudaStreamSynchronize(st));
-  const double up = (double)words / std::min<double>(words, (double)sel.count);
-  S.est_s = up * (double)h[0];
-  S.est_d = up * (double)h[2];
-  S.est_xd = up * (double)h[4];
-  const double t = lists_us(a->n_rows, a->length, up * (double)(h[3] + h[4]));
-  S.verdict = t < 0.9 * dense_us(a->n_rows, a->length, (uint32_t)a->planes) ? 1 : -1;
+  const double inner = sel.words - sel.edges();
+  const double up = sel.stride > 1 ? inner / std::min<double>(inner, sel.count - sel.edges()) : 1.0;
+  const double more = (double)rows / (double)have;
+  auto est = [&](int k) { return (double)h[k] + up * (double)h[5 + k]; };
+  S.est_s = more * est(0);
+  S.est_d = more * est(2);
+  S.est_xd = more * more * est(4);
+  const double t = lists_us(rows, a->length, more * more * (est(3) + est(4)));
+  S.verdict = t < 0.9 * dense_us(rows, a->length, (uint32_t)a->planes) ? 1 : -1;
   return S.verdict > 0;
 }
 
@@ -706,7 +707,7 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
   HD_CUDA(cudaMemsetAsync(sums, 0, sizeof(BuildSums), st));
   HD_CUDA(cudaMemsetAsync(S.weight.p, 0, a->n_rows * 4, st));
   const Planes p = planes_of(a);
-  const Words sel{words, 1, words};
+  const Words sel = Words::of(words, 1);
   k_site_ref<<<(unsigned)ceil_div((uint64_t)words, (uint64_t)2), 256, 0, st>>>(
       p, a->n_rows, sel, r0, r1);
   HD_LAUNCHED(ctx);

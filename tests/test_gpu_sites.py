@@ -89,3 +89,26 @@ def test_file_in_row_ranges(ctx, monkeypatch, tmp_path):
     monkeypatch.delenv("HAMMINGDIST_KERNEL")
     aln.free()
     assert (tmp_path / "a.txt").read_bytes() == (tmp_path / "b.txt").read_bytes()
+
+
+@pytest.mark.parametrize("n,L,kind", [(1600, 8300, "alike"), (1100, 45000, "random4")])
+@pytest.mark.parametrize("dup", [False, True])
+def test_streamed_file(tmp_path, monkeypatch, n, L, kind, dup):
+    # the lists of a file's parts, and a file whose rows turn out too different
+    hd = pytest.importorskip("hammingdist_gb300")
+    from gpu_util import write
+
+    rng = np.random.default_rng(n)
+    rows = (rng.choice(np.frombuffer(b"ACGT", np.uint8), (n, L)) if kind == "random4"
+            else _rows(n, L, kind, 3))
+    rows[n // 2:n // 2 + 40] = rows[:40]
+    path = write(tmp_path, "s.fasta", synth.to_fasta(rows))
+    monkeypatch.setenv("HAMMINGDIST_STREAM_MIN_BYTES", "0")
+    got = []
+    for env in ("HAMMINGDIST_SITE_LISTS", "HAMMINGDIST_KERNEL"):
+        monkeypatch.setenv(env, {"HAMMINGDIST_KERNEL": "lop3"}.get(env, "1"))
+        ds = hd.from_fasta_large(path, remove_duplicates=dup, use_gpu=True)
+        got.append(np.array(ds.lt_array))
+        monkeypatch.delenv(env)
+        os.utime(path, ns=(1, len(got)))  # read again, not the file already on the device
+    np.testing.assert_array_equal(got[0], got[1])
