@@ -222,11 +222,11 @@ struct SiteLists {
   }
 };
 // A selection of a row's 32-site words: with stride 1 all of them, else the
-// first and the last 32 (an alignment's ends have most of its '-') and four
+// first and the last 16 (an alignment's ends have most of its '-') and four
 // neighbouring ones of every 4 stride between them.
 struct Words {
   uint32_t words, stride, count;  // of a row; selected (some may be past the last: at >= words)
-  static constexpr uint32_t kEdge = 32;
+  static constexpr uint32_t kEdge = 16;
   __host__ __device__ uint32_t edges() const { return stride == 1 ? 0u : 2 * kEdge; }
   __host__ __device__ uint32_t at(uint32_t k) const {
     if (stride == 1) return k;
@@ -236,7 +236,7 @@ struct Words {
     const uint32_t w = kEdge + (k >> 2) * 4 * stride + (k & 3u);
     return w < words - kEdge ? w : words;
   }
-  // stride > 1 needs more than 64 words
+  // stride > 1 needs more than 32 words
   static Words of(uint32_t words, uint32_t stride) {
     Words s{words, stride, words};
     if (stride > 1) s.count = 2 * kEdge + 4 * ((words - 2 * kEdge + 4 * stride - 1) / (4 * stride));

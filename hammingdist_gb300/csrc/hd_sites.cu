@@ -49,6 +49,7 @@ constexpr uint32_t kOffLater = kOffPitch, kOffDash = 2 * kOffPitch, kOffSlot = 3
 constexpr uint32_t kRefRows = 64;            // rows that the reference is taken from
 constexpr int kPairThreads = 768;
 constexpr uint32_t kPending = 64;            // sites a warp gathers before it takes 32 of them
+constexpr uint32_t kStepSites = 128;         // of one range, a warp's step: four to a lane
 constexpr uint32_t kPairSmem = kT * kPitch * 4 + kPairThreads / 32 * kPending * 8;
 // an entry: site in its range (10 bits), row in its tile (8), code (6), 1 bit:
 // a '-' counts against it, 1 bit: the site's r is 0, and for code 0 where r is
@@ -222,10 +223,12 @@ struct BuildSums {
   uint32_t max_weight, pad[3];
 };
 
-// The lists of one (range, tile): a warp takes a row at a time, a lane a word.
-// The block counts the entries of its sites, places them and, reading the
-// rows again (from the caches), files them. weight: sum of m per row.
-__global__ void __launch_bounds__(256)
+// The lists of one (range, tile): a warp takes four rows at a time, a lane a
+// word. The block counts the entries of its sites, places them and, reading
+// the rows again (from the caches), files them. weight: sum of m per row.
+// What bounds it is the latency of the rows: LISTFIG
+template <bool kWide>  // more than four planes
+__global__ void __launch_bounds__(256, 4)
     k_site_lists(Planes p, uint64_t n, uint64_t L, uint32_t words, const uint4 *r0, const uint2 *r1,
                  uint32_t ranges, uint64_t cap_s, uint64_t cap_d, uint4 *base, uint16_t *off,
                  uint32_t *es, uint8_t *ed, uint32_t *weight, BuildSums *sums) {
@@ -247,16 +250,31 @@ __global__ void __launch_bounds__(256)
   }
   const uint32_t zero = valid & ~(ra.x | ra.y | ra.z | ra.w | rb.x | rb.y);
   __syncthreads();
+  constexpr uint32_t kBatch = 4;
+  const uint32_t planes = kWide ? p.planes : 4u;
+  // rows i, i + 8, ... of a batch: this lane's words, and for each row f(row,
+  // words, diff) by the whole warp; a lane past the row's words has none
+  auto each_row = [&](auto &&f) {
+    for (uint32_t i0 = warp; i0 < rows; i0 += 8 * kBatch) {
+      uint4 a[kBatch];
+      uint2 b[kBatch];
+#pragma unroll
+      for (uint32_t k = 0; k < kBatch; ++k) {
+        a[k] = ra;  // no entries
+        b[k] = rb;
+        if (valid && i0 + 8 * k < rows) {
+          a[k] = __ldg(p.g0 + (row0 + i0 + 8 * k) * p.pitch + w);
+          if (kWide) b[k] = __ldg(reinterpret_cast<const uint2 *>(p.g1 + (row0 + i0 + 8 * k) * p.pitch + w));
+        }
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kBatch; ++k)
+        if (i0 + 8 * k < rows) f(i0 + 8 * k, a[k], b[k], diff_of(a[k], b[k], ra, rb, planes, valid));
+    }
+  };
   // a word with entries at a time, a lane a site: a run of 'N' or '-' costs no
   // more than one entry
-  for (uint32_t i = warp; i < rows; i += 8) {
-    Diff f{0u, 0u, 0u, 0u};
-    if (valid) {
-      uint4 a;
-      uint2 b;
-      p.load(row0 + i, w, a, b);
-      f = diff_of(a, b, ra, rb, p.planes, valid);
-    }
+  each_row([&](uint32_t i, const uint4 &, const uint2 &, const Diff &f) {
     for (uint32_t on = __ballot_sync(0xffffffffu, f.s | f.d); on; on &= on - 1) {
       const int src = __ffs(on) - 1;
       const uint32_t ms = __shfl_sync(0xffffffffu, f.s, src), md = __shfl_sync(0xffffffffu, f.d, src);
@@ -266,7 +284,7 @@ __global__ void __launch_bounds__(256)
     }
     const uint32_t m = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(f.s & ~zero));
     if (lane == 0 && m) atomicAdd(&weight[row0 + i], m);
-  }
+  });
   if (tile == 0 && warp == 0) {
     const uint32_t z = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(zero));
     if (lane == 0 && z) atomicAdd(&sums->zero, z);
@@ -311,14 +329,7 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
   if (!fits) return;
-  for (uint32_t i = warp; i < rows; i += 8) {
-    uint4 a = make_uint4(0u, 0u, 0u, 0u);
-    uint2 b = make_uint2(0u, 0u);
-    Diff f{0u, 0u, 0u, 0u};
-    if (valid) {
-      p.load(row0 + i, w, a, b);
-      f = diff_of(a, b, ra, rb, p.planes, valid);
-    }
+  each_row([&](uint32_t i, const uint4 &a, const uint2 &b, const Diff &f) {
     for (uint32_t on = __ballot_sync(0xffffffffu, f.s | f.d); on; on &= on - 1) {
       const int src = __ffs(on) - 1;
       const uint32_t ms = __shfl_sync(0xffffffffu, f.s, src), md = __shfl_sync(0xffffffffu, f.d, src);
@@ -330,7 +341,7 @@ __global__ void __launch_bounds__(256)
                         ((__shfl_sync(0xffffffffu, a.y, src) >> lane) & 1u) << 1 |
                         ((__shfl_sync(0xffffffffu, a.z, src) >> lane) & 1u) << 2 |
                         ((__shfl_sync(0xffffffffu, a.w, src) >> lane) & 1u) << 3;
-        if (p.planes > 4)
+        if (kWide)
           code |= ((__shfl_sync(0xffffffffu, b.x, src) >> lane) & 1u) << 4 |
                   ((__shfl_sync(0xffffffffu, b.y, src) >> lane) & 1u) << 5;
         if (ms >> lane & 1u)
@@ -345,7 +356,7 @@ __global__ void __launch_bounds__(256)
       }
       if (md >> lane & 1u) ed[at_d + atomicAdd(at, 1u)] = (uint8_t)i;
     }
-  }
+  });
 }
 
 // The pairs of s entries that meet over all tiles, and the largest weight
@@ -372,29 +383,39 @@ __global__ void __launch_bounds__(256)
   if ((threadIdx.x & 31) == 0) atomicMax(&sums->max_weight, m);
 }
 
-template <class T>
-__device__ __forceinline__ void store_rows(const SiteJob &J, const uint32_t *acc, uint32_t ti,
+// The tile pair's distances from its counters: a warp a row, a lane a column of
+// every 32. kDiag: the pair of a tile with itself, whose rows end at themselves.
+template <class T, bool kDiag>
+__device__ __forceinline__ void store_tile(const SiteJob &J, const uint32_t *acc, uint32_t ti,
                                            uint32_t tj) {
-  const uint32_t lane = threadIdx.x & 31;
+  constexpr uint32_t kWarps = kPairThreads / 32;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t half = (lane & 1u) ? 0x4432u : 0x4410u;  // its 16 bits of a counter word
   uint32_t wj[kT / 32];
 #pragma unroll
   for (uint32_t k = 0; k < kT / 32; ++k) {
     const uint64_t j = (uint64_t)tj * kT + 32 * k + lane;
-    wj[k] = j < J.n ? J.weight[j] + J.zero : 0u;
+    wj[k] = j < J.n ? __ldg(J.weight + j) + J.zero : 0u;
   }
-  for (uint32_t i = threadIdx.x >> 5; i < kT; i += kPairThreads / 32) {
-    const uint64_t r = (uint64_t)ti * kT + i;
+  const uint64_t r0 = (uint64_t)ti * kT;
+  for (uint32_t i = warp; i < kT; i += kWarps) {
+    const uint64_t r = r0 + i;
     if (r < J.row_lo || r >= J.row_hi) continue;
-    const uint32_t cols = ti == tj ? i : kT, wi = J.weight[r];
-    T *out = static_cast<T *>(J.out) + (r * (r - 1) / 2 + (uint64_t)tj * kT - J.out_base);
+    const uint32_t wi = __ldg(J.weight + r);
+    T *out = static_cast<T *>(J.out) + (r * (r - 1) / 2 + (uint64_t)tj * kT - J.out_base) + lane;
+    const uint32_t *row = acc + i * kPitch + (lane >> 1);
 #pragma unroll
     for (uint32_t k = 0; k < kT / 32; ++k) {
-      const uint32_t j = 32 * k + lane;
-      const uint32_t a = (acc[i * kPitch + (j >> 1)] >> (16u * (j & 1u))) & 0xFFFFu;
-      const uint32_t d = wi + wj[k] - a;
-      if (j < cols) out[j] = (T)(d < J.max_dist ? d : J.max_dist);
+      const uint32_t d = wi + wj[k] - __byte_perm(row[16 * k], 0u, half);
+      if (!kDiag || 32 * k + lane < i) out[32 * k] = (T)min(d, J.max_dist);
     }
   }
+}
+template <class T>
+__device__ __forceinline__ void store_rows(const SiteJob &J, const uint32_t *acc, uint32_t ti,
+                                           uint32_t tj) {
+  if (ti == tj) store_tile<T, true>(J, acc, ti, tj);
+  else store_tile<T, false>(J, acc, ti, tj);
 }
 
 // 1 to every '-' entry's counter: column j (row i) of the list's rows, for up
@@ -456,7 +477,8 @@ __device__ __forceinline__ void meet_sites(uint32_t *acc, const uint2 *sites, ui
 // each: the longest steps), then 128 sites at a time the s entries that meet,
 // which 32 lanes share evenly. What bounds it is the instructions
 // of finding the meetings (IPC 3.3 of 4). 14,000 rows of 29,903 sites, one
-// substitution per 1,000: 330 us, where the tensor-core engine takes 1,910. A
+// substitution per 1,000: 300 us (about 30 for the '-', 110 for the meetings,
+// 65 to gather their sites, 30 to store), where the tensor-core engine takes 1,910. A
 // lane an entry of the row tile instead, which looks its site up, took 655
 // (the blocks' warps waited half of the time for those with '-' entries), 32
 // sites at a time without gathering them and with every pair of a run 410.
@@ -492,7 +514,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_site_pairs(SiteJob J) {
   }
   __syncthreads();
   const uint32_t ci = chunks[0][J.ranges], cd = ci + chunks[1][J.ranges];
-  const uint32_t steps = cd + J.ranges * (kRange / 128);
+  const uint32_t steps = cd + J.ranges * (kRange / kStepSites);
   for (;;) {
     uint32_t c = 0;
     if (lane == 0) c = atomicAdd(&queue, 1u);
@@ -527,9 +549,10 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_site_pairs(SiteJob J) {
       }
       continue;
     }
-    // 128 sites, four to a lane: the sites with entries in both tiles are
+    // a step's sites, four to a lane: those with entries in both tiles are
     // gathered, and taken 32 at a time
-    const uint32_t k = c - cd, r = k / (kRange / 128), s0 = (k % (kRange / 128)) * 128;
+    const uint32_t k = c - cd, r = k / (kRange / kStepSites), s0 = (k % (kRange / kStepSites)) * kStepSites;
+    const uint32_t *li = J.es + bi[r].x, *lj = J.es + bj[r].x;
     const uint16_t *a = oi + (uint64_t)r * kOffSlot + s0 + 4 * lane;
     const uint16_t *b = oj + (uint64_t)r * kOffSlot + s0 + 4 * lane;
     const uint2 af = __ldg(reinterpret_cast<const uint2 *>(a));
@@ -542,7 +565,6 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_site_pairs(SiteJob J) {
       an = a[4];
       bn = b[4];
     }
-    const uint32_t *li = J.es + bi[r].x, *lj = J.es + bj[r].x;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const uint32_t a0 = (q & 1) ? (q < 2 ? af.x : af.y) >> 16 : (q < 2 ? af.x : af.y) & 0xFFFFu;
@@ -559,15 +581,13 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_site_pairs(SiteJob J) {
             make_uint2(a0 | b0 << 16, (a1 - a0) | (a2 - a1) << 8 | (b1 - b0) << 16 | (b2 - b1) << 24);
       count += __popc(mask);
       __syncwarp();
-      if (count >= 32 || (q == 3 && count)) {
-        // the sites gathered last; those left move up below
-        const uint32_t take = count < 32u ? count : 32u;
-        count -= take;
-        meet_sites(acc, pending + count, take, li, lj, lane);
+      if (count >= 32) {  // the sites gathered last
+        count -= 32;
+        meet_sites(acc, pending + count, 32, li, lj, lane);
         __syncwarp();
       }
     }
-    if (count) {  // what the last site words added past 32
+    if (count) {
       meet_sites(acc, pending, count, li, lj, lane);
       __syncwarp();
       count = 0;
@@ -625,7 +645,7 @@ Words sites_sample(hd_ctx *ctx, const hd_alignment *a, uint64_t rows) {
   // they save (about 100 us)
   if (f == 0 && dense_us(rows, a->length, (uint32_t)a->planes) < 200.0) return Words{};
   const uint32_t w = (uint32_t)ceil_div(a->length, (uint64_t)32);
-  return Words::of(w, w < 256 ? 1 : 8);
+  return Words::of(w, w < 256 ? 1 : w < 512 ? 8 : 16);
 }
 
 bool sites_likely(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st, uint64_t have, uint64_t rows) {
@@ -716,7 +736,7 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
     Planes q = p;
     q.g0 += row * p.pitch;
     if (q.g1) q.g1 += row * p.pitch;
-    k_site_lists<<<dim3(ranges, (unsigned)tn), 256, 0, st>>>(
+    (q.planes > 4 ? k_site_lists<true> : k_site_lists<false>)<<<dim3(ranges, (unsigned)tn), 256, 0, st>>>(
         q, a->n_rows - row, a->length, words, r0, r1, ranges, cap_s, cap_d,
         S.base.as<uint4>() + t0 * ranges, S.off.as<uint16_t>() + t0 * ranges * kOffSlot,
         S.es.as<uint32_t>(), S.ed.as<uint8_t>(), S.weight.as<uint32_t>() + row, sums);
