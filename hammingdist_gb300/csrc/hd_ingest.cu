@@ -1146,27 +1146,62 @@ void IncDedupe::rows(hd_ctx *ctx, std::vector<uint64_t> &seqidx) {
 }
 
 // -------------------------------------------------------------- consensus
-constexpr int kColRows = 128;
+// 0x01 in every byte of w that equals the byte of x
+__device__ __forceinline__ uint32_t equal_bytes(uint32_t w, uint32_t x) {
+  const uint32_t z = w ^ x, ne = ((z & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | z;
+  return ~(ne >> 7) & 0x01010101u;
+}
 
-__global__ void k_colcount(const uint8_t *base, const uint64_t *rs, const uint64_t *rows,
-                           uint64_t n_rows, uint64_t L, unsigned int *counts) {
-  uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (s >= L) return;
-  uint64_t u0 = (uint64_t)blockIdx.y * kColRows;
-  uint64_t u1 = u0 + kColRows < n_rows ? u0 + kColRows : n_rows;
-  unsigned a = 0, c = 0, g = 0, t = 0;
-  for (uint64_t u = u0; u < u1; ++u) {
-    uint64_t r = rows ? rows[u] : u;
-    uint8_t ch = base[rs[r] + s];
-    a += ch == 'A';
-    c += ch == 'C';
-    g += ch == 'G';
-    t += ch == 'T';
+// Counts of A, C, G and T per site over a share of at most 128 rows: a thread
+// takes four neighbouring sites, whose counts are the bytes of four words, and
+// a share is small enough to use all SMs: 120 rows of 1,273 sites take 5.5 us
+// (17 with a byte a load and shares of 128), 2,000 of 29,903 57 (57).
+constexpr uint32_t kColRows = 128;
+__global__ void __launch_bounds__(256)
+    k_colcount(const uint8_t *base, uint64_t bytes, const uint64_t *rs, const uint64_t *rows,
+               uint64_t n_rows, uint32_t share, uint64_t L, unsigned int *counts) {
+  __shared__ uint64_t start[kColRows];
+  const uint64_t u0 = (uint64_t)blockIdx.y * share;
+  const uint32_t m = (uint32_t)(n_rows - u0 < share ? n_rows - u0 : share);
+  const uint64_t lo = reinterpret_cast<uint64_t>(base), hi = lo + bytes;
+  for (uint32_t u = threadIdx.x; u < m; u += blockDim.x) start[u] = lo + rs[rows ? rows[u0 + u] : u0 + u];
+  __syncthreads();
+  const uint64_t s = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) * 4;
+  if ((s & ~127ull) >= L) return;  // warp-uniform
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t c[4] = {0u, 0u, 0u, 0u};
+  constexpr int kAhead = 8;
+  for (uint32_t u = 0; u < m; u += kAhead) {
+    uint32_t v[kAhead], n[kAhead], sh[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      v[k] = n[k] = sh[k] = 0u;  // past the share: no symbol
+      if (u + k < m) {
+        const uint64_t P = start[u + k] + s, A = P & ~3ull;
+        sh[k] = 8u * (uint32_t)(P - A);
+        // the warp's 128 bytes, and the word after them for lane 31
+        const bool in = A - 4 * lane >= lo && A - 4 * lane + 132 <= hi;  // warp-uniform
+        v[k] = in ? __ldg(reinterpret_cast<const uint32_t *>(A)) : load4_in(A, lo, hi);
+        if (lane == 31 && sh[k])
+          n[k] = in ? __ldg(reinterpret_cast<const uint32_t *>(A + 4)) : load4_in(A + 4, lo, hi);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint32_t next = __shfl_down_sync(0xffffffffu, v[k], 1);
+      const uint32_t w = __funnelshift_r(v[k], lane == 31 ? n[k] : next, sh[k]);
+      c[0] += equal_bytes(w, 0x41414141u);
+      c[1] += equal_bytes(w, 0x43434343u);
+      c[2] += equal_bytes(w, 0x47474747u);
+      c[3] += equal_bytes(w, 0x54545454u);
+    }
   }
-  if (a) atomicAdd(&counts[4 * s + 0], a);
-  if (c) atomicAdd(&counts[4 * s + 1], c);
-  if (g) atomicAdd(&counts[4 * s + 2], g);
-  if (t) atomicAdd(&counts[4 * s + 3], t);
+  for (int k = 0; k < 4 && s + k < L; ++k)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t t = (c[j] >> (8 * k)) & 0xFFu;
+      if (t) atomicAdd(&counts[4 * (s + k) + j], t);
+    }
 }
 
 __global__ void k_colmax_sum(const unsigned int *counts, uint64_t L, unsigned long long *sum) {
@@ -1190,14 +1225,18 @@ uint64_t consensus_matches(hd_ctx *ctx, const Records &rec, const uint64_t *d_ro
   DevBuf counts(L * 16, st), sum(8, st);
   HD_CUDA(cudaMemsetAsync(counts.p, 0, L * 16, st));
   HD_CUDA(cudaMemsetAsync(sum.p, 0, 8, st));
-  uint64_t chunks = ceil_div(n_rows, kColRows);
+  // shares of 128 rows, or fewer where that leaves SMs without a block
+  const uint64_t X = ceil_div(L, (uint64_t)1024);
+  const uint64_t want = ceil_div((uint64_t)ctx->sm_count * 4, X);
+  const uint32_t share = (uint32_t)std::min<uint64_t>(kColRows, std::max<uint64_t>(8, n_rows / want));
+  const uint64_t chunks = ceil_div(n_rows, (uint64_t)share);
   for (uint64_t c0 = 0; c0 < chunks; c0 += 65535) {
     uint64_t cn = chunks - c0 < 65535 ? chunks - c0 : 65535;
-    dim3 grid((unsigned)ceil_div(L, 256), (unsigned)cn);
-    const uint64_t *rows = d_rows ? d_rows + c0 * kColRows : nullptr;
-    // without a row list the rows are records [c0*kColRows, ...): shift the starts
-    const uint64_t *rs = rec.rec_start.as<uint64_t>() + (d_rows ? 0 : c0 * kColRows);
-    k_colcount<<<grid, 256, 0, st>>>(rec.base, rs, rows, n_rows - c0 * kColRows, L,
+    dim3 grid((unsigned)X, (unsigned)cn);
+    const uint64_t *rows = d_rows ? d_rows + c0 * share : nullptr;
+    // without a row list the rows are records [c0 * share, ...): shift the starts
+    const uint64_t *rs = rec.rec_start.as<uint64_t>() + (d_rows ? 0 : c0 * share);
+    k_colcount<<<grid, 256, 0, st>>>(rec.base, rec.bytes, rs, rows, n_rows - c0 * share, share, L,
                                      counts.as<unsigned int>());
     HD_LAUNCHED(ctx);
   }
