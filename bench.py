@@ -208,14 +208,17 @@ def measured_peaks():
 # the distance kernel on this workload's 14,000 distinct rows at L=29,903,
 # from one ncu capture (one launch, one pass):
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none
-#       -k regex:k_pairwise_mma -s 1 -c 1
+#       -k regex:k_site_pairs -s 1 -c 1
 #       python bench.py --kernel-only --n 14000 --steps 1 --warmup 1
-# bench.py cannot run ncu itself, so the figure is a constant of the kernel
-# build it was measured on (KERNEL_DRAM_SOURCE).
-KERNEL_DRAM_BYTES = 7_754_952_192
-KERNEL_DRAM_SOURCE = ("ncu capture of k_pairwise_mma (FP4 operand, 240-column items, dash "
-                      "products of marked chunks only), n=14000 L=29903, one launch: 7.658 GB "
-                      "read + 0.097 GB written")
+# (k_pairwise_mma with HAMMINGDIST_SITE_LISTS=0 for the tensor-core engine).
+# bench.py cannot run ncu itself, so the figures are constants of the kernel
+# build they were measured on.
+KERNEL_DRAM_BYTES = 60_078_336
+KERNEL_DRAM_SOURCE = ("ncu capture of k_site_pairs, n=14000 L=29903, one launch: 16 MB "
+                      "read + 44 MB written (the rest of the matrix was still in L2)")
+MMA_DRAM_BYTES = 6_373_476_608
+MMA_DRAM_SOURCE = ("ncu capture of k_pairwise_mma (FP4 operand, CTA pairs, items of 256 rows x "
+                   "496 columns), n=14000 L=29903, one launch: 6.195 GB read + 0.179 GB written")
 
 
 # ------------------------------------------------------------------ CPU leg
@@ -416,19 +419,39 @@ def run_ours(args):
         exact = all(checks.values())
         entries_equal = int(np.count_nonzero(lt_dev == lt_o)) if lt_dev.size == lt_o.size else 0
 
-        # roofline of the dominant kernel, the tensor-core engine: per pair,
+        # roofline of the distance kernel. The tensor-core engine: per pair,
         # matches = <planes, planes'> - 3 <dash, dash'>, 4 multiply-adds per
-        # site for the planes and 1 more per site of the 256-site chunks that
+        # site for the planes and 1 more per site of the 192-site chunks that
         # hold a '-' (the library reports the launch's multiply-adds), in
-        # E2M1 (FP4) operands against the device's measured FP4 MMA rate
+        # E2M1 (FP4) operands against the device's measured FP4 MMA rate. The
+        # site lists do no multiply-adds: what they cannot do without is the
+        # matrix written, against the measured copy rate; what bounds them is
+        # the instructions that find where two rows both differ.
         peaks = ctx.measure_int_peaks()
         fp4_peak = ctx.measure_mma_peak()
         ctx.close()
         kern_s = statistics.mean(pair_ms) / 1e3
         flop_per_launch = 2.0 * r["mma_macs"]
-        achieved = flop_per_launch / kern_s / 1e12
-        peak = fp4_peak / 1e12
         bf16 = measured_peaks().get("bf16_tflops")
+        if flop_per_launch:
+            achieved, peak = flop_per_launch / kern_s / 1e12, fp4_peak / 1e12
+            roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                        "frac": achieved / peak, "traffic": MMA_DRAM_BYTES,
+                        "traffic_source": MMA_DRAM_SOURCE,
+                        "peak_source": "in-run FP4 (E2M1, kind::mxf4) tcgen05 MMA "
+                                       "microbenchmark, CTA pairs, M=256 N=256+240 K=96 "
+                                       "(hd_measure_mma_peak); MEASURED_PEAKS.json has "
+                                       "bf16 only",
+                        "flop_per_pair_site": flop_per_launch / (pairs * L)}
+        else:
+            achieved, peak = pairs / kern_s / 1e9, measured_peaks().get("hbm_gbs") or 6800.0
+            roofline = {"bound": "issue", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                        "frac": achieved / peak, "traffic": KERNEL_DRAM_BYTES,
+                        "traffic_source": KERNEL_DRAM_SOURCE,
+                        "peak_source": "measured copy rate; achieved counts the bytes of the "
+                                       "matrix written. The kernel is bound by instruction "
+                                       "issue (IPC 3.3 of 4, ncu)",
+                        "fp4_peak_TF": fp4_peak / 1e12}
         busy = sum(phases.values())
 
         if rank == 0:
@@ -447,16 +470,8 @@ def run_ours(args):
                            "distances equal the oracle (resident and e2e results)"
                            % (entries_equal, lt_o.size, len(idx_o), len(rd_o)))
                 if exact else "MISMATCH " + json.dumps(checks),
-                "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak,
-                             "unit": "TFLOP/s", "frac": achieved / peak,
-                             "traffic": KERNEL_DRAM_BYTES, "traffic_source": KERNEL_DRAM_SOURCE,
-                             "kernel_ms": kern_s * 1e3,
-                             "peak_source": "in-run FP4 (E2M1, kind::mxf4) tcgen05 MMA "
-                                            "microbenchmark, M=128 N=256 K=64 "
-                                            "(hd_measure_mma_peak); MEASURED_PEAKS.json has "
-                                            "bf16 only",
+                "roofline": {**roofline, "kernel_ms": kern_s * 1e3,
                              "bf16_measured_TF": bf16,
-                             "flop_per_pair_site": flop_per_launch / (pairs * L),
                              "kernel_pair_sites_T": pairs * L / kern_s / 1e12,
                              "hbm_write_GBs": pairs / kern_s / 1e9,
                              "lop3_engine_bound_T": min(8 * peaks["lop3_per_s"],
