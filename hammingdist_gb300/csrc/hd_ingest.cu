@@ -1539,17 +1539,12 @@ __global__ void k_query(const uint4 *g0, uint64_t words, uint64_t n_rows, const 
 
 void query_distances_async(hd_ctx *ctx, const hd_alignment *aln, const uint8_t *d_query,
                            uint32_t *d_out_rows, DevBuf &q_planes) {
-  // pack the query with the alignment's AND codes (one row), then one warp per row
-  Table256 t;
-  code_table(kCodesAnd, t.v);
+  // pack the query with the AND codes (one row: 3 us), then one warp per row
   q_planes = DevBuf(aln->words * 16, ctx->stream);
-  DevBuf rs(8, ctx->stream);  // record start 0, freed after the kernels in stream order
-  HD_CUDA(cudaMemsetAsync(rs.p, 0, 8, ctx->stream));
-  k_pack<4><<<grid_for(hd::ceil_div((aln->words + 31) / 32, (uint64_t)kPackCPG) * 32, kPackThreads),
-              kPackThreads, 0, ctx->stream>>>(
-      d_query, rs.as<uint64_t>(), nullptr, 1, aln->length, aln->words, t, q_planes.as<uint4>(),
-      nullptr);
-  HD_LAUNCHED(ctx);
+  Records q;  // one record, at the start
+  q.base = d_query;
+  q.bytes = aln->length;
+  pack_planes(ctx, q, nullptr, 1, aln->length, aln->words, q_planes.as<uint4>(), nullptr);
   k_query<<<grid_for(aln->n_rows * 32, 256), 256, 0, ctx->stream>>>(
       static_cast<const uint4 *>(aln->planes_ptr(0)), aln->words, aln->n_rows,
       q_planes.as<uint4>(), d_out_rows);

@@ -33,13 +33,14 @@
 // cores read without a swizzle: for 8 rows (a row group) and 192 sites, the P
 // planes (1.0), the dash as 1.0 (read for rows) and the dash as -(P - 1)
 // (read for columns; -4 and -1 for P = 6) are blocks of 768 bytes, each six
-// 128-byte core matrices (8 rows x 16 bytes = 32 sites). Sites past L are 0. A
+// 128-byte core matrices (8 rows x 16 bytes = 32 sites). Sites past L are 0; the
+// dash blocks are written for the listed chunks only. A
 // row group's blocks follow one another, so a TMA box of 16 groups brings one
 // block of 128 rows. An alignment caches its operand; a view of a resident
 // alignment (a serving window) gets one of its own rows.
 //
 // One launch serves a job table of matrices. Persistent pairs of CTAs (a
-// cluster of two SMs, 320 threads each) walk a list of items: 256 rows x up to
+// cluster of two SMs, 352 threads each) walk a list of items: 256 rows x up to
 // 496 columns of one job, in bands of tile rows, column-major within a band,
 // so that resident pairs share operands in L2.
 //  * warps 0 and 10 (one thread each) take turns to issue the TMA loads of one
@@ -133,9 +134,11 @@ constexpr uint32_t kNoSlot = 0xFFFFFFFFu;             // an item that covers all
 // A split tile's partial distances of one K piece: 16-bit pairs, per CTA,
 // column half, lane quarter and word the 32 lanes of a warp
 constexpr uint64_t kSlotBytes = 2ull * 2 * 4 * kHalfWords * 32 * 4;
-// K pieces of fewer chunks than this cost more in barriers and workspace
-// traffic than they spread (three chunks of four planes run 3 us)
-constexpr uint32_t kMinPart = 3;
+// K pieces of fewer chunks than this cost more in barriers, workspace traffic
+// and k_pair_fix than they spread (six chunks of four planes run 6.5 us). A call
+// with pieces of 3, 6 and 10 chunks: 700 rows of 8,000 sites 72.2, 66.7 and
+// 74.2 us, 1,500 of 1,273 (7 chunks) 63.5, 62.3 and 61.8.
+constexpr uint32_t kMinPart = 6;
 // blocks of 192 sites per row and chunk in the operand: the P planes, the row
 // side's dash and the column side's dash (two blocks for P = 6: -4 and -1)
 __host__ __device__ constexpr uint32_t op_blocks(uint32_t planes) {
@@ -354,7 +357,7 @@ __device__ __forceinline__ void pack_sites(const uint32_t *v, uint32_t db, uint3
 
 // The text of rows [row_lo, row_hi) of the AND rule -> their plane words and
 // the plane blocks of their E2M1 operand rows, in one pass: row row_lo + i is
-// record rows[i] (none: i). Thread and store layout as in k_expand_op; the
+// record rows[i] (none: i; no rs: one record, at the start). Thread and store layout as in k_expand_op; the
 // sites past L are '-' in the planes and 0 in the operand. A thread reads the
 // 32 bytes of its sites as aligned 16-byte vectors. Eight sites' codes are
 // one word of nibbles z, in site order, in which plane p's E2M1 ones are the
@@ -386,7 +389,7 @@ __global__ void __launch_bounds__(256, 6)
   // the record starts of a group's rows are fetched one group ahead
   auto start_of = [&](uint64_t r) -> uint64_t {
     if (!valid || r < row_lo || r >= row_hi) return 0;
-    return lo + s0 + rs[rows ? rows[r - row_lo] : r - row_lo];
+    return lo + s0 + (rs ? rs[rows ? rows[r - row_lo] : r - row_lo] : 0);
   };
   uint64_t r = row_lo / 8 * 8 + blockIdx.y * 8 + row;
   uint64_t next = start_of(r);

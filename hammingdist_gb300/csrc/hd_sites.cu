@@ -226,7 +226,9 @@ struct BuildSums {
 // The lists of one (range, tile): a warp takes four rows at a time, a lane a
 // word. The block counts the entries of its sites, places them and, reading
 // the rows again (from the caches), files them. weight: sum of m per row.
-// What bounds it is the latency of the rows: LISTFIG
+// 14,000 rows of 29,903 sites: 150 us, bound by the instructions and the chains
+// of ballots, shuffles and atomics of a row's entries (a lane a word's entries
+// instead, one after another: 217 us; a row at a time: 173).
 template <bool kWide>  // more than four planes
 __global__ void __launch_bounds__(256, 4)
     k_site_lists(Planes p, uint64_t n, uint64_t L, uint32_t words, const uint4 *r0, const uint2 *r1,
