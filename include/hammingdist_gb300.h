@@ -414,10 +414,10 @@ void hd_server_free(hd_server *s);
  * (n bucket <= max_n_bucket, L bucket, dtype) with the GPU filled, and keeps
  * the fastest per bucket in the context: for the bit-plane engine the tile
  * edge (64/128 = 4/8 rows per thread) and TMA staging depth (2-4), for the
- * tensor-core engine the L2 band (8, 16 or 32 tile rows) and the item shape
- * (one or two 128-row tiles). Then, per L bucket, it times single matrices
- * of growing size on both engines and keeps the launch size (single-row-tile
- * items) from which the tensor-core engine wins. Without a table (or with
+ * tensor-core engine the L2 band (8, 16 or 32 item rows of 256) and the item
+ * shape (one or two column halves). Then, per L bucket, it times single
+ * matrices of growing size on both engines and keeps the launch size (tiles
+ * of 128 x 240 pairs) from which the tensor-core engine wins. Without a table (or with
  * HAMMINGDIST_TILE=<tile>x<stages>, HAMMINGDIST_MMA_BAND, HAMMINGDIST_MMA_ROWS,
  * HAMMINGDIST_MMA_MIN_ITEMS) built-in choices apply. No reference
  * counterpart (the reference has one kernel shape,
@@ -426,7 +426,7 @@ int hd_autotune(hd_ctx *ctx, uint64_t max_n_bucket);
 int hd_tune_lookup(hd_ctx *ctx, uint64_t n_rows, uint64_t length,
                    int dtype_bytes, int *tile, int *stages);
 /* The tensor-core engine's settings that apply to a matrix of n_rows x length
- * sites: L2 band (tile rows), row tiles per item (1 or 2) and the launch
+ * sites: L2 band (item rows), column halves per item (1 or 2) and the launch
  * size from which a launch goes to that engine. No reference counterpart. */
 int hd_tune_lookup_mma(hd_ctx *ctx, uint64_t n_rows, uint64_t length,
                        int dtype_bytes, int *band, int *rows, uint64_t *min_items);
@@ -452,10 +452,10 @@ const char *hd_trace_last(const hd_ctx *ctx);
  * IMAD per 32 pair-sites; pair-sites per second). No reference counterpart. */
 int hd_measure_int_peaks(hd_ctx *ctx, double *lop3_per_s, double *popc_per_s,
                          double *mix_pair_sites_per_s);
-/* Dense FP4 tensor-core rate of this device (FLOP per second): one CTA per SM
- * issues back-to-back tcgen05.mma.kind::mxf4.block_scale (E2M1, M=128,
- * N=256, K=64) on shared-memory operands, the instruction of the
- * tensor-core distance engine. No reference counterpart. */
+/* Dense FP4 tensor-core rate of this device (FLOP per second): CTA pairs
+ * issue back-to-back tcgen05.mma.cta_group::2.kind::mxf4.block_scale (E2M1,
+ * M=256, N=256 and 240, K=96) on shared-memory operands, the instructions of
+ * the tensor-core distance engine. No reference counterpart. */
 int hd_measure_mma_peak(hd_ctx *ctx, double *fp4_flop_per_s);
 /* Failure-path self-test: a kernel waits, with the bounded wait of the
  * pairwise kernel and a limit of limit_ns (<= 1 s), on an mbarrier that is
