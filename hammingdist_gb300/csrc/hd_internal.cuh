@@ -213,7 +213,8 @@ namespace hd {
 // sites said about them.
 struct SiteLists {
   int verdict = 0;  // 0: not looked at, 1: the distances use them, -1: they do not
-  double est_s = 0, est_d = 0, est_xd = 0;  // entries, and meetings with '-', from the sample
+  // from the sample: entries, those that a '-' counts against, '-', and their meetings
+  double est_s = 0, est_x = 0, est_d = 0, est_xd = 0;
   uint32_t tiles = 0, ranges = 0;           // tiles > 0: built
   uint32_t zero = 0;                        // sites that every pair mismatches in
   DevBuf base, off, es, ed, weight;

@@ -218,9 +218,10 @@ __global__ void __launch_bounds__(1024)
 struct BuildSums {
   unsigned long long s, d;     // entries
   unsigned long long pairs;    // of s entries that meet
+  unsigned long long dashes;   // of an s and a '-' entry of one site
   uint32_t full;               // some list did not fit
   uint32_t zero;               // sites where r is 0
-  uint32_t max_weight, pad[3];
+  uint32_t max_weight, pad;
 };
 
 // The lists of one (range, tile): a warp takes four rows at a time, a lane a
@@ -361,28 +362,42 @@ __global__ void __launch_bounds__(256, 4)
   });
 }
 
-// The pairs of s entries that meet over all tiles, and the largest weight
+// The pairs of s entries that meet over all tiles, of s and '-' entries, and
+// the largest weight. A lane takes a site, the block's warps a share of the
+// tiles each.
 __global__ void __launch_bounds__(256)
     k_site_check(const uint16_t *off, uint32_t tiles, uint32_t ranges, const uint32_t *weight,
                  uint64_t n, BuildSums *sums) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  unsigned long long pairs = 0;
-  if (i < (uint64_t)ranges * kRange) {
-    const uint32_t range = (uint32_t)(i / kRange), s = (uint32_t)(i % kRange);
-    unsigned long long k = 0, l = 0;
-    for (uint32_t t = 0; t < tiles; ++t) {
-      const uint16_t *o = off + ((uint64_t)t * ranges + range) * kOffSlot + s;
-      k += (uint32_t)o[1] - o[0];
-      l += (uint32_t)o[1] - o[kOffLater];
-    }
-    pairs = (k * k - l * l) / 2;
+  __shared__ uint32_t part[3][8][32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t range = blockIdx.x / (kRange / 32), s = (blockIdx.x % (kRange / 32)) * 32 + lane;
+  uint32_t k = 0, l = 0, d = 0;
+  for (uint32_t t = warp; t < tiles; t += 8) {
+    const uint16_t *o = off + ((uint64_t)t * ranges + range) * kOffSlot + s;
+    k += (uint32_t)o[1] - o[0];
+    l += (uint32_t)o[1] - o[kOffLater];
+    d += (uint32_t)o[kOffDash + 1] - o[kOffDash];
   }
-  pairs = warp_sum(pairs);
-  if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&sums->pairs, pairs);
+  part[0][warp][lane] = k;
+  part[1][warp][lane] = l;
+  part[2][warp][lane] = d;
+  __syncthreads();
+  if (warp == 0) {
+    unsigned long long v[3] = {0, 0, 0};
+#pragma unroll
+    for (int w = 0; w < 8; ++w)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) v[j] += part[j][w][lane];
+    const unsigned long long pairs = warp_sum((v[0] * v[0] - v[1] * v[1]) / 2);
+    const unsigned long long dashes = warp_sum(v[0] * v[2]);
+    if (lane == 0 && pairs) atomicAdd(&sums->pairs, pairs);
+    if (lane == 0 && dashes) atomicAdd(&sums->dashes, dashes);
+  }
   uint32_t m = 0;
-  for (uint64_t r = i; r < n; r += (uint64_t)gridDim.x * blockDim.x) m = max(m, weight[r]);
+  for (uint64_t r = blockIdx.x * 256ull + threadIdx.x; r < n; r += gridDim.x * 256ull)
+    m = max(m, weight[r]);
   m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) atomicMax(&sums->max_weight, m);
+  if (lane == 0 && m) atomicMax(&sums->max_weight, m);
 }
 
 // The tile pair's distances from its counters: a warp a row, a lane a column of
@@ -676,7 +691,8 @@ bool sites_likely(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st, uint64_t 
   k_site_ref<<<(unsigned)ceil_div((uint64_t)sel.count, (uint64_t)2), 256, 0, st>>>(p, have, sel, r0,
                                                                                    r1);
   HD_LAUNCHED(ctx);
-  const uint64_t shares = std::min<uint64_t>(ceil_div(have, (uint64_t)512), 64);
+  // two rounds of a block's 64 rows: the rows' latency is most of its time
+  const uint64_t shares = std::min<uint64_t>(ceil_div(have, (uint64_t)128), 65535);
   k_site_count<<<dim3(quads, (unsigned)shares), 256, 0, st>>>(p, have, a->length, sel, r0, r1, counts);
   HD_LAUNCHED(ctx);
   k_site_cost<<<1, 1024, 0, st>>>(counts, 32 * sel.edges(), quads * 128, sums);
@@ -689,6 +705,7 @@ bool sites_likely(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st, uint64_t 
   const double more = (double)rows / (double)have;
   auto est = [&](int k) { return (double)h[k] + up * (double)h[5 + k]; };
   S.est_s = more * est(0);
+  S.est_x = more * est(1);
   S.est_d = more * est(2);
   S.est_xd = more * more * est(4);
   const double t = lists_us(rows, a->length, more * more * (est(3) + est(4)));
@@ -744,7 +761,7 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
         S.es.as<uint32_t>(), S.ed.as<uint8_t>(), S.weight.as<uint32_t>() + row, sums);
     HD_LAUNCHED(ctx);
   }
-  k_site_check<<<(unsigned)ceil_div((uint64_t)ranges * kRange, (uint64_t)256), 256, 0, st>>>(
+  k_site_check<<<ranges * (kRange / 32), 256, 0, st>>>(
       S.off.as<uint16_t>(), (uint32_t)tiles, ranges, S.weight.as<uint32_t>(), a->n_rows, sums);
   HD_LAUNCHED(ctx);
   auto *h = reinterpret_cast<BuildSums *>(pinned_words(ctx));
@@ -753,7 +770,10 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
   // every list fits, a pair's sum of c (at most the distance's other terms)
   // fits 16 bits, and the true count of pairs still costs less than the engine
   const bool fits = !h->full && 2ull * h->max_weight + h->zero <= 65535;
-  const double t = lists_us(a->n_rows, a->length, (double)h->pairs + S.est_xd);
+  // meetings with '-': the pairs found, by the sample's share of s entries that
+  // do meet a '-', if the sample saw fewer
+  const double dash = std::max(S.est_xd, (double)h->dashes * S.est_x / std::max(1.0, S.est_s));
+  const double t = lists_us(a->n_rows, a->length, (double)h->pairs + dash);
   if (!fits || (forced() == 0 && t > dense_us(a->n_rows, a->length, (uint32_t)a->planes))) {
     S.release();
     return false;
