@@ -227,6 +227,8 @@ struct BuildSums {
 // The lists of one (range, tile): a warp takes four rows at a time, a lane a
 // word. The block counts the entries of its sites, places them and, reading
 // the rows again (from the caches), files them. weight: sum of m per row.
+// first_rows: block row 0 is the alignment's first tile (not that of a later
+// launch), which counts the sites where r is 0.
 // 14,000 rows of 29,903 sites: 150 us, bound by the instructions and the chains
 // of ballots, shuffles and atomics of a row's entries (a lane a word's entries
 // instead, one after another: 217 us; a row at a time: 173).
@@ -234,7 +236,7 @@ template <bool kWide>  // more than four planes
 __global__ void __launch_bounds__(256, 4)
     k_site_lists(Planes p, uint64_t n, uint64_t L, uint32_t words, const uint4 *r0, const uint2 *r1,
                  uint32_t ranges, uint64_t cap_s, uint64_t cap_d, uint4 *base, uint16_t *off,
-                 uint32_t *es, uint8_t *ed, uint32_t *weight, BuildSums *sums) {
+                 uint32_t *es, uint8_t *ed, uint32_t *weight, bool first_rows, BuildSums *sums) {
   __shared__ uint32_t cnt[3][kRange];  // first entries, later ones of runs, '-'
   __shared__ uint64_t tmp[33];
   __shared__ unsigned long long at_s, at_d;
@@ -288,7 +290,7 @@ __global__ void __launch_bounds__(256, 4)
     const uint32_t m = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(f.s & ~zero));
     if (lane == 0 && m) atomicAdd(&weight[row0 + i], m);
   });
-  if (tile == 0 && warp == 0) {
+  if (first_rows && tile == 0 && warp == 0) {
     const uint32_t z = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(zero));
     if (lane == 0 && z) atomicAdd(&sums->zero, z);
   }
@@ -758,7 +760,7 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
     (q.planes > 4 ? k_site_lists<true> : k_site_lists<false>)<<<dim3(ranges, (unsigned)tn), 256, 0, st>>>(
         q, a->n_rows - row, a->length, words, r0, r1, ranges, cap_s, cap_d,
         S.base.as<uint4>() + t0 * ranges, S.off.as<uint16_t>() + t0 * ranges * kOffSlot,
-        S.es.as<uint32_t>(), S.ed.as<uint8_t>(), S.weight.as<uint32_t>() + row, sums);
+        S.es.as<uint32_t>(), S.ed.as<uint8_t>(), S.weight.as<uint32_t>() + row, t0 == 0, sums);
     HD_LAUNCHED(ctx);
   }
   k_site_check<<<ranges * (kRange / 32), 256, 0, st>>>(
