@@ -280,10 +280,10 @@ struct hd_alignment {
   mutable uint64_t op_rows = 0, op_cap = 0;
   // per 192-site chunk of the operand (uint32 each): 0, or the extension of
   // the operand (1, 2, ...) whose rows had the chunk's first '-' (the chunks
-  // whose dash products count, and whose dash blocks are written)
+  // whose dash products count, and whose dash blocks are written); then the
+  // marked chunks' list and ranks after the first extension
   mutable hd::DevBuf op_dash;
-  // the marked chunks' list and ranks after each extension of the operand,
-  // the last one current
+  // the list and ranks after each later extension, the last one current
   mutable std::vector<hd::DevBuf> op_lists;
   // built on first use, where the distances use them (hd_sites.cu)
   mutable std::unique_ptr<hd::SiteLists> sites;

@@ -260,42 +260,54 @@ __global__ void k_expand_op(const uint4 *__restrict__ g0, const uint4 *__restric
   }
 }
 
-// The dash blocks of the marked chunks (list[0 .. *n)): of rows [row_lo,
+// One extension of an operand whose marked chunks are to be listed and their
+// dash blocks written: rows [row_lo, row_hi) of the planes g0, g1, now in x.
+struct DashJob {
+  const uint4 *g0, *g1;
+  uint8_t *x;
+  const uint32_t *marks;
+  uint32_t *list;  // the marked chunks, then the listed ones before each chunk (chunks + 1)
+  unsigned long long row_lo, row_hi, sites;
+  uint32_t planes, words, ext, pad;
+};
+
+// The dash blocks of the marked chunks (the job's list): of rows [row_lo,
 // row_hi), and for a chunk that extension `ext` marked first of the rows
 // before them, which have no '-' there. The other chunks' blocks are never
 // read, and stay unwritten: two of an operand's six blocks (four planes),
 // 0.4 of 1.3 GB for 14,000 rows of 29,903 sites. A thread per (row, word):
-// 48 threads take one row group of a chunk.
+// 48 threads take one row group of a chunk. Block row y takes job y of `jobs`,
+// or `one` without them.
 constexpr uint32_t kDashGroups = 4;  // row groups per block
 __global__ void __launch_bounds__(kDashGroups * 8 * kChunkWords)
-    k_dash_blocks(const uint4 *__restrict__ g0, const uint4 *__restrict__ g1, uint32_t planes,
-                  uint32_t words, uint64_t row_lo, uint64_t row_hi, uint64_t L,
-                  uint8_t *__restrict__ x, const uint32_t *__restrict__ marks, uint32_t ext,
-                  const uint32_t *__restrict__ list, const uint32_t *__restrict__ n) {
+    k_dash_blocks(DashJob one, const DashJob *__restrict__ jobs, uint32_t n_jobs) {
   const uint32_t sub = threadIdx.x / (8 * kChunkWords), u = threadIdx.x % (8 * kChunkWords);
-  const uint32_t nb = op_blocks(planes);
-  const uint64_t group_bytes = op_group_bytes(planes, L);
-  const uint64_t batches = ((row_hi + 7) / 8 + kDashGroups - 1) / kDashGroups;
-  const uint64_t jobs = batches * *n;
-  for (uint64_t job = blockIdx.x; job < jobs; job += gridDim.x) {
-    const uint64_t i = job / batches, g = (job - i * batches) * kDashGroups + sub;
-    const uint32_t c = list[i], w = c * kChunkWords + u / 8;
-    const uint64_t r = g * 8 + (u & 7u), s0 = (uint64_t)w * 32;
-    if (r >= row_hi || (r < row_lo && marks[c] != ext)) continue;
-    uint32_t dash = s0 >= L ? 0u : (L - s0 >= 32 ? 0xffffffffu : ((1u << (L - s0)) - 1u));
-    if (w < words) {
-      const uint4 p = g0[r * words + w];
-      dash &= p.x & p.y & p.z & p.w;
-      if (planes > 4) {
-        const uint4 p1 = g1[r * words + w];
-        dash &= p1.x;
-        if (planes > 5) dash &= p1.y;
+  for (uint32_t q = blockIdx.y; q < n_jobs; q += gridDim.y) {
+    const DashJob j = jobs ? jobs[q] : one;
+    const uint32_t nb = op_blocks(j.planes), chunks = op_chunks(j.sites);
+    const uint64_t group_bytes = op_group_bytes(j.planes, j.sites);
+    const uint64_t batches = ((j.row_hi + 7) / 8 + kDashGroups - 1) / kDashGroups;
+    const uint64_t work = batches * j.list[2 * chunks];
+    for (uint64_t t = blockIdx.x; t < work; t += gridDim.x) {
+      const uint64_t i = t / batches, g = (t - i * batches) * kDashGroups + sub;
+      const uint32_t c = j.list[i], w = c * kChunkWords + u / 8;
+      const uint64_t r = g * 8 + (u & 7u), s0 = (uint64_t)w * 32;
+      if (r >= j.row_hi || (r < j.row_lo && j.marks[c] != j.ext)) continue;
+      uint32_t dash = s0 >= j.sites ? 0u : (j.sites - s0 >= 32 ? 0xffffffffu : ((1u << (j.sites - s0)) - 1u));
+      if (w < j.words) {
+        const uint4 p = j.g0[r * j.words + w];
+        dash &= p.x & p.y & p.z & p.w;
+        if (j.planes > 4) {
+          const uint4 p1 = j.g1[r * j.words + w];
+          dash &= p1.x;
+          if (j.planes > 5) dash &= p1.y;
+        }
       }
+      uint8_t *blk = j.x + g * group_bytes + ((uint64_t)c * nb + j.planes) * kGroupBytes + u * 16u;
+      put16(blk, dash, kE2M1One);                         // 1.0: the row side
+      put16(blk + kGroupBytes, dash, dash_neg(j.planes));  // the column side
+      if (j.planes == 6) put16(blk + 2 * kGroupBytes, dash, kE2M1Neg1);
     }
-    uint8_t *blk = x + g * group_bytes + ((uint64_t)c * nb + planes) * kGroupBytes + u * 16u;
-    put16(blk, dash, kE2M1One);                       // 1.0: the row side
-    put16(blk + kGroupBytes, dash, dash_neg(planes));  // the column side
-    if (planes == 6) put16(blk + 2 * kGroupBytes, dash, kE2M1Neg1);
   }
 }
 
@@ -1193,17 +1205,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1)
 }
 
 // The ascending list of the chunks whose mark is set, and for every chunk the
-// listed ones before it (one block).
-__global__ void __launch_bounds__(512)
-    k_dash_list(const uint32_t *marks, uint32_t chunks, uint32_t *list, uint32_t *before) {
+// listed ones before it (a block per job of `jobs`, or one block for `one`).
+__global__ void __launch_bounds__(512) k_dash_list(DashJob one, const DashJob *__restrict__ jobs) {
   __shared__ uint32_t tmp[33];
-  uint32_t n = 0;
+  const DashJob j = jobs ? jobs[blockIdx.x] : one;
+  const uint32_t chunks = op_chunks(j.sites);
+  uint32_t *before = j.list + chunks, n = 0;
   for (uint32_t c0 = 0; c0 < chunks; c0 += blockDim.x) {
     const uint32_t c = c0 + threadIdx.x;
-    const uint32_t on = c < chunks && marks[c] != 0u ? 1u : 0u;
+    const uint32_t on = c < chunks && j.marks[c] != 0u ? 1u : 0u;
     uint32_t total;
     const uint32_t at = n + block_excl_scan<uint32_t>(on, tmp, total);
-    if (on) list[at] = c;
+    if (on) j.list[at] = c;
     if (c < chunks) before[c] = at;
     n += total;
   }
@@ -1240,34 +1253,67 @@ void make_tmap_op(hd_ctx *ctx, CUtensorMap *tm, const void *base, uint32_t plane
 uint64_t mark_words(uint64_t sites) { return op_chunks(sites); }
 uint64_t list_words(uint64_t sites) { return 2 * (uint64_t)op_chunks(sites) + 1; }
 
-// The list of the marked chunks, and their dash blocks (k_dash_blocks).
-void dash_rows(hd_ctx *ctx, const uint4 *g0, const uint4 *g1, uint32_t planes, uint64_t words,
-               uint64_t lo, uint64_t hi, uint64_t sites, uint8_t *x, uint32_t *marks, uint32_t ext,
-               uint32_t *list, cudaStream_t stream) {
-  const uint32_t chunks = op_chunks(sites);
-  k_dash_list<<<1, 512, 0, stream>>>(marks, chunks, list, list + chunks);
-  HD_LAUNCHED(ctx);
-  const uint64_t jobs = ceil_div(ceil_div(hi, (uint64_t)8), (uint64_t)kDashGroups) * chunks;
-  k_dash_blocks<<<(unsigned)std::min<uint64_t>(jobs, (uint64_t)ctx->sm_count * 8),
-                  kDashGroups * 8 * kChunkWords, 0, stream>>>(
-      g0, g1, planes, (uint32_t)words, lo, hi, sites, x, marks, ext, list, list + 2 * chunks);
-  HD_LAUNCHED(ctx);
+// The list of a job's marked chunks, and their dash blocks.
+void dash_rows(const DashJob &j, int sm_count, cudaStream_t stream) {
+  k_dash_list<<<1, 512, 0, stream>>>(j, nullptr);
+  const uint64_t work = ceil_div(ceil_div((uint64_t)j.row_hi, (uint64_t)8), (uint64_t)kDashGroups) *
+                        op_chunks(j.sites);
+  k_dash_blocks<<<(unsigned)std::min<uint64_t>(work, (uint64_t)sm_count * 8),
+                  kDashGroups * 8 * kChunkWords, 0, stream>>>(j, nullptr, 1);
 }
+
+// The jobs of a plan whose chunks are not listed yet: two launches for all of
+// them instead of two for each (first run of a batch of 200 matrices of 20 to
+// 128 rows: 1.6 ms, with two for each 3.2; 50 served windows of 100 rows 1.57
+// and 1.84). Left early, each is listed by itself: their alignments count the
+// rows as there.
+struct DashJobs {
+  hd_ctx *ctx;
+  cudaStream_t stream;
+  std::vector<DashJob> jobs;
+  ~DashJobs() {
+    for (const DashJob &j : jobs) dash_rows(j, ctx->sm_count, stream);
+  }
+  // d_jobs: their copy on the device
+  void launch(const DashJob *d_jobs) {
+    const uint32_t n = (uint32_t)jobs.size();
+    if (!n) return;
+    k_dash_list<<<n, 512, 0, stream>>>(DashJob{}, d_jobs);
+    HD_LAUNCHED(ctx);
+    const unsigned y = std::min(n, 65535u);
+    const unsigned x = (unsigned)ceil_div((uint64_t)ctx->sm_count * 32, (uint64_t)y);
+    k_dash_blocks<<<dim3(x, y), kDashGroups * 8 * kChunkWords, 0, stream>>>(DashJob{}, d_jobs, n);
+    HD_LAUNCHED(ctx);
+    jobs.clear();
+  }
+};
+
 dim3 op_grid(uint64_t words, uint64_t lo, uint64_t hi) {
   const uint64_t groups = ceil_div(hi, (uint64_t)8) - lo / 8;
   return dim3((unsigned)ceil_div(words, (uint64_t)32),
               (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(groups, 65535)));
 }
 
-// Expands rows [lo, hi) of the planes into the operand x, as its extension
-// `ext`, marks the chunks with a '-' and lists the marked ones.
-void expand_rows(hd_ctx *ctx, const uint4 *g0, const uint4 *g1, uint32_t planes, uint64_t words,
-                 uint64_t lo, uint64_t hi, uint64_t sites, uint8_t *x, uint32_t *marks,
-                 uint32_t ext, uint32_t *list, cudaStream_t stream) {
-  k_expand_op<<<op_grid((uint64_t)op_chunks(sites) * kChunkWords, lo, hi), 256, 0, stream>>>(
-      g0, g1, planes, (uint32_t)words, lo, hi, sites, x, marks, ext);
+// Lists the job's chunks with the plan's others, or now.
+void list_chunks(hd_ctx *ctx, const DashJob &j, cudaStream_t stream, DashJobs *later) {
+  if (later) {
+    later->jobs.push_back(j);
+    return;
+  }
+  dash_rows(j, ctx->sm_count, stream);
+  check_cuda(cudaGetLastError(), "kernel launch");
+  ctx->launches += 2;
+}
+
+// Expands the job's rows of the planes into its operand, marks the chunks with
+// a '-' and lists the marked ones.
+void expand_rows(hd_ctx *ctx, const DashJob &j, uint32_t *marks, cudaStream_t stream,
+                 DashJobs *later) {
+  k_expand_op<<<op_grid((uint64_t)op_chunks(j.sites) * kChunkWords, j.row_lo, j.row_hi), 256, 0,
+                stream>>>(j.g0, j.g1, j.planes, j.words, j.row_lo, j.row_hi, j.sites, j.x, marks,
+                          j.ext);
   HD_LAUNCHED(ctx);
-  dash_rows(ctx, g0, g1, planes, words, lo, hi, sites, x, marks, ext, list, stream);
+  list_chunks(ctx, j, stream, later);
 }
 
 }  // namespace
@@ -1321,29 +1367,51 @@ bool grow_operand(hd_ctx *ctx, const hd_alignment *o, uint64_t rows, cudaStream_
     o->op = std::move(grown);
     o->op_cap = cap;
   }
+  // a list of its own for every extension (the first one's after the marks):
+  // launches on other streams may still read an earlier one
   if (!o->op_dash.p) {
-    o->op_dash = DevBuf(mark_words(o->length) * 4, stream);
-    HD_CUDA(cudaMemsetAsync(o->op_dash.p, 0, mark_words(o->length) * 4, stream));
+    const uint64_t marks = mark_words(o->length);
+    o->op_dash = DevBuf((marks + list_words(o->length)) * 4, stream);
+    HD_CUDA(cudaMemsetAsync(o->op_dash.p, 0, marks * 4, stream));
+  } else {
+    o->op_lists.emplace_back(list_words(o->length) * 4, stream);
   }
-  // a list of its own for every extension: launches on other streams may
-  // still read an earlier one
-  o->op_lists.emplace_back(list_words(o->length) * 4, stream);
+  return true;
+}
+// The list of the operand's last extension
+uint32_t *last_list(const hd_alignment *o) {
+  return o->op_lists.empty() ? o->op_dash.as<uint32_t>() + mark_words(o->length)
+                             : o->op_lists.back().as<uint32_t>();
+}
+// The extension to rows [op_rows, rows) that grow_operand made room for
+DashJob extension_of(const hd_alignment *o, uint64_t rows) {
+  DashJob j{};
+  j.g0 = o->plane_buf[0].as<uint4>();
+  j.g1 = o->planes > 4 ? o->plane_buf[1].as<uint4>() : nullptr;
+  j.x = o->op.as<uint8_t>();
+  j.marks = o->op_dash.as<uint32_t>();
+  j.list = last_list(o);
+  j.row_lo = o->op_rows;
+  j.row_hi = rows;
+  j.sites = o->length;
+  j.planes = (uint32_t)o->planes;
+  j.words = (uint32_t)o->words;
+  j.ext = (uint32_t)o->op_lists.size() + 1;
+  return j;
+}
+bool extend_operand(hd_ctx *ctx, const hd_alignment *o, uint64_t rows, cudaStream_t stream,
+                    uint64_t cap_hint, DashJobs *later) {
+  if (o->op_rows >= rows) return true;
+  if (!grow_operand(ctx, o, rows, stream, cap_hint)) return false;
+  expand_rows(ctx, extension_of(o, rows), o->op_dash.as<uint32_t>(), stream, later);
+  o->op_rows = rows;
   return true;
 }
 }  // namespace
 
 bool ensure_operand(hd_ctx *ctx, const hd_alignment *aln, uint64_t rows, cudaStream_t stream,
                     uint64_t cap_hint) {
-  const hd_alignment *o = aln->base ? aln->base : aln;
-  if (o->op_rows >= rows) return true;
-  if (!grow_operand(ctx, o, rows, stream, cap_hint)) return false;
-  const uint32_t P = (uint32_t)o->planes;
-  expand_rows(ctx, o->plane_buf[0].as<uint4>(), P > 4 ? o->plane_buf[1].as<uint4>() : nullptr, P,
-              o->words, o->op_rows, rows, o->length, o->op.as<uint8_t>(),
-              o->op_dash.as<uint32_t>(), (uint32_t)o->op_lists.size(),
-              o->op_lists.back().as<uint32_t>(), stream);
-  o->op_rows = rows;
-  return true;
+  return extend_operand(ctx, aln->base ? aln->base : aln, rows, stream, cap_hint, nullptr);
 }
 
 namespace {
@@ -1371,17 +1439,14 @@ bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const
                   uint64_t lo, uint64_t hi, uint4 *copy, cudaStream_t stream, uint64_t cap_hint) {
   if (aln->base || aln->planes != 4 || aln->op_rows != lo || hi <= lo) return false;
   if (!grow_operand(ctx, aln, hi, stream, cap_hint)) return false;
-  const uint32_t ext = (uint32_t)aln->op_lists.size();
-  uint4 *g0 = aln->plane_buf[0].as<uint4>();
-  uint8_t *x = aln->op.as<uint8_t>();
-  uint32_t *marks = aln->op_dash.as<uint32_t>();
+  const DashJob j = extension_of(aln, hi);
   const uint64_t op_words = (uint64_t)op_chunks(aln->length) * kChunkWords;
   k_pack_op<true><<<pack_grid(ctx, std::max(aln->words, op_words), lo, hi), 256, 0, stream>>>(
       rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), d_rows, lo, hi, aln->length,
-      (uint32_t)aln->words, g0, copy, x, marks, ext, Words::of(0, 1));
+      (uint32_t)aln->words, aln->plane_buf[0].as<uint4>(), copy, j.x, aln->op_dash.as<uint32_t>(),
+      j.ext, Words::of(0, 1));
   HD_LAUNCHED(ctx);
-  dash_rows(ctx, g0, nullptr, 4, aln->words, lo, hi, aln->length, x, marks, ext,
-            aln->op_lists.back().as<uint32_t>(), stream);
+  list_chunks(ctx, j, stream, nullptr);
   aln->op_rows = hi;
   return true;
 }
@@ -1417,19 +1482,19 @@ double measure_mma_peak(hd_ctx *ctx) {
 // until the kernel has run (a serving window must not expand a large base).
 // False if there is no memory for it.
 bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLaunchPlan *plan,
-                 const uint8_t *&op, const uint32_t *&dash) {
+                 const uint8_t *&op, const uint32_t *&dash, DashJobs *later) {
   const hd_alignment *o = a->base ? a->base : a;
   if (!a->base) {
-    if (!ensure_operand(ctx, a, a->n_rows, stream)) return false;
+    if (!extend_operand(ctx, a, a->n_rows, stream, 0, later)) return false;
     op = a->op.as<uint8_t>();
-    dash = a->op_lists.back().as<uint32_t>();
+    dash = last_list(a);
     return true;
   }
   if (a->row0 == 0 && o->op.p && o->op_rows >= a->n_rows) {
     // the base's listed chunks cover its other rows too: a chunk listed for
     // them only adds dash products of 0
     op = o->op.as<uint8_t>();
-    dash = o->op_lists.back().as<uint32_t>();
+    dash = last_list(o);
     return true;
   }
   const uint32_t P = (uint32_t)o->planes;
@@ -1446,12 +1511,21 @@ bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLa
   }
   uint32_t *flags = reinterpret_cast<uint32_t *>(tmp.as<uint8_t>() + bytes);
   HD_CUDA(cudaMemsetAsync(flags, 0, marks * 4, stream));
-  expand_rows(ctx, static_cast<const uint4 *>(a->planes_ptr(0)),
-              P > 4 ? static_cast<const uint4 *>(a->planes_ptr(1)) : nullptr, P, o->words, 0,
-              a->n_rows, o->length, tmp.as<uint8_t>(), flags, 1, flags + marks, stream);
-  op = tmp.as<uint8_t>();
-  dash = flags + marks;
+  DashJob j{};
+  j.g0 = static_cast<const uint4 *>(a->planes_ptr(0));
+  j.g1 = P > 4 ? static_cast<const uint4 *>(a->planes_ptr(1)) : nullptr;
+  j.x = tmp.as<uint8_t>();
+  j.marks = flags;
+  j.list = flags + marks;
+  j.row_hi = a->n_rows;
+  j.sites = o->length;
+  j.planes = P;
+  j.words = (uint32_t)o->words;
+  j.ext = 1;
   plan->blocks.push_back(std::move(tmp));
+  expand_rows(ctx, j, flags, stream, later);
+  op = j.x;
+  dash = j.list;
   return true;
 }
 
@@ -1621,6 +1695,7 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     double cost;
   };
   std::vector<Job> js;
+  DashJobs unlisted{ctx, stream, {}};
   // A small launch leaves SMs idle: below a minimum size, counted in tiles of
   // 128 x kMmaCols pairs (mma_min_items_for, autotuned per row length), the
   // bit-plane engine's finer tiles finish first; a batch of small matrices
@@ -1646,7 +1721,7 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     const uint64_t edge = sp.cfg.tile > 0 ? (uint64_t)sp.cfg.tile : kTile;
     const uint64_t row_lo = sp.tile_lo * edge, row_hi = std::min<uint64_t>(sp.tile_hi * edge, a->n_rows);
     if (row_lo % kTM || row_hi <= row_lo) continue;
-    if (!operand_for(ctx, a, stream, plan, ops[k], dash_lists[k])) continue;
+    if (!operand_for(ctx, a, stream, plan, ops[k], dash_lists[k], &unlisted)) continue;
     const uint32_t lo = (uint32_t)(row_lo / kTM), hi = (uint32_t)ceil_div(row_hi, kTM);
     js.push_back({k, lo, hi, (double)a->words * ((double)hi * hi - (double)lo * lo)});
     taken[k] = 1;
@@ -1737,12 +1812,13 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     }
   }
   // one device block: [tensor maps (2 per job)][jobs][items][split tiles]
-  // [queue counter]
+  // [queue counter][chunks to list]
   const size_t tm_bytes = nj * 2 * sizeof(CUtensorMap);
   const size_t job_at = tm_bytes, item_at = job_at + round_up(nj * sizeof(MmaJob), 64);
   const size_t fix_at = item_at + mp.items.size() * sizeof(MmaItem);
   const size_t counter_at = fix_at + round_up(mp.fix.size() * sizeof(MmaFix), 16);
-  std::vector<uint8_t> host(counter_at + 16, 0);
+  const size_t dash_at = counter_at + 16;
+  std::vector<uint8_t> host(dash_at + unlisted.jobs.size() * sizeof(DashJob), 0);
   DevBuf dev(host.size(), stream);
   auto *tms = reinterpret_cast<CUtensorMap *>(host.data());
   auto *jobs = reinterpret_cast<MmaJob *>(host.data() + job_at);
@@ -1768,9 +1844,11 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
   }
   std::memcpy(host.data() + item_at, mp.items.data(), mp.items.size() * sizeof(MmaItem));
   std::memcpy(host.data() + fix_at, mp.fix.data(), mp.fix.size() * sizeof(MmaFix));
+  std::memcpy(host.data() + dash_at, unlisted.jobs.data(), unlisted.jobs.size() * sizeof(DashJob));
   // staged in pinned memory (pageable for a large table): `host` may go when this returns
   upload_table(ctx, dev.p, host.data(), host.size(), stream);
   uint8_t *d = dev.as<uint8_t>();
+  unlisted.launch(reinterpret_cast<const DashJob *>(d + dash_at));
   PairLaunchPlan::Launch L;
   L.mma = true;
   L.fn = reinterpret_cast<const void *>(k_pairwise_mma);
