@@ -47,6 +47,12 @@ uint64_t mma_items_of(uint64_t n) {
     items += ((I + 1) * kTile - 2) / kMmaCols + 1;
   return items;
 }
+// What the tensor-core fields of a saved table (mma_band, mma_rows,
+// mma_min_items) mean and were measured with: 2 is items of 256 rows x 496
+// columns on CTA pairs, bands in item rows, mma_rows the column halves of an
+// item. A table that hd_tune_save wrote ("sm_count" is in it) without this
+// number counted rows of 128 and row tiles, and was measured on another kernel.
+constexpr int kMmaEngine = 2;
 uint32_t key_of(int nb, int lb, int dtype) { return (uint32_t)(nb * 100 + lb * 10 + dtype); }
 
 bool env_override(TileConfig &c) {
@@ -275,7 +281,7 @@ extern "C" int hd_tune_save(hd_ctx *ctx, const char *path) {
     std::ofstream f(path);
     if (!f) hd::fail(HD_ERR_IO, std::string("Error: Failed to open file '") + path + "'");
     f << "{\"device\": \"" << prop.name << "\", \"sm_count\": " << ctx->sm_count
-      << ", \"mma_min_items\": [";
+      << ", \"mma_engine\": " << hd::kMmaEngine << ", \"mma_min_items\": [";
     for (int lb = 0; lb < 4; ++lb) f << (lb ? ", " : "") << ctx->tune.mma_min_items[lb];
     f << "], \"entries\": [";
     for (size_t k = 0; k < ctx->tune.entries.size(); ++k) {
@@ -309,6 +315,10 @@ extern "C" int hd_tune_load(hd_ctx *ctx, const char *path) {
       v = std::atoi(s.c_str() + p + 1);
       return true;
     };
+    // tensor-core settings of another engine are left out (built-in ones apply)
+    int saved = 0, engine = 0;
+    const bool mma_fields = !field("sm_count", 0, s.size(), saved) ||
+                            (field("mma_engine", 0, s.size(), engine) && engine == hd::kMmaEngine);
     size_t pos = 0;
     while ((pos = s.find("\"n_bucket\"", pos)) != std::string::npos) {
       const size_t begin = s.rfind('{', pos);
@@ -327,8 +337,10 @@ extern "C" int hd_tune_load(hd_ctx *ctx, const char *path) {
       hd::TileConfig c;
       c.tile = tile;
       c.stages = st;
-      c.mma_band = band;
-      c.mma_rows = rows;
+      if (mma_fields) {
+        c.mma_band = band;
+        c.mma_rows = rows;
+      }
       table.entries.push_back({hd::key_of(nb, lb, dt), c});
       pos = end;
     }
@@ -336,7 +348,7 @@ extern "C" int hd_tune_load(hd_ctx *ctx, const char *path) {
     const size_t mi = s.find("\"mma_min_items\"");
     const size_t open_b = mi == std::string::npos ? mi : s.find('[', mi);
     const size_t close_b = open_b == std::string::npos ? open_b : s.find(']', open_b);
-    if (close_b != std::string::npos) {
+    if (mma_fields && close_b != std::string::npos) {
       size_t q = open_b + 1;
       for (int lb = 0; lb < 4 && q < close_b; ++lb) {
         table.mma_min_items[lb] = (uint64_t)std::strtoull(s.c_str() + q, nullptr, 10);
