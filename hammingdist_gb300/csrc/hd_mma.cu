@@ -1664,6 +1664,19 @@ void plan_queue(std::vector<MmaItem> &list, uint32_t units, const std::vector<ui
   plan.pairs = (uint32_t)std::min<uint64_t>(units, plan.items.size());
 }
 
+// The item, or (halves) its column halves as items of their own.
+void push_item(std::vector<MmaItem> &list, MmaItem it, bool halves) {
+  if (halves && it.n1_16) {
+    MmaItem first = it;
+    first.n1_16 = 0;
+    list.push_back(first);
+    it.col0 += it.n0();
+    it.n0_16 = it.n1_16;
+    it.n1_16 = 0;
+  }
+  list.push_back(it);
+}
+
 }  // namespace
 
 // Size of the tile rows [lo, hi) in tiles of 128 x kMmaCols pairs: what the
@@ -1771,13 +1784,7 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
           const uint32_t n0 = std::min(need, kN0), n1 = need - n0;
           MmaItem it{q, r, col, (uint8_t)(n0 / 16), (uint8_t)(n1 / 16), (uint8_t)planes[q], 0, 0,
                      chunks, kNoSlot, 0};
-          if (halves && n1) {
-            it.n1_16 = 0;
-            list.push_back(it);
-            it.col0 = col + n0;
-            it.n0_16 = (uint8_t)(n1 / 16);
-          }
-          list.push_back(it);
+          push_item(list, it, halves);
         }
     }
   }
@@ -1785,6 +1792,14 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
   // matrices always go through the queue)
   const int sms = sm_limit > 0 && sm_limit < ctx->sm_count ? sm_limit : ctx->sm_count;
   const uint32_t units = (uint32_t)std::max(1, sms / 2);
+  // 32-bit outputs are not split along K: where two thirds of an item's time
+  // for twice the items leave every pair one at most, they are cut into column
+  // halves (a call with 1,000 rows of 29,903 sites 233 -> 177 us)
+  if (nj == 1 && specs[js[0].k].dtype == 4 && 2 * list.size() <= units) {
+    std::vector<MmaItem> cut;
+    for (const MmaItem &it : list) push_item(cut, it, true);
+    list.swap(cut);
+  }
   bool queue = nj > 1;
   if (const char *e = std::getenv("HAMMINGDIST_MMA_SCHEDULE"))
     queue = queue || std::string(e) == "queue";
