@@ -82,7 +82,9 @@
 // Pairs halve the column bytes an SM loads and its MMAs read.
 #include <algorithm>
 #include <cstdlib>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -217,59 +219,96 @@ __device__ __forceinline__ void put16(uint8_t *dst, uint32_t w, uint32_t v) {
                  nib8(w >> 24, v));
 }
 
-// Rows [row_lo, row_hi) of a P-plane alignment (P = 4: the AND rule; 5, 6:
-// the sparse rules, planes 4-5 in the second group) -> the plane blocks of
-// their E2M1 operand rows. One thread per (row, 32-site word): 16 or 32 bytes
-// read, 16 bytes written per block. A warp takes one row group x 4 words, lane
-// l row l % 8, so that each of its stores fills whole 128-byte core matrices;
-// a block of 256 threads takes 32 words. The words past the alignment's, up to
-// whole chunks, are written as 0. The dash is the AND of the P planes ('-' has
-// every plane); a chunk where some row has its first '-' is marked with `ext`.
-__global__ void k_expand_op(const uint4 *__restrict__ g0, const uint4 *__restrict__ g1,
-                            uint32_t planes, uint32_t words, uint64_t row_lo, uint64_t row_hi,
-                            uint64_t L, uint8_t *__restrict__ x, uint32_t *dash_chunk,
-                            uint32_t ext) {
-  const uint32_t nb = op_blocks(planes), chunks = op_chunks(L);
+// the dash blocks' 16 bytes of a word
+__device__ __forceinline__ void put_dash(uint8_t *dst, uint32_t dash, uint32_t planes) {
+  put16(dst, dash, kE2M1One);                       // 1.0: the row side
+  put16(dst + kGroupBytes, dash, dash_neg(planes));  // the column side
+  if (planes == 6) put16(dst + 2 * kGroupBytes, dash, kE2M1Neg1);
+}
+
+// One extension of an operand: rows [row_lo, row_hi) of the planes g0, g1 in x.
+struct OpRows {
+  const uint4 *g0, *g1;
+  uint8_t *x;
+  uint32_t *marks;  // per chunk, and a count of k_expand_op's blocks (0 between launches)
+  uint32_t *list;   // the marked chunks, then the listed ones before each chunk (chunks + 1)
+  unsigned long long row_lo, row_hi, sites;
+  uint32_t planes, words, ext;
+  uint32_t blocks;  // the listed chunks' dash blocks are to be written (k_dash_blocks)
+};
+
+// The ascending list of the chunks whose mark is set, and for every chunk the
+// listed ones before it; by a whole block.
+__device__ __forceinline__ void list_marked(const OpRows &o, uint32_t *tmp /*[33]*/) {
+  const uint32_t chunks = op_chunks(o.sites);
+  uint32_t *before = o.list + chunks, n = 0;
+  for (uint32_t c0 = 0; c0 < chunks; c0 += blockDim.x) {
+    const uint32_t c = c0 + threadIdx.x;
+    const uint32_t on = c < chunks && __ldcg(o.marks + c) != 0u ? 1u : 0u;
+    uint32_t total;
+    const uint32_t at = n + block_excl_scan<uint32_t>(on, tmp, total);
+    if (on) o.list[at] = c;
+    if (c < chunks) before[c] = at;
+    n += total;
+  }
+  if (threadIdx.x == 0) before[chunks] = n;
+}
+
+// Rows of a P-plane alignment (P = 4: the AND rule; 5, 6: the sparse rules,
+// planes 4-5 in the second group) -> the plane blocks of their E2M1 operand
+// rows, and unless k_dash_blocks follows the dash blocks of every chunk. One thread per (row,
+// 32-site word): 16 or 32 bytes read, 16 bytes written per block. A warp takes
+// one row group x 4 words, lane l row l % 8, so that each of its stores fills
+// whole 128-byte core matrices; a block of 256 threads takes 32 words. The
+// words past the alignment's, up to whole chunks, are written as 0. The dash is
+// the AND of the P planes ('-' has every plane); a chunk where some row has its
+// first '-' is marked with `ext`. The block that ends last lists the marked
+// chunks (kList).
+template <bool kList>
+__global__ void __launch_bounds__(256) k_expand_op(OpRows o) {
+  __shared__ uint32_t tmp[33];
+  __shared__ bool last;
+  const uint32_t nb = op_blocks(o.planes), chunks = op_chunks(o.sites);
   const uint32_t w = blockIdx.x * 32 + threadIdx.x / 8;
-  if (w >= chunks * kChunkWords) return;
   const uint32_t c = w / kChunkWords;
   const uint64_t s0 = (uint64_t)w * 32;
-  const uint32_t valid = s0 >= L ? 0u : (L - s0 >= 32 ? 0xffffffffu : ((1u << (L - s0)) - 1u));
+  const uint32_t valid = s0 >= o.sites ? 0u : (o.sites - s0 >= 32 ? 0xffffffffu : ((1u << (o.sites - s0)) - 1u));
   const uint64_t in_group = (uint64_t)c * nb * kGroupBytes + (w - c * kChunkWords) * 128u +
                             (threadIdx.x & 7u) * 16u;
-  const uint64_t group_bytes = op_group_bytes(planes, L);
-  for (uint64_t g = row_lo / 8 + blockIdx.y; g * 8 < row_hi; g += gridDim.y) {
+  const uint64_t group_bytes = op_group_bytes(o.planes, o.sites);
+  for (uint64_t g = o.row_lo / 8 + blockIdx.y; c < chunks && g * 8 < o.row_hi; g += gridDim.y) {
     const uint64_t r = g * 8 + (threadIdx.x & 7u);
-    if (r < row_lo || r >= row_hi) continue;
+    if (r < o.row_lo || r >= o.row_hi) continue;
     uint4 p = make_uint4(0u, 0u, 0u, 0u), p1 = p;
-    if (w < words) {
-      p = g0[r * words + w];
-      if (planes > 4) p1 = g1[r * words + w];
+    if (w < o.words) {
+      p = __ldg(o.g0 + r * o.words + w);
+      if (o.planes > 4) p1 = __ldg(o.g1 + r * o.words + w);
     }
     uint32_t dash = p.x & p.y & p.z & p.w & valid;
-    if (planes > 4) dash &= p1.x;
-    if (planes > 5) dash &= p1.y;
-    uint8_t *blk = x + g * group_bytes + in_group;
+    if (o.planes > 4) dash &= p1.x;
+    if (o.planes > 5) dash &= p1.y;
+    uint8_t *blk = o.x + g * group_bytes + in_group;
     put16(blk, p.x & valid, kE2M1One);
     put16(blk + kGroupBytes, p.y & valid, kE2M1One);
     put16(blk + 2 * kGroupBytes, p.z & valid, kE2M1One);
     put16(blk + 3 * kGroupBytes, p.w & valid, kE2M1One);
-    if (planes > 4) put16(blk + 4 * kGroupBytes, p1.x & valid, kE2M1One);
-    if (planes > 5) put16(blk + 5 * kGroupBytes, p1.y & valid, kE2M1One);
-    if (dash && !dash_chunk[c]) dash_chunk[c] = ext;  // every writer stores the same
+    if (o.planes > 4) put16(blk + 4 * kGroupBytes, p1.x & valid, kE2M1One);
+    if (o.planes > 5) put16(blk + 5 * kGroupBytes, p1.y & valid, kE2M1One);
+    if (!o.blocks) put_dash(blk + o.planes * kGroupBytes, dash, o.planes);
+    if (dash && !o.marks[c]) o.marks[c] = o.ext;  // every writer stores the same
   }
+  if (!kList) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();  // the block's marks, before its count
+    last = atomicAdd(o.marks + chunks, 1u) == gridDim.x * gridDim.y - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  list_marked(o, tmp);
+  if (threadIdx.x == 0) o.marks[chunks] = 0;
 }
-
-// One extension of an operand whose marked chunks are to be listed and their
-// dash blocks written: rows [row_lo, row_hi) of the planes g0, g1, now in x.
-struct DashJob {
-  const uint4 *g0, *g1;
-  uint8_t *x;
-  const uint32_t *marks;
-  uint32_t *list;  // the marked chunks, then the listed ones before each chunk (chunks + 1)
-  unsigned long long row_lo, row_hi, sites;
-  uint32_t planes, words, ext, pad;
-};
 
 // The dash blocks of the marked chunks (the job's list): of rows [row_lo,
 // row_hi), and for a chunk that extension `ext` marked first of the rows
@@ -280,10 +319,11 @@ struct DashJob {
 // or `one` without them.
 constexpr uint32_t kDashGroups = 4;  // row groups per block
 __global__ void __launch_bounds__(kDashGroups * 8 * kChunkWords)
-    k_dash_blocks(DashJob one, const DashJob *__restrict__ jobs, uint32_t n_jobs) {
+    k_dash_blocks(OpRows one, const OpRows *__restrict__ jobs, uint32_t n_jobs) {
   const uint32_t sub = threadIdx.x / (8 * kChunkWords), u = threadIdx.x % (8 * kChunkWords);
   for (uint32_t q = blockIdx.y; q < n_jobs; q += gridDim.y) {
-    const DashJob j = jobs ? jobs[q] : one;
+    const OpRows j = jobs ? jobs[q] : one;
+    if (!j.blocks) continue;
     const uint32_t nb = op_blocks(j.planes), chunks = op_chunks(j.sites);
     const uint64_t group_bytes = op_group_bytes(j.planes, j.sites);
     const uint64_t batches = ((j.row_hi + 7) / 8 + kDashGroups - 1) / kDashGroups;
@@ -304,9 +344,7 @@ __global__ void __launch_bounds__(kDashGroups * 8 * kChunkWords)
         }
       }
       uint8_t *blk = j.x + g * group_bytes + ((uint64_t)c * nb + j.planes) * kGroupBytes + u * 16u;
-      put16(blk, dash, kE2M1One);                         // 1.0: the row side
-      put16(blk + kGroupBytes, dash, dash_neg(j.planes));  // the column side
-      if (j.planes == 6) put16(blk + 2 * kGroupBytes, dash, kE2M1Neg1);
+      put_dash(blk, dash, j.planes);
     }
   }
 }
@@ -1204,23 +1242,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1)
   }
 }
 
-// The ascending list of the chunks whose mark is set, and for every chunk the
-// listed ones before it (a block per job of `jobs`, or one block for `one`).
-__global__ void __launch_bounds__(512) k_dash_list(DashJob one, const DashJob *__restrict__ jobs) {
+// The list of the marked chunks (a block for each of `jobs`, or one for `one`)
+__global__ void __launch_bounds__(512) k_dash_list(OpRows one, const OpRows *__restrict__ jobs) {
   __shared__ uint32_t tmp[33];
-  const DashJob j = jobs ? jobs[blockIdx.x] : one;
-  const uint32_t chunks = op_chunks(j.sites);
-  uint32_t *before = j.list + chunks, n = 0;
-  for (uint32_t c0 = 0; c0 < chunks; c0 += blockDim.x) {
-    const uint32_t c = c0 + threadIdx.x;
-    const uint32_t on = c < chunks && j.marks[c] != 0u ? 1u : 0u;
-    uint32_t total;
-    const uint32_t at = n + block_excl_scan<uint32_t>(on, tmp, total);
-    if (on) j.list[at] = c;
-    if (c < chunks) before[c] = at;
-    n += total;
-  }
-  if (threadIdx.x == 0) before[chunks] = n;
+  const OpRows o = jobs ? jobs[blockIdx.x] : one;
+  list_marked(o, tmp);
 }
 
 void set_smem_once() {
@@ -1249,42 +1275,48 @@ void make_tmap_op(hd_ctx *ctx, CUtensorMap *tm, const void *base, uint32_t plane
     fail(HD_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
 }
 
-// uint32s of the marks, and of the list and ranks k_dash_list makes of them
-uint64_t mark_words(uint64_t sites) { return op_chunks(sites); }
+// uint32s of the marks and the block count, and of the list and ranks made of them
+uint64_t mark_words(uint64_t sites) { return (uint64_t)op_chunks(sites) + 1; }
 uint64_t list_words(uint64_t sites) { return 2 * (uint64_t)op_chunks(sites) + 1; }
 
-// The list of a job's marked chunks, and their dash blocks.
-void dash_rows(const DashJob &j, int sm_count, cudaStream_t stream) {
-  k_dash_list<<<1, 512, 0, stream>>>(j, nullptr);
-  const uint64_t work = ceil_div(ceil_div((uint64_t)j.row_hi, (uint64_t)8), (uint64_t)kDashGroups) *
-                        op_chunks(j.sites);
+// The list of the extension's marked chunks, and their dash blocks if they are
+// not written: launches
+uint64_t list_chunks(const OpRows &o, int sm_count, cudaStream_t stream) {
+  k_dash_list<<<1, 512, 0, stream>>>(o, nullptr);
+  if (!o.blocks) return 1;
+  const uint64_t work = ceil_div(ceil_div((uint64_t)o.row_hi, (uint64_t)8), (uint64_t)kDashGroups) *
+                        op_chunks(o.sites);
   k_dash_blocks<<<(unsigned)std::min<uint64_t>(work, (uint64_t)sm_count * 8),
-                  kDashGroups * 8 * kChunkWords, 0, stream>>>(j, nullptr, 1);
+                  kDashGroups * 8 * kChunkWords, 0, stream>>>(o, nullptr, 1);
+  return 2;
 }
 
-// The jobs of a plan whose chunks are not listed yet: two launches for all of
-// them instead of two for each (first run of a batch of 200 matrices of 20 to
-// 128 rows: 1.6 ms, with two for each 3.2; 50 served windows of 100 rows 1.57
-// and 1.84). Left early, each is listed by itself: their alignments count the
-// rows as there.
-struct DashJobs {
+// A plan's extensions whose marked chunks are not listed yet, and the large ones'
+// dash blocks not written: two launches for all of them. A list by each one's
+// last block costs 2 us a matrix there, since the launches follow one another
+// (first run of a batch of 200 matrices of 20 to 128 rows: 2.0 ms, with one
+// launch for all lists 1.6, with two launches for each matrix 3.2; 50 served
+// windows of 100 rows 1.63, 1.57, 1.84). Left early, each has its own launches:
+// their alignments count the rows as there.
+struct DashLater {
   hd_ctx *ctx;
   cudaStream_t stream;
-  std::vector<DashJob> jobs;
-  ~DashJobs() {
-    for (const DashJob &j : jobs) dash_rows(j, ctx->sm_count, stream);
+  std::vector<OpRows> jobs;
+  ~DashLater() {
+    for (const OpRows &o : jobs) list_chunks(o, ctx->sm_count, stream);
   }
   // d_jobs: their copy on the device
-  void launch(const DashJob *d_jobs) {
-    const uint32_t n = (uint32_t)jobs.size();
-    if (!n) return;
-    k_dash_list<<<n, 512, 0, stream>>>(DashJob{}, d_jobs);
+  void launch(const OpRows *d_jobs) {
+    if (jobs.empty()) return;
+    const unsigned n = (unsigned)jobs.size(), y = std::min(n, 65535u);
+    k_dash_list<<<n, 512, 0, stream>>>(OpRows{}, d_jobs);
     HD_LAUNCHED(ctx);
-    const unsigned y = std::min(n, 65535u);
-    const unsigned x = (unsigned)ceil_div((uint64_t)ctx->sm_count * 32, (uint64_t)y);
-    k_dash_blocks<<<dim3(x, y), kDashGroups * 8 * kChunkWords, 0, stream>>>(DashJob{}, d_jobs, n);
-    HD_LAUNCHED(ctx);
+    const bool blocks = std::any_of(jobs.begin(), jobs.end(), [](const OpRows &o) { return o.blocks != 0; });
     jobs.clear();
+    if (!blocks) return;
+    const unsigned x = (unsigned)ceil_div((uint64_t)ctx->sm_count * 32, (uint64_t)y);
+    k_dash_blocks<<<dim3(x, y), kDashGroups * 8 * kChunkWords, 0, stream>>>(OpRows{}, d_jobs, n);
+    HD_LAUNCHED(ctx);
   }
 };
 
@@ -1294,26 +1326,26 @@ dim3 op_grid(uint64_t words, uint64_t lo, uint64_t hi) {
               (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(groups, 65535)));
 }
 
-// Lists the job's chunks with the plan's others, or now.
-void list_chunks(hd_ctx *ctx, const DashJob &j, cudaStream_t stream, DashJobs *later) {
-  if (later) {
-    later->jobs.push_back(j);
-    return;
-  }
-  dash_rows(j, ctx->sm_count, stream);
-  check_cuda(cudaGetLastError(), "kernel launch");
-  ctx->launches += 2;
-}
-
-// Expands the job's rows of the planes into its operand, marks the chunks with
-// a '-' and lists the marked ones.
-void expand_rows(hd_ctx *ctx, const DashJob &j, uint32_t *marks, cudaStream_t stream,
-                 DashJobs *later) {
-  k_expand_op<<<op_grid((uint64_t)op_chunks(j.sites) * kChunkWords, j.row_lo, j.row_hi), 256, 0,
-                stream>>>(j.g0, j.g1, j.planes, j.words, j.row_lo, j.row_hi, j.sites, j.x, marks,
-                          j.ext);
+// Expands the rows and lists the chunks with a '-', now or with the plan's
+// others. Where the dash blocks of all chunks are few bytes they are written with
+// the others and the last block makes the list: one launch instead of three. A
+// first call with 1,500 rows of 1,273 sites takes 103 us, with three launches
+// 113; with 3,000 of 3,000 (9 MB) 123 and 136. On large operands the blocks'
+// counting costs more than the launches (14,000 rows of 29,903 sites: 60 us).
+constexpr uint64_t kDashBytes = 16ull << 20;
+void expand_rows(hd_ctx *ctx, OpRows o, cudaStream_t stream, DashLater *later) {
+  const uint64_t bytes = (o.row_hi - o.row_lo) * op_chunks(o.sites) * (op_blocks(o.planes) - o.planes) * kBlockK;
+  o.blocks = bytes > kDashBytes ? 1u : 0u;
+  const bool list = !later && !o.blocks;
+  (list ? k_expand_op<true> : k_expand_op<false>)<<<
+      op_grid((uint64_t)op_chunks(o.sites) * kChunkWords, o.row_lo, o.row_hi), 256, 0, stream>>>(o);
   HD_LAUNCHED(ctx);
-  list_chunks(ctx, j, stream, later);
+  if (later) {
+    later->jobs.push_back(o);
+  } else if (!list) {
+    ctx->launches += list_chunks(o, ctx->sm_count, stream);
+    check_cuda(cudaGetLastError(), "kernel launch");
+  }
 }
 
 }  // namespace
@@ -1384,8 +1416,8 @@ uint32_t *last_list(const hd_alignment *o) {
                              : o->op_lists.back().as<uint32_t>();
 }
 // The extension to rows [op_rows, rows) that grow_operand made room for
-DashJob extension_of(const hd_alignment *o, uint64_t rows) {
-  DashJob j{};
+OpRows extension_of(const hd_alignment *o, uint64_t rows) {
+  OpRows j{};
   j.g0 = o->plane_buf[0].as<uint4>();
   j.g1 = o->planes > 4 ? o->plane_buf[1].as<uint4>() : nullptr;
   j.x = o->op.as<uint8_t>();
@@ -1397,13 +1429,14 @@ DashJob extension_of(const hd_alignment *o, uint64_t rows) {
   j.planes = (uint32_t)o->planes;
   j.words = (uint32_t)o->words;
   j.ext = (uint32_t)o->op_lists.size() + 1;
+  j.blocks = 1;
   return j;
 }
 bool extend_operand(hd_ctx *ctx, const hd_alignment *o, uint64_t rows, cudaStream_t stream,
-                    uint64_t cap_hint, DashJobs *later) {
+                    uint64_t cap_hint, DashLater *later) {
   if (o->op_rows >= rows) return true;
   if (!grow_operand(ctx, o, rows, stream, cap_hint)) return false;
-  expand_rows(ctx, extension_of(o, rows), o->op_dash.as<uint32_t>(), stream, later);
+  expand_rows(ctx, extension_of(o, rows), stream, later);
   o->op_rows = rows;
   return true;
 }
@@ -1439,14 +1472,15 @@ bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const
                   uint64_t lo, uint64_t hi, uint4 *copy, cudaStream_t stream, uint64_t cap_hint) {
   if (aln->base || aln->planes != 4 || aln->op_rows != lo || hi <= lo) return false;
   if (!grow_operand(ctx, aln, hi, stream, cap_hint)) return false;
-  const DashJob j = extension_of(aln, hi);
+  const OpRows j = extension_of(aln, hi);
   const uint64_t op_words = (uint64_t)op_chunks(aln->length) * kChunkWords;
   k_pack_op<true><<<pack_grid(ctx, std::max(aln->words, op_words), lo, hi), 256, 0, stream>>>(
       rec.base, rec.bytes, rec.rec_start.as<uint64_t>(), d_rows, lo, hi, aln->length,
-      (uint32_t)aln->words, aln->plane_buf[0].as<uint4>(), copy, j.x, aln->op_dash.as<uint32_t>(),
-      j.ext, Words::of(0, 1));
+      (uint32_t)aln->words, aln->plane_buf[0].as<uint4>(), copy, j.x, j.marks, j.ext,
+      Words::of(0, 1));
   HD_LAUNCHED(ctx);
-  list_chunks(ctx, j, stream, nullptr);
+  ctx->launches += list_chunks(j, ctx->sm_count, stream);
+  check_cuda(cudaGetLastError(), "kernel launch");
   aln->op_rows = hi;
   return true;
 }
@@ -1482,7 +1516,7 @@ double measure_mma_peak(hd_ctx *ctx) {
 // until the kernel has run (a serving window must not expand a large base).
 // False if there is no memory for it.
 bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLaunchPlan *plan,
-                 const uint8_t *&op, const uint32_t *&dash, DashJobs *later) {
+                 const uint8_t *&op, const uint32_t *&dash, DashLater *later) {
   const hd_alignment *o = a->base ? a->base : a;
   if (!a->base) {
     if (!extend_operand(ctx, a, a->n_rows, stream, 0, later)) return false;
@@ -1511,7 +1545,7 @@ bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLa
   }
   uint32_t *flags = reinterpret_cast<uint32_t *>(tmp.as<uint8_t>() + bytes);
   HD_CUDA(cudaMemsetAsync(flags, 0, marks * 4, stream));
-  DashJob j{};
+  OpRows j{};
   j.g0 = static_cast<const uint4 *>(a->planes_ptr(0));
   j.g1 = P > 4 ? static_cast<const uint4 *>(a->planes_ptr(1)) : nullptr;
   j.x = tmp.as<uint8_t>();
@@ -1523,7 +1557,7 @@ bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLa
   j.words = (uint32_t)o->words;
   j.ext = 1;
   plan->blocks.push_back(std::move(tmp));
-  expand_rows(ctx, j, flags, stream, later);
+  expand_rows(ctx, j, stream, later);
   op = j.x;
   dash = j.list;
   return true;
@@ -1586,20 +1620,31 @@ void plan_static(std::vector<MmaItem> &list, uint32_t units, uint32_t planes, bo
   // a pair's share: the average, at least the shortest piece of a full tile
   const uint64_t share = std::max<uint64_t>(ceil_div(total, units), 3ull * planes * kMinPart);
   const size_t whole = std::min<size_t>(m, (size_t)(total / units / most) * units);
-  std::vector<std::vector<MmaItem>> of(units);
+  // items in the order that their pairs take them, and each one's pair
+  std::vector<MmaItem> out;
+  std::vector<uint32_t> owner;
   std::vector<uint64_t> load(units, 0);
+  out.reserve(m + 2 * units);
+  owner.reserve(m + 2 * units);
   for (size_t k = 0; k < whole; ++k) {
-    of[k % units].push_back(list[k]);
+    out.push_back(list[k]);
+    owner.push_back((uint32_t)(k % units));
     load[k % units] += cost_of(list[k]);
   }
   // 250 cycles are 0.12 us
   const uint64_t unsplit = (whole / units + ceil_div(m - whole, (size_t)units)) * most;
   const bool split = may_split && (double)(unsplit - std::min(unsplit, share)) * 0.12 > 8.0;
   if (!split) {
+    // each to the least loaded pair, the first of equals
+    using Load = std::pair<uint64_t, uint32_t>;
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+    for (uint32_t v = 0; v < units; ++v) least.push({load[v], v});
     for (size_t k = whole; k < m; ++k) {
-      const size_t u = std::min_element(load.begin(), load.end()) - load.begin();
-      of[u].push_back(list[k]);
-      load[u] += cost_of(list[k]);
+      const Load v = least.top();
+      least.pop();
+      out.push_back(list[k]);
+      owner.push_back(v.second);
+      least.push({v.first + cost_of(list[k]), v.second});
     }
   } else {
     // the rest as one row of chunks; pair u's end on it is the sum of the room
@@ -1607,10 +1652,11 @@ void plan_static(std::vector<MmaItem> &list, uint32_t units, uint32_t planes, bo
     auto room = [&](uint32_t v) { return load[v] < share ? share - load[v] : 0; };
     uint32_t u = 0;
     uint64_t at = 0, end = room(0);
+    std::vector<uint32_t> cuts;
     for (size_t k = whole; k < m; ++k) {
       const MmaItem &it = list[k];
       const uint64_t per = block_cost(it) * planes;  // cost of one chunk
-      std::vector<uint32_t> cuts{it.c_lo}, owner;
+      cuts.assign(1, it.c_lo);
       for (uint32_t c = it.c_lo; c < it.c_hi;) {
         const uint32_t left = it.c_hi - c;
         uint64_t take = end > at ? (end - at + per / 2) / per : 0;
@@ -1624,21 +1670,22 @@ void plan_static(std::vector<MmaItem> &list, uint32_t units, uint32_t planes, bo
         cuts.push_back(c);
         owner.push_back(u);
       }
-      std::vector<MmaItem> pieces;
-      plan.add_pieces(it, cuts, pieces);
-      for (size_t q = 0; q < pieces.size(); ++q) of[owner[q]].push_back(pieces[q]);
+      plan.add_pieces(it, cuts, out);
     }
   }
-  size_t depth = 0;
+  std::vector<uint32_t> depth(units, 0);
+  for (uint32_t v : owner) ++depth[v];
+  uint32_t deepest = 0;
   for (uint32_t v = 0; v < units; ++v) {
-    depth = std::max(depth, of[v].size());
-    if (!of[v].empty()) plan.pairs = v + 1;
+    deepest = std::max(deepest, depth[v]);
+    if (depth[v]) plan.pairs = v + 1;
   }
   MmaItem none{};
   none.job = kNoItem;
-  plan.items.assign(depth * plan.pairs, none);
-  for (uint32_t v = 0; v < plan.pairs; ++v)
-    for (size_t k = 0; k < of[v].size(); ++k) plan.items[k * plan.pairs + v] = of[v][k];
+  plan.items.assign((size_t)deepest * plan.pairs, none);
+  std::fill(depth.begin(), depth.end(), 0u);
+  for (size_t k = 0; k < out.size(); ++k)
+    plan.items[(size_t)depth[owner[k]]++ * plan.pairs + owner[k]] = out[k];
 }
 
 // Several matrices: the pairs draw items from a queue, the costliest first
@@ -1708,7 +1755,7 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     double cost;
   };
   std::vector<Job> js;
-  DashJobs unlisted{ctx, stream, {}};
+  DashLater dash_later{ctx, stream, {}};
   // A small launch leaves SMs idle: below a minimum size, counted in tiles of
   // 128 x kMmaCols pairs (mma_min_items_for, autotuned per row length), the
   // bit-plane engine's finer tiles finish first; a batch of small matrices
@@ -1734,7 +1781,8 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     const uint64_t edge = sp.cfg.tile > 0 ? (uint64_t)sp.cfg.tile : kTile;
     const uint64_t row_lo = sp.tile_lo * edge, row_hi = std::min<uint64_t>(sp.tile_hi * edge, a->n_rows);
     if (row_lo % kTM || row_hi <= row_lo) continue;
-    if (!operand_for(ctx, a, stream, plan, ops[k], dash_lists[k], &unlisted)) continue;
+    if (!operand_for(ctx, a, stream, plan, ops[k], dash_lists[k], specs.size() > 1 ? &dash_later : nullptr))
+      continue;
     const uint32_t lo = (uint32_t)(row_lo / kTM), hi = (uint32_t)ceil_div(row_hi, kTM);
     js.push_back({k, lo, hi, (double)a->words * ((double)hi * hi - (double)lo * lo)});
     taken[k] = 1;
@@ -1827,13 +1875,13 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     }
   }
   // one device block: [tensor maps (2 per job)][jobs][items][split tiles]
-  // [queue counter][chunks to list]
+  // [queue counter][dash blocks to write]
   const size_t tm_bytes = nj * 2 * sizeof(CUtensorMap);
   const size_t job_at = tm_bytes, item_at = job_at + round_up(nj * sizeof(MmaJob), 64);
   const size_t fix_at = item_at + mp.items.size() * sizeof(MmaItem);
   const size_t counter_at = fix_at + round_up(mp.fix.size() * sizeof(MmaFix), 16);
   const size_t dash_at = counter_at + 16;
-  std::vector<uint8_t> host(dash_at + unlisted.jobs.size() * sizeof(DashJob), 0);
+  std::vector<uint8_t> host(dash_at + dash_later.jobs.size() * sizeof(OpRows), 0);
   DevBuf dev(host.size(), stream);
   auto *tms = reinterpret_cast<CUtensorMap *>(host.data());
   auto *jobs = reinterpret_cast<MmaJob *>(host.data() + job_at);
@@ -1859,11 +1907,11 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
   }
   std::memcpy(host.data() + item_at, mp.items.data(), mp.items.size() * sizeof(MmaItem));
   std::memcpy(host.data() + fix_at, mp.fix.data(), mp.fix.size() * sizeof(MmaFix));
-  std::memcpy(host.data() + dash_at, unlisted.jobs.data(), unlisted.jobs.size() * sizeof(DashJob));
+  std::memcpy(host.data() + dash_at, dash_later.jobs.data(), dash_later.jobs.size() * sizeof(OpRows));
   // staged in pinned memory (pageable for a large table): `host` may go when this returns
   upload_table(ctx, dev.p, host.data(), host.size(), stream);
   uint8_t *d = dev.as<uint8_t>();
-  unlisted.launch(reinterpret_cast<const DashJob *>(d + dash_at));
+  dash_later.launch(reinterpret_cast<const OpRows *>(d + dash_at));
   PairLaunchPlan::Launch L;
   L.mma = true;
   L.fn = reinterpret_cast<const void *>(k_pairwise_mma);

@@ -1,0 +1,55 @@
+"""Operands whose dash blocks are written with the plane blocks (up to 16 MB of
+them) and those whose listed chunks' blocks follow: the launches of a first
+call, and both kinds in one plan, against the bit-plane engine bit for bit."""
+import numpy as np
+import pytest
+
+from hammingdist_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def ctx(monkeypatch):
+    from hammingdist_gb300 import abi
+
+    monkeypatch.setenv("HAMMINGDIST_MMA_MIN_ITEMS", "1")
+    c = abi.Context(0)
+    yield c
+    c.close()
+
+
+def _alignment(ctx, n, L, seed):
+    rows, _, _ = synth.alignment(n, L, p=0.1, seed=seed, dash_max=min(200, L // 4))
+    rows[n // 2, L // 2: L // 2 + 9] = ord("-")
+    return ctx.alignment_from_sequences([r.tobytes() for r in rows])
+
+
+def _bit_planes(ctx, monkeypatch, aln):
+    monkeypatch.setenv("HAMMINGDIST_KERNEL", "lop3")
+    want = ctx.pairwise_lt(aln, dtype=np.uint16, max_distance=65535)
+    monkeypatch.delenv("HAMMINGDIST_KERNEL")
+    return want
+
+
+# 16 MB: 87,381 rows of one chunk, 560 of 156
+@pytest.mark.parametrize("n,L,launches", [(40, 150, 2), (257, 1273, 2), (559, 29903, 3), (561, 29903, 5)])
+def test_launches_of_a_first_call(ctx, monkeypatch, n, L, launches):
+    aln = _alignment(ctx, n, L, n)
+    before = ctx.kernel_launches
+    got = ctx.pairwise_lt(aln, dtype=np.uint16, max_distance=65535)
+    # rows and chunk list (or rows, list, listed blocks), distances (and the sums of
+    # tiles split along K)
+    assert ctx.kernel_launches - before == launches
+    np.testing.assert_array_equal(got, _bit_planes(ctx, monkeypatch, aln))
+
+
+def test_both_kinds_in_one_plan(ctx, monkeypatch):
+    alns = [_alignment(ctx, n, L, n + L) for n, L in [(60, 500), (620, 29903), (300, 3000), (900, 20000)]]
+    b = ctx.batch()
+    for a in alns:
+        b.add(a, dtype=np.uint16, max_distance=65535)
+    for _ in range(2):
+        for a, g in zip(alns, b.run()):
+            np.testing.assert_array_equal(g, _bit_planes(ctx, monkeypatch, a))
+    b.free()
