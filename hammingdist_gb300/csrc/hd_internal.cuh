@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/hammingdist_gb300.h"
+#include "hd_device_once.h"
 
 namespace hd {
 

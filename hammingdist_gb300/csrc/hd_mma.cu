@@ -83,7 +83,6 @@
 #include <algorithm>
 #include <cstdlib>
 #include <functional>
-#include <mutex>
 #include <queue>
 #include <string>
 #include <type_traits>
@@ -1249,14 +1248,11 @@ __global__ void __launch_bounds__(512) k_dash_list(OpRows one, const OpRows *__r
   list_marked(o, tmp);
 }
 
-void set_smem_once() {
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(k_pairwise_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kMmaSmem);
+void set_smem_once(int device) {
+  static OncePerDevice once;
+  once.run(device, [] {
+    HD_CUDA(cudaFuncSetAttribute(k_pairwise_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem));
   });
-  HD_CUDA(err);
 }
 
 // Map of an operand's row groups: boxes of one block of `box_rows` rows.
@@ -1490,12 +1486,10 @@ uint64_t mma_operand_bytes(uint32_t planes, uint64_t sites, uint64_t rows) {
 }
 
 double measure_mma_peak(hd_ctx *ctx) {
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(k_peak_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem);
+  static OncePerDevice once;
+  once.run(ctx->device, [] {
+    HD_CUDA(cudaFuncSetAttribute(k_peak_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmem));
   });
-  HD_CUDA(err);
   const uint32_t rounds = 4096, pairs = std::max(1, ctx->sm_count / 2);
   k_peak_mma<<<2 * pairs, 128, kMmaSmem, ctx->stream>>>(256, ctx->d_status);  // warm-up
   HD_LAUNCHED(ctx);
@@ -1935,7 +1929,7 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
 }
 
 void launch_mma(hd_ctx *ctx, const PairLaunchPlan::Launch &L, cudaStream_t stream) {
-  set_smem_once();
+  set_smem_once(ctx->device);
   // the item queue starts empty at every launch (also when a graph replays it)
   if (L.queue) HD_CUDA(cudaMemsetAsync(L.d_counter, 0, sizeof(unsigned), stream));
   k_pairwise_mma<<<(unsigned)L.grid, kMmaThreads, kMmaSmem, stream>>>(

@@ -325,17 +325,21 @@ const Variant &find_variant(int tile, int stages, int planes) {
   fail(HD_ERR_ARG, "no pairwise kernel variant for this configuration");
 }
 
-int resident_ctas(const Variant &v) {
+int resident_ctas(const Variant &v, int device) {
   static std::mutex mu;
-  static std::vector<std::pair<KernelFn, int>> cache;  // per variant
+  struct Entry {
+    KernelFn fn;
+    int device, per_sm;
+  };
+  static std::vector<Entry> cache;  // per variant and device
   std::lock_guard<std::mutex> lk(mu);
   for (auto &e : cache)
-    if (e.first == v.fn) return e.second;
+    if (e.fn == v.fn && e.device == device) return e.per_sm;
   HD_CUDA(cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
   int per_sm = 0;
   HD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v.fn, kThreads, v.smem));
   if (per_sm < 1) fail(HD_ERR_CUDA, "pairwise kernel does not fit on an SM");
-  cache.emplace_back(v.fn, per_sm);
+  cache.push_back({v.fn, device, per_sm});
   return per_sm;
 }
 
@@ -435,7 +439,7 @@ void prepare_pairwise_jobs(hd_ctx *ctx, std::vector<PairJobSpec> &specs, cudaStr
     L.tiles = tiles;
     L.d_jobs = dev.as<uint8_t>() + tm_bytes;
     L.d_counter = reinterpret_cast<unsigned long long *>(dev.as<uint8_t>() + tm_bytes + job_bytes);
-    const int per_sm = resident_ctas(v);
+    const int per_sm = resident_ctas(v, ctx->device);
     // sm_limit > 0 leaves the other SMs to kernels of other streams
     const int sms = sm_limit > 0 && sm_limit < ctx->sm_count ? sm_limit : ctx->sm_count;
     L.grid = std::min<uint64_t>(tiles, (uint64_t)per_sm * sms);

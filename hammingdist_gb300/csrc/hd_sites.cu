@@ -30,7 +30,6 @@
 // the two tiles' lists have at one site.
 #include <algorithm>
 #include <cstdlib>
-#include <mutex>
 
 #include "hd_internal.cuh"
 
@@ -826,12 +825,10 @@ void prepare_site_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaS
 }
 
 void launch_sites(hd_ctx *ctx, const PairLaunchPlan::Launch &L, cudaStream_t stream) {
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(k_site_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+  static OncePerDevice once;
+  once.run(ctx->device, [] {
+    HD_CUDA(cudaFuncSetAttribute(k_site_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
   });
-  HD_CUDA(err);
   k_site_pairs<<<(unsigned)L.grid, kPairThreads, kPairSmem, stream>>>(L.site);
   HD_LAUNCHED(ctx);
   ctx->last_pair_tiles += L.tiles;
