@@ -1585,17 +1585,21 @@ struct MmaPlan {
   }
 };
 
-// Cost of an item per K block, in units of 250 cycles: 745 cycles of MMAs for
-// both column halves; one half alone waits for its loads (36.9 KB at the 72 B
-// per cycle and SM that the L2 gives), about 510.
+// Cost of an item per K block, in units of 177 cycles (0.09 us): 531 cycles for
+// both column halves; one half alone waits for its loads (24.6 KB at the 72 B
+// per cycle and SM that the L2 gives), about 340.
+constexpr double kCostUs = 0.09;
+// What splitting costs: the pieces' workspace traffic and one more launch. Calls,
+// split and whole: 1,000 rows of 2,400 sites (7.5 us of pieces' gain) 80 and 75
+// us, of 3,000 (10.8) 73 and 77, of 5,000 74 and 89; 3,000 rows of 4,000 (9.0) 97
+// and 86, of 5,000 (11.6) 92 and 93, of 8,000 (18) 106 and 109.
+constexpr double kSplitUs = 10.0;
 uint64_t block_cost(const MmaItem &it) { return it.n1_16 ? 3 : 2; }
 
 // One matrix: every pair of CTAs gets the same share of the work to within a
 // chunk. Whole items go round in list order while every pair has one more;
-// the rest is dealt out in K pieces that fill each pair up to the average.
-// Splitting costs the pieces' workspace traffic and one more launch, about 8
-// us, so it is left out where it would gain less (then the rest goes to the
-// least loaded pairs). n=1,000 x 29,903, 10 items: 35 us split, 160 us whole.
+// the rest is dealt out in K pieces that fill each pair up to the average, unless
+// that gains less than it costs: then the rest goes to the least loaded pairs.
 void plan_static(std::vector<MmaItem> &list, uint32_t units, uint32_t planes, bool may_split,
                  MmaPlan &plan) {
   // The items of both column halves first: they all take the same time, so
@@ -1625,9 +1629,8 @@ void plan_static(std::vector<MmaItem> &list, uint32_t units, uint32_t planes, bo
     owner.push_back((uint32_t)(k % units));
     load[k % units] += cost_of(list[k]);
   }
-  // 250 cycles are 0.12 us
   const uint64_t unsplit = (whole / units + ceil_div(m - whole, (size_t)units)) * most;
-  const bool split = may_split && (double)(unsplit - std::min(unsplit, share)) * 0.12 > 8.0;
+  const bool split = may_split && (double)(unsplit - std::min(unsplit, share)) * kCostUs > kSplitUs;
   if (!split) {
     // each to the least loaded pair, the first of equals
     using Load = std::pair<uint64_t, uint32_t>;
@@ -1695,8 +1698,8 @@ void plan_queue(std::vector<MmaItem> &list, uint32_t units, const std::vector<ui
     const uint32_t n = it.c_hi - it.c_lo;
     const uint64_t cost = block_cost(it) * planes[it.job] * n;
     uint64_t parts = may_split[it.job] ? std::min<uint64_t>(cost / half, n / kMinPart) : 1;
-    // below 8 us a split gains less than it costs
-    if ((double)(cost - std::min(cost, half)) * 0.12 < 8.0) parts = 1;
+    // (between 2 and 12 us this line makes no difference to a batch)
+    if ((double)(cost - std::min(cost, half)) * kCostUs < kSplitUs) parts = 1;
     std::vector<uint32_t> cuts{it.c_lo};
     for (uint64_t k = 1; k <= std::max<uint64_t>(parts, 1); ++k)
       cuts.push_back(it.c_lo + (uint32_t)(n * k / std::max<uint64_t>(parts, 1)));
