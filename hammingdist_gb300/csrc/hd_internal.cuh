@@ -12,6 +12,7 @@
 #include <cstring>
 #include <chrono>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -138,6 +139,16 @@ struct TuneTable {
 };
 }  // namespace hd
 
+namespace hd {
+// A point on a stream that other streams wait for
+struct StreamMark {
+  cudaEvent_t ev = nullptr;
+  ~StreamMark() {
+    if (ev) cudaEventDestroy(ev);
+  }
+};
+}  // namespace hd
+
 struct hd_ctx {
   int device = 0;
   int sm_count = 0;
@@ -184,6 +195,8 @@ struct hd_ctx {
   bool expect_pairwise = false;
   // pinned words that small results are copied to (pinned_words)
   uint64_t *words = nullptr;
+  // the last operand rows written on `stream` (the alignments keep it too)
+  std::shared_ptr<hd::StreamMark> op_mark;
   hd::Trace trace;
 };
 
@@ -274,6 +287,9 @@ struct hd_alignment {
   hd::DevBuf plane_buf[2];
   std::vector<uint64_t> seqidx;  // host, n_input entries (empty = identity)
   hd::DevBuf d_seqidx;           // device copy (serving / reference queries)
+  // What is built on first use, below: several threads, each with a context of
+  // its own, may compare one alignment, and a server its windows meanwhile
+  mutable std::recursive_mutex lazy;
   // E2M1 (FP4) operand of the tensor-core engine (hd_mma.cu), rows [0, op_rows)
   // expanded so far out of op_cap; built on first use, freed with the
   // alignment
@@ -286,6 +302,10 @@ struct hd_alignment {
   mutable hd::DevBuf op_dash;
   // the list and ranks after each later extension, the last one current
   mutable std::vector<hd::DevBuf> op_lists;
+  // the stream that the rows were written on, and the point there after which
+  // they and the last list are: other streams wait for it
+  mutable cudaStream_t op_stream = nullptr;
+  mutable std::shared_ptr<hd::StreamMark> op_mark;
   // built on first use, where the distances use them (hd_sites.cu)
   mutable std::unique_ptr<hd::SiteLists> sites;
   // Freed on the null stream: every API call has synchronised its own stream

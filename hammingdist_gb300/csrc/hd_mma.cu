@@ -1287,6 +1287,27 @@ uint64_t list_chunks(const OpRows &o, int sm_count, cudaStream_t stream) {
   return 2;
 }
 
+// The operand's rows and its last list are written by what is queued on the
+// stream so far: other streams wait for that.
+void mark_operand(hd_ctx *ctx, const hd_alignment *o, cudaStream_t stream,
+                  std::shared_ptr<StreamMark> &mark) {
+  if (!mark) {
+    mark = stream == ctx->stream ? ctx->op_mark : nullptr;
+    if (!mark) {
+      mark = std::make_shared<StreamMark>();
+      HD_CUDA(cudaEventCreateWithFlags(&mark->ev, cudaEventDisableTiming));
+      if (stream == ctx->stream) ctx->op_mark = mark;
+    }
+    HD_CUDA(cudaEventRecord(mark->ev, stream));
+  }
+  o->op_mark = mark;
+  o->op_stream = stream;
+}
+// The stream's next work follows what wrote the operand.
+void follow_operand(const hd_alignment *o, cudaStream_t stream) {
+  if (o->op_mark && o->op_stream != stream) HD_CUDA(cudaStreamWaitEvent(stream, o->op_mark->ev, 0));
+}
+
 // A plan's extensions whose marked chunks are not listed yet, and the large ones'
 // dash blocks not written: two launches for all of them. A list by each one's
 // last block costs 2 us a matrix there, since the launches follow one another
@@ -1298,8 +1319,19 @@ struct DashLater {
   hd_ctx *ctx;
   cudaStream_t stream;
   std::vector<OpRows> jobs;
+  std::vector<const hd_alignment *> owners;  // the alignments among them
+  void mark() {
+    std::shared_ptr<StreamMark> at;
+    for (const hd_alignment *o : owners) mark_operand(ctx, o, stream, at);
+    owners.clear();
+  }
   ~DashLater() {
     for (const OpRows &o : jobs) list_chunks(o, ctx->sm_count, stream);
+    try {
+      mark();
+    } catch (const Error &) {
+      cudaStreamSynchronize(stream);
+    }
   }
   // d_jobs: their copy on the device
   void launch(const OpRows *d_jobs) {
@@ -1308,11 +1340,13 @@ struct DashLater {
     k_dash_list<<<n, 512, 0, stream>>>(OpRows{}, d_jobs);
     HD_LAUNCHED(ctx);
     const bool blocks = std::any_of(jobs.begin(), jobs.end(), [](const OpRows &o) { return o.blocks != 0; });
+    if (blocks) {
+      const unsigned x = (unsigned)ceil_div((uint64_t)ctx->sm_count * 32, (uint64_t)y);
+      k_dash_blocks<<<dim3(x, y), kDashGroups * 8 * kChunkWords, 0, stream>>>(OpRows{}, d_jobs, n);
+      HD_LAUNCHED(ctx);
+    }
     jobs.clear();
-    if (!blocks) return;
-    const unsigned x = (unsigned)ceil_div((uint64_t)ctx->sm_count * 32, (uint64_t)y);
-    k_dash_blocks<<<dim3(x, y), kDashGroups * 8 * kChunkWords, 0, stream>>>(OpRows{}, d_jobs, n);
-    HD_LAUNCHED(ctx);
+    mark();
   }
 };
 
@@ -1430,10 +1464,15 @@ OpRows extension_of(const hd_alignment *o, uint64_t rows) {
 }
 bool extend_operand(hd_ctx *ctx, const hd_alignment *o, uint64_t rows, cudaStream_t stream,
                     uint64_t cap_hint, DashLater *later) {
+  std::lock_guard<std::recursive_mutex> lk(o->lazy);
+  follow_operand(o, stream);
   if (o->op_rows >= rows) return true;
   if (!grow_operand(ctx, o, rows, stream, cap_hint)) return false;
   expand_rows(ctx, extension_of(o, rows), stream, later);
   o->op_rows = rows;
+  std::shared_ptr<StreamMark> mark;
+  if (later) later->owners.push_back(o);
+  else mark_operand(ctx, o, stream, mark);
   return true;
 }
 }  // namespace
@@ -1467,6 +1506,8 @@ void pack_planes(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, uint64
 bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const hd_alignment *aln,
                   uint64_t lo, uint64_t hi, uint4 *copy, cudaStream_t stream, uint64_t cap_hint) {
   if (aln->base || aln->planes != 4 || aln->op_rows != lo || hi <= lo) return false;
+  std::lock_guard<std::recursive_mutex> lk(aln->lazy);
+  follow_operand(aln, stream);
   if (!grow_operand(ctx, aln, hi, stream, cap_hint)) return false;
   const OpRows j = extension_of(aln, hi);
   const uint64_t op_words = (uint64_t)op_chunks(aln->length) * kChunkWords;
@@ -1478,6 +1519,8 @@ bool pack_operand(hd_ctx *ctx, const Records &rec, const uint64_t *d_rows, const
   ctx->launches += list_chunks(j, ctx->sm_count, stream);
   check_cuda(cudaGetLastError(), "kernel launch");
   aln->op_rows = hi;
+  std::shared_ptr<StreamMark> mark;
+  mark_operand(ctx, aln, stream, mark);
   return true;
 }
 
@@ -1514,17 +1557,22 @@ bool operand_for(hd_ctx *ctx, const hd_alignment *a, cudaStream_t stream, PairLa
   const hd_alignment *o = a->base ? a->base : a;
   if (!a->base) {
     if (!extend_operand(ctx, a, a->n_rows, stream, 0, later)) return false;
+    std::lock_guard<std::recursive_mutex> lk(a->lazy);
     op = a->op.as<uint8_t>();
     dash = last_list(a);
     return true;
   }
+  std::unique_lock<std::recursive_mutex> lk(o->lazy, std::defer_lock);
+  if (a->row0 == 0) lk.lock();
   if (a->row0 == 0 && o->op.p && o->op_rows >= a->n_rows) {
+    follow_operand(o, stream);
     // the base's listed chunks cover its other rows too: a chunk listed for
     // them only adds dash products of 0
     op = o->op.as<uint8_t>();
     dash = last_list(o);
     return true;
   }
+  if (lk) lk.unlock();
   const uint32_t P = (uint32_t)o->planes;
   const uint64_t bytes = op_bytes(P, o->length, a->n_rows);
   const uint64_t marks = mark_words(o->length), flag_bytes = (marks + list_words(o->length)) * 4;
@@ -1752,7 +1800,10 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
     double cost;
   };
   std::vector<Job> js;
-  DashLater dash_later{ctx, stream, {}};
+  // Rows whose lists follow with the plan's others are nobody else's to read
+  // until then: their alignments stay locked (in the order of their addresses)
+  std::vector<std::unique_lock<std::recursive_mutex>> locks;
+  DashLater dash_later{ctx, stream, {}, {}};
   // A small launch leaves SMs idle: below a minimum size, counted in tiles of
   // 128 x kMmaCols pairs (mma_min_items_for, autotuned per row length), the
   // bit-plane engine's finer tiles finish first; a batch of small matrices
@@ -1770,6 +1821,15 @@ void prepare_mma_jobs(hd_ctx *ctx, const std::vector<PairJobSpec> &specs, cudaSt
   }
   const uint64_t min_items = ctx->engine_force == 1 ? 0 : mma_min_items_for(ctx, max_len);
   if (items_total < min_items) return;
+  if (specs.size() > 1) {
+    std::vector<const hd_alignment *> shared;
+    for (const PairJobSpec &sp : specs)
+      if (!sp.aln->base || sp.aln->row0 == 0) shared.push_back(sp.aln->base ? sp.aln->base : sp.aln);
+    std::sort(shared.begin(), shared.end(), std::less<const hd_alignment *>());
+    shared.erase(std::unique(shared.begin(), shared.end()), shared.end());
+    locks.reserve(shared.size());
+    for (const hd_alignment *o : shared) locks.emplace_back(o->lazy);
+  }
   for (size_t k = 0; k < specs.size(); ++k) {
     const PairJobSpec &sp = specs[k];
     const hd_alignment *a = sp.aln;

@@ -671,6 +671,7 @@ bool sites_likely(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st, uint64_t 
   if (!have) have = rows;
   const Words sel = sites_sample(ctx, a, rows);
   if (!sel.stride) return false;
+  std::lock_guard<std::recursive_mutex> lk(a->lazy);
   if (a->sites && a->sites->verdict) return a->sites->verdict > 0;
   if (!a->sites) a->sites = std::make_unique<SiteLists>();
   SiteLists &S = *a->sites;
@@ -714,7 +715,11 @@ bool sites_likely(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st, uint64_t 
   return S.verdict > 0;
 }
 
+// (the stream is waited for before the lists count as there, for other threads
+// and streams too)
 bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
+  if (!sites_sample(ctx, a).stride) return false;
+  std::lock_guard<std::recursive_mutex> lk(a->lazy);
   if (!sites_likely(ctx, a, st)) return false;
   SiteLists &S = *a->sites;
   if (S.tiles) return true;
