@@ -1202,11 +1202,11 @@ int hd_pairwise_lt_fasta_file(hd_ctx *ctx, const char *path, int remove_duplicat
     // after the given fractions of its bytes. After each part its new records
     // are deduplicated against the earlier ones (first occurrences keep their
     // order, so earlier unique rows keep their positions) and the new unique
-    // rows are packed; the tile rows that are complete then run on the side
-    // stream, with 16 SMs left for the next part's ingest. The last part's
-    // tile rows run as two launches, split at 90% of the tile rows, so that
-    // the copy of every finished range to the host overlaps the rest of the
-    // distances.
+    // rows are packed. On the engines the tile rows that are complete then run
+    // on the side stream, with 16 SMs left for the next part's ingest, and the
+    // last part's run as two launches, split at 90% of the tile rows; site lists
+    // are built after the last part, and all rows run in four ranges. The copy of
+    // every finished range to the host overlaps the rest of the distances.
     // part ends as fractions of the file (HAMMINGDIST_STREAM_SPLITS="f1,f2,...",
     // increasing, at most 3). At n=20,000 x L=29,903 the file-to-host step
     // (with the reference distances) took 7.17-7.21 ms with splits at 35% and

@@ -34,10 +34,10 @@
 // planes (1.0), the dash as 1.0 (read for rows) and the dash as -(P - 1)
 // (read for columns; -4 and -1 for P = 6) are blocks of 768 bytes, each six
 // 128-byte core matrices (8 rows x 16 bytes = 32 sites). Sites past L are 0; the
-// dash blocks are written for the listed chunks only. A
-// row group's blocks follow one another, so a TMA box of 16 groups brings one
-// block of 128 rows. An alignment caches its operand; a view of a resident
-// alignment (a serving window) gets one of its own rows.
+// dash blocks of a large operand are written for the listed chunks only. A row
+// group's blocks follow one another, so a TMA box of 16 groups brings one block
+// of 128 rows. An alignment caches its operand; a view of a resident alignment (a
+// serving window) gets one of its own rows.
 //
 // One launch serves a job table of matrices. Persistent pairs of CTAs (a
 // cluster of two SMs, 352 threads each) walk a list of items: 256 rows x up to

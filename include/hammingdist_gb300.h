@@ -430,6 +430,10 @@ int hd_tune_lookup(hd_ctx *ctx, uint64_t n_rows, uint64_t length,
  * size from which a launch goes to that engine. No reference counterpart. */
 int hd_tune_lookup_mma(hd_ctx *ctx, uint64_t n_rows, uint64_t length,
                        int dtype_bytes, int *band, int *rows, uint64_t *min_items);
+/* The table as JSON. A saved table names the tensor-core engine it was measured
+ * on ("mma_engine"); of a table saved on another one hd_tune_load takes the
+ * bit-plane settings only. A table written by hand ("sm_count" not in it) is
+ * taken as it is, in this engine's units. */
 int hd_tune_save(hd_ctx *ctx, const char *path);
 int hd_tune_load(hd_ctx *ctx, const char *path);
 
@@ -464,12 +468,14 @@ int hd_measure_mma_peak(hd_ctx *ctx, double *fp4_flop_per_s);
  * the context stays usable. No reference counterpart. */
 int hd_selftest_wait_timeout(hd_ctx *ctx, uint64_t limit_ns, int *status,
                              double *waited_ms);
-/* Device time of the last pairwise kernel launch sequence (ms, CUDA events on
- * the launching stream) and the number of tiles it processed. */
+/* Device time of the last hd_pairwise_lt's distance launches (ms, CUDA events on
+ * the launching stream) and the number of tiles they processed. What a first
+ * call builds before them (site lists, the tensor-core operand, job tables) is
+ * not in it; the trace has it. */
 int hd_last_pairwise_timing(const hd_ctx *ctx, double *ms, uint64_t *tiles);
 /* Tensor-core work of the last hd_pairwise_lt: the multiply-adds its
  * launches performed for the lower triangle (pairs x operand values per
- * pair; 0 if the bit-plane engine computed it). No reference counterpart. */
+ * pair; 0 if site lists or the bit-plane engine computed it). No reference counterpart. */
 int hd_last_pairwise_work(const hd_ctx *ctx, double *mma_macs);
 
 #ifdef __cplusplus
