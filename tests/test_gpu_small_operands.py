@@ -53,3 +53,13 @@ def test_both_kinds_in_one_plan(ctx, monkeypatch):
         for a, g in zip(alns, b.run()):
             np.testing.assert_array_equal(g, _bit_planes(ctx, monkeypatch, a))
     b.free()
+
+
+# 32-bit outputs: column halves while twice the items leave every pair of SMs one at
+# most (a few thousand rows), whole items above
+@pytest.mark.parametrize("n", [2, 257, 512, 2304, 2560, 2816, 3100])
+def test_wide_outputs(ctx, monkeypatch, n):
+    aln = _alignment(ctx, n, 450, n)
+    got = ctx.pairwise_lt(aln, dtype=np.uint32, max_distance=2**32 - 1)
+    monkeypatch.setenv("HAMMINGDIST_KERNEL", "lop3")
+    np.testing.assert_array_equal(got, ctx.pairwise_lt(aln, dtype=np.uint32, max_distance=2**32 - 1))
