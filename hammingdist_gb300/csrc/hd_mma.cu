@@ -255,14 +255,14 @@ __device__ __forceinline__ void list_marked(const OpRows &o, uint32_t *tmp /*[33
 
 // Rows of a P-plane alignment (P = 4: the AND rule; 5, 6: the sparse rules,
 // planes 4-5 in the second group) -> the plane blocks of their E2M1 operand
-// rows, and unless k_dash_blocks follows the dash blocks of every chunk. One thread per (row,
-// 32-site word): 16 or 32 bytes read, 16 bytes written per block. A warp takes
-// one row group x 4 words, lane l row l % 8, so that each of its stores fills
-// whole 128-byte core matrices; a block of 256 threads takes 32 words. The
-// words past the alignment's, up to whole chunks, are written as 0. The dash is
-// the AND of the P planes ('-' has every plane); a chunk where some row has its
-// first '-' is marked with `ext`. The block that ends last lists the marked
-// chunks (kList).
+// rows and, unless k_dash_blocks follows, the dash blocks of every chunk. One
+// thread per (row, 32-site word): 16 or 32 bytes read, 16 bytes written per block.
+// A warp takes one row group x 4 words, lane l row l % 8, so that each of its
+// stores fills whole 128-byte core matrices; a block of 256 threads takes 32
+// words. The words past the alignment's, up to whole chunks, are written as 0.
+// The dash is the AND of the P planes ('-' has every plane); a chunk where some
+// row has its first '-' is marked with `ext`. The block that ends last lists the
+// marked chunks (kList).
 template <bool kList>
 __global__ void __launch_bounds__(256) k_expand_op(OpRows o) {
   __shared__ uint32_t tmp[33];
@@ -1362,10 +1362,12 @@ dim3 op_grid(uint64_t words, uint64_t lo, uint64_t hi) {
 // first call with 1,500 rows of 1,273 sites takes 103 us, with three launches
 // 113; with 3,000 of 3,000 (9 MB) 123 and 136. On large operands the blocks'
 // counting costs more than the launches (14,000 rows of 29,903 sites: 60 us).
+// Rows after others go the longer way: a chunk that they mark first needs dash
+// blocks of the earlier rows too.
 constexpr uint64_t kDashBytes = 16ull << 20;
 void expand_rows(hd_ctx *ctx, OpRows o, cudaStream_t stream, DashLater *later) {
   const uint64_t bytes = (o.row_hi - o.row_lo) * op_chunks(o.sites) * (op_blocks(o.planes) - o.planes) * kBlockK;
-  o.blocks = bytes > kDashBytes ? 1u : 0u;
+  o.blocks = bytes > kDashBytes || o.row_lo > 0 ? 1u : 0u;
   const bool list = !later && !o.blocks;
   (list ? k_expand_op<true> : k_expand_op<false>)<<<
       op_grid((uint64_t)op_chunks(o.sites) * kChunkWords, o.row_lo, o.row_hi), 256, 0, stream>>>(o);

@@ -63,3 +63,29 @@ def test_wide_outputs(ctx, monkeypatch, n):
     got = ctx.pairwise_lt(aln, dtype=np.uint32, max_distance=2**32 - 1)
     monkeypatch.setenv("HAMMINGDIST_KERNEL", "lop3")
     np.testing.assert_array_equal(got, ctx.pairwise_lt(aln, dtype=np.uint32, max_distance=2**32 - 1))
+
+
+# an operand whose first rows' dash blocks were written for their listed chunks only,
+# extended by few rows that have the first '-' of other chunks; and the other way round
+@pytest.mark.parametrize("first", [640, 40])
+def test_extended_operand(ctx, monkeypatch, first):
+    import ctypes
+
+    from hammingdist_gb300 import abi
+
+    n, L = 700, 29903
+    rows, _, _ = synth.alignment(n, L, p=0.1, seed=first, dash_max=0)
+    rows[: first, 100:140] = ord("-")
+    rows[first:, 100:120] = ord("N")
+    rows[first + 3, 9000:9300] = rows[first + 9, 29900:] = ord("-")
+    # the memory that the operand will take holds dash blocks of '-' in every site
+    dirty = ctx.alignment_from_sequences([b"-" * L] * n)
+    assert not ctx.pairwise_lt(dirty).any()
+    dirty.free()
+    aln = ctx.alignment_from_sequences([r.tobytes() for r in rows])
+    fn = getattr(abi.lib(), "_ZN2hd14ensure_operandEP6hd_ctxPK12hd_alignmentmP11CUstream_stm")
+    fn.restype = ctypes.c_bool
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_uint64]
+    assert fn(ctx.h, aln.h, first, ctx.stream, n)
+    got = ctx.pairwise_lt(aln, dtype=np.uint16, max_distance=65535)
+    np.testing.assert_array_equal(got, _bit_planes(ctx, monkeypatch, aln))
