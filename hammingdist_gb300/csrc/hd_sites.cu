@@ -7,7 +7,7 @@
 // few sites per thousand, so that nearly all site pairs that a dense
 // comparison takes are equal to the reference in both rows.
 //
-// Per site, r is the commonest code of 64 rows (any choice gives the same
+// Per site, r is the commonest code of some rows (any choice gives the same
 // distances). Two rows' codes a, b mismatch at a site where a & b == 0. With
 //   k = [r & r == 0] (1 where r is the code 0 that matches nothing),
 //   m(a) = [a & r == 0] - k,
@@ -100,50 +100,88 @@ __device__ __forceinline__ Diff diff_of(const uint4 &a, const uint2 &b, const ui
   return o;
 }
 
-// The reference: four warps take a word, 16 rows each, a lane a site. The
-// commonest code of up to 64 rows, '-' left out (r has at most one bit).
+// Rows of a word's sites, `each` a warp from the q0-th of them on, counted by
+// code: 8 bits a slot (bits 0-5, none, '-')
+template <uint32_t kEach, class RowOf>
+__device__ __forceinline__ unsigned long long count_codes(const Planes &p, uint64_t n, uint32_t w,
+                                                          uint32_t lane, RowOf &&row_of) {
+  unsigned long long cnt = 0;
+#pragma unroll 1
+  for (uint32_t h = 0; h < kEach; h += 8) {
+    uint4 a[8];
+    uint2 b[8];
+    uint64_t row[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+      row[q] = row_of(h + q);
+      a[q] = make_uint4(0u, 0u, 0u, 0u);
+      b[q] = make_uint2(0u, 0u);
+      if (row[q] < n) p.load(row[q], w, a[q], b[q]);
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) {
+      const uint32_t code = ((a[q].x >> lane) & 1u) | ((a[q].y >> lane) & 1u) << 1 |
+                            ((a[q].z >> lane) & 1u) << 2 | ((a[q].w >> lane) & 1u) << 3 |
+                            ((b[q].x >> lane) & 1u) << 4 | ((b[q].y >> lane) & 1u) << 5;
+      const uint32_t slot = code == 0 ? 6u : code & (code - 1u) ? 7u : (uint32_t)__ffs(code) - 1u;
+      if (row[q] < n) cnt += 1ull << (8u * slot);
+    }
+  }
+  return cnt;
+}
+
+// The reference: four warps take a word, 16 rows each, a lane a site: the
+// commonest code with one bit (r has at most one) of 64 rows. Where r is 0 a '-'
+// is an s entry, so r is 0 only where there are more rows of code 0 than of that
+// code and '-' together. Near an alignment's ends the 64 rows can all be '-' at a
+// site, or one of them 'N': words with sites that no row gives a code with a bit
+// look at 192 rows more. (r taken to be 0 at four sites where all rows but a few
+// are '-': 11.3 ms for 14,000 rows instead of 0.3; a code that is not the rows' at
+// 18 sites, where 2-12% have one: 0.7 ms.)
 __global__ void __launch_bounds__(256)
     k_site_ref(Planes p, uint64_t n, Words sel, uint4 *r0, uint2 *r1) {
   __shared__ unsigned long long part[8][32];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ uint32_t more[2];  // the sites of each word to look at again
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quarter = warp & 3u;
   const uint32_t k = blockIdx.x * 2 + (warp >> 2), w = k < sel.count ? sel.at(k) : sel.words;
-  unsigned long long cnt = 0;  // 8 bits per code: bits 0-5, none, '-'
-  if (w < sel.words) {         // warp-uniform
-    constexpr uint32_t kEach = kRefRows / 4;
-    uint4 a[kEach / 2];
-    uint2 b[kEach / 2];
-    for (uint32_t h = 0; h < 2; ++h) {
-      const uint32_t q0 = (warp & 3u) * kEach + h * (kEach / 2);
-#pragma unroll
-      for (uint32_t q = 0; q < kEach / 2; ++q) {
-        const uint64_t row = n < kRefRows ? q0 + q : n * (q0 + q) / kRefRows;
-        a[q] = make_uint4(~0u, ~0u, ~0u, ~0u);  // a '-', which does not count
-        b[q] = make_uint2(~0u, ~0u);
-        if (row < n) p.load(row, w, a[q], b[q]);
-      }
-#pragma unroll
-      for (uint32_t q = 0; q < kEach / 2; ++q) {
-        const uint32_t code = ((a[q].x >> lane) & 1u) | ((a[q].y >> lane) & 1u) << 1 |
-                              ((a[q].z >> lane) & 1u) << 2 | ((a[q].w >> lane) & 1u) << 3 |
-                              ((b[q].x >> lane) & 1u) << 4 | ((b[q].y >> lane) & 1u) << 5;
-        const uint32_t slot = code == 0 ? 6u : code & (code - 1u) ? 7u : (uint32_t)__ffs(code) - 1u;
-        cnt += 1ull << (8u * slot);
-      }
-    }
-  }
-  part[warp][lane] = cnt;
+  const bool here = w < sel.words;  // warp-uniform
+  part[warp][lane] = !here ? 0ull : count_codes<kRefRows / 4>(p, n, w, lane, [&](uint32_t q) {
+    q += quarter * (kRefRows / 4);
+    return n < kRefRows ? (uint64_t)q : n * q / kRefRows;
+  });
   __syncthreads();
-  if ((warp & 3u) || w >= sel.words) return;
-  cnt = part[warp][lane] + part[warp + 1][lane] + part[warp + 2][lane] + part[warp + 3][lane];
-  uint32_t best = 0, most = (uint32_t)(cnt & 255u);
+  auto sum = [&] {
+    return part[warp][lane] + part[warp + 1][lane] + part[warp + 2][lane] + part[warp + 3][lane];
+  };
+  auto slot = [](unsigned long long c, uint32_t s) { return (uint32_t)(c >> (8u * s)) & 255u; };
+  uint32_t best = 0, most = 0;
+  auto choose = [&](unsigned long long c) {
+    most = slot(c, 0);
 #pragma unroll
-  for (uint32_t s = 1; s < 7; ++s) {
-    const uint32_t c = (uint32_t)(cnt >> (8u * s)) & 255u;
-    if (c > most) {
-      most = c;
-      best = s;
-    }
+    for (uint32_t s = 1; s < 6; ++s)
+      if (slot(c, s) > most) {
+        most = slot(c, s);
+        best = s;
+      }
+    if (slot(c, 6) > most + slot(c, 7)) best = 6;
+  };
+  uint32_t again = 0;
+  if (quarter == 0) {
+    choose(sum());
+    again = __ballot_sync(0xffffffffu, here && n > kRefRows && most == 0 && best != 6);
+    if (lane == 0) more[warp >> 2] = again;
   }
+  __syncthreads();
+  if (more[warp >> 2]) {
+    constexpr uint32_t kMore = 192;
+    part[warp][lane] = count_codes<kMore / 4>(p, n, w, lane, [&](uint32_t q) {
+      q += quarter * (kMore / 4);
+      return n < kRefRows + kMore ? (uint64_t)kRefRows + q : n * (2 * q + 1) / (2 * kMore);
+    });
+  }
+  __syncthreads();
+  if (quarter || !here) return;
+  if (again >> lane & 1u) choose(sum());
   uint32_t bits[6];
 #pragma unroll
   for (uint32_t s = 0; s < 6; ++s) bits[s] = __ballot_sync(0xffffffffu, best == s);

@@ -86,31 +86,34 @@ def test_what_lists_do_not_hold(ctx, monkeypatch, n, L, share):
 
 def _sums_fit(rows):
     """Whether twice the largest sum of m over a row, and the sites of code 0, stay
-    within 16 bits, with the commonest code of the (at most 64) rows but '-'."""
+    within 16 bits, with the commonest code of one bit of the (at most 64) rows, or 0
+    where more rows have that than this code and '-'."""
     code = np.zeros(256, np.uint8)
     for c, v in zip(b"ACGT-", (1, 2, 4, 8, 15)):
         code[c] = v
     x = code[rows]
-    order = np.array([1, 2, 4, 8, 0])  # of equally common codes the first
-    r = order[np.argmax(np.stack([(x == v).sum(0) for v in order]), axis=0)]
+    order = np.array([1, 2, 4, 8])  # of equally common codes the first
+    count = np.stack([(x == v).sum(0) for v in order])
+    r = order[np.argmax(count, axis=0)]
+    r[(x == 0).sum(0) > count.max(0) + (x == 15).sum(0)] = 0
     weight = ((x & r) == 0).sum(1) - (r == 0).sum()
     return 2 * int(weight.max()) + int((r == 0).sum()) <= 65535
 
 
-@pytest.mark.parametrize("equal", [0, 3])
-def test_sums_past_16_bits(ctx, monkeypatch, equal):
-    # rows unlike one another; two rows unlike four equal ones, in 3/4 of the sites
+@pytest.mark.parametrize("kind", ["unlike", "two unlike four", "alike"])
+def test_sums_past_16_bits(ctx, monkeypatch, kind):
+    # rows unlike one another; two rows unlike four equal ones, in 3/4 of the sites;
+    # rows that differ in half of the sites at most
     monkeypatch.setenv("HAMMINGDIST_SITE_LISTS", "1")
-    if equal:
+    if kind == "two unlike four":
         rng = np.random.default_rng(1)
         rows = rng.choice(np.frombuffer(b"ACGT", np.uint8), (6, 65536))
         rows[3:] = rows[0]
     else:
-        rows = _mixed(6, 65536, 1.0, 6)
+        rows = _mixed(6, 65536, 1.0 if kind == "unlike" else 0.3, 6)
     aln = _pack(ctx, rows)
     got, listed = _listed(ctx, aln, np.uint32)
-    assert listed == _sums_fit(rows)
-    assert _sums_fit(rows) == (equal == 0)
+    assert listed == _sums_fit(rows) == (kind == "alike")
     np.testing.assert_array_equal(got, _bit_planes(ctx, monkeypatch, aln, np.uint32))
 
 
