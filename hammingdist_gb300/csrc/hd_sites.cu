@@ -49,6 +49,8 @@ constexpr uint32_t kRefRows = 64;            // rows that the reference is taken
 constexpr int kPairThreads = 768;
 constexpr uint32_t kPending = 64;            // sites a warp gathers before it takes 32 of them
 constexpr uint32_t kStepSites = 128;         // of one range, a warp's step: four to a lane
+constexpr uint32_t kMaxSteps = kMaxRanges * (kRange / kStepSites);
+constexpr uint32_t kHeavy = 4096;            // meetings of 32 gathered sites that the block's warps share
 constexpr uint32_t kPairSmem = kT * kPitch * 4 + kPairThreads / 32 * kPending * 8;
 // an entry: site in its range (10 bits), row in its tile (8), code (6), 1 bit:
 // a '-' counts against it, 1 bit: the site's r is 0, and for code 0 where r is
@@ -492,14 +494,18 @@ __device__ __forceinline__ void meet_dashes(uint32_t *acc, const uint8_t *list, 
 
 // The entries of n <= 32 sites of one range that meet, one a lane at a time:
 // per site, the first entries of the row tile's list with all of the column
-// tile's, and its later ones with the column tile's first ones.
-__device__ __forceinline__ void meet_sites(uint32_t *acc, const uint2 *sites, uint32_t n,
+// tile's, and its later ones with the column tile's first ones. kShare: one warp's
+// part of them, every 24th 32 meetings; else false, and nothing is done, if there
+// are more than kHeavy.
+template <bool kShare>
+__device__ __forceinline__ bool meet_sites(uint32_t *acc, const uint2 *sites, uint32_t n,
                                            const uint32_t *li, const uint32_t *lj, uint32_t lane) {
   const uint2 me = lane < n ? sites[lane] : make_uint2(0u, 0u);
   const uint32_t fa = me.y & 255u, la = (me.y >> 8) & 255u, fb = (me.y >> 16) & 255u, lb = me.y >> 24;
   const uint32_t mine = fa * (fb + lb) + la * fb;
   const uint32_t inc = warp_incl_scan(mine), total = __shfl_sync(0xffffffffu, inc, 31);
-  for (uint32_t m0 = 0; m0 < total; m0 += 32) {
+  if (!kShare && total > kHeavy) return false;
+  for (uint32_t m0 = kShare ? threadIdx.x & ~31u : 0u; m0 < total; m0 += kShare ? kPairThreads : 32) {
     const uint32_t m = m0 + lane;
     uint32_t src = 0;  // the lane whose site the m-th meeting is of
 #pragma unroll
@@ -525,14 +531,65 @@ __device__ __forceinline__ void meet_sites(uint32_t *acc, const uint2 *sites, ui
       if (w) atomicAdd(&acc[e_row(e) * kPitch + (j >> 1)], w << (16u * (j & 1u)));
     }
   }
+  return true;
+}
+
+// A step's sites, four to a lane: those with entries in both tiles are gathered in
+// `pending` and taken in batches of 32, take(bit, sites, n) for the batch (bit q: of
+// those a lane's q-th sites complete, 4: the rest).
+template <class Take>
+__device__ __forceinline__ void gather_sites(const uint16_t *a, const uint16_t *b, uint2 *pending,
+                                             uint32_t lane, Take &&take) {
+  uint32_t count = 0;
+  const uint2 af = __ldg(reinterpret_cast<const uint2 *>(a));
+  const uint2 al = __ldg(reinterpret_cast<const uint2 *>(a + kOffLater));
+  const uint2 bf = __ldg(reinterpret_cast<const uint2 *>(b));
+  const uint2 bl = __ldg(reinterpret_cast<const uint2 *>(b + kOffLater));
+  uint32_t an = __shfl_down_sync(0xffffffffu, af.x, 1) & 0xFFFFu;
+  uint32_t bn = __shfl_down_sync(0xffffffffu, bf.x, 1) & 0xFFFFu;
+  if (lane == 31) {
+    an = a[4];
+    bn = b[4];
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t a0 = (q & 1) ? (q < 2 ? af.x : af.y) >> 16 : (q < 2 ? af.x : af.y) & 0xFFFFu;
+    const uint32_t b0 = (q & 1) ? (q < 2 ? bf.x : bf.y) >> 16 : (q < 2 ? bf.x : bf.y) & 0xFFFFu;
+    const uint32_t a1 = (q & 1) ? (q < 2 ? al.x : al.y) >> 16 : (q < 2 ? al.x : al.y) & 0xFFFFu;
+    const uint32_t b1 = (q & 1) ? (q < 2 ? bl.x : bl.y) >> 16 : (q < 2 ? bl.x : bl.y) & 0xFFFFu;
+    const uint32_t a2 = q == 0 ? af.x >> 16 : q == 1 ? af.y & 0xFFFFu : q == 2 ? af.y >> 16 : an;
+    const uint32_t b2 = q == 0 ? bf.x >> 16 : q == 1 ? bf.y & 0xFFFFu : q == 2 ? bf.y >> 16 : bn;
+    // some first entry here, and some entry there
+    const bool on = (a1 > a0 && b2 > b0) || (b1 > b0 && a2 > a0);
+    const uint32_t mask = __ballot_sync(0xffffffffu, on);
+    if (on)
+      pending[count + __popc(mask & ((1u << lane) - 1u))] =
+          make_uint2(a0 | b0 << 16, (a1 - a0) | (a2 - a1) << 8 | (b1 - b0) << 16 | (b2 - b1) << 24);
+    count += __popc(mask);
+    __syncwarp();
+    if (count >= 32) {  // the sites gathered last
+      count -= 32;
+      take(q, pending + count, 32u);
+      __syncwarp();
+    }
+  }
+  if (count) {
+    take(4, pending, count);
+    __syncwarp();
+  }
 }
 
 // The distances of a tile pair (see the top of the file). The warps draw steps
 // from a queue: first the s entries that a '-' counts against, 32 at a time, in
 // the ranges where the other tile has '-' entries (a list of up to 224 rows
 // each: the longest steps), then 128 sites at a time the s entries that meet,
-// which 32 lanes share evenly. What bounds it is the instructions
-// of finding the meetings (IPC 3.3 of 4). 14,000 rows of 29,903 sites, one
+// which 32 lanes share evenly. Where many rows of both tiles differ from the
+// reference (a lineage's substitutions), one warp would be at a batch long after the
+// others' steps: batches of more than 4,096 meetings are left to the end, and all
+// warps share them (10 neighbouring sites where half of the rows differ: 7.2 -> 1.06
+// ms, 60 of a clade of a tenth of the rows 23.8 -> 1.69; lines at 8,192 and 16,384:
+// 400 sites with a tenth 1.69, 1.98 and 3.25). What bounds the kernel is the
+// instructions of finding the meetings (IPC 3.3 of 4). 14,000 rows of 29,903 sites, one
 // substitution per 1,000: 300 us (about 30 for the '-', 110 for the meetings,
 // 65 to gather their sites, 30 to store), where the tensor-core engine takes 1,910. A
 // lane an entry of the row tile instead, which looks its site up, took 655
@@ -541,10 +598,10 @@ __device__ __forceinline__ void meet_sites(uint32_t *acc, const uint2 *sites, ui
 __global__ void __launch_bounds__(kPairThreads, 2) k_site_pairs(SiteJob J) {
   extern __shared__ __align__(16) uint32_t acc[];
   __shared__ uint32_t chunks[2][kMaxRanges + 1];  // 32-entry chunks before each range
-  __shared__ uint32_t queue;
+  __shared__ uint32_t queue, some_left;
+  __shared__ __align__(4) uint8_t left[kMaxSteps];  // a step's batches of more than kHeavy meetings
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint2 *pending = reinterpret_cast<uint2 *>(acc + kT * kPitch) + warp * kPending;
-  uint32_t count = 0;
   const uint64_t idx = J.first + blockIdx.x;
   uint32_t ti = (uint32_t)((sqrtf(8.0f * (float)idx + 1.0f) - 1.0f) * 0.5f);
   while ((uint64_t)ti * (ti + 1) / 2 > idx) --ti;
@@ -552,7 +609,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_site_pairs(SiteJob J) {
   const uint32_t tj = (uint32_t)(idx - (uint64_t)ti * (ti + 1) / 2);
   for (uint32_t i = threadIdx.x; i < kT * kPitch / 4; i += kPairThreads)
     reinterpret_cast<uint4 *>(acc)[i] = make_uint4(0u, 0u, 0u, 0u);
-  if (threadIdx.x == 0) queue = 0;
+  if (threadIdx.x == 0) queue = some_left = 0;
+  for (uint32_t i = threadIdx.x; i < kMaxSteps / 4; i += kPairThreads) reinterpret_cast<uint32_t *>(left)[i] = 0u;
   const uint4 *bi = J.base + (uint64_t)ti * J.ranges, *bj = J.base + (uint64_t)tj * J.ranges;
   const uint16_t *oi = J.off + (uint64_t)ti * J.ranges * kOffSlot;
   const uint16_t *oj = J.off + (uint64_t)tj * J.ranges * kOffSlot;
@@ -605,64 +663,48 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_site_pairs(SiteJob J) {
       }
       continue;
     }
-    // a step's sites, four to a lane: those with entries in both tiles are
-    // gathered, and taken 32 at a time
-    const uint32_t k = c - cd, r = k / (kRange / kStepSites), s0 = (k % (kRange / kStepSites)) * kStepSites;
+    const uint32_t k = c - cd, r = k / (kRange / kStepSites);
+    const uint32_t at = r * kOffSlot + (k % (kRange / kStepSites)) * kStepSites + 4 * lane;
     const uint32_t *li = J.es + bi[r].x, *lj = J.es + bj[r].x;
-    const uint16_t *a = oi + (uint64_t)r * kOffSlot + s0 + 4 * lane;
-    const uint16_t *b = oj + (uint64_t)r * kOffSlot + s0 + 4 * lane;
-    const uint2 af = __ldg(reinterpret_cast<const uint2 *>(a));
-    const uint2 al = __ldg(reinterpret_cast<const uint2 *>(a + kOffLater));
-    const uint2 bf = __ldg(reinterpret_cast<const uint2 *>(b));
-    const uint2 bl = __ldg(reinterpret_cast<const uint2 *>(b + kOffLater));
-    uint32_t an = __shfl_down_sync(0xffffffffu, af.x, 1) & 0xFFFFu;
-    uint32_t bn = __shfl_down_sync(0xffffffffu, bf.x, 1) & 0xFFFFu;
-    if (lane == 31) {
-      an = a[4];
-      bn = b[4];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t a0 = (q & 1) ? (q < 2 ? af.x : af.y) >> 16 : (q < 2 ? af.x : af.y) & 0xFFFFu;
-      const uint32_t b0 = (q & 1) ? (q < 2 ? bf.x : bf.y) >> 16 : (q < 2 ? bf.x : bf.y) & 0xFFFFu;
-      const uint32_t a1 = (q & 1) ? (q < 2 ? al.x : al.y) >> 16 : (q < 2 ? al.x : al.y) & 0xFFFFu;
-      const uint32_t b1 = (q & 1) ? (q < 2 ? bl.x : bl.y) >> 16 : (q < 2 ? bl.x : bl.y) & 0xFFFFu;
-      const uint32_t a2 = q == 0 ? af.x >> 16 : q == 1 ? af.y & 0xFFFFu : q == 2 ? af.y >> 16 : an;
-      const uint32_t b2 = q == 0 ? bf.x >> 16 : q == 1 ? bf.y & 0xFFFFu : q == 2 ? bf.y >> 16 : bn;
-      // some first entry here, and some entry there
-      const bool on = (a1 > a0 && b2 > b0) || (b1 > b0 && a2 > a0);
-      const uint32_t mask = __ballot_sync(0xffffffffu, on);
-      if (on)
-        pending[count + __popc(mask & ((1u << lane) - 1u))] =
-            make_uint2(a0 | b0 << 16, (a1 - a0) | (a2 - a1) << 8 | (b1 - b0) << 16 | (b2 - b1) << 24);
-      count += __popc(mask);
-      __syncwarp();
-      if (count >= 32) {  // the sites gathered last
-        count -= 32;
-        meet_sites(acc, pending + count, 32, li, lj, lane);
-        __syncwarp();
+    gather_sites(oi + at, oj + at, pending, lane, [&](int bit, const uint2 *sites, uint32_t n) {
+      if (!meet_sites<false>(acc, sites, n, li, lj, lane) && lane == 0) {
+        left[k] |= (uint8_t)(1u << bit);
+        some_left = 1;
       }
-    }
-    if (count) {
-      meet_sites(acc, pending, count, li, lj, lane);
-      __syncwarp();
-      count = 0;
-    }
+    });
   }
   __syncthreads();
+  if (some_left) {  // block-uniform: the batches left, shared by all warps
+    for (uint32_t k0 = 0; k0 < steps - cd; k0 += 32) {
+      uint32_t on = __ballot_sync(0xffffffffu, k0 + lane < steps - cd && left[k0 + lane] != 0);
+      for (; on; on &= on - 1) {
+        const uint32_t k = k0 + __ffs(on) - 1, r = k / (kRange / kStepSites);
+        const uint32_t at = r * kOffSlot + (k % (kRange / kStepSites)) * kStepSites + 4 * lane;
+        const uint32_t *li = J.es + bi[r].x, *lj = J.es + bj[r].x;
+        gather_sites(oi + at, oj + at, pending, lane, [&](int bit, const uint2 *sites, uint32_t n) {
+          if (left[k] >> bit & 1u) meet_sites<true>(acc, sites, n, li, lj, lane);
+        });
+      }
+    }
+    __syncthreads();
+  }
   if (J.dtype == 1) store_rows<uint8_t>(J, acc, ti, tj);
   else if (J.dtype == 2) store_rows<uint16_t>(J, acc, ti, tj);
   else store_rows<uint32_t>(J, acc, ti, tj);
 }
 
-// Estimated times in us, from measurements (dense / lists, us):
-//   n = 14,000, L = 29,903: 2,025 / 315 at one substitution per 10,000 sites,
-//     368 at 1e-3, 533 at 3e-3, 1,410 at 1e-2, 6,180 at 3e-2
-//   n = 5,000, L = 29,903: 430 / 76, 86, 123, 292, 1,122
-//   n = 14,000, L = 3,000: 331 / 192, 215, 253, 433, 1,215
-//   n = 14,000, L = 600: 207 / 125, 138, 168, 233, 632
-// pairs: meetings of entries. Building the lists costs about what expanding
-// the operand does.
+// Estimated times of a call in us, from measurements. The distances alone (dense /
+// lists, us) at 1e-3, 3e-3, 1e-2, 1.5e-2 and 3e-2 substitutions per site:
+//   n = 14,000, L = 29,903: 1,920 / 295, 471, 1,331, 2,188, 6,112
+//   n = 5,000, L = 29,903: 363 / 55, 92, 256, 407, 1,097
+//   n = 14,000, L = 3,000: 254 / 129, 182, 372, 540, 1,173
+//   n = 8,000, L = 10,000: 261 / 65, 98, 245, 383, 965
+//   n = 16,000, L = 600: 168 / 107, 147, 227, 324, 733
+// and at 1e-3 with 10, 20 and 40 sites where half of 14,000 rows differ 1,193,
+// 2,068 and 3,823. pairs: meetings of entries by the sample, which also counts those
+// of 'N' runs and '-' (2.5e-6 us each puts the line between 1.2e-2 and 1.5e-2; 2e-6
+// took the lists at 1.5e-2, 3.2e-6 the dense kernel at 1.2e-2).
+// Building the lists costs about what expanding the operand does.
 double dense_us(uint64_t n, uint64_t L, uint32_t planes) {
   const double pairs = 0.5 * (double)n * (double)n;
   return 60.0 + 1e-6 * pairs + 6.2e-10 * pairs * (double)L * (double)planes / 4.0;
@@ -670,7 +712,7 @@ double dense_us(uint64_t n, uint64_t L, uint32_t planes) {
 double lists_us(uint64_t n, uint64_t L, double pairs) {
   const double tiles = (double)ceil_div(n, (uint64_t)kT), ranges = (double)ceil_div(L, (uint64_t)kRange);
   return 40.0 + 0.95e-6 * 0.5 * (double)n * (double)n +
-         3.3e-3 * 0.5 * tiles * (tiles + 1) * ranges + 2e-6 * pairs;
+         3.3e-3 * 0.5 * tiles * (tiles + 1) * ranges + 2.5e-6 * pairs;
 }
 
 Planes planes_of(const hd_alignment *a) {
