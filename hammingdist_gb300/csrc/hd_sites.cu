@@ -137,7 +137,7 @@ __device__ __forceinline__ unsigned long long count_codes(const Planes &p, uint6
 // is an s entry, so r is 0 only where there are more rows of code 0 than of that
 // code and '-' together. Near an alignment's ends the 64 rows can all be '-' at a
 // site, or one of them 'N': words with sites that no row gives a code with a bit
-// look at 192 rows more. (r taken to be 0 at four sites where all rows but a few
+// look at 96 rows more. (r taken to be 0 at four sites where all rows but a few
 // are '-': 11.3 ms for 14,000 rows instead of 0.3; a code that is not the rows' at
 // 18 sites, where 2-12% have one: 0.7 ms.)
 __global__ void __launch_bounds__(256)
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
   if (more[warp >> 2]) {
-    constexpr uint32_t kMore = 192;
+    constexpr uint32_t kMore = 96;
     part[warp][lane] = count_codes<kMore / 4>(p, n, w, lane, [&](uint32_t q) {
       q += quarter * (kMore / 4);
       return n < kRefRows + kMore ? (uint64_t)kRefRows + q : n * (2 * q + 1) / (2 * kMore);
@@ -260,7 +260,8 @@ struct BuildSums {
   unsigned long long dashes;   // of an s and a '-' entry of one site
   uint32_t full;               // some list did not fit
   uint32_t zero;               // sites where r is 0
-  uint32_t max_weight, pad;
+  uint32_t max_weight;
+  uint32_t peak;               // most meetings of a tile with itself, of its sites with many
 };
 
 // The lists of one (range, tile): a warp takes four rows at a time, a lane a
@@ -403,20 +404,24 @@ __global__ void __launch_bounds__(256, 4)
   });
 }
 
-// The pairs of s entries that meet over all tiles, of s and '-' entries, and
-// the largest weight. A lane takes a site, the block's warps a share of the
-// tiles each.
+// The pairs of s entries that meet over all tiles, of s and '-' entries, the
+// largest weight, and the tile whose own entries meet most (no pair of tiles has
+// more), by the 32 neighbouring sites that have many: tile_sum, one a tile, starts
+// at 0. A lane takes a site, the block's warps a share of the tiles each.
 __global__ void __launch_bounds__(256)
     k_site_check(const uint16_t *off, uint32_t tiles, uint32_t ranges, const uint32_t *weight,
-                 uint64_t n, BuildSums *sums) {
+                 uint64_t n, uint32_t *tile_sum, BuildSums *sums) {
   __shared__ uint32_t part[3][8][32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t range = blockIdx.x / (kRange / 32), s = (blockIdx.x % (kRange / 32)) * 32 + lane;
   uint32_t k = 0, l = 0, d = 0;
   for (uint32_t t = warp; t < tiles; t += 8) {
     const uint16_t *o = off + ((uint64_t)t * ranges + range) * kOffSlot + s;
-    k += (uint32_t)o[1] - o[0];
-    l += (uint32_t)o[1] - o[kOffLater];
+    const uint32_t kt = (uint32_t)o[1] - o[0], lt = (uint32_t)o[1] - o[kOffLater];
+    const uint32_t own = __reduce_add_sync(0xffffffffu, kt * kt - lt * lt);
+    if (own >= 1024 && lane == 0) atomicMax(&sums->peak, atomicAdd(&tile_sum[t], own) + own);
+    k += kt;
+    l += lt;
     d += (uint32_t)o[kOffDash + 1] - o[kOffDash];
   }
   part[0][warp][lane] = k;
@@ -812,13 +817,14 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
   const uint64_t cap_d = std::min<uint64_t>(all, (uint64_t)(2.0 * S.est_d) + 64 * a->n_rows + 65536);
   if (cap_s > 0xFFFFFFFFull || cap_d > 0xFFFFFFFFull) return false;
   DevBuf ref;
+  const uint64_t tile_bytes = round_up(tiles * 4, 16);
   try {
     S.off = DevBuf(slots * kOffSlot * 2, st, true);
     S.base = DevBuf(slots * 16, st, true);
     S.es = DevBuf(cap_s * 4, st, true);
     S.ed = DevBuf(cap_d + 16, st, true);
     S.weight = DevBuf(a->n_rows * 4, st, true);
-    ref = DevBuf(ref_bytes(a) + sizeof(BuildSums), st, true);
+    ref = DevBuf(ref_bytes(a) + sizeof(BuildSums) + tile_bytes, st, true);
   } catch (const Error &e) {
     if (e.code != HD_ERR_OOM) throw;
     cudaGetLastError();
@@ -826,10 +832,11 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
     return false;  // the engines need less memory
   }
   auto *sums = ref.as<BuildSums>();
-  uint4 *r0 = reinterpret_cast<uint4 *>(sums + 1);
+  uint32_t *tile_sum = reinterpret_cast<uint32_t *>(sums + 1);
+  uint4 *r0 = reinterpret_cast<uint4 *>(ref.as<uint8_t>() + sizeof(BuildSums) + tile_bytes);
   uint2 *r1 = reinterpret_cast<uint2 *>(r0 + a->words);
   static_assert(sizeof(BuildSums) % 16 == 0, "the reference follows");
-  HD_CUDA(cudaMemsetAsync(sums, 0, sizeof(BuildSums), st));
+  HD_CUDA(cudaMemsetAsync(sums, 0, sizeof(BuildSums) + tile_bytes, st));
   HD_CUDA(cudaMemsetAsync(S.weight.p, 0, a->n_rows * 4, st));
   const Planes p = planes_of(a);
   const Words sel = Words::of(words, 1);
@@ -848,7 +855,7 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
     HD_LAUNCHED(ctx);
   }
   k_site_check<<<ranges * (kRange / 32), 256, 0, st>>>(
-      S.off.as<uint16_t>(), (uint32_t)tiles, ranges, S.weight.as<uint32_t>(), a->n_rows, sums);
+      S.off.as<uint16_t>(), (uint32_t)tiles, ranges, S.weight.as<uint32_t>(), a->n_rows, tile_sum, sums);
   HD_LAUNCHED(ctx);
   auto *h = reinterpret_cast<BuildSums *>(pinned_words(ctx));
   HD_CUDA(cudaMemcpyAsync(h, sums, sizeof(BuildSums), cudaMemcpyDeviceToHost, st));
@@ -859,7 +866,10 @@ bool ensure_sites(hd_ctx *ctx, const hd_alignment *a, cudaStream_t st) {
   // meetings with '-': the pairs found, by the sample's share of s entries that
   // do meet a '-', if the sample saw fewer
   const double dash = std::max(S.est_xd, (double)h->dashes * S.est_x / std::max(1.0, S.est_s));
-  const double t = lists_us(a->n_rows, a->length, (double)h->pairs + dash);
+  // a block with `peak` meetings takes 0.5 ns each, beyond the average ones': 40
+  // lineages of 350 neighbouring rows, 60 sites each, take 2.6-3.0 ms, and 1.9 on the
+  // tensor cores
+  const double t = lists_us(a->n_rows, a->length, (double)h->pairs + dash) + 0.5e-3 * h->peak;
   if (!fits || (forced() == 0 && t > dense_us(a->n_rows, a->length, (uint32_t)a->planes))) {
     S.release();
     return false;

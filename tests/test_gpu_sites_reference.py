@@ -7,7 +7,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [65, 255, 256, 257, 700])
+@pytest.mark.parametrize("n", [65, 159, 160, 161, 255, 256, 257, 700])
 @pytest.mark.parametrize("seen", [b"N", b"-", b"NN-"])
 def test_ends_that_few_rows_reach(monkeypatch, n, seen):
     from hammingdist_gb300 import abi
