@@ -198,10 +198,12 @@ __global__ void __launch_bounds__(kRdThreads)
         value = __dp4a(digits, 0x00010A64u >> (8 * (3 - len)), 0u);
         value = value > kMax ? kMax : value;
       } else {
-        uint64_t end = x + k;
-        while (end < n && !is_sep(p[end])) ++end;
+        // its own end stops every phase of std::stoi but the whitespace (a '\n'
+        // is one): nothing after the number is read, however long the field
+        uint64_t s = x + k;
+        while (s < n && (p[s] == ' ' || (p[s] >= '\t' && p[s] <= '\r' && p[s] != '\n'))) ++s;
         int r_v = 0;
-        const int r = dev_stoi(p, x + k, end, &r_v);
+        const int r = s < n && !is_sep(p[s]) ? dev_stoi(p, s, n, &r_v) : 1;
         if (r) note_error(err, base + idx, r);
         value = r ? 0u : (uint32_t)safe_cast<T>(r_v);
       }
